@@ -153,7 +153,9 @@ int wf_add_trimesh(wf_domain* d, const double* nodes, int32_t nn, const int32_t*
  *   particle, as Energy.cu:270-276; 1: each particle's own; both forms),
  *   contact_dx (0),
  *   contact_stiffness (0.1), contact_vreg (1e-3), contact_heat_fraction (1),
- *   fuse_heat (1), fuse_integrate (1), tile_staging (0; 1: the mixed pair passes
+ *   fuse_heat (1), fuse_integrate (1), pair_cache (1; 0: the FP64 passes of a
+ *   step each compute the pair geometry instead of keeping it, 1.2 KB less per
+ *   particle, same results), tile_staging (0; 1: the mixed pair passes
  *   read neighbours from per-tile halos in shared memory; same results),
  *   tile_cap_max (2048: largest halo staged), list_prefetch (2: L2 prefetch of
  *   the neighbour lists that many blocks ahead; 0 off), state_prefetch (1: L2 prefetch, before

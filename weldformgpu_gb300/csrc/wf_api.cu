@@ -118,6 +118,15 @@ struct wf_domain {
   bool l16_built = false;
   int32_t* l16_base = nullptr;
   uint16_t* l16_off = nullptr;
+  // FP64 form: the pair geometry and per-particle quotients kept between the
+  // passes of a step (Work64), allocated at the first FP64 solve
+  double* work64 = nullptr;
+  int64_t work64_pad = 0;      // padded slots it was allocated for (the cache's may be more)
+  bool work64_tried = false;
+  bool pair_cache = true;      // option "pair_cache"
+  int rr_cur = 0;              // which of the two 1/rho arrays is current
+  bool geo_valid = false;      // gk, r2: of the current positions and lists
+  bool rr_valid = false;       // rr: of the current density
   int tile_cap_max = WF_TILE_HALO_MAX;   // option "tile_cap_max": largest halo staged
   int tile_cap = 0;            // halo capacity the current tiles were built for (0: none)
   int tile_hmax = 0;           // largest halo of the last build (read at the next rebuild)
@@ -458,6 +467,8 @@ struct ArenaCache {
   size_t bytes = 0;
   int dev = -1;
   int* h_status = nullptr;
+  double* work64 = nullptr;    // an FP64 domain's work arrays, sized by its npad
+  int64_t npad = 0;
 };
 static std::mutex g_cache_mu;
 static ArenaCache g_cache;
@@ -468,6 +479,7 @@ static void cache_free_locked() {
     cudaGetDevice(&cur);
     cudaSetDevice(g_cache.dev);
     cudaFree(g_cache.arena);
+    if (g_cache.work64) cudaFree(g_cache.work64);
     cudaSetDevice(cur);
   }
   if (g_cache.h_status) cudaFreeHost(g_cache.h_status);
@@ -484,6 +496,8 @@ static void cache_take(wf_domain* d) {
   d->arena = g_cache.arena;
   d->arena_alloc = g_cache.bytes;
   d->h_status = g_cache.h_status;
+  d->work64 = g_cache.work64;
+  d->work64_pad = g_cache.npad;
   g_cache = ArenaCache{};
 }
 static void cache_put(wf_domain* d) {
@@ -494,6 +508,9 @@ static void cache_put(wf_domain* d) {
   g_cache.bytes = d->arena_alloc;
   g_cache.dev = d->dev;
   g_cache.h_status = d->h_status;
+  g_cache.work64 = d->work64;
+  g_cache.npad = d->work64_pad;
+  d->work64 = nullptr;
   d->arena = nullptr;
   d->h_status = nullptr;
 }
@@ -506,6 +523,8 @@ static StepParams make_params(const wf_domain* d) {
   P.npad = d->npad;
   P.h = d->h;
   P.gkC = 1.0 / (d->h * d->h * d->h * d->h * WF_PI);   // Functions.cu:83 with h_ = h
+  P.invh = 1.0 / d->h;
+  P.h_known = d->h > 1.0e-100 && d->h < 1.0e100;
   P.dt = d->dt;
   P.Cs = d->Cs;
   P.G = d->G;
@@ -712,6 +731,41 @@ static int ensure_cells(wf_domain* d, int64_t ncell) {
   return WF_OK;
 }
 
+// The FP64 form's work arrays.  Without them (not enough memory) the passes
+// compute the pair geometry themselves.
+static void work64_alloc(wf_domain* d) {
+  if (d->work64_tried) return;
+  d->work64_tried = true;
+  if (d->work64) {             // taken over from the cache
+    if (d->work64_pad >= d->npad) return;
+    cudaFree(d->work64);
+    d->work64 = nullptr;
+  }
+  const size_t words = (size_t)(2 * WF_NB_ALLOC + 9) * (size_t)d->npad;
+  d->work64_pad = d->npad;
+  if (cudaMalloc((void**)&d->work64, sizeof(double) * words) != cudaSuccess) {
+    cudaGetLastError();
+    d->work64 = nullptr;
+  }
+}
+// Kept values are of this call's own steps only: anything may have changed
+// between two calls and in the step hook.
+static void work64_drop(wf_domain* d) { d->geo_valid = d->rr_valid = false; }
+static Work64 work64_of(const wf_domain* d) {
+  Work64 W{};
+  if (!d->work64 || !d->work64_tried || !d->pair_cache) return W;
+  const int64_t e = (int64_t)WF_NB_ALLOC * d->npad, n = d->npad;
+  W.gk = d->work64;
+  W.r2 = W.gk + e;
+  W.mr = W.r2 + e;
+  W.rr = W.mr + n + d->rr_cur * n;
+  W.rr_out = W.mr + n + (1 - d->rr_cur) * n;
+  W.sa6 = W.mr + 3 * n;
+  W.geo = d->geo_valid;
+  W.recip = d->rr_valid;
+  return W;
+}
+
 constexpr int kReorderEvery = 20;   // physical reorder at every 20th rebuild of a solve
 
 static int rebuild(wf_domain* d, bool use_current, bool light = false) {
@@ -720,6 +774,7 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
     if (rc) return rc;
   }
   KTimer t(d, KID_REBUILD);
+  work64_drop(d);
   const int64_t n = d->n;
   cudaStream_t s = d->stream;
   Fields& A = d->F[d->cur];
@@ -1063,6 +1118,7 @@ static int solve_begin(wf_domain* d, double dt_out) {
 
 static int solve_step_launches(wf_domain* d) {
   cudaStream_t s = d->stream;
+  if (d->precision == 0 && d->pair_cache && !d->capturing) work64_alloc(d);
   bool rb;
   if (d->rb_dep > 0.0) {
     // adaptive: rebuild once the plastic strain grew by rb_dep anywhere since
@@ -1110,9 +1166,13 @@ static int solve_step_launches(wf_domain* d) {
                     (mixed && d->tile_staging && !P.contact) ? d->tile_cap : 0};
   const List16 L16{(mixed && d->list16 && d->l16_built) ? d->l16_base : nullptr, d->l16_off};
   if (!mixed) {
-    { KTimer t(d, KID_DENSITY); launch_fp64_density(P, F, d->vd2, N, s); }          // :193-202
-    { KTimer t(d, KID_STRESS); launch_fp64_stress(P, F, d->vd2, N, d->d_status, s); }  // :204-218
-    { KTimer t(d, KID_ACCEL); launch_fp64_accel(P, F, d->vd2, N, s); }               // :221
+    const Work64 W = work64_of(d);
+    { KTimer t(d, KID_DENSITY); launch_fp64_density(P, F, W, d->vd2, N, s); }       // :193-202
+    { KTimer t(d, KID_STRESS);                                                      // :204-218
+      d->launches += launch_fp64_stress(P, F, W, d->vd2, N, d->d_status, s) - 1; }
+    { KTimer t(d, KID_ACCEL); launch_fp64_accel(P, F, W, d->vd2, N, s); }            // :221
+    d->rr_cur ^= 1;
+    d->rr_valid = W.gk != nullptr;
   } else {
     {
       KTimer t(d, KID_DENSITY);
@@ -1145,6 +1205,7 @@ static int solve_step_launches(wf_domain* d) {
   if (!integrated) {   // :273-287
     KTimer t(d, KID_INTEGRATE);
     launch_integrate(P, F, d->vd2, mixed ? d->a32 : nullptr, s);
+    d->geo_valid = false;
   }
   d->launches += integrated ? 3 : 4;
   if (d->thermal) {                                                                   // :285
@@ -1153,7 +1214,10 @@ static int solve_step_launches(wf_domain* d) {
       d->heat_pending_first = d->isfirst;
     } else {
       KTimer t(d, KID_THERMAL);
-      launch_thermal(P, F, N, d->isfirst ? 1 : 0, d->chi > 0.0 ? 1 : 0, mixed ? 1 : 0, s);
+      Work64 W = work64_of(d);
+      W.mr_heat = W.mr;                  // the density pass's m / rho
+      launch_thermal(P, F, W, N, d->isfirst ? 1 : 0, d->chi > 0.0 ? 1 : 0, mixed ? 1 : 0, s);
+      d->geo_valid = !mixed && W.gk;     // of the new positions: the next step's
       d->launches += 2;
     }
   }
@@ -1217,6 +1281,7 @@ static int solve_step(wf_domain* d) {
   d->in_callback = true;
   const int r = d->after_fn(d, d->after_user);
   d->in_callback = false;
+  work64_drop(d);
   if (r) return wf_fail(d, WF_ERR_STATE, "step callback returned " + std::to_string(r));
   return WF_OK;
 }
@@ -1227,8 +1292,8 @@ static void flush_heat(wf_domain* d) {
   StepParams P = make_params(d);
   NbBuffers N{d->nb, d->nbc};
   KTimer t(d, KID_THERMAL);
-  launch_thermal(P, d->F[d->cur], N, d->heat_pending_first ? 1 : 0, d->chi > 0.0 ? 1 : 0, 1,
-                 d->stream);
+  launch_thermal(P, d->F[d->cur], Work64{}, N, d->heat_pending_first ? 1 : 0,
+                 d->chi > 0.0 ? 1 : 0, 1, d->stream);
   d->launches += 2;
   d->heat_pending = false;
 }
@@ -1321,6 +1386,7 @@ int wf_destroy(wf_domain* d) {
                   M.off32, M.cvert, M.cursor, M.scan_tmp};
     for (void* p : mp) if (p) cudaFree(p);
   }
+  if (d->work64) cudaFree(d->work64);
   if (d->d_maxdep) cudaFree(d->d_maxdep);
   if (d->h_maxdep) cudaFreeHost(d->h_maxdep);
   if (d->cnb) cudaFree(d->cnb);
@@ -1735,6 +1801,10 @@ int wf_set_option(wf_domain* d, const char* key, double v) {
       WF_CUDA_OK(dalloc(&d->log_count, 1, d->stream));
     }
   }
+  else if (k == "pair_cache") {
+    d->pair_cache = v != 0;
+    work64_drop(d);
+  }
   else if (k == "tile_staging") d->tile_staging = v != 0;   // takes effect at the next rebuild
   else if (k == "list_prefetch") d->list_prefetch = std::max(0, std::min((int)v, WF_NB_BLOCKS));
   else if (k == "state_prefetch") d->state_prefetch = v != 0;
@@ -1780,6 +1850,7 @@ int wf_step(wf_domain* d, int64_t nsteps) {
     int rc = solve_begin(d, d->output_interval);
     if (rc) return rc;
   }
+  work64_drop(d);
   for (int64_t k = 0; k < nsteps; k++) {
     int rc = solve_step(d);
     if (rc) return rc;
@@ -1819,7 +1890,8 @@ int wf_thermal_solve(wf_domain* d, double tf) {
   while (d->time < tf) {
     {
       KTimer t(d, KID_THERMAL);
-      launch_thermal(P, CF(d), N, d->isfirst ? 1 : 0, 0, d->precision == 1 ? 1 : 0, d->stream);
+      launch_thermal(P, CF(d), Work64{}, N, d->isfirst ? 1 : 0, 0, d->precision == 1 ? 1 : 0,
+                     d->stream);
     }
     d->launches += 2;
     d->isfirst = false;
@@ -2203,6 +2275,7 @@ int wf_time_steps(wf_domain* d, int64_t nsteps, double* elapsed_ms, double* kern
   cudaEventRecord(e0, d->stream);
   int rc = WF_OK;
   d->timing = true;
+  work64_drop(d);
   for (int64_t k = 0; k < nsteps && rc == WF_OK; k++) rc = solve_step(d);
   flush_heat(d);   // the timed steps include their whole heat work
   if (rc == WF_OK) rc = segment_end(d);

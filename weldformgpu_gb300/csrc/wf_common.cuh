@@ -170,6 +170,8 @@ struct StepParams {
   int64_t n_solid;      // original ids below this are solid (solid_part_count)
   int64_t npad;         // slot stride of the neighbour-list blocks (nb_at)
   double h, gkC;        // smoothing length (uniform) and 1/(h^4 pi)
+  double invh;          // 1/h rounded to nearest (FP64 form's division by h)
+  int h_known;          // h is far enough inside the range for that division
   double dt;
   double Cs, G, rho0;   // uniform sound speed, shear modulus, reference density
   double alpha, beta;   // Monaghan artificial viscosity
@@ -306,16 +308,32 @@ struct NbBuffers {
   int32_t* cnt;     // [npad]
 };
 
-void launch_fp64_density(const StepParams& P, const Fields& F, double4* vd2, const NbBuffers& N,
-                         cudaStream_t s);
-void launch_fp64_stress(const StepParams& P, const Fields& F, const double4* vd2,
-                        const NbBuffers& N, int* status, cudaStream_t s);
-void launch_fp64_accel(const StepParams& P, const Fields& F, const double4* vd2,
+// Work arrays of the FP64 form (wf_step_fp64.cu); all null when they could not
+// be allocated (the passes then compute everything per pair).
+struct Work64 {
+  double* gk;        // per list entry (nb_at): kernel factor GK
+  double* r2;        // per list entry: r_ij^2
+  double* mr;        // m / rho of the step's new density
+  double* rr;        // 1 / rho of the density the step starts from
+  double* rr_out;    // 1 / rho of the new density, rr of the next step
+  double* sa6;       // sigma / rho^2, 6 per slot
+  double* mr_heat;   // m / rho as the heat pass needs it (mr behind a step; null: divide)
+  int geo;           // gk and r2 hold the current positions' and lists' values
+  int recip;         // rr holds the current density's reciprocals
+};
+void launch_fp64_density(const StepParams& P, const Fields& F, const Work64& W, double4* vd2,
+                         const NbBuffers& N, cudaStream_t s);
+// returns the number of kernels launched
+int launch_fp64_stress(const StepParams& P, const Fields& F, const Work64& W, const double4* vd2,
+                       const NbBuffers& N, int* status, cudaStream_t s);
+void launch_fp64_accel(const StepParams& P, const Fields& F, const Work64& W, const double4* vd2,
                        const NbBuffers& N, cudaStream_t s);
+void launch_fp64_heat_rate(const StepParams& P, const Fields& F, const Work64& W,
+                           const NbBuffers& N, int plastic_heat, cudaStream_t s);
 void launch_integrate(const StepParams& P, const Fields& F, const double4* vd2,
                       const float4* a32, cudaStream_t s);
-void launch_thermal(const StepParams& P, const Fields& F, const NbBuffers& N, int first,
-                    int plastic_heat, int mixed, cudaStream_t s);
+void launch_thermal(const StepParams& P, const Fields& F, const Work64& W, const NbBuffers& N,
+                    int first, int plastic_heat, int mixed, cudaStream_t s);
 
 // contact (wf_contact.cu): surface tagging, contact list (when `list`) and
 // penalty forces after the acceleration pass; mesh motion and rigid particles

@@ -28,6 +28,26 @@ __device__ __forceinline__ double heat_rate_mixed(const StepParams& P, const Fie
   return (double)sm;
 }
 
+// dT/dt of the FP64 form from the flux sum s: the reference's arithmetic in
+// its order (ThermalSolveKernel's scaling, plastic heat, CalcConvHeatKernel,
+// src/cuda/Thermal.cu:36-64, :101-142).  For units compiled with -fmad=false.
+__device__ __forceinline__ double heat_rate_fp64(const StepParams& P, const Fields& F, int64_t i,
+                                                 double s, double rhoi, double mass, double Ti,
+                                                 int plastic_heat) {
+  s *= 1. / (rhoi * F.cpT[i]);
+  if (plastic_heat && F.perm[i] < P.n_solid) {
+    const double dep = F.dep[i];
+    if (dep > 0.0) s += P.chi * F.sy[i] * dep / (rhoi * F.cpT[i] * P.dt);
+  }
+  if (F.qf && F.qf[i] > 0.0) s += F.qf[i] / (mass * F.cpT[i]);   // frictional heat, law 1
+  if (F.bct[i] == 1) {
+    const double dS2 = pow(mass / rhoi, 0.666666666);
+    const double q_conv = P.h_conv * dS2 * (P.T_inf - Ti) / mass;
+    s += 1. / F.cpT[i] * q_conv;
+  }
+  return s;
+}
+
 // TempCalcLeapfrogFirst / TempCalcLeapfrog (src/cuda/Thermal.cu:16-31) for
 // one particle; returns the new temperature (unchanged on the first step).
 __device__ __forceinline__ double heat_leapfrog_one(const StepParams& P, const Fields& F,

@@ -56,47 +56,6 @@ __global__ void __launch_bounds__(256) k_integrate(StepParams P, Fields F,
   F.a[i] = make_double4(ax, ay, az, 0.0);
 }
 
-// ---- heat: ThermalSolveKernel + plastic heat + CalcConvHeatKernel -------
-// src/cuda/Thermal.cu:101-142 and :36-64, FP64 form: the reference's
-// arithmetic in its order.  The mixed form's heat pass is k_heat32
-// (wf_step_fp32.cu): pair flux in FP32 with the temperature difference taken
-// from the (hi, lo) float pair; dT/dt and T stay FP64.
-__global__ void __launch_bounds__(128) k_heat_rate(StepParams P, Fields F,
-                                                   const int32_t* __restrict__ nb,
-                                                   const int32_t* __restrict__ cnt,
-                                                   int plastic_heat) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= P.n) return;
-  const double4 xi = F.xm[i];
-  const double rhoi = F.vd[i].w;
-  const double Ti = F.T[i], ki = F.kT[i];
-  const int c = cnt[i];
-  double s = 0.0;
-  for (int k = 0; k < c; k++) {
-    const int j = __ldg(nb + nb_at(P.npad, i, k));
-    const double4 xj = F.xm[j];
-    const double rhoj = F.vd[j].w;
-    const double kj = F.kT[j];
-    const double xx = xi.x - xj.x, xy = xi.y - xj.y, xz = xi.z - xj.z;
-    const double nxij = sqrt(xx * xx + xy * xy + xz * xz);
-    const double GK = gradK64(nxij / P.h, P.h, P.gkC);
-    s += xj.w / rhoj * (4.0 * ki * kj / (ki + kj) * (Ti - F.T[j])) *
-         (xx * (xx * GK) + xy * (xy * GK) + xz * (xz * GK)) / (nxij * nxij);
-  }
-  s *= 1. / (rhoi * F.cpT[i]);
-  if (plastic_heat && F.perm[i] < P.n_solid) {
-    const double dep = F.dep[i];
-    if (dep > 0.0) s += P.chi * F.sy[i] * dep / (rhoi * F.cpT[i] * P.dt);
-  }
-  if (F.qf && F.qf[i] > 0.0) s += F.qf[i] / (xi.w * F.cpT[i]);   // frictional heat, law 1
-  if (F.bct[i] == 1) {
-    const double dS2 = pow(xi.w / rhoi, 0.666666666);
-    const double q_conv = P.h_conv * dS2 * (P.T_inf - Ti) / xi.w;
-    s += 1. / F.cpT[i] * q_conv;
-  }
-  F.dTdt[i] = s;
-}
-
 // TempCalcLeapfrogFirst / TempCalcLeapfrog (src/cuda/Thermal.cu:16-31)
 __global__ void __launch_bounds__(256) k_heat_leapfrog(StepParams P, Fields F, int first,
                                                        int mixed) {
@@ -118,9 +77,9 @@ void launch_integrate(const StepParams& P, const Fields& F, const double4* vd2,
   k_integrate<<<blocks_for(P.n, 256), 256, 0, s>>>(P, F, vd2, a32);
 }
 
-void launch_thermal(const StepParams& P, const Fields& F, const NbBuffers& N, int first,
-                    int plastic_heat, int mixed, cudaStream_t s) {
+void launch_thermal(const StepParams& P, const Fields& F, const Work64& W, const NbBuffers& N,
+                    int first, int plastic_heat, int mixed, cudaStream_t s) {
   if (mixed) launch_fp32_heat(P, F, N, plastic_heat, s);
-  else k_heat_rate<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, N.nb, N.cnt, plastic_heat);
+  else launch_fp64_heat_rate(P, F, W, N, plastic_heat, s);
   k_heat_leapfrog<<<blocks_for(P.n, 256), 256, 0, s>>>(P, F, first, mixed);
 }
