@@ -118,11 +118,12 @@ struct wf_domain {
   bool l16_built = false;
   int32_t* l16_base = nullptr;
   uint16_t* l16_off = nullptr;
-  // FP64 form: the pair geometry and per-particle quotients kept between the
-  // passes of a step (Work64), allocated at the first FP64 solve
-  double* work64 = nullptr;
-  int64_t work64_pad = 0;      // padded slots it was allocated for (the cache's may be more)
-  bool work64_tried = false;
+  // pair work arrays, allocated when a solve first needs them: what the passes
+  // of an FP64 step keep for one another (Work64), or a heat solve for its
+  // steps (HeatWork64, HeatWork32)
+  char* work = nullptr;
+  size_t work_bytes = 0;       // allocated
+  size_t work_refused = 0;     // a size the device had no memory for
   bool pair_cache = true;      // option "pair_cache"
   int rr_cur = 0;              // which of the two 1/rho arrays is current
   bool geo_valid = false;      // gk, r2: of the current positions and lists
@@ -467,8 +468,8 @@ struct ArenaCache {
   size_t bytes = 0;
   int dev = -1;
   int* h_status = nullptr;
-  double* work64 = nullptr;    // an FP64 domain's work arrays, sized by its npad
-  int64_t npad = 0;
+  char* work = nullptr;        // the domain's pair work arrays
+  size_t work_bytes = 0;
 };
 static std::mutex g_cache_mu;
 static ArenaCache g_cache;
@@ -479,7 +480,7 @@ static void cache_free_locked() {
     cudaGetDevice(&cur);
     cudaSetDevice(g_cache.dev);
     cudaFree(g_cache.arena);
-    if (g_cache.work64) cudaFree(g_cache.work64);
+    if (g_cache.work) cudaFree(g_cache.work);
     cudaSetDevice(cur);
   }
   if (g_cache.h_status) cudaFreeHost(g_cache.h_status);
@@ -496,8 +497,8 @@ static void cache_take(wf_domain* d) {
   d->arena = g_cache.arena;
   d->arena_alloc = g_cache.bytes;
   d->h_status = g_cache.h_status;
-  d->work64 = g_cache.work64;
-  d->work64_pad = g_cache.npad;
+  d->work = g_cache.work;
+  d->work_bytes = g_cache.work_bytes;
   g_cache = ArenaCache{};
 }
 static void cache_put(wf_domain* d) {
@@ -508,9 +509,9 @@ static void cache_put(wf_domain* d) {
   g_cache.bytes = d->arena_alloc;
   g_cache.dev = d->dev;
   g_cache.h_status = d->h_status;
-  g_cache.work64 = d->work64;
-  g_cache.npad = d->work64_pad;
-  d->work64 = nullptr;
+  g_cache.work = d->work;
+  g_cache.work_bytes = d->work_bytes;
+  d->work = nullptr;
   d->arena = nullptr;
   d->h_status = nullptr;
 }
@@ -731,31 +732,38 @@ static int ensure_cells(wf_domain* d, int64_t ncell) {
   return WF_OK;
 }
 
-// The FP64 form's work arrays.  Without them (not enough memory) the passes
-// compute the pair geometry themselves.
-static void work64_alloc(wf_domain* d) {
-  if (d->work64_tried) return;
-  d->work64_tried = true;
-  if (d->work64) {             // taken over from the cache
-    if (d->work64_pad >= d->npad) return;
-    cudaFree(d->work64);
-    d->work64 = nullptr;
+// Work arrays of at least `bytes`; false when there is no memory for them (the
+// passes then compute the pair geometry themselves).  Not inside a capture.
+static bool work_reserve(wf_domain* d, size_t bytes) {
+  if (!d->pair_cache) return false;
+  if (d->work && d->work_bytes >= bytes) return true;
+  if (d->capturing || (d->work_refused && bytes >= d->work_refused)) return false;
+  if (d->work) {
+    cudaStreamSynchronize(d->stream);   // the passes that still read it
+    cudaFree(d->work);
+    d->work = nullptr;
+    d->geo_valid = d->rr_valid = false;
   }
-  const size_t words = (size_t)(2 * WF_NB_ALLOC + 9) * (size_t)d->npad;
-  d->work64_pad = d->npad;
-  if (cudaMalloc((void**)&d->work64, sizeof(double) * words) != cudaSuccess) {
+  if (cudaMalloc((void**)&d->work, bytes) != cudaSuccess) {
     cudaGetLastError();
-    d->work64 = nullptr;
+    d->work = nullptr;
+    d->work_refused = bytes;
+    return false;
   }
+  d->work_bytes = bytes;
+  return true;
+}
+static size_t work64_bytes(const wf_domain* d) {
+  return sizeof(double) * (size_t)(2 * WF_NB_ALLOC + 9) * (size_t)d->npad;
 }
 // Kept values are of this call's own steps only: anything may have changed
 // between two calls and in the step hook.
 static void work64_drop(wf_domain* d) { d->geo_valid = d->rr_valid = false; }
 static Work64 work64_of(const wf_domain* d) {
   Work64 W{};
-  if (!d->work64 || !d->work64_tried || !d->pair_cache) return W;
+  if (!d->pair_cache || !d->work || d->work_bytes < work64_bytes(d)) return W;
   const int64_t e = (int64_t)WF_NB_ALLOC * d->npad, n = d->npad;
-  W.gk = d->work64;
+  W.gk = reinterpret_cast<double*>(d->work);
   W.r2 = W.gk + e;
   W.mr = W.r2 + e;
   W.rr = W.mr + n + d->rr_cur * n;
@@ -1118,7 +1126,7 @@ static int solve_begin(wf_domain* d, double dt_out) {
 
 static int solve_step_launches(wf_domain* d) {
   cudaStream_t s = d->stream;
-  if (d->precision == 0 && d->pair_cache && !d->capturing) work64_alloc(d);
+  if (d->precision == 0 && !d->capturing) work_reserve(d, work64_bytes(d));
   bool rb;
   if (d->rb_dep > 0.0) {
     // adaptive: rebuild once the plastic strain grew by rb_dep anywhere since
@@ -1386,7 +1394,7 @@ int wf_destroy(wf_domain* d) {
                   M.off32, M.cvert, M.cursor, M.scan_tmp};
     for (void* p : mp) if (p) cudaFree(p);
   }
-  if (d->work64) cudaFree(d->work64);
+  if (d->work) cudaFree(d->work);
   if (d->d_maxdep) cudaFree(d->d_maxdep);
   if (d->h_maxdep) cudaFreeHost(d->h_maxdep);
   if (d->cnb) cudaFree(d->cnb);
@@ -1887,13 +1895,44 @@ int wf_thermal_solve(wf_domain* d, double tf) {
   if (d->precision == 1) k_mixed_init<<<nblk(d->n), 256, 0, d->stream>>>(d->n, CF(d));
   StepParams P = make_params(d);
   NbBuffers N{d->nb, d->nbc};
+  work64_drop(d);
+  const bool mixed = d->precision == 1;
+  const int64_t entries = (int64_t)WF_NB_ALLOC * d->npad, n = d->npad;
+  const bool kept = d->time < tf &&
+                    work_reserve(d, mixed ? (size_t)(4 * entries + 16 * n)
+                                          : sizeof(double) * (size_t)(3 * entries + 5 * n));
+  HeatWork64 H64{};
+  HeatWork32 H32{};
+  if (kept && mixed) {
+    H32.own = reinterpret_cast<float4*>(d->work);
+    H32.mg = reinterpret_cast<float*>(H32.own + n);
+    launch_heat_pairs32(P, CF(d), H32, N, d->stream);
+    d->launches += 1;
+  } else if (kept) {
+    double* w = reinterpret_cast<double*>(d->work);
+    H64.dot = w; H64.r2 = w + entries; H64.ir2 = w + 2 * entries;
+    w += 3 * entries;
+    H64.mr = w; H64.scale = w + n; H64.icp = w + 2 * n; H64.conv = w + 3 * n; H64.fric = w + 4 * n;
+    launch_heat_pairs64(P, CF(d), H64, N, d->stream);
+    d->launches += 1;
+  }
   while (d->time < tf) {
     {
       KTimer t(d, KID_THERMAL);
-      launch_thermal(P, CF(d), Work64{}, N, d->isfirst ? 1 : 0, 0, d->precision == 1 ? 1 : 0,
-                     d->stream);
+      Fields& A = d->F[d->cur];
+      Fields& B = d->F[1 - d->cur];      // its T and th32 take the new temperatures
+      if (kept && mixed) {
+        launch_heat_step32(P, A, H32, B.th32, N, d->isfirst ? 1 : 0, !(d->time + d->dt < tf),
+                           d->stream);
+        std::swap(A.th32, B.th32);
+      } else if (kept) {
+        launch_heat_step64(P, A, H64, B.T, N, d->isfirst ? 1 : 0, d->stream);
+        std::swap(A.T, B.T);
+      } else {
+        launch_thermal(P, A, Work64{}, N, d->isfirst ? 1 : 0, 0, mixed ? 1 : 0, d->stream);
+      }
     }
-    d->launches += 2;
+    d->launches += kept ? 1 : 2;
     d->isfirst = false;
     d->time += d->dt;
     d->step++;

@@ -321,6 +321,27 @@ struct Work64 {
   int geo;           // gk and r2 hold the current positions' and lists' values
   int recip;         // rr holds the current density's reciprocals
 };
+// What a heat solve keeps for its steps (ThermalSolve: positions, densities
+// and lists are fixed inside one solve).
+struct HeatWork64 {
+  double *dot, *r2, *ir2;            // per list entry: x_ij . grad W, r^2, 1 / r^2
+  double *mr, *scale, *icp, *conv, *fric;   // per slot: m/rho, 1/(rho cp), 1/cp, h_conv dS^2,
+                                            // frictional heat rate
+};
+struct HeatWork32 {
+  float* mg;       // per list entry: m_j / rho_j GK
+  float4* own;     // per slot: rho cp, h_conv dS^2 (0: no convection), m cp, frictional heat rate
+};
+void launch_heat_pairs64(const StepParams& P, const Fields& F, const HeatWork64& H,
+                         const NbBuffers& N, cudaStream_t s);
+// one step with its leapfrog update: F.T -> T_out
+void launch_heat_step64(const StepParams& P, const Fields& F, const HeatWork64& H, double* T_out,
+                        const NbBuffers& N, int first, cudaStream_t s);
+void launch_heat_pairs32(const StepParams& P, const Fields& F, const HeatWork32& H,
+                         const NbBuffers& N, cudaStream_t s);
+// one step with its leapfrog update: F.th32 -> th_out; `last`: F.T, F.Tb, F.dTdt are written
+void launch_heat_step32(const StepParams& P, const Fields& F, const HeatWork32& H, float2* th_out,
+                        const NbBuffers& N, int first, int last, cudaStream_t s);
 void launch_fp64_density(const StepParams& P, const Fields& F, const Work64& W, double4* vd2,
                          const NbBuffers& N, cudaStream_t s);
 // returns the number of kernels launched

@@ -335,6 +335,101 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_heat32(StepParams P, Fi
   F.dTdt[i] = heat_rate_mixed(P, F, i, P.k2f * sf, F.vd[i].w, F.xm[i].w, F.T[i], plastic_heat);
 }
 
+// ---- ThermalSolve in the mixed form (src/cuda/Thermal.cu:188-260) ---------
+// Positions, densities and lists do not change inside a heat solve, so the
+// pair factor m_j / rho_j GK of heat_pairs is computed once per solve (one
+// float per list entry, padding entries 0) and a step gathers 8 bytes a
+// neighbour, its temperature, instead of 28; the particle's own factors are
+// kept too (heat_rate_mixed), and the leapfrog update rides in the same pass:
+// the neighbours' temperatures are read from one mirror while the new ones go
+// to another.  T, Tb and dT/dt feed nothing inside a solve and are written by
+// its last step only.  Same operations in the same order as k_heat32 and
+// k_heat_leapfrog.
+__global__ void __launch_bounds__(128) k_heat_pairs32(StepParams P, Fields F, HeatWork32 H,
+                                                      const int32_t* __restrict__ nb,
+                                                      const int32_t* __restrict__ cnt) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= P.n) return;
+  const float4 pi = F.p32[i];
+  const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
+  const int c = cnt[i];
+  const NbList32 list{nb, P.npad, i};
+  for (int b = 0; WF_NB_BLK * b < c; b++) {
+    int js[WF_NB_BLK];
+    float mg[WF_NB_BLK];
+    list.block(b, js);
+#pragma unroll
+    for (int q = 0; q < WF_NB_BLK; q++) {
+      const float4 pj = F.p32[js[q]];
+      const float rj = __ldg(&F.v32[js[q]].w);
+      const float xx = pi.x - pj.x, xy = pi.y - pj.y, xz = pi.z - pj.z;
+      const float GK = gk32_r2(xx * xx + xy * xy + xz * xz, invh, Ch, C);
+      mg[q] = __fdividef(pj.w, rj) * GK;
+    }
+    float4* out = reinterpret_cast<float4*>(H.mg + ((int64_t)b * P.npad + i) * WF_NB_BLK);
+    out[0] = make_float4(mg[0], mg[1], mg[2], mg[3]);
+    out[1] = make_float4(mg[4], mg[5], mg[6], mg[7]);
+  }
+  const float rf = (float)F.vd[i].w, cpf = (float)F.cpT[i], mf = (float)F.xm[i].w;
+  float conv = 0.0f, fric = 0.0f;
+  if (F.bct[i] == 1) conv = P.h_convf * powf(mf / rf, 0.666666666f);
+  if (F.qf && F.qf[i] > 0.0) fric = (float)F.qf[i] / (mf * cpf);
+  H.own[i] = make_float4(rf * cpf, conv, mf * cpf, fric);
+}
+
+__global__ void __launch_bounds__(128) k_heat_step32(StepParams P, Fields F, HeatWork32 H,
+                                                     const float2* __restrict__ th,
+                                                     float2* __restrict__ th_out,
+                                                     const int32_t* __restrict__ nb,
+                                                     const int32_t* __restrict__ cnt, int first,
+                                                     int last) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= P.n) return;
+  const float2 ti = th[i];
+  const int c = cnt[i];
+  const NbList32 list{nb, P.npad, i};
+  float sf = 0.0f;
+  int nx[WF_NB_BLK];
+  if (c > 0) list.block(0, nx);
+  for (int b = 0; WF_NB_BLK * b < c; b++) {
+    float2 tj[WF_NB_BLK];
+#pragma unroll
+    for (int q = 0; q < WF_NB_BLK; q++) tj[q] = __ldg(th + nx[q]);
+    const float4* m4 =
+        reinterpret_cast<const float4*>(H.mg + ((int64_t)b * P.npad + i) * WF_NB_BLK);
+    const float4 ma = __ldg(m4), mb = __ldg(m4 + 1);
+    if (c > WF_NB_BLK * (b + 1)) list.block(b + 1, nx);
+    const float mg[WF_NB_BLK] = {ma.x, ma.y, ma.z, ma.w, mb.x, mb.y, mb.z, mb.w};
+#pragma unroll
+    for (int q = 0; q < WF_NB_BLK; q++) {
+      const float dT = (ti.x - tj[q].x) + (ti.y - tj[q].y);
+      sf += mg[q] * dT;
+    }
+  }
+  const float4 own = H.own[i];
+  float sm = P.k2f * sf / own.x;
+  if (own.w > 0.0f) sm += own.w;
+  if (own.y != 0.0f) sm += own.y * (P.T_inff - ti.x) / own.z;
+  const double rate = (double)sm, dt = P.dt;
+  if (first) {
+    F.Ta[i] = __dsub_rn(F.T[i], __dmul_rn(dt / 2.0, rate));
+    if (last) F.dTdt[i] = rate;
+    th_out[i] = ti;
+    return;
+  }
+  const double ta = F.Ta[i];
+  const double ta2 = __dadd_rn(ta, __dmul_rn(rate, dt));
+  F.Ta[i] = ta2;
+  const double T = __dmul_rn(__dadd_rn(ta2, ta), 0.5);
+  const float thi = (float)T;
+  th_out[i] = make_float2(thi, (float)(T - (double)thi));
+  if (last) {
+    F.T[i] = T;
+    F.Tb[i] = ta;
+    F.dTdt[i] = rate;
+  }
+}
+
 // Johnson-Cook consistent return map of the mixed form, solved for the
 // increment.  With the cached power pwn = ep^n and u = dl / ep,
 //   f(dl) = d0 - 3G dl - B RT pwn ((1 + u)^n - 1),   d0 = st - (A + B pwn) RT,
@@ -1038,6 +1133,15 @@ void launch_fp32_heat(const StepParams& P, const Fields& F, const NbBuffers& N, 
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
       k_heat32, 128, 0, 1, &c_smem, &c_val));
   k_heat32<<<blocks_for(P.n, 128), 128, 0, s>>>(Q, F, N.nb, N.cnt, plastic_heat);
+}
+void launch_heat_pairs32(const StepParams& P, const Fields& F, const HeatWork32& H,
+                         const NbBuffers& N, cudaStream_t s) {
+  k_heat_pairs32<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, H, N.nb, N.cnt);
+}
+void launch_heat_step32(const StepParams& P, const Fields& F, const HeatWork32& H, float2* th_out,
+                        const NbBuffers& N, int first, int last, cudaStream_t s) {
+  k_heat_step32<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, H, F.th32, th_out, N.nb, N.cnt, first,
+                                                     last);
 }
 void launch_fp32_stress(const StepParams& P, const Fields& F, const float4* v32b, float* sigr32,
                         const NbBuffers& N, int* status, const void* mlp_packed,

@@ -581,6 +581,101 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_rate(StepParams P, F
   F.dTdt[i] = heat_rate_fp64(P, F, i, s, rhoi, xi.w, Ti, plastic_heat);
 }
 
+
+// ---- ThermalSolve in FP64 (src/cuda/Thermal.cu:188-260) --------------------
+// Positions, densities and lists do not change inside a heat solve, so what a
+// pair contributes apart from the temperatures is computed once per solve:
+// the product of the position difference with the kernel gradient, r^2 and
+// its reciprocal (three arrays of the lists' layout), m / rho, and the
+// particle's own factors.  A step is then eight FP64 operations a pair instead
+// of 90 (the FP64 pipe bounds both: 64,000 particles 761 -> 68 us a step, 80 %
+// of the pipe's peak; the factors take 364 us a solve) and takes the leapfrog
+// update with it; the neighbours' temperatures are read
+// from one array while the new ones go to another.
+__global__ void __launch_bounds__(64) k_heat_pairs64(StepParams P, Fields F, HeatWork64 H,
+                                                     const int32_t* __restrict__ nb,
+                                                     const int32_t* __restrict__ cnt) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= P.n) return;
+  const double4 xi = F.xm[i];
+  const double rhoi = F.vd[i].w, cp = F.cpT[i];
+  H.mr[i] = xi.w / rhoi;
+  H.scale[i] = 1. / (rhoi * cp);
+  H.icp[i] = 1. / cp;
+  H.conv[i] = F.bct[i] == 1 ? P.h_conv * pow(xi.w / rhoi, 0.666666666) : 0.0;
+  H.fric[i] = F.qf && F.qf[i] > 0.0 ? F.qf[i] / (xi.w * cp) : 0.0;
+  const int c = cnt[i];
+  for (int k = 0; k < c; k++) {
+    const int64_t e = nb_at(P.npad, i, k);
+    const double4 xj = F.xm[__ldg(nb + e)];
+    const double xx = xi.x - xj.x, xy = xi.y - xj.y, xz = xi.z - xj.z;
+    double GK, r2;
+    pair_geometry(P, xx, xy, xz, GK, r2);
+    H.dot[e] = xx * (xx * GK) + xy * (xy * GK) + xz * (xz * GK);
+    H.r2[e] = r2;
+    H.ir2[e] = 1.0 / r2;
+  }
+}
+
+__device__ __forceinline__ double heat_step_term(const HeatWork64& H, const double* __restrict__ T,
+                                                 int64_t e, int j, double Ti, double kk) {
+  const double num = __ldg(H.mr + j) * (kk * (Ti - __ldg(T + j))) * __ldg(H.dot + e);
+  const double r2 = __ldg(H.r2 + e), y = __ldg(H.ir2 + e);
+  // zero and the middle of the range divide by the known reciprocal
+  const bool easy = mid_range(num) || ((__double2hiint(num) << 1) | __double2loint(num)) == 0;
+  return easy && mid_range(y) ? div_known(num, r2, y) : num / r2;
+}
+
+template <int kG>
+__global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_step64(StepParams P, Fields F,
+                                                     HeatWork64 H, const double* __restrict__ T,
+                                                     double* __restrict__ T_out,
+                                                     const int32_t* __restrict__ nb,
+                                                     const int32_t* __restrict__ cnt, int first) {
+  int g;
+  const int64_t i0 = slot64<kG>(g);
+  if (kG == 1 && i0 >= P.n) return;
+  const bool valid = i0 < P.n;
+  const int64_t i = valid ? i0 : 0;
+  const double Ti = T[i], ki = F.kT[i];
+  const double kk = 4.0 * ki * ki / (ki + ki);
+  const int c = valid ? cnt[i] : 0;
+  double s = 0.0;
+  if constexpr (kG == 1) {
+    for (int k = 0; k < c; k++) {
+      const int64_t e = nb_at(P.npad, i, k);
+      s += heat_step_term(H, T, e, __ldg(nb + e), Ti, kk);
+    }
+  } else {
+    const int blocks = warp_blocks(c);
+    for (int b = 0; b < blocks; b++) {
+      double t = 0.0;
+      if (WF_NB_BLK * b + g < c) {
+        const int64_t e = nb_at(P.npad, i, WF_NB_BLK * b + g);
+        t = heat_step_term(H, T, e, __ldg(nb + e), Ti, kk);
+      }
+      s = add_in_order(s, t);
+    }
+    if (!valid || g != 0) return;
+  }
+  // heat_rate_fp64 without plastic heat, from the kept factors
+  s *= H.scale[i];
+  const double fric = H.fric[i];
+  if (fric > 0.0) s += fric;
+  if (F.bct[i] == 1) s += H.icp[i] * (H.conv[i] * (P.T_inf - Ti) / F.xm[i].w);
+  F.dTdt[i] = s;
+  if (first) {
+    F.Ta[i] = Ti - P.dt / 2.0 * s;
+    T_out[i] = Ti;
+    return;
+  }
+  const double ta = F.Ta[i];
+  F.Tb[i] = ta;
+  const double ta2 = ta + s * P.dt;
+  F.Ta[i] = ta2;
+  T_out[i] = (ta2 + ta) / 2.;
+}
+
 }  // namespace
 
 static inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
@@ -625,4 +720,16 @@ void launch_fp64_heat_rate(const StepParams& P, const Fields& F, const Work64& W
                            const NbBuffers& N, int plastic_heat, cudaStream_t s) {
   if (W.gk) WF_LAUNCH64(k_heat_rate, GEO_STORE, N.nb, N.cnt, plastic_heat);
   else WF_LAUNCH64(k_heat_rate, GEO_NONE, N.nb, N.cnt, plastic_heat);
+}
+void launch_heat_pairs64(const StepParams& P, const Fields& F, const HeatWork64& H,
+                         const NbBuffers& N, cudaStream_t s) {
+  k_heat_pairs64<<<blocks_for(P.n, 64), 64, 0, s>>>(P, F, H, N.nb, N.cnt);
+}
+void launch_heat_step64(const StepParams& P, const Fields& F, const HeatWork64& H, double* T_out,
+                        const NbBuffers& N, int first, cudaStream_t s) {
+  if (P.n < kWide64)
+    k_heat_step64<kLanes64><<<blocks_for(P.n * kLanes64, 32), 32, 0, s>>>(P, F, H, F.T, T_out,
+                                                                          N.nb, N.cnt, first);
+  else
+    k_heat_step64<1><<<blocks_for(P.n, 64), 64, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
 }
