@@ -7,6 +7,7 @@
 // return (src/cuda/Mechanical.cu:503-536) with no iterative solve.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -165,118 +166,226 @@ __global__ void __launch_bounds__(128) k_mlp_newton_iters(StepParams P, double G
 }
 
 // ---- training: loss and gradient of the mean squared error -------------------
-// Block of 128 threads = 128 samples.  Shared memory: the parameters, the
-// layer-1 pre-activations and activations, and the layer-2 gradients of the
-// block's samples; weight gradients are reduced over the block's samples from
-// shared memory and added to the global gradient once per block.
-constexpr int TB = 128;
-constexpr int LD = WF_MLP_H + 1;
+// FP32 throughout.  A block of 512 threads takes tiles of 32 samples (a batch
+// of 4,096 is 128 blocks, nearly one per SM; larger sets loop) and keeps its
+// weight gradients in registers over its tiles: thread (ts, to) holds one
+// sample by four units in the products with W2 and a 2 x 4 block of W2's
+// gradient, operands read from shared memory as float4 without bank conflicts.
+// Each block writes its sums to its own row of `part`; the rows are added in a
+// fixed order by the kernel that uses them (k_adam, k_grad_total), so a run
+// gives the same bits every time.  What bounds a training step at this size is
+// the latency of its two kernels, not arithmetic (0.1 GFLOP) or memory.  The
+// kernel before this one took a sample per thread and walked 64 x 64 products
+// serially on 32 blocks: 372 -> 16 us per 4,096 samples (a step with Adam 382
+// -> 21 us; 256 threads per block: 17 us).
+constexpr int kTile = 32;              // samples per tile
+constexpr int kGradThreads = 512;
+constexpr int kGradBlocks = 304;       // most blocks (rows of partial sums): 2 per SM
+constexpr int LDA = WF_MLP_H + 4;      // row stride of the tile arrays (16-byte aligned rows)
+constexpr int kPartRow = (WF_MLP_NPARAM + 1 + 31) / 32 * 32;   // gradient, then the loss
 
-__global__ void __launch_bounds__(TB) k_mlp_grad(const float* __restrict__ P,
-                                                 const float4* __restrict__ X,
-                                                 const float* __restrict__ Yt, int64_t n,
-                                                 int64_t offset, int64_t count, float inv_total,
-                                                 float* __restrict__ grad, float* __restrict__ loss) {
-  extern __shared__ float sm[];
-  float* Ps = sm;                                  // WF_MLP_NPARAM
-  float* Z1 = Ps + ((WF_MLP_NPARAM + 3) & ~3);     // TB x LD
-  float* H1 = Z1 + TB * LD;                        // TB x LD
-  float* G2 = H1 + TB * LD;                        // TB x LD
-  float* Xs = G2 + TB * LD;                        // TB x 4
-  float* red = Xs + TB * 4;                        // 2 x WF_MLP_H + 2
-  for (int k = threadIdx.x; k < WF_MLP_NPARAM; k += TB) Ps[k] = P[k];
-  for (int k = threadIdx.x; k < 2 * WF_MLP_H + 2; k += TB) red[k] = 0.0f;
-  __syncthreads();
-  const float* W1 = Ps + WF_MLP_OFF_W1;
-  const float* b1 = Ps + WF_MLP_OFF_B1;
-  const float* W2 = Ps + WF_MLP_OFF_W2;
-  const float* b2 = Ps + WF_MLP_OFF_B2;
-  const float* w3 = Ps + WF_MLP_OFF_W3;
-  const int s = threadIdx.x;
-  const int64_t gi = offset + (int64_t)blockIdx.x * TB + s;
-  const int nvalid = (int)min((int64_t)TB, count - (int64_t)blockIdx.x * TB);
-  const bool valid = s < nvalid && gi < n;
-  float* z1 = Z1 + s * LD;
-  float* h1 = H1 + s * LD;
-  float* g2 = G2 + s * LD;
-  if (valid) {
-    const float4 x4 = X[gi];
-    const float x[4] = {x4.x, x4.y, x4.z, x4.w};
-    Xs[s * 4 + 0] = x[0]; Xs[s * 4 + 1] = x[1]; Xs[s * 4 + 2] = x[2]; Xs[s * 4 + 3] = x[3];
-    for (int o = 0; o < WF_MLP_H; o++) {
-      float z = b1[o];
-      for (int k = 0; k < 4; k++) z += W1[o * 4 + k] * x[k];
-      z1[o] = z;
-      h1[o] = z / (1.0f + expf(-z));
-    }
-    float y = Ps[WF_MLP_OFF_B3];
-    for (int o = 0; o < WF_MLP_H; o++) {
-      float z = b2[o];
-      for (int k = 0; k < WF_MLP_H; k++) z += W2[o * WF_MLP_H + k] * h1[k];
-      g2[o] = z;                                   // z2 for now
-      y += w3[o] * (z / (1.0f + expf(-z)));
-    }
-    const float e = y - Yt[gi];
-    atomicAdd(loss, e * e * inv_total);
-    const float gy = 2.0f * e * inv_total;
-    atomicAdd(red + 2 * WF_MLP_H, gy);             // gb3
-    for (int o = 0; o < WF_MLP_H; o++) {
-      const float z = g2[o];
-      const float sg = 1.0f / (1.0f + expf(-z));
-      atomicAdd(red + o, gy * z * sg);             // gW3
-      g2[o] = gy * w3[o] * sg * (1.0f + z * (1.0f - sg));
-    }
-  } else {
-    for (int o = 0; o < WF_MLP_H; o++) { z1[o] = 0.f; h1[o] = 0.f; g2[o] = 0.f; }
-    Xs[s * 4 + 0] = Xs[s * 4 + 1] = Xs[s * 4 + 2] = Xs[s * 4 + 3] = 0.f;
-  }
-  __syncthreads();
-  // gW2[o][k] = sum_s g2[s][o] h1[s][k]; gb2[o] = sum_s g2[s][o]
-  for (int e = s; e < WF_MLP_H * WF_MLP_H; e += TB) {
-    const int o = e / WF_MLP_H, k = e % WF_MLP_H;
-    float acc = 0.0f;
-    for (int q = 0; q < TB; q++) acc += G2[q * LD + o] * H1[q * LD + k];
-    atomicAdd(grad + WF_MLP_OFF_W2 + e, acc);
-  }
-  if (s < WF_MLP_H) {
-    float acc = 0.0f;
-    for (int q = 0; q < TB; q++) acc += G2[q * LD + s];
-    atomicAdd(grad + WF_MLP_OFF_B2 + s, acc);
-    atomicAdd(grad + WF_MLP_OFF_W3 + s, red[s]);
-  }
-  if (s == 0) atomicAdd(grad + WF_MLP_OFF_B3, red[2 * WF_MLP_H]);
-  // g1 = (W2^T g2) * silu'(z1), into z1
-  float g1[WF_MLP_H];
-  for (int k = 0; k < WF_MLP_H; k++) {
-    float acc = 0.0f;
-    for (int o = 0; o < WF_MLP_H; o++) acc += W2[o * WF_MLP_H + k] * g2[o];
-    const float z = z1[k];
-    const float sg = 1.0f / (1.0f + expf(-z));
-    g1[k] = acc * sg * (1.0f + z * (1.0f - sg));
-  }
-  __syncthreads();
-  for (int k = 0; k < WF_MLP_H; k++) z1[k] = g1[k];
-  __syncthreads();
-  // gW1[o][k] = sum_s g1[s][o] x[s][k]; gb1[o] = sum_s g1[s][o]
-  for (int e = s; e < WF_MLP_H * 4; e += TB) {
-    const int o = e / 4, k = e % 4;
-    float acc = 0.0f;
-    for (int q = 0; q < TB; q++) acc += Z1[q * LD + o] * Xs[q * 4 + k];
-    atomicAdd(grad + WF_MLP_OFF_W1 + e, acc);
-  }
-  if (s < WF_MLP_H) {
-    float acc = 0.0f;
-    for (int q = 0; q < TB; q++) acc += Z1[q * LD + s];
-    atomicAdd(grad + WF_MLP_OFF_B1 + s, acc);
-  }
+struct GradShared {
+  float W2[WF_MLP_H * LDA];            // [o][k]
+  float W1[WF_MLP_H * 4], b1[WF_MLP_H], b2[WF_MLP_H], w3[WF_MLP_H];
+  float H1[kTile * LDA], D1[kTile * LDA], G2[kTile * LDA];
+  float4 X[kTile];
+};
+
+__device__ __forceinline__ void fma4(float4& acc, float a, const float4& b) {
+  acc.x += a * b.x; acc.y += a * b.y; acc.z += a * b.z; acc.w += a * b.w;
+}
+__device__ __forceinline__ float dot4(float acc, const float4& a, const float4& b) {
+  acc += a.x * b.x; acc += a.y * b.y; acc += a.z * b.z; acc += a.w * b.w;
+  return acc;
 }
 
-__global__ void k_adam(float* __restrict__ P, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, int np, float lr, float b1, float b2, float eps,
-                       float c1, float c2) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= np) return;
-  const float gk = g[k];
+__global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const float* __restrict__ P,
+                                                          const float4* __restrict__ X,
+                                                          const float* __restrict__ Yt,
+                                                          int64_t offset, int64_t count,
+                                                          float inv_total,
+                                                          float* __restrict__ part) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  GradShared& S = *reinterpret_cast<GradShared*>(smem_raw);
+  const int t = threadIdx.x;
+  for (int k = t; k < WF_MLP_H * WF_MLP_H; k += kGradThreads)
+    S.W2[(k / WF_MLP_H) * LDA + k % WF_MLP_H] = P[WF_MLP_OFF_W2 + k];
+  if (t < 4 * WF_MLP_H) S.W1[t] = P[WF_MLP_OFF_W1 + t];
+  if (t < WF_MLP_H) {
+    S.b1[t] = P[WF_MLP_OFF_B1 + t];
+    S.b2[t] = P[WF_MLP_OFF_B2 + t];
+    S.w3[t] = P[WF_MLP_OFF_W3 + t];
+  }
+  const float b3 = P[WF_MLP_OFF_B3];
+  const int ts = t >> 4, to = t & 15;          // sample ts; 16 threads share it
+  float4 gW2[2] = {}, gW1[4] = {};             // gW2 rows 2 ts + r, columns 4 to; gW1 of unit 4 to + r
+  float4 gb1 = {};                             // units 4 to ..
+  float gb2[4] = {}, gw3[4] = {};              // units to + 16 r
+  float gb3 = 0.0f, loss = 0.0f;
+  const int64_t tiles = (count + kTile - 1) / kTile;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t gi = tile * kTile + ts;
+    const bool valid = gi < count;
+    const float4 x = valid ? X[offset + gi] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float target = valid ? Yt[offset + gi] : 0.0f;
+    __syncthreads();                           // the last tile's arrays are done with
+    if (to == 0) S.X[ts] = x;
+    {  // layer 1: units 4 to .. 4 to + 3
+      float h[4], d[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int o = 4 * to + q;
+        const float4 w = *reinterpret_cast<const float4*>(S.W1 + 4 * o);
+        const float z = dot4(S.b1[o], w, x);
+        const float sg = 1.0f / (1.0f + expf(-z));
+        h[q] = valid ? z * sg : 0.0f;
+        d[q] = sg * (1.0f + z * (1.0f - sg));
+      }
+      *reinterpret_cast<float4*>(S.H1 + ts * LDA + 4 * to) = make_float4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<float4*>(S.D1 + ts * LDA + 4 * to) = make_float4(d[0], d[1], d[2], d[3]);
+    }
+    __syncthreads();
+    {  // layer 2, output and its gradient: z2 = b2 + W2 h1 for units to + 16 r
+      float z[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) z[r] = S.b2[to + 16 * r];
+#pragma unroll 4
+      for (int k = 0; k < WF_MLP_H; k += 4) {
+        const float4 h = *reinterpret_cast<const float4*>(S.H1 + ts * LDA + k);
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          z[r] = dot4(z[r], *reinterpret_cast<const float4*>(S.W2 + (to + 16 * r) * LDA + k), h);
+      }
+      float h2[4], d2[4], y = 0.0f;
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const float w3 = S.w3[to + 16 * r];
+        const float sg = 1.0f / (1.0f + expf(-z[r]));
+        h2[r] = z[r] * sg;
+        d2[r] = w3 * sg * (1.0f + z[r] * (1.0f - sg));
+        y += w3 * h2[r];
+      }
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+      const float e = valid ? y + b3 - target : 0.0f;
+      const float gy = 2.0f * e * inv_total;
+      loss += e * e * inv_total;
+      gb3 += gy;
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const float g = gy * d2[r];
+        gw3[r] += gy * h2[r];
+        gb2[r] += g;
+        S.G2[ts * LDA + to + 16 * r] = g;
+      }
+    }
+    __syncthreads();
+    {  // layer 1's gradient: g1 = (W2^T g2) silu'(z1); gW1 = sum_s g1 x, gb1 = sum_s g1
+      float4 g1 = {};
+#pragma unroll 4
+      for (int o = 0; o < WF_MLP_H; o += 4) {
+        const float4 ga = *reinterpret_cast<const float4*>(S.G2 + ts * LDA + o);
+        const float av[4] = {ga.x, ga.y, ga.z, ga.w};
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          fma4(g1, av[q], *reinterpret_cast<const float4*>(S.W2 + (o + q) * LDA + 4 * to));
+      }
+      const float4 d = *reinterpret_cast<const float4*>(S.D1 + ts * LDA + 4 * to);
+      const float g[4] = {g1.x * d.x, g1.y * d.y, g1.z * d.z, g1.w * d.w};
+#pragma unroll
+      for (int q = 0; q < 4; q++) fma4(gW1[q], g[q], x);
+      gb1.x += g[0]; gb1.y += g[1]; gb1.z += g[2]; gb1.w += g[3];
+    }
+    // gW2[o][k] = sum_s g2[s][o] h1[s][k]
+#pragma unroll 8
+    for (int s = 0; s < kTile; s++) {
+      const float2 g = *reinterpret_cast<const float2*>(S.G2 + s * LDA + 2 * ts);
+      const float4 h = *reinterpret_cast<const float4*>(S.H1 + s * LDA + 4 * to);
+      fma4(gW2[0], g.x, h);
+      fma4(gW2[1], g.y, h);
+    }
+  }
+  float* row = part + (int64_t)blockIdx.x * kPartRow;
+#pragma unroll
+  for (int r = 0; r < 2; r++)
+    *reinterpret_cast<float4*>(row + WF_MLP_OFF_W2 + (2 * ts + r) * WF_MLP_H + 4 * to) = gW2[r];
+  // the sums held per sample: over the two samples of the warp, then over the
+  // warps through shared memory (448 values and two scalars per warp)
+  constexpr int kRed = 7 * WF_MLP_H + 2;
+  float* red = reinterpret_cast<float*>(smem_raw) + (t >> 5) * kRed;
+  float v[30] = {gb1.x,    gb1.y,    gb1.z,    gb1.w,    gb2[0],   gb2[1],   gb2[2],   gb2[3],
+                 gw3[0],   gw3[1],   gw3[2],   gw3[3],   gW1[0].x, gW1[0].y, gW1[0].z, gW1[0].w,
+                 gW1[1].x, gW1[1].y, gW1[1].z, gW1[1].w, gW1[2].x, gW1[2].y, gW1[2].z, gW1[2].w,
+                 gW1[3].x, gW1[3].y, gW1[3].z, gW1[3].w, gb3,      loss};
+#pragma unroll
+  for (int q = 0; q < 30; q++) v[q] += __shfl_xor_sync(0xffffffffu, v[q], 16);
+  __syncthreads();                             // the tile arrays become the reduction buffer
+  if ((t & 31) < 16) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      red[4 * to + q] = v[q];
+      red[WF_MLP_H + to + 16 * q] = v[4 + q];
+      red[2 * WF_MLP_H + to + 16 * q] = v[8 + q];
+    }
+#pragma unroll
+    for (int q = 0; q < 16; q++) red[3 * WF_MLP_H + 16 * to + q] = v[12 + q];
+    if (to == 0) {
+      red[kRed - 2] = v[28];
+      red[kRed - 1] = v[29];
+    }
+  }
+  __syncthreads();
+  if (t >= kRed) return;
+  const float* all = reinterpret_cast<const float*>(smem_raw) + t;
+  float a = 0.0f;
+#pragma unroll
+  for (int w = 0; w < kGradThreads / 32; w++) a += all[w * kRed];
+  const int at = t < WF_MLP_H        ? WF_MLP_OFF_B1 + t
+                 : t < 2 * WF_MLP_H  ? WF_MLP_OFF_B2 + t - WF_MLP_H
+                 : t < 3 * WF_MLP_H  ? WF_MLP_OFF_W3 + t - 2 * WF_MLP_H
+                 : t < 7 * WF_MLP_H  ? WF_MLP_OFF_W1 + t - 3 * WF_MLP_H
+                 : t == 7 * WF_MLP_H ? WF_MLP_OFF_B3
+                                     : WF_MLP_NPARAM;
+  row[at] = a;
+}
+
+// The rows' sum of value k on the first 32 threads of a block of 256, value
+// 32 blockIdx.x + lane: eight threads per value, each every eighth row.
+__device__ __forceinline__ float total_of_rows(const float* __restrict__ part, int rows) {
+  __shared__ float sum[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float* p = part + blockIdx.x * 32 + lane;
+  float a = 0.0f;
+#pragma unroll 8
+  for (int r = w; r < rows; r += 8) a += p[(int64_t)r * kPartRow];
+  sum[w][lane] = a;
+  __syncthreads();
+  a = 0.0f;
+  for (int k = 0; k < 8; k++) a += sum[k][lane];
+  return a;
+}
+
+__global__ void __launch_bounds__(256) k_grad_total(const float* __restrict__ part, int rows,
+                                                    float* __restrict__ grad,
+                                                    float* __restrict__ loss) {
+  const float a = total_of_rows(part, rows);
+  const int k = blockIdx.x * 32 + threadIdx.x;
+  if (threadIdx.x >= 32) return;
+  if (k < WF_MLP_NPARAM) grad[k] = a;
+  else if (k == WF_MLP_NPARAM) *loss = a;
+}
+
+// one Adam step from the blocks' partial sums
+__global__ void __launch_bounds__(256) k_adam(float* __restrict__ P, const float* __restrict__ part,
+                                              int rows, float* __restrict__ m,
+                                              float* __restrict__ v, float* __restrict__ loss,
+                                              float lr, float b1, float b2, float eps, float c1,
+                                              float c2) {
+  const float gk = total_of_rows(part, rows);
+  const int k = blockIdx.x * 32 + threadIdx.x;
+  if (threadIdx.x >= 32) return;
+  if (k == WF_MLP_NPARAM) *loss = gk;
+  if (k >= WF_MLP_NPARAM) return;
   const float mk = b1 * m[k] + (1.0f - b1) * gk;
   const float vk = b2 * v[k] + (1.0f - b2) * gk * gk;
   m[k] = mk;
@@ -284,8 +393,14 @@ __global__ void k_adam(float* __restrict__ P, const float* __restrict__ g, float
   P[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
 }
 
-size_t grad_smem_bytes() {
-  return sizeof(float) * (((WF_MLP_NPARAM + 3) & ~3) + 3 * TB * LD + TB * 4 + 2 * WF_MLP_H + 2);
+// partial-sum rows (blocks) of a gradient over `count` samples
+int grad_rows(int64_t count) {
+  return (int)std::min<int64_t>((count + kTile - 1) / kTile, kGradBlocks);
+}
+// the opt-in for the gradient kernel's shared memory, on the current device
+cudaError_t grad_ready() {
+  return cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(GradShared));
 }
 
 StepParams jc_params(const wf_material* m, double rtol) {
@@ -374,11 +489,12 @@ int wf_mlp_grad(const float* params, const float* X, const float* Y, int64_t n, 
   cudaMemcpy(dP, params, sizeof(float) * WF_MLP_NPARAM, cudaMemcpyHostToDevice);
   cudaMemcpy(dX, X, sizeof(float) * 4 * n, cudaMemcpyHostToDevice);
   cudaMemcpy(dY, Y, sizeof(float) * n, cudaMemcpyHostToDevice);
-  cudaMemset(dG, 0, sizeof(float) * WF_MLP_NPARAM);
-  cudaMemset(dL, 0, sizeof(float));
-  const size_t smem = grad_smem_bytes();
-  cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_mlp_grad<<<nb(n, TB), TB, smem>>>(dP, dX, dY, n, 0, n, 1.0f / (float)n, dG, dL);
+  const int rows = grad_rows(n);
+  float* dR = B.get<float>((size_t)rows * kPartRow);
+  if (!dR) return WF_ERR_ALLOC;
+  if (grad_ready() != cudaSuccess) return WF_ERR_CUDA;
+  k_mlp_grad<<<rows, kGradThreads, sizeof(GradShared)>>>(dP, dX, dY, 0, n, 1.0f / (float)n, dR);
+  k_grad_total<<<kPartRow / 32, 256>>>(dR, rows, dG, dL);
   cudaMemcpy(grad, dG, sizeof(float) * WF_MLP_NPARAM, cudaMemcpyDeviceToHost);
   if (cudaMemcpy(loss, dL, sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) return WF_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? WF_OK : WF_ERR_CUDA;
@@ -387,36 +503,40 @@ int wf_mlp_grad(const float* params, const float* X, const float* Y, int64_t n, 
 int wf_mlp_train(float* params, const float* X, const float* Y, int64_t n, int64_t steps,
                  int64_t batch, float lr, float* final_loss) {
   if (!params || !X || !Y || n <= 0 || steps <= 0 || batch <= 0) return WF_ERR_ARG;
+  // one device block: samples, targets, parameters and moments, partial sums, losses
+  const int most = grad_rows(std::min<int64_t>(batch, n));
+  const auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t bX = up(sizeof(float4) * n), bY = up(sizeof(float) * n),
+               bP = up(sizeof(float) * WF_MLP_NPARAM), bR = up(sizeof(float) * most * kPartRow);
   DevBufs B;
-  float* dP = B.get<float>(WF_MLP_NPARAM);
-  float4* dX = B.get<float4>(n);
-  float* dY = B.get<float>(n);
-  float* dG = B.get<float>(WF_MLP_NPARAM);
-  float* dM = B.get<float>(WF_MLP_NPARAM);
-  float* dV = B.get<float>(WF_MLP_NPARAM);
-  float* dL = B.get<float>(steps);
-  if (!dP || !dX || !dY || !dG || !dM || !dV || !dL) return WF_ERR_ALLOC;
+  char* base = B.get<char>(bX + bY + 3 * bP + bR + sizeof(float) * steps);
+  if (!base) return WF_ERR_ALLOC;
+  float4* dX = (float4*)base;
+  float* dY = (float*)(base + bX);
+  float* dP = (float*)(base + bX + bY);
+  float* dM = (float*)((char*)dP + bP);
+  float* dV = (float*)((char*)dM + bP);
+  float* dR = (float*)((char*)dV + bP);
+  float* dL = (float*)((char*)dR + bR);
   cudaMemcpy(dP, params, sizeof(float) * WF_MLP_NPARAM, cudaMemcpyHostToDevice);
   cudaMemcpy(dX, X, sizeof(float) * 4 * n, cudaMemcpyHostToDevice);
   cudaMemcpy(dY, Y, sizeof(float) * n, cudaMemcpyHostToDevice);
-  cudaMemset(dM, 0, sizeof(float) * WF_MLP_NPARAM);
-  cudaMemset(dV, 0, sizeof(float) * WF_MLP_NPARAM);
-  cudaMemset(dL, 0, sizeof(float) * steps);
-  const size_t smem = grad_smem_bytes();
-  cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaMemset(dM, 0, 2 * bP);
+  if (grad_ready() != cudaSuccess) return WF_ERR_CUDA;
   const float b1 = 0.9f, b2 = 0.999f;
   double p1 = 1.0, p2 = 1.0;
   int64_t off = 0;
   for (int64_t st = 0; st < steps; st++) {
     const int64_t cnt = std::min<int64_t>(batch, n - off);
-    cudaMemsetAsync(dG, 0, sizeof(float) * WF_MLP_NPARAM);
-    k_mlp_grad<<<nb(cnt, TB), TB, smem>>>(dP, dX, dY, n, off, cnt, 1.0f / (float)cnt, dG, dL + st);
+    const int rows = grad_rows(cnt);
+    k_mlp_grad<<<rows, kGradThreads, sizeof(GradShared)>>>(dP, dX, dY, off, cnt, 1.0f / (float)cnt,
+                                                          dR);
     p1 *= b1;
     p2 *= b2;
     // cosine decay of the learning rate
     const float lr_t = lr * 0.5f * (1.0f + cosf(3.14159265f * (float)st / (float)steps));
-    k_adam<<<nb(WF_MLP_NPARAM, 256), 256>>>(dP, dG, dM, dV, WF_MLP_NPARAM, lr_t, b1, b2, 1e-8f,
-                                            (float)(1.0 - p1), (float)(1.0 - p2));
+    k_adam<<<kPartRow / 32, 256>>>(dP, dR, rows, dM, dV, dL + st, lr_t, b1, b2, 1e-8f,
+                                   (float)(1.0 - p1), (float)(1.0 - p2));
     off += cnt;
     if (off >= n) off = 0;
   }
