@@ -73,7 +73,7 @@ struct wf_domain {
   Fields F[2]{};
   int cur = 0;
   double4* vd2 = nullptr;
-  float4* v32b = nullptr;
+  Rec32* pvb = nullptr;        // the mirrors with the new density, for the later passes of a step
   float4* a32 = nullptr;       // mixed-form acceleration
   float* sigr32 = nullptr;
   float* mlp_w = nullptr;      // device MLP parameters (FP32, packed layout of wf_mlp.cuh)
@@ -273,8 +273,8 @@ __global__ void k_mixed_init(int64_t n, Fields F) {
   int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
   double4 x = F.xm[s], v = F.vd[s];
-  F.p32[s] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
-  F.v32[s] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)v.w);
+  F.pv[s].p = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
+  F.pv[s].v = make_float4((float)v.x, (float)v.y, (float)v.z, (float)v.w);
   for (int c = 0; c < 6; c++) F.ss32[s * 6 + c] = (float)F.ss6[s * 6 + c];
   const double T = F.T[s];
   const float thi = (float)T;
@@ -424,10 +424,10 @@ static void layout_arena(wf_domain* d, Arena& A) {
     A.take(&F.T, n); A.take(&F.Ta, n); A.take(&F.Tb, n); A.take(&F.dTdt, n);
     A.take(&F.kT, n); A.take(&F.cpT, n);
     A.take(&F.id, n); A.take(&F.bct, n); A.take(&F.perm, n); A.take(&F.nw, n);
-    A.take(&F.xh, n); A.take(&F.p32, n); A.take(&F.v32, n); A.take(&F.ss32, 6 * n);
-    A.take(&F.th32, n); A.take(&F.pwn, n); A.take(&F.p32n, n);
+    A.take(&F.xh, n); A.take(&F.pv, n); A.take(&F.ss32, 6 * n);
+    A.take(&F.th32, n); A.take(&F.pwn, n);
   }
-  A.take(&d->vd2, n); A.take(&d->v32b, n); A.take(&d->a32, n); A.take(&d->sigr32, 8 * n);
+  A.take(&d->vd2, n); A.take(&d->pvb, n); A.take(&d->a32, n); A.take(&d->sigr32, 8 * n);
   A.take(&d->nb, (int64_t)WF_NB_ALLOC * n); A.take(&d->nbc, n); A.take(&d->inv, n);
   A.take(&d->pf, n); A.take(&d->pf2, n); A.take(&d->cellid, n); A.take(&d->s_src, n);
   A.take(&d->s_orig, n); A.take(&d->d_mm, 8); A.take(&d->d_status, WF_STATUS_WORDS);
@@ -1185,24 +1185,23 @@ static int solve_step_launches(wf_domain* d) {
     {
       KTimer t(d, KID_DENSITY);
       if (d->heat_pending)
-        launch_fp32_density_heat(P, F, d->vd2, d->v32b, N, d->heat_pending_first ? 1 : 0,
+        launch_fp32_density_heat(P, F, d->vd2, d->pvb, N, d->heat_pending_first ? 1 : 0,
                                  d->chi > 0.0 ? 1 : 0, TH, L16, s);
       else
-        launch_fp32_density(P, F, d->vd2, d->v32b, N, L16, s);
+        launch_fp32_density(P, F, d->vd2, d->pvb, N, L16, s);
       d->heat_pending = false;
     }
     { KTimer t(d, KID_STRESS);
-      launch_fp32_stress(P, F, d->v32b, d->sigr32, N, d->d_status,
+      launch_fp32_stress(P, F, d->pvb, d->sigr32, N, d->d_status,
                          (d->mlp_on && d->mlp_loaded) ? d->mlp_packed : nullptr, &d->mlp_l1, TH, L16,
                          s); }
     if (!P.contact && d->fuse_integrate) {
       { KTimer t(d, KID_ACCEL);
-        launch_fp32_accel_integrate(P, F, d->v32b, d->sigr32, d->vd2, N, TH, L16, s); }
-      std::swap(d->F[d->cur].p32, d->F[d->cur].p32n);   // the new positions become current
+        launch_fp32_accel_integrate(P, F, d->pvb, d->sigr32, d->vd2, N, TH, L16, s); }
       integrated = true;
     } else {
       KTimer t(d, KID_ACCEL);
-      launch_fp32_accel(P, F, d->v32b, d->sigr32, d->a32, N, s);
+      launch_fp32_accel(P, F, d->pvb, d->sigr32, d->a32, N, s);
     }
   }
   if (P.contact) {                                                                    // :233-257

@@ -78,6 +78,22 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 // over its zone before the BC is imposed (3 each)].
 #define WF_ROW_FIXED 11
 
+// A particle's FP32 mirror, one 32-byte sector: the pair passes gather it with a
+// single 256-bit load (rec_load).
+struct __align__(32) Rec32 {
+  float4 p;         // position xyz, mass w
+  float4 v;         // velocity xyz, density w
+};
+
+__device__ __forceinline__ Rec32 rec_load(const Rec32* a) {
+  Rec32 r;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(r.p.x), "=f"(r.p.y), "=f"(r.p.z), "=f"(r.p.w), "=f"(r.v.x), "=f"(r.v.y), "=f"(r.v.z),
+        "=f"(r.v.w)
+      : "l"(a));
+  return r;
+}
+
 // All per-slot arrays that move with the particles at a reorder.
 struct Fields {
   double4* xm;      // position xyz, mass w
@@ -109,11 +125,9 @@ struct Fields {
   uint8_t* nw;      // not_write_surf_ID
   float4* xh;       // float positions the next neighbour rebuild reads (x_h)
   // mixed-precision mirrors (written by the integration kernel)
-  float4* p32;      // position xyz, mass w
-  float4* v32;      // velocity xyz, density w
+  Rec32* pv;        // position, mass, velocity, density in FP32
   float* ss32;      // deviatoric stress FP32 state (mixed form), 6 per slot
   float2* th32;     // heat-flux mirror (mixed form): T as a float pair (hi, lo)
-  float4* p32n;     // next positions of the fused acceleration + integration pass
   double* pwn;      // cached eps_p^n of the Johnson-Cook law (< 0: not cached yet)
   // contact (allocated when a rigid mesh is added)
   double4* nrm;     // surface normal (solid particles) / element normal (rigid particles)
@@ -366,11 +380,11 @@ void launch_mesh_plane(const StepParams& P, cudaStream_t s);
 struct TileHalo;
 struct List16;
 // density pass alone (mixed form; a call's first step, or heat off)
-void launch_fp32_density(const StepParams& P, const Fields& F, double4* vd2, float4* v32b,
+void launch_fp32_density(const StepParams& P, const Fields& F, double4* vd2, Rec32* pvb,
                          const NbBuffers& N, const List16& L16, cudaStream_t s);
 // density pass of this step with the previous step's heat pass (mixed form);
 // T: tile halos (T.cap = 0: none), L16: 16-bit lists (L16.base null: none)
-void launch_fp32_density_heat(const StepParams& P, const Fields& F, double4* vd2, float4* v32b,
+void launch_fp32_density_heat(const StepParams& P, const Fields& F, double4* vd2, Rec32* pvb,
                               const NbBuffers& N, int first, int plastic_heat, const TileHalo& T,
                               const List16& L16, cudaStream_t s);
 struct MlpL1;
@@ -379,12 +393,12 @@ struct MlpL1;
 // the mixed heat pass alone (a call's last step; the mixed ThermalSolve)
 void launch_fp32_heat(const StepParams& P, const Fields& F, const NbBuffers& N, int plastic_heat,
                       cudaStream_t s);
-void launch_fp32_stress(const StepParams& P, const Fields& F, const float4* v32b,
+void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb,
                         float* sigr32, const NbBuffers& N, int* status, const void* mlp_packed,
                         const MlpL1* mlp_l1, const TileHalo& T, const List16& L16,
                         cudaStream_t s);
-void launch_fp32_accel(const StepParams& P, const Fields& F, const float4* v32b,
+void launch_fp32_accel(const StepParams& P, const Fields& F, const Rec32* pvb,
                        const float* sigr32, float4* a32, const NbBuffers& N, cudaStream_t s);
-void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const float4* v32b,
+void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec32* pvb,
                                  const float* sigr32, const double4* vd2, const NbBuffers& N,
                                  const TileHalo& T, const List16& L16, cudaStream_t s);

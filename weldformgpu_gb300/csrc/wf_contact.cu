@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(128) k_contact_law1(StepParams P, Fields F, fl
   // skip all FP64 work.  The mixed form keeps an FP32 position mirror.
   float px, py, pz;
   if (a32) {
-    const float4 p = F.p32[i];
+    const float4 p = F.pv[i].p;
     px = p.x; py = p.y; pz = p.z;
   } else {
     const double4 p = F.xm[i];
@@ -511,7 +511,7 @@ __global__ void k_contact_particles(StepParams P, Fields F, MeshDev M, int mixed
   F.vd[s] = d4(v, rho);
   F.a[s] = make_double4(0.0, 0.0, 0.0, 0.0);
   F.nrm[s] = M.normal[e];
-  if (mixed) F.v32[s] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)rho);
+  if (mixed) F.pv[s].v = make_float4((float)v.x, (float)v.y, (float)v.z, (float)rho);
 }
 
 inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }

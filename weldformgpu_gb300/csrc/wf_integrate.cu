@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(256) k_integrate(StepParams P, Fields F,
   if (a32) {
     // rigid (non-solid) slots keep the acceleration the BCs left (zero)
     const float4 af = F.perm[i] < P.n_solid ? a32[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    integrate_mixed_one(P, F, vd2, i, af, F.p32);
+    integrate_mixed_one(P, F, vd2, i, af);
     return;
   }
   double4 xm = F.xm[i];

@@ -29,11 +29,11 @@ __device__ __forceinline__ void apply_bc(const StepParams& P, int32_t id, double
 
 // Mixed form: the increments in FP32 (relative error ~1e-7 of the increment),
 // added to the FP64 positions, displacements and velocities; then the FP32
-// mirrors (positions to p32_out, velocities, temperature pair).  af is the
+// mirrors (positions, velocities, temperature pair).  af is the
 // acceleration of the step (zero for rigid slots).
 __device__ __forceinline__ void integrate_mixed_one(const StepParams& P, const Fields& F,
                                                     const double4* __restrict__ vd2, int64_t i,
-                                                    float4 af, float4* __restrict__ p32_out) {
+                                                    float4 af) {
   double4 xm = F.xm[i];
   const double4 v4 = vd2[i];
   const int32_t id = F.id[i];
@@ -59,8 +59,8 @@ __device__ __forceinline__ void integrate_mixed_one(const StepParams& P, const F
   // energy_mode 0: particle 0's S:D of this step (written by the stress pass)
   // for every particle, as k_integrate's FP64 form
   if (P.energy_mode == 0) F.eint[i] += xm.w / v4.w * *P.e0 * P.dt;
-  p32_out[i] = make_float4((float)xm.x, (float)xm.y, (float)xm.z, (float)xm.w);
-  F.v32[i] = make_float4((float)vx, (float)vy, (float)vz, (float)v4.w);
+  F.pv[i].p = make_float4((float)xm.x, (float)xm.y, (float)xm.z, (float)xm.w);
+  F.pv[i].v = make_float4((float)vx, (float)vy, (float)vz, (float)v4.w);
   const double T = F.T[i];
   const float thi = (float)T;
   F.th32[i] = make_float2(thi, (float)(T - (double)thi));

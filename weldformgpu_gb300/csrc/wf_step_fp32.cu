@@ -5,8 +5,9 @@
 // ~1e-7 s increments over long runs): positions, displacements, velocities
 // and their update, density accumulation, equivalent plastic strain, yield
 // stress and the Newton residual, and every reduction.  The gathered
-// neighbour data are FP32 mirrors written by the integration kernel:
-// p32 = (x, m), v32 = (v, rho), and (after the density pass) v32b = (v, rho_new).
+// neighbour data are FP32 mirrors written by the integration kernel, one 32-byte
+// record per particle: pv = (x, m, v, rho), and (after the density pass)
+// pvb = (x, m, v, rho_new).
 // All FP32 constants arrive precomputed in StepParams: on GB300 a per-thread
 // FP64 division or conversion costs as much as the whole FP32 pair loop.
 #include "wf_common.cuh"
@@ -36,6 +37,18 @@ __device__ __forceinline__ T3f mul_ref_f(const T3f& a, const T3f& b) {
   r.zz = a.zx * b.zx + a.zy * b.zy + a.zz * b.zz;
   return r;
 }
+
+// Neighbour records by slot from global memory or by halo rank from a staged
+// tile's shared memory.
+struct RecGlobal {
+  const Rec32* r;
+  __device__ __forceinline__ Rec32 get(int j) const { return rec_load(r + j); }
+};
+struct RecShared {
+  const float4* p;
+  const float4* v;
+  __device__ __forceinline__ Rec32 get(int j) const { return Rec32{p[j], v[j]}; }
+};
 
 // ---- A32: density rate + update (InteractionAlt.cu:166-246, Mechanical.cu:198) --
 // Lane groups of the pair passes: kLanes consecutive lanes share one particle;
@@ -69,13 +82,12 @@ constexpr int kDensBatch = 4;
 // n+1 the heat flux of step n uses the new list (built for these positions).
 // The pair loop of the density + heat pass over the neighbour list L: its
 // entries are slots (NbList32 / NbList16: records gathered from the global
-// arrays gp, gv, gt) or ranks in the tile's halo (NbListS: the arrays are its
+// arrays) or ranks in the tile's halo (NbListS: the arrays are its
 // shared-memory copies).
-template <class L, bool kHeat = true>
+template <class L, class R, bool kHeat = true>
 __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fields& F,
-                                                   const float4* __restrict__ gp,
-                                                   const float4* __restrict__ gv,
-                                                   const float2* __restrict__ gt, const L& list,
+                                                   const R& rec, const float2* __restrict__ gt,
+                                                   const L& list,
                                                    int g, int c, float4 pi, float4 vi, float2 ti,
                                                    bool solid, int32_t idi, float& drho_out,
                                                    float& sf_out) {
@@ -98,8 +110,9 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
       float2 tj[NB];
 #pragma unroll
       for (int q = 0; q < NB; q++) {
-        pj[q] = gp[js[h + q]];
-        vj[q] = gv[js[h + q]];
+        const Rec32 r = rec.get(js[h + q]);
+        pj[q] = r.p;
+        vj[q] = r.v;
         if constexpr (kHeat) tj[q] = gt[js[h + q]];
       }
 #pragma unroll
@@ -136,7 +149,7 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
 // step; every step when heat is off): the density sum of density_heat_pairs.
 __global__ void __launch_bounds__(128, kDensMinBlocks) k_density32(StepParams P, Fields F,
                                                                   double4* __restrict__ vd2,
-                                                                  float4* __restrict__ v32b,
+                                                                  Rec32* __restrict__ pvb,
                                                                   const int32_t* __restrict__ nb,
                                                                   const int32_t* __restrict__ cnt,
                                                                   const List16 L16) {
@@ -147,25 +160,26 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density32(StepParams P,
   if (P.pf_ahead > 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(F.p32 + ia); prefetch_l2(F.v32 + ia); prefetch_l2(cnt + ia);
+      prefetch_l2(F.pv + ia); prefetch_l2(cnt + ia);
       prefetch_l2(F.perm + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 4);
     }
   }
-  const float4 pi = F.p32[i];
-  const float4 vi = F.v32[i];
+  const Rec32 own = rec_load(F.pv + i);
+  const float4 pi = own.p, vi = own.v;
   const int c = solid ? cnt[i] : 0;
   const int32_t idi = F.id[i];
   float drho = 0.0f, sf = 0.0f;
   const int b16 = L16.base ? L16.base[i / WF_TILE] : -1;     // uniform over the block
   const float2 t0 = make_float2(0.f, 0.f);
   if (b16 >= 0)
-    density_heat_pairs<NbList16, false>(P, F, F.p32, F.v32, nullptr,
-                                        NbList16{L16.off, P.npad, i, b16}, 0, c, pi, vi, t0, solid,
-                                        idi, drho, sf);
+    density_heat_pairs<NbList16, RecGlobal, false>(P, F, RecGlobal{F.pv}, nullptr,
+                                                   NbList16{L16.off, P.npad, i, b16}, 0, c, pi, vi,
+                                                   t0, solid, idi, drho, sf);
   else
-    density_heat_pairs<NbList32, false>(P, F, F.p32, F.v32, nullptr, NbList32{nb, P.npad, i}, 0,
-                                        c, pi, vi, t0, solid, idi, drho, sf);
+    density_heat_pairs<NbList32, RecGlobal, false>(P, F, RecGlobal{F.pv}, nullptr,
+                                                   NbList32{nb, P.npad, i}, 0, c, pi, vi, t0, solid,
+                                                   idi, drho, sf);
   const double4 vdi = F.vd[i];
   double rho_new = vdi.w;
   if (solid) {
@@ -173,12 +187,12 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density32(StepParams P,
     rho_new = vdi.w + P.dt * (double)drho;
   }
   vd2[i] = make_double4(vdi.x, vdi.y, vdi.z, rho_new);
-  v32b[i] = make_float4(vi.x, vi.y, vi.z, (float)rho_new);
+  pvb[i] = Rec32{pi, make_float4(vi.x, vi.y, vi.z, (float)rho_new)};
 }
 
 __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepParams P, Fields F,
                                                         double4* __restrict__ vd2,
-                                                        float4* __restrict__ v32b,
+                                                        Rec32* __restrict__ pvb,
                                                         const int32_t* __restrict__ nb,
                                                         const int32_t* __restrict__ cnt,
                                                         int first, int plastic_heat,
@@ -191,15 +205,14 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
   uint16_t* sl = reinterpret_cast<uint16_t*>(st + T.cap);
   int staged = -1;
   if (kDensLanes == 1 && T.cap > 0) {
-    float4* dst[2] = {sp, sv};
-    const float4* src[2] = {F.p32, F.v32};
+    const float4* src = reinterpret_cast<const float4*>(F.pv);
     const int H = T.hcnt[blockIdx.x];
     if (H >= 0 && H <= T.cap) {                 // uniform over the block
       const int32_t* hs = T.halo + T.hoff[blockIdx.x];
       for (int k = threadIdx.x; k < H; k += blockDim.x) {
         const int s = hs[k];
-        cp_async16(dst[0] + k, src[0] + s);
-        cp_async16(dst[1] + k, src[1] + s);
+        cp_async16(sp + k, src + 2 * (int64_t)s);
+        cp_async16(sv + k, src + 2 * (int64_t)s + 1);
         cp_async8(st + k, F.th32 + s);
       }
       stage_lists(T.nbl, P.npad, blockIdx.x, sl);
@@ -212,8 +225,8 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
   const int g = (int)(t & (kDensLanes - 1));
   const int64_t i = t / kDensLanes;
   if (i >= P.n) return;
-  const float4 pi = F.p32[i];
-  const float4 vi = F.v32[i];
+  const Rec32 own = rec_load(F.pv + i);
+  const float4 pi = own.p, vi = own.v;
   const float2 ti = F.th32[i];
   const bool solid = F.perm[i] < P.n_solid;
   const int32_t idi = F.id[i];
@@ -224,7 +237,7 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
   if (P.pf_ahead > 0 && g == 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(F.p32 + ia); prefetch_l2(F.v32 + ia); prefetch_l2(F.th32 + ia);
+      prefetch_l2(F.pv + ia); prefetch_l2(F.th32 + ia);
       prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 4);
     }
@@ -233,13 +246,13 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
   const int c = cnt[i];
   const int b16 = L16.base ? L16.base[i / WF_TILE] : -1;     // uniform over the block
   if (staged >= 0)
-    density_heat_pairs(P, F, sp, sv, st, NbListS{sl, (int)threadIdx.x}, g, c, pi, vi, ti, solid,
-                       idi, drho, sf);
+    density_heat_pairs(P, F, RecShared{sp, sv}, st, NbListS{sl, (int)threadIdx.x}, g, c, pi, vi, ti,
+                       solid, idi, drho, sf);
   else if (b16 >= 0)
-    density_heat_pairs(P, F, F.p32, F.v32, F.th32, NbList16{L16.off, P.npad, i, b16}, g, c, pi, vi,
+    density_heat_pairs(P, F, RecGlobal{F.pv}, F.th32, NbList16{L16.off, P.npad, i, b16}, g, c, pi, vi,
                        ti, solid, idi, drho, sf);
   else
-    density_heat_pairs(P, F, F.p32, F.v32, F.th32, NbList32{nb, P.npad, i}, g, c, pi, vi, ti, solid,
+    density_heat_pairs(P, F, RecGlobal{F.pv}, F.th32, NbList32{nb, P.npad, i}, g, c, pi, vi, ti, solid,
                        idi, drho, sf);
   if constexpr (kDensLanes > 1) {
     const unsigned mask = group_mask<kDensLanes>();
@@ -262,17 +275,15 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
     rho_new = vdi.w + P.dt * (double)drho;
   }
   vd2[i] = make_double4(vdi.x, vdi.y, vdi.z, rho_new);
-  v32b[i] = make_float4(vi.x, vi.y, vi.z, (float)rho_new);
+  pvb[i] = Rec32{pi, make_float4(vi.x, vi.y, vi.z, (float)rho_new)};
 }
 
 // ---- the heat pass alone (ThermalSolveKernel, src/cuda/Thermal.cu:101-142) --
 // A call's last heat pass and every step of the mixed ThermalSolve: the heat
 // sum of density_heat_pairs, the same operations in the same neighbour order
-// (so a separate pass gives the fused pass's sum bit for bit), with the
-// neighbour's density read as one float of its velocity record.
+// (so a separate pass gives the fused pass's sum bit for bit).
 template <class L>
-__device__ __forceinline__ float heat_pairs(const StepParams& P, const float4* __restrict__ gp,
-                                            const float4* __restrict__ gv,
+__device__ __forceinline__ float heat_pairs(const StepParams& P, const Rec32* __restrict__ pv,
                                             const float2* __restrict__ gt, const L& list, int c,
                                             float4 pi, float2 ti) {
   constexpr int NB = kDensBatch;
@@ -293,8 +304,9 @@ __device__ __forceinline__ float heat_pairs(const StepParams& P, const float4* _
       float2 tj[NB];
 #pragma unroll
       for (int q = 0; q < NB; q++) {
-        pj[q] = gp[js[h + q]];
-        rj[q] = __ldg(&gv[js[h + q]].w);
+        const Rec32 r = rec_load(pv + js[h + q]);
+        pj[q] = r.p;
+        rj[q] = r.v.w;
         tj[q] = gt[js[h + q]];
       }
 #pragma unroll
@@ -324,14 +336,14 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_heat32(StepParams P, Fi
   if (P.pf_ahead > 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(F.p32 + ia); prefetch_l2(F.th32 + ia); prefetch_l2(cnt + ia);
+      prefetch_l2(F.pv + ia); prefetch_l2(F.th32 + ia); prefetch_l2(cnt + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 4);
     }
   }
-  const float4 pi = F.p32[i];
+  const float4 pi = F.pv[i].p;
   const float2 ti = F.th32[i];
   const int c = cnt[i];
-  const float sf = heat_pairs(P, F.p32, F.v32, F.th32, NbList32{nb, P.npad, i}, c, pi, ti);
+  const float sf = heat_pairs(P, F.pv, F.th32, NbList32{nb, P.npad, i}, c, pi, ti);
   F.dTdt[i] = heat_rate_mixed(P, F, i, P.k2f * sf, F.vd[i].w, F.xm[i].w, F.T[i], plastic_heat);
 }
 
@@ -350,7 +362,7 @@ __global__ void __launch_bounds__(128) k_heat_pairs32(StepParams P, Fields F, He
                                                       const int32_t* __restrict__ cnt) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= P.n) return;
-  const float4 pi = F.p32[i];
+  const float4 pi = F.pv[i].p;
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
   const int c = cnt[i];
   const NbList32 list{nb, P.npad, i};
@@ -360,8 +372,9 @@ __global__ void __launch_bounds__(128) k_heat_pairs32(StepParams P, Fields F, He
     list.block(b, js);
 #pragma unroll
     for (int q = 0; q < WF_NB_BLK; q++) {
-      const float4 pj = F.p32[js[q]];
-      const float rj = __ldg(&F.v32[js[q]].w);
+      const Rec32 r = rec_load(F.pv + js[q]);
+      const float4 pj = r.p;
+      const float rj = r.v.w;
       const float xx = pi.x - pj.x, xy = pi.y - pj.y, xz = pi.z - pj.z;
       const float GK = gk32_r2(xx * xx + xy * xy + xz * xz, invh, Ch, C);
       mg[q] = __fdividef(pj.w, rj) * GK;
@@ -508,15 +521,14 @@ constexpr float kMlpSteep = 0.02f;
 
 // The rate-tensor pair loop of the stress pass (CalcRateTensors,
 // InteractionAlt.cu:262-383, in FP32) over the neighbour list L (slots into
-// the global arrays gp, gv, or ranks into the tile's halo in shared memory).
+// the global array, or ranks into the tile's halo in shared memory).
 // acc = D xx yy zz xy yz xz, W xy yz xz, with the off-diagonal sums doubled
 // (halved by the caller).  The off-diagonal terms of a pair are a + b (D) and
 // a - b (W) of two products a = s_k x_l, b = s_l x_k: their two sums are
 // accumulated (one FMA each) and combined once after the loop.
-template <class L>
-__device__ __forceinline__ void stress_pairs(const StepParams& P, const Fields& F,
-                                             const float4* __restrict__ gp,
-                                             const float4* __restrict__ gv, const L& list, int c,
+template <class L, class R>
+__device__ __forceinline__ void stress_pairs(const StepParams& P, const Fields& F, const R& rec,
+                                             const L& list, int c,
                                              float4 pi, float4 vi, float* acc) {
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
   float Dxx = 0.f, Dyy = 0.f, Dzz = 0.f;
@@ -535,8 +547,9 @@ __device__ __forceinline__ void stress_pairs(const StepParams& P, const Fields& 
       float4 pj[kStressBatch], vj[kStressBatch];
 #pragma unroll
       for (int q = 0; q < kStressBatch; q++) {
-        pj[q] = gp[js[h + q]];
-        vj[q] = gv[js[h + q]];
+        const Rec32 r = rec.get(js[h + q]);
+        pj[q] = r.p;
+        vj[q] = r.v;
       }
 #pragma unroll
       for (int q = 0; q < kStressBatch; q++) {
@@ -574,17 +587,17 @@ __device__ __forceinline__ void stress_pairs(const StepParams& P, const Fields& 
 // Copies the tile's halo records and local lists into shared memory (every
 // thread of the block takes part; asynchronous 16-byte copies, then one
 // barrier).  Returns the halo size, or -1 when the tile is not staged (the
-// block then gathers from global memory).  n_arr arrays: dst[a][k] =
-// src[a][halo[k]]; the lists go to sl.
-__device__ __forceinline__ int stage_halo16(const TileHalo& T, int64_t npad, int tile, int n_arr,
-                                            float4* const* dst, const float4* const* src,
-                                            uint16_t* sl) {
+// block then gathers from global memory): sp[k], sv[k] = the two halves of
+// rec[halo[k]]; the lists go to sl.
+__device__ __forceinline__ int stage_halo16(const TileHalo& T, int64_t npad, int tile, float4* sp,
+                                            float4* sv, const Rec32* rec, uint16_t* sl) {
   const int H = T.cap > 0 ? T.hcnt[tile] : -1;
   if (H < 0 || H > T.cap) return -1;        // uniform over the block
   const int32_t* hs = T.halo + T.hoff[tile];
   for (int k = threadIdx.x; k < H; k += blockDim.x) {
-    const int s = hs[k];
-    for (int a = 0; a < n_arr; a++) cp_async16(dst[a] + k, src[a] + s);
+    const float4* src = reinterpret_cast<const float4*>(rec + hs[k]);
+    cp_async16(sp + k, src);
+    cp_async16(sv + k, src + 1);
   }
   stage_lists(T.nbl, npad, tile, sl);
   cp_async_wait_all();
@@ -599,7 +612,7 @@ __device__ __forceinline__ int stage_halo16(const TileHalo& T, int64_t npad, int
 // memory per block, and 0.2335 -> 0.226 ms once it took 17 KB).
 template <bool kMlp>
 __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
-                                                  const float4* __restrict__ v32b,
+                                                  const Rec32* __restrict__ pvb,
                                                   float* __restrict__ sigr32,
                                                   const int32_t* __restrict__ nb,
                                                   const int32_t* __restrict__ cnt,
@@ -617,17 +630,12 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
   float4* sp = reinterpret_cast<float4*>(smlp + (kMlp ? WF_UMMA_SMEM : 0));
   float4* sv = sp + T.cap;
   uint16_t* sl = reinterpret_cast<uint16_t*>(sv + T.cap);
-  int staged;
-  {
-    float4* dst[2] = {sp, sv};
-    const float4* src[2] = {F.p32, v32b};
-    staged = stage_halo16(T, P.npad, blockIdx.x, 2, dst, src, sl);
-  }
+  const int staged = stage_halo16(T, P.npad, blockIdx.x, sp, sv, pvb, sl);
   const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const bool valid = i0 < P.n;
   const int64_t i = valid ? i0 : 0;
-  const float4 pi = F.p32[i];
-  const float4 vi = v32b[i];
+  const Rec32 own = rec_load(pvb + i);
+  const float4 pi = own.p, vi = own.v;
   const double rho_new = F.vd[i].w + P.dt * F.drho[i];
   const double p = 0.0 + (P.Cs * P.Cs) * (rho_new - P.rho0);   // FP64: small density change
   if (valid) F.p[i] = p;
@@ -640,7 +648,7 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
   if (P.pf_ahead > 0) {
     const int64_t ia = i0 + P.pf_ahead;     // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(F.p32 + ia); prefetch_l2(v32b + ia); prefetch_l2(F.vd + ia);
+      prefetch_l2(pvb + ia); prefetch_l2(F.vd + ia);
       prefetch_l2(F.drho + ia); prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 4);
     }
@@ -649,11 +657,11 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
   float acc[9];
   const int b16 = L16.base ? L16.base[i0 / WF_TILE] : -1;    // uniform over the block
   if (staged >= 0)
-    stress_pairs(P, F, sp, sv, NbListS{sl, (int)threadIdx.x}, c, pi, vi, acc);
+    stress_pairs(P, F, RecShared{sp, sv}, NbListS{sl, (int)threadIdx.x}, c, pi, vi, acc);
   else if (b16 >= 0)
-    stress_pairs(P, F, F.p32, v32b, NbList16{L16.off, P.npad, i, b16}, c, pi, vi, acc);
+    stress_pairs(P, F, RecGlobal{pvb}, NbList16{L16.off, P.npad, i, b16}, c, pi, vi, acc);
   else
-    stress_pairs(P, F, F.p32, v32b, NbList32{nb, P.npad, i}, c, pi, vi, acc);
+    stress_pairs(P, F, RecGlobal{pvb}, NbList32{nb, P.npad, i}, c, pi, vi, acc);
   float Dxx = acc[0], Dyy = acc[1], Dzz = acc[2], Dxy = acc[3], Dyz = acc[4], Dxz = acc[5];
   float Wxy = acc[6], Wyz = acc[7], Wxz = acc[8];
   Dxy *= 0.5f; Dxz *= 0.5f; Dyz *= 0.5f;
@@ -822,7 +830,7 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
 }
 
 __global__ void __launch_bounds__(128, 6) k_stress32_mlp(StepParams P, Fields F,
-                                                      const float4* __restrict__ v32b,
+                                                      const Rec32* __restrict__ pvb,
                                                       float* __restrict__ sigr32,
                                                       const int32_t* __restrict__ nb,
                                                       const int32_t* __restrict__ cnt,
@@ -830,16 +838,16 @@ __global__ void __launch_bounds__(128, 6) k_stress32_mlp(StepParams P, Fields F,
                                                       const uint4* __restrict__ mlp,
                                                       const MlpL1 l1, const TileHalo T,
                                                       const List16 L16) {
-  stress32_body<true>(P, F, v32b, sigr32, nb, cnt, status, mlp, l1, T, L16);
+  stress32_body<true>(P, F, pvb, sigr32, nb, cnt, status, mlp, l1, T, L16);
 }
 __global__ void __launch_bounds__(128, 6) k_stress32(StepParams P, Fields F,
-                                                     const float4* __restrict__ v32b,
+                                                     const Rec32* __restrict__ pvb,
                                                      float* __restrict__ sigr32,
                                                      const int32_t* __restrict__ nb,
                                                      const int32_t* __restrict__ cnt,
                                                      int* __restrict__ status,
                                                      const TileHalo T, const List16 L16) {
-  stress32_body<false>(P, F, v32b, sigr32, nb, cnt, status, nullptr, MlpL1{}, T, L16);
+  stress32_body<false>(P, F, pvb, sigr32, nb, cnt, status, nullptr, MlpL1{}, T, L16);
 }
 
 // ---- C32: acceleration + Monaghan viscosity (InteractionAlt.cu:18-150) ----
@@ -855,22 +863,22 @@ static_assert(WF_NB_BLK / kAccelLanes >= kAccelBatch, "batch within the lane's s
 
 // Neighbour records of the acceleration pass, from global memory (the slot
 // arrays) or from the tile's halo in shared memory (indexed by local list).
+template <class R>
 struct AccelSrc {
-  const float4* p;
-  const float4* v;
+  R rec;
   const float4* sa;
   const float2* sb;
 };
 
-template <class L>
+template <class L, class R>
 __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields& F,
-                                              const float4* __restrict__ v32b,
+                                              const Rec32* __restrict__ pvb,
                                               const float* __restrict__ sigr32,
                                               const int32_t* __restrict__ cnt, int64_t i, int g,
-                                              const AccelSrc& src, const L& list) {
+                                              const AccelSrc<R>& src, const L& list) {
   constexpr int W = WF_NB_BLK / kAccelLanes;
-  const float4 pi = F.p32[i];
-  const float4 vi = v32b[i];
+  const Rec32 own = rec_load(pvb + i);
+  const float4 pi = own.p, vi = own.v;
   const int32_t idi = F.id[i];
   const float4* sga;
   const float2* sgb;
@@ -898,8 +906,9 @@ __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields&
 #pragma unroll
       for (int q = 0; q < kAccelBatch; q++) {
         const int j = js[hh + q];
-        pj[q] = src.p[j];
-        vj[q] = src.v[j];
+        const Rec32 r = src.rec.get(j);
+        pj[q] = r.p;
+        vj[q] = r.v;
         t0[q] = src.sa[j];
         t1[q] = src.sb[j];
       }
@@ -954,7 +963,7 @@ __device__ __forceinline__ int64_t accel_slot(int& g) {
 }
 
 __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
-                                                 const float4* __restrict__ v32b,
+                                                 const Rec32* __restrict__ pvb,
                                                  const float* __restrict__ sigr32,
                                                  float4* __restrict__ a32,
                                                  const int32_t* __restrict__ nb,
@@ -968,7 +977,7 @@ __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
   if (P.pf_ahead > 0 && g == 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(F.p32 + ia); prefetch_l2(v32b + ia); prefetch_l2(sga + ia);
+      prefetch_l2(pvb + ia); prefetch_l2(sga + ia);
       prefetch_l2(sgb + ia); prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
       prefetch_l2(F.id + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++)
@@ -976,38 +985,36 @@ __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
     }
   }
   if (F.perm[i] >= P.n_solid) return;
-  const AccelSrc src{F.p32, v32b, sga, sgb};
-  const float4 af = accel_value(P, F, v32b, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
+  const AccelSrc<RecGlobal> src{{pvb}, sga, sgb};
+  const float4 af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
   if (g == 0) a32[i] = af;
 }
 
 // The acceleration pass with the integration of the same slot behind it
 // (no contact stage in between): one pass instead of two, the integration's
 // FP64 work and traffic overlapping the other warps' neighbour gathers.
-// Neighbours' positions are read from F.p32 while the new positions go to
-// p32n (the two are swapped by the host after the launch); the other mirrors
-// written here (v32, th32) are not read by this pass.
+// Neighbours are read from pvb (the density pass's copy of the mirrors) while
+// the new mirrors go to F.pv and th32, which this pass does not read.
 __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
-                                                     const float4* __restrict__ v32b,
+                                                     const Rec32* __restrict__ pvb,
                                                      const float* __restrict__ sigr32,
                                                      const double4* __restrict__ vd2,
                                                      const int32_t* __restrict__ nb,
-                                                     const int32_t* __restrict__ cnt,
-                                                     float4* __restrict__ p32n, const List16 L16) {
+                                                     const int32_t* __restrict__ cnt, const List16 L16) {
   int g;
   const int64_t i = accel_slot(g);
   if (i >= P.n) return;
   const float4* sga;
   const float2* sgb;
   sigr32_split(sigr32, P.npad, sga, sgb);
-  const AccelSrc src{F.p32, v32b, sga, sgb};
+  const AccelSrc<RecGlobal> src{{pvb}, sga, sgb};
   if (P.state_pf && g == 0) {
     prefetch_l2(F.xm + i); prefetch_l2(vd2 + i); prefetch_l2(F.u + i); prefetch_l2(F.T + i);
   }
   if (P.pf_ahead > 0 && g == 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(F.p32 + ia); prefetch_l2(v32b + ia); prefetch_l2(sga + ia);
+      prefetch_l2(pvb + ia); prefetch_l2(sga + ia);
       prefetch_l2(sgb + ia); prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
       prefetch_l2(F.id + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 2 * kAccelLanes);
@@ -1018,11 +1025,11 @@ __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
   if (F.perm[i] < P.n_solid) {
     const int b16 = L16.base ? L16.base[i / WF_TILE] : -1;   // uniform over the block
     if (b16 >= 0)
-      af = accel_value(P, F, v32b, sigr32, cnt, i, g, src, NbList16{L16.off, P.npad, i, b16});
+      af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList16{L16.off, P.npad, i, b16});
     else
-      af = accel_value(P, F, v32b, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
+      af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
   }
-  if (g == 0) integrate_mixed_one(P, F, vd2, i, af, p32n);
+  if (g == 0) integrate_mixed_one(P, F, vd2, i, af);
 }
 
 // The same pass for staged tiles: a block of 2 x 128 threads is one tile;
@@ -1030,9 +1037,9 @@ __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
 // shared memory, then reads the neighbours from there through the local
 // lists.  Tiles that are not staged gather from global memory.
 __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
-    StepParams P, Fields F, const float4* __restrict__ v32b, const float* __restrict__ sigr32,
+    StepParams P, Fields F, const Rec32* __restrict__ pvb, const float* __restrict__ sigr32,
     const double4* __restrict__ vd2, const int32_t* __restrict__ nb,
-    const int32_t* __restrict__ cnt, float4* __restrict__ p32n, const TileHalo T) {
+    const int32_t* __restrict__ cnt, const TileHalo T) {
   static_assert(kAccelLanes == 2, "one tile per block of 2 lanes per slot");
   extern __shared__ __align__(16) uint8_t sac[];
   const float4* sga;
@@ -1050,8 +1057,9 @@ __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
       const int32_t* hs = T.halo + T.hoff[blockIdx.x];
       for (int k = threadIdx.x; k < H; k += blockDim.x) {
         const int s = hs[k];
-        cp_async16(sp + k, F.p32 + s);
-        cp_async16(sv + k, v32b + s);
+        const float4* rec = reinterpret_cast<const float4*>(pvb + s);
+        cp_async16(sp + k, rec);
+        cp_async16(sv + k, rec + 1);
         cp_async16(ssa + k, sga + s);
         cp_async8(ssb + k, sgb + s);
       }
@@ -1067,14 +1075,14 @@ __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
   float4 af = make_float4(0.f, 0.f, 0.f, 0.f);   // rigid (non-solid) slots: moved by their BCs
   if (F.perm[i] < P.n_solid) {
     if (staged >= 0) {
-      const AccelSrc src{sp, sv, ssa, ssb};
-      af = accel_value(P, F, v32b, sigr32, cnt, i, g, src, NbListS{sl, (int)(threadIdx.x >> 1)});
+      const AccelSrc<RecShared> src{{sp, sv}, ssa, ssb};
+      af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbListS{sl, (int)(threadIdx.x >> 1)});
     } else {
-      const AccelSrc src{F.p32, v32b, sga, sgb};
-      af = accel_value(P, F, v32b, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
+      const AccelSrc<RecGlobal> src{{pvb}, sga, sgb};
+      af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
     }
   }
-  if (g == 0) integrate_mixed_one(P, F, vd2, i, af, p32n);
+  if (g == 0) integrate_mixed_one(P, F, vd2, i, af);
 }
 
 }  // namespace
@@ -1099,16 +1107,16 @@ static int64_t wave_slots(K kernel, int threads, size_t smem, int lanes, size_t*
   return *c_val;
 }
 
-void launch_fp32_density(const StepParams& P, const Fields& F, double4* vd2, float4* v32b,
+void launch_fp32_density(const StepParams& P, const Fields& F, double4* vd2, Rec32* pvb,
                          const NbBuffers& N, const List16& L16, cudaStream_t s) {
   static size_t c_smem = 0;
   static int64_t c_val = 0;
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
       k_density32, 128, 0, 1, &c_smem, &c_val));
-  k_density32<<<blocks_for(P.n, 128), 128, 0, s>>>(Q, F, vd2, v32b, N.nb, N.cnt, L16);
+  k_density32<<<blocks_for(P.n, 128), 128, 0, s>>>(Q, F, vd2, pvb, N.nb, N.cnt, L16);
 }
-void launch_fp32_density_heat(const StepParams& P, const Fields& F, double4* vd2, float4* v32b,
+void launch_fp32_density_heat(const StepParams& P, const Fields& F, double4* vd2, Rec32* pvb,
                               const NbBuffers& N, int first, int plastic_heat, const TileHalo& T,
                               const List16& L16, cudaStream_t s) {
   TileHalo Tl = T;
@@ -1123,7 +1131,7 @@ void launch_fp32_density_heat(const StepParams& P, const Fields& F, double4* vd2
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
       k_density_heat32, 128, smem, kDensLanes, &c_smem, &c_val));
   k_density_heat32<<<blocks_for(P.n * kDensLanes, 128), 128, smem, s>>>(
-      Q, F, vd2, v32b, N.nb, N.cnt, first, plastic_heat, Tl, L16);
+      Q, F, vd2, pvb, N.nb, N.cnt, first, plastic_heat, Tl, L16);
 }
 void launch_fp32_heat(const StepParams& P, const Fields& F, const NbBuffers& N, int plastic_heat,
                       cudaStream_t s) {
@@ -1143,7 +1151,7 @@ void launch_heat_step32(const StepParams& P, const Fields& F, const HeatWork32& 
   k_heat_step32<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, H, F.th32, th_out, N.nb, N.cnt, first,
                                                      last);
 }
-void launch_fp32_stress(const StepParams& P, const Fields& F, const float4* v32b, float* sigr32,
+void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, float* sigr32,
                         const NbBuffers& N, int* status, const void* mlp_packed,
                         const MlpL1* mlp_l1, const TileHalo& T, const List16& L16,
                         cudaStream_t s) {
@@ -1159,26 +1167,26 @@ void launch_fp32_stress(const StepParams& P, const Fields& F, const float4* v32b
     opt_in_smem(k_stress32_mlp, smem, opted[1]);
     Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
         k_stress32_mlp, 128, smem, 1, &c_smem[1], &c_val[1]));
-    k_stress32_mlp<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, v32b, sigr32, N.nb, N.cnt,
+    k_stress32_mlp<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, pvb, sigr32, N.nb, N.cnt,
                                                            status, W, l1, T, L16);
   } else {
     opt_in_smem(k_stress32, smem, opted[0]);
     Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
         k_stress32, 128, smem, 1, &c_smem[0], &c_val[0]));
-    k_stress32<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, v32b, sigr32, N.nb, N.cnt, status,
+    k_stress32<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, pvb, sigr32, N.nb, N.cnt, status,
                                                        T, L16);
   }
 }
-void launch_fp32_accel(const StepParams& P, const Fields& F, const float4* v32b,
+void launch_fp32_accel(const StepParams& P, const Fields& F, const Rec32* pvb,
                        const float* sigr32, float4* a32, const NbBuffers& N, cudaStream_t s) {
   static size_t c_smem = 0;
   static int64_t c_val = 0;
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
       k_accel32, 128, 0, kAccelLanes, &c_smem, &c_val));
-  k_accel32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, v32b, sigr32, a32, N.nb, N.cnt);
+  k_accel32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sigr32, a32, N.nb, N.cnt);
 }
-void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const float4* v32b,
+void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec32* pvb,
                                  const float* sigr32, const double4* vd2, const NbBuffers& N,
                                  const TileHalo& T, const List16& L16, cudaStream_t s) {
   if (T.cap > 0) {
@@ -1186,7 +1194,7 @@ void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const flo
     static size_t opted[64] = {};
     opt_in_smem(k_accel_int32_tiles, smem, opted);
     k_accel_int32_tiles<<<blocks_for(P.n * kAccelLanes, 2 * WF_TILE), 2 * WF_TILE, smem, s>>>(
-        P, F, v32b, sigr32, vd2, N.nb, N.cnt, F.p32n, T);
+        P, F, pvb, sigr32, vd2, N.nb, N.cnt, T);
     return;
   }
   static size_t c_smem = 0;
@@ -1194,6 +1202,6 @@ void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const flo
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
       k_accel_int32, 128, 0, kAccelLanes, &c_smem, &c_val));
-  k_accel_int32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, v32b, sigr32, vd2, N.nb,
-                                                                   N.cnt, F.p32n, L16);
+  k_accel_int32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sigr32, vd2, N.nb,
+                                                                   N.cnt, L16);
 }
