@@ -73,9 +73,9 @@ struct wf_domain {
   Fields F[2]{};
   int cur = 0;
   double4* vd2 = nullptr;
-  Rec32* pvb = nullptr;        // the mirrors with the new density, for the later passes of a step
+  Rec32* pvb = nullptr;        // position, mass | velocity, new density: the later passes of a step
   float4* a32 = nullptr;       // mixed-form acceleration
-  float* sigr32 = nullptr;
+  Rec32* sigr32 = nullptr;     // stress / rho^2: xx yy zz xy | yz xz
   float* mlp_w = nullptr;      // device MLP parameters (FP32, packed layout of wf_mlp.cuh)
   void* mlp_packed = nullptr;  // BF16 tensor-core fragment image of mlp_w
   MlpL1 mlp_l1{};              // layer 1 of mlp_w (a kernel parameter of the stress pass)
@@ -273,12 +273,15 @@ __global__ void k_mixed_init(int64_t n, Fields F) {
   int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
   double4 x = F.xm[s], v = F.vd[s];
-  F.pv[s].p = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
-  F.pv[s].v = make_float4((float)v.x, (float)v.y, (float)v.z, (float)v.w);
+  const float m = (float)x.w;
   for (int c = 0; c < 6; c++) F.ss32[s * 6 + c] = (float)F.ss6[s * 6 + c];
   const double T = F.T[s];
-  const float thi = (float)T;
-  F.th32[s] = make_float2(thi, (float)(T - (double)thi));
+  const float thi = (float)T, tlo = (float)(T - (double)thi);
+  F.m32[s] = m;
+  F.pv[s].p = make_float4((float)x.x, (float)x.y, (float)x.z, __fdividef(m, (float)v.w));
+  F.pv[s].v = make_float4((float)v.x, (float)v.y, (float)v.z, thi);
+  F.tl32[s] = tlo;
+  F.th32[s] = make_float2(thi, tlo);
 }
 // FP64 copy of the FP32 deviatoric state (mixed -> plain switch)
 __global__ void k_mixed_to_fp64(int64_t n, Fields F) {
@@ -424,10 +427,10 @@ static void layout_arena(wf_domain* d, Arena& A) {
     A.take(&F.T, n); A.take(&F.Ta, n); A.take(&F.Tb, n); A.take(&F.dTdt, n);
     A.take(&F.kT, n); A.take(&F.cpT, n);
     A.take(&F.id, n); A.take(&F.bct, n); A.take(&F.perm, n); A.take(&F.nw, n);
-    A.take(&F.xh, n); A.take(&F.pv, n); A.take(&F.ss32, 6 * n);
+    A.take(&F.xh, n); A.take(&F.pv, n); A.take(&F.tl32, n); A.take(&F.m32, n); A.take(&F.ss32, 6 * n);
     A.take(&F.th32, n); A.take(&F.pwn, n);
   }
-  A.take(&d->vd2, n); A.take(&d->pvb, n); A.take(&d->a32, n); A.take(&d->sigr32, 8 * n);
+  A.take(&d->vd2, n); A.take(&d->pvb, n); A.take(&d->a32, n); A.take(&d->sigr32, n);
   A.take(&d->nb, (int64_t)WF_NB_ALLOC * n); A.take(&d->nbc, n); A.take(&d->inv, n);
   A.take(&d->pf, n); A.take(&d->pf2, n); A.take(&d->cellid, n); A.take(&d->s_src, n);
   A.take(&d->s_orig, n); A.take(&d->d_mm, 8); A.take(&d->d_status, WF_STATUS_WORDS);

@@ -78,11 +78,14 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 // over its zone before the BC is imposed (3 each)].
 #define WF_ROW_FIXED 11
 
-// A particle's FP32 mirror, one 32-byte sector: the pair passes gather it with a
-// single 256-bit load (rec_load).
+// A particle's FP32 data as the mixed pair passes gather them: one 32-byte
+// sector, read with a single 256-bit load (rec_load).  What bounds those passes
+// is the L1 data pipe, one access per distinct 128-byte line that a warp's
+// gather touches (ncu: 71-88 % of its peak), so each pass's neighbour data
+// sit in as few and as small records as its arithmetic allows.
 struct __align__(32) Rec32 {
-  float4 p;         // position xyz, mass w
-  float4 v;         // velocity xyz, density w
+  float4 p;
+  float4 v;
 };
 
 __device__ __forceinline__ Rec32 rec_load(const Rec32* a) {
@@ -125,9 +128,11 @@ struct Fields {
   uint8_t* nw;      // not_write_surf_ID
   float4* xh;       // float positions the next neighbour rebuild reads (x_h)
   // mixed-precision mirrors (written by the integration kernel)
-  Rec32* pv;        // position, mass, velocity, density in FP32
+  Rec32* pv;        // FP32: position, m / rho | velocity, T (high part of the pair)
+  float* tl32;      // FP32 low part of T: T = v.w + tl32 to ~48 bits
+  float* m32;       // FP32 mass
   float* ss32;      // deviatoric stress FP32 state (mixed form), 6 per slot
-  float2* th32;     // heat-flux mirror (mixed form): T as a float pair (hi, lo)
+  float2* th32;     // T as a float pair (hi, lo), ThermalSolve's own mirror
   double* pwn;      // cached eps_p^n of the Johnson-Cook law (< 0: not cached yet)
   // contact (allocated when a rigid mesh is added)
   double4* nrm;     // surface normal (solid particles) / element normal (rigid particles)
@@ -394,11 +399,11 @@ struct MlpL1;
 void launch_fp32_heat(const StepParams& P, const Fields& F, const NbBuffers& N, int plastic_heat,
                       cudaStream_t s);
 void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb,
-                        float* sigr32, const NbBuffers& N, int* status, const void* mlp_packed,
+                        Rec32* sigr32, const NbBuffers& N, int* status, const void* mlp_packed,
                         const MlpL1* mlp_l1, const TileHalo& T, const List16& L16,
                         cudaStream_t s);
 void launch_fp32_accel(const StepParams& P, const Fields& F, const Rec32* pvb,
-                       const float* sigr32, float4* a32, const NbBuffers& N, cudaStream_t s);
+                       const Rec32* sigr32, float4* a32, const NbBuffers& N, cudaStream_t s);
 void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec32* pvb,
-                                 const float* sigr32, const double4* vd2, const NbBuffers& N,
+                                 const Rec32* sigr32, const double4* vd2, const NbBuffers& N,
                                  const TileHalo& T, const List16& L16, cudaStream_t s);

@@ -511,7 +511,10 @@ __global__ void k_contact_particles(StepParams P, Fields F, MeshDev M, int mixed
   F.vd[s] = d4(v, rho);
   F.a[s] = make_double4(0.0, 0.0, 0.0, 0.0);
   F.nrm[s] = M.normal[e];
-  if (mixed) F.pv[s].v = make_float4((float)v.x, (float)v.y, (float)v.z, (float)rho);
+  if (mixed) {
+    float4& m = F.pv[s].v;
+    m.x = (float)v.x; m.y = (float)v.y; m.z = (float)v.z;
+  }
 }
 
 inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }

@@ -64,7 +64,8 @@ __global__ void __launch_bounds__(256) k_heat_leapfrog(StepParams P, Fields F, i
   const double T = heat_leapfrog_one(P, F, i, F.dTdt[i], first);
   if (mixed && !first) {
     const float thi = (float)T;
-    F.th32[i] = make_float2(thi, (float)(T - (double)thi));
+    F.pv[i].v.w = thi;
+    F.tl32[i] = (float)(T - (double)thi);
   }
 }
 

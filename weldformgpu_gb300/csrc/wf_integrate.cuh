@@ -59,9 +59,11 @@ __device__ __forceinline__ void integrate_mixed_one(const StepParams& P, const F
   // energy_mode 0: particle 0's S:D of this step (written by the stress pass)
   // for every particle, as k_integrate's FP64 form
   if (P.energy_mode == 0) F.eint[i] += xm.w / v4.w * *P.e0 * P.dt;
-  F.pv[i].p = make_float4((float)xm.x, (float)xm.y, (float)xm.z, (float)xm.w);
-  F.pv[i].v = make_float4((float)vx, (float)vy, (float)vz, (float)v4.w);
   const double T = F.T[i];
   const float thi = (float)T;
-  F.th32[i] = make_float2(thi, (float)(T - (double)thi));
+  const float m = (float)xm.w;
+  F.m32[i] = m;
+  F.pv[i].p = make_float4((float)xm.x, (float)xm.y, (float)xm.z, __fdividef(m, (float)v4.w));
+  F.pv[i].v = make_float4((float)vx, (float)vy, (float)vz, thi);
+  F.tl32[i] = (float)(T - (double)thi);
 }

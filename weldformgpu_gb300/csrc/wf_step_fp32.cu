@@ -5,9 +5,10 @@
 // ~1e-7 s increments over long runs): positions, displacements, velocities
 // and their update, density accumulation, equivalent plastic strain, yield
 // stress and the Newton residual, and every reduction.  The gathered
-// neighbour data are FP32 mirrors written by the integration kernel, one 32-byte
-// record per particle: pv = (x, m, v, rho), and (after the density pass)
-// pvb = (x, m, v, rho_new).
+// neighbour data are 32-byte FP32 records (Rec32): pv = (x, m/rho | v, T_hi) with
+// T_lo beside it, written by the integration, for the density + heat pass;
+// pvb = (x, m | v, rho_new), written by the density pass, for the stress and
+// acceleration passes; sigr32 = stress / rho^2, written by the stress pass.
 // All FP32 constants arrive precomputed in StepParams: on GB300 a per-thread
 // FP64 division or conversion costs as much as the whole FP32 pair loop.
 #include "wf_common.cuh"
@@ -86,9 +87,9 @@ constexpr int kDensBatch = 4;
 // shared-memory copies).
 template <class L, class R, bool kHeat = true>
 __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fields& F,
-                                                   const R& rec, const float2* __restrict__ gt,
-                                                   const L& list,
-                                                   int g, int c, float4 pi, float4 vi, float2 ti,
+                                                   const R& rec, const float* __restrict__ gt,
+                                                   const L& list, int g, int c, float4 pi,
+                                                   float4 vi, float2 ti,
                                                    bool solid, int32_t idi, float& drho_out,
                                                    float& sf_out) {
   constexpr int W = WF_NB_BLK / kDensLanes;
@@ -107,7 +108,7 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
 #pragma unroll
     for (int h = 0; h < W; h += NB) {
       float4 pj[NB], vj[NB];
-      float2 tj[NB];
+      float tj[NB];
 #pragma unroll
       for (int q = 0; q < NB; q++) {
         const Rec32 r = rec.get(js[h + q]);
@@ -124,11 +125,11 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
         const float xx = pi.x - pj[q].x, xy = pi.y - pj[q].y, xz = pi.z - pj[q].z;
         const float GK = gk32_r2(xx * xx + xy * xy + xz * xz, invh, Ch, C);
         // m_j / rho_j GK, shared by both sums
-        const float mg = __fdividef(pj[q].w, vj[q].w) * GK;
+        const float mg = pj[q].w * GK;
         // heat flux (every particle, no contact filter); the pair
         // conductivity 4 k_i k_j / (k_i + k_j) = 2k multiplies the sum
         if constexpr (kHeat) {
-          const float dT = (ti.x - tj[q].x) + (ti.y - tj[q].y);
+          const float dT = (ti.x - vj[q].w) + (ti.y - tj[q]);
           sf += mg * dT;
         }
         // density rate (solid particles, contact filter); rho_i multiplies the sum
@@ -141,7 +142,7 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
       }
     }
   }
-  drho_out = drho * vi.w;
+  drho_out = drho;             // rho_i multiplies it (caller)
   sf_out = sf;
 }
 
@@ -181,13 +182,15 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density32(StepParams P,
                                                    NbList32{nb, P.npad, i}, 0, c, pi, vi, t0, solid,
                                                    idi, drho, sf);
   const double4 vdi = F.vd[i];
+  drho *= (float)vdi.w;
   double rho_new = vdi.w;
   if (solid) {
     F.drho[i] = (double)drho;
     rho_new = vdi.w + P.dt * (double)drho;
   }
   vd2[i] = make_double4(vdi.x, vdi.y, vdi.z, rho_new);
-  pvb[i] = Rec32{pi, make_float4(vi.x, vi.y, vi.z, (float)rho_new)};
+  pvb[i] = Rec32{make_float4(pi.x, pi.y, pi.z, F.m32[i]),
+                 make_float4(vi.x, vi.y, vi.z, (float)rho_new)};
 }
 
 __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepParams P, Fields F,
@@ -201,8 +204,8 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
   extern __shared__ __align__(16) uint8_t sdh[];
   float4* sp = reinterpret_cast<float4*>(sdh);
   float4* sv = sp + T.cap;
-  float2* st = reinterpret_cast<float2*>(sv + T.cap);
-  uint16_t* sl = reinterpret_cast<uint16_t*>(st + T.cap);
+  float* st = reinterpret_cast<float*>(sv + T.cap);
+  uint16_t* sl = reinterpret_cast<uint16_t*>(st + ((T.cap + 3) & ~3));
   int staged = -1;
   if (kDensLanes == 1 && T.cap > 0) {
     const float4* src = reinterpret_cast<const float4*>(F.pv);
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
         const int s = hs[k];
         cp_async16(sp + k, src + 2 * (int64_t)s);
         cp_async16(sv + k, src + 2 * (int64_t)s + 1);
-        cp_async8(st + k, F.th32 + s);
+        cp_async4(st + k, F.tl32 + s);
       }
       stage_lists(T.nbl, P.npad, blockIdx.x, sl);
       cp_async_wait_all();
@@ -227,7 +230,7 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
   if (i >= P.n) return;
   const Rec32 own = rec_load(F.pv + i);
   const float4 pi = own.p, vi = own.v;
-  const float2 ti = F.th32[i];
+  const float2 ti = make_float2(vi.w, F.tl32[i]);
   const bool solid = F.perm[i] < P.n_solid;
   const int32_t idi = F.id[i];
   if (P.state_pf && g == 0) {
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
   if (P.pf_ahead > 0 && g == 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(F.pv + ia); prefetch_l2(F.th32 + ia);
+      prefetch_l2(F.pv + ia); prefetch_l2(F.tl32 + ia);
       prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 4);
     }
@@ -249,10 +252,10 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
     density_heat_pairs(P, F, RecShared{sp, sv}, st, NbListS{sl, (int)threadIdx.x}, g, c, pi, vi, ti,
                        solid, idi, drho, sf);
   else if (b16 >= 0)
-    density_heat_pairs(P, F, RecGlobal{F.pv}, F.th32, NbList16{L16.off, P.npad, i, b16}, g, c, pi, vi,
+    density_heat_pairs(P, F, RecGlobal{F.pv}, F.tl32, NbList16{L16.off, P.npad, i, b16}, g, c, pi, vi,
                        ti, solid, idi, drho, sf);
   else
-    density_heat_pairs(P, F, RecGlobal{F.pv}, F.th32, NbList32{nb, P.npad, i}, g, c, pi, vi, ti, solid,
+    density_heat_pairs(P, F, RecGlobal{F.pv}, F.tl32, NbList32{nb, P.npad, i}, g, c, pi, vi, ti, solid,
                        idi, drho, sf);
   if constexpr (kDensLanes > 1) {
     const unsigned mask = group_mask<kDensLanes>();
@@ -264,8 +267,10 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
   }
   if (g != 0) return;
   const double4 vdi = F.vd[i];
+  drho *= (float)vdi.w;
   // heat of the previous step: rate and leapfrog, own particle only
-  const double dTdt = heat_rate_mixed(P, F, i, P.k2f * sf, vdi.w, (double)pi.w, F.T[i], plastic_heat);
+  const double dTdt = heat_rate_mixed(P, F, i, P.k2f * sf, vdi.w, (double)F.m32[i], F.T[i],
+                                      plastic_heat);
   F.dTdt[i] = dTdt;
   heat_leapfrog_one(P, F, i, dTdt, first);
   // density of this step
@@ -275,7 +280,8 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
     rho_new = vdi.w + P.dt * (double)drho;
   }
   vd2[i] = make_double4(vdi.x, vdi.y, vdi.z, rho_new);
-  pvb[i] = Rec32{pi, make_float4(vi.x, vi.y, vi.z, (float)rho_new)};
+  pvb[i] = Rec32{make_float4(pi.x, pi.y, pi.z, F.m32[i]),
+                 make_float4(vi.x, vi.y, vi.z, (float)rho_new)};
 }
 
 // ---- the heat pass alone (ThermalSolveKernel, src/cuda/Thermal.cu:101-142) --
@@ -284,7 +290,7 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
 // (so a separate pass gives the fused pass's sum bit for bit).
 template <class L>
 __device__ __forceinline__ float heat_pairs(const StepParams& P, const Rec32* __restrict__ pv,
-                                            const float2* __restrict__ gt, const L& list, int c,
+                                            const float* __restrict__ gt, const L& list, int c,
                                             float4 pi, float2 ti) {
   constexpr int NB = kDensBatch;
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
@@ -300,21 +306,19 @@ __device__ __forceinline__ float heat_pairs(const StepParams& P, const Rec32* __
 #pragma unroll
     for (int h = 0; h < WF_NB_BLK; h += NB) {
       float4 pj[NB];
-      float rj[NB];
       float2 tj[NB];
 #pragma unroll
       for (int q = 0; q < NB; q++) {
         const Rec32 r = rec_load(pv + js[h + q]);
         pj[q] = r.p;
-        rj[q] = r.v.w;
-        tj[q] = gt[js[h + q]];
+        tj[q] = make_float2(r.v.w, gt[js[h + q]]);
       }
 #pragma unroll
       for (int q = 0; q < NB; q++) {
         // padding entries (the particle's own slot) add exact zeros (gk32_r2)
         const float xx = pi.x - pj[q].x, xy = pi.y - pj[q].y, xz = pi.z - pj[q].z;
         const float GK = gk32_r2(xx * xx + xy * xy + xz * xz, invh, Ch, C);
-        const float mg = __fdividef(pj[q].w, rj[q]) * GK;
+        const float mg = pj[q].w * GK;
         const float dT = (ti.x - tj[q].x) + (ti.y - tj[q].y);
         sf += mg * dT;
       }
@@ -336,14 +340,15 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_heat32(StepParams P, Fi
   if (P.pf_ahead > 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(F.pv + ia); prefetch_l2(F.th32 + ia); prefetch_l2(cnt + ia);
+      prefetch_l2(F.pv + ia); prefetch_l2(F.tl32 + ia); prefetch_l2(cnt + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 4);
     }
   }
-  const float4 pi = F.pv[i].p;
-  const float2 ti = F.th32[i];
+  const Rec32 own = rec_load(F.pv + i);
+  const float4 pi = own.p;
+  const float2 ti = make_float2(own.v.w, F.tl32[i]);
   const int c = cnt[i];
-  const float sf = heat_pairs(P, F.pv, F.th32, NbList32{nb, P.npad, i}, c, pi, ti);
+  const float sf = heat_pairs(P, F.pv, F.tl32, NbList32{nb, P.npad, i}, c, pi, ti);
   F.dTdt[i] = heat_rate_mixed(P, F, i, P.k2f * sf, F.vd[i].w, F.xm[i].w, F.T[i], plastic_heat);
 }
 
@@ -372,12 +377,10 @@ __global__ void __launch_bounds__(128) k_heat_pairs32(StepParams P, Fields F, He
     list.block(b, js);
 #pragma unroll
     for (int q = 0; q < WF_NB_BLK; q++) {
-      const Rec32 r = rec_load(F.pv + js[q]);
-      const float4 pj = r.p;
-      const float rj = r.v.w;
+      const float4 pj = __ldg(&F.pv[js[q]].p);
       const float xx = pi.x - pj.x, xy = pi.y - pj.y, xz = pi.z - pj.z;
       const float GK = gk32_r2(xx * xx + xy * xy + xz * xz, invh, Ch, C);
-      mg[q] = __fdividef(pj.w, rj) * GK;
+      mg[q] = pj.w * GK;
     }
     float4* out = reinterpret_cast<float4*>(H.mg + ((int64_t)b * P.npad + i) * WF_NB_BLK);
     out[0] = make_float4(mg[0], mg[1], mg[2], mg[3]);
@@ -502,17 +505,6 @@ __device__ __forceinline__ bool jc_return_inc32(const StepParams& P, float st, f
 
 // ---- B32: rate tensors + EOS + stress (InteractionAlt.cu:262-383,
 //      Mechanical.cu:289-298, :458-554), energy (Energy.cu:5-19, own tensors)
-// The acceleration pass's per-particle stress / rho^2: the buffer of 8 floats
-// per padded slot holds a float4 array (xx, yy, zz, xy) followed by a float2
-// array (yz, xz).  Separate arrays, 16 and 8 bytes per particle, put more
-// particles in each cache line than one 32-byte record: a warp's gather of
-// its neighbours' stress touches about a quarter fewer L1 lines.
-template <class F4, class F2, class T>
-__device__ __forceinline__ void sigr32_split(T* base, int64_t npad, F4*& a, F2*& b) {
-  a = reinterpret_cast<F4*>(base);
-  b = reinterpret_cast<F2*>(base + 4 * npad);
-}
-
 // neighbours gathered per batch in the stress pass (position and velocity)
 constexpr int kStressBatch = 4;
 // hardening slope over 3G above which the warm-start network is asked: the
@@ -613,7 +605,7 @@ __device__ __forceinline__ int stage_halo16(const TileHalo& T, int64_t npad, int
 template <bool kMlp>
 __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
                                                   const Rec32* __restrict__ pvb,
-                                                  float* __restrict__ sigr32,
+                                                  Rec32* __restrict__ sigr32,
                                                   const int32_t* __restrict__ nb,
                                                   const int32_t* __restrict__ cnt,
                                                   int* __restrict__ status,
@@ -798,16 +790,13 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
   ssp[0] = make_float2(Sn.xx, Sn.yy);
   ssp[1] = make_float2(Sn.zz, Sn.xy);
   ssp[2] = make_float2(Sn.yz, Sn.xz);
-  // stress / rho^2 for the acceleration pass: (xx, yy, zz, xy) in one float4
-  // array and (yz, xz) in a float2 array behind it (sigr32_split)
+  // stress / rho^2 for the acceleration pass
   const float pf = (float)p;
   const float rf = vi.w;
   const float ir2 = 1.0f / (rf * rf);
-  float4* sga;
-  float2* sgb;
-  sigr32_split(sigr32, P.npad, sga, sgb);
-  sga[i] = make_float4((Sn.xx - pf) * ir2, (Sn.yy - pf) * ir2, (Sn.zz - pf) * ir2, Sn.xy * ir2);
-  sgb[i] = make_float2(Sn.yz * ir2, Sn.xz * ir2);
+  sigr32[i] = Rec32{make_float4((Sn.xx - pf) * ir2, (Sn.yy - pf) * ir2, (Sn.zz - pf) * ir2,
+                                Sn.xy * ir2),
+                    make_float4(Sn.yz * ir2, Sn.xz * ir2, 0.f, 0.f)};
   F.eps_p[i] = eps_p;
   F.sy[i] = sy;
   F.seq[i] = seq;
@@ -831,7 +820,7 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
 
 __global__ void __launch_bounds__(128, 6) k_stress32_mlp(StepParams P, Fields F,
                                                       const Rec32* __restrict__ pvb,
-                                                      float* __restrict__ sigr32,
+                                                      Rec32* __restrict__ sigr32,
                                                       const int32_t* __restrict__ nb,
                                                       const int32_t* __restrict__ cnt,
                                                       int* __restrict__ status,
@@ -842,7 +831,7 @@ __global__ void __launch_bounds__(128, 6) k_stress32_mlp(StepParams P, Fields F,
 }
 __global__ void __launch_bounds__(128, 6) k_stress32(StepParams P, Fields F,
                                                      const Rec32* __restrict__ pvb,
-                                                     float* __restrict__ sigr32,
+                                                     Rec32* __restrict__ sigr32,
                                                      const int32_t* __restrict__ nb,
                                                      const int32_t* __restrict__ cnt,
                                                      int* __restrict__ status,
@@ -865,26 +854,22 @@ static_assert(WF_NB_BLK / kAccelLanes >= kAccelBatch, "batch within the lane's s
 // arrays) or from the tile's halo in shared memory (indexed by local list).
 template <class R>
 struct AccelSrc {
-  R rec;
-  const float4* sa;
-  const float2* sb;
+  R rec, sig;
 };
 
 template <class L, class R>
 __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields& F,
                                               const Rec32* __restrict__ pvb,
-                                              const float* __restrict__ sigr32,
+                                              const Rec32* __restrict__ sigr32,
                                               const int32_t* __restrict__ cnt, int64_t i, int g,
                                               const AccelSrc<R>& src, const L& list) {
   constexpr int W = WF_NB_BLK / kAccelLanes;
   const Rec32 own = rec_load(pvb + i);
   const float4 pi = own.p, vi = own.v;
   const int32_t idi = F.id[i];
-  const float4* sga;
-  const float2* sgb;
-  sigr32_split(sigr32, P.npad, sga, sgb);
-  const float4 s0 = sga[i];
-  const float2 s1 = sgb[i];
+  const Rec32 own_sig = rec_load(sigr32 + i);
+  const float4 s0 = own_sig.p;
+  const float2 s1 = make_float2(own_sig.v.x, own_sig.v.y);
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
   const float h = P.hf, Cs = P.Csf, alpha = P.alphaf, beta = P.betaf, eps = P.epsf;
   const bool av = alpha != 0.0f || beta != 0.0f;
@@ -909,8 +894,9 @@ __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields&
         const Rec32 r = src.rec.get(j);
         pj[q] = r.p;
         vj[q] = r.v;
-        t0[q] = src.sa[j];
-        t1[q] = src.sb[j];
+        const Rec32 u = src.sig.get(j);
+        t0[q] = u.p;
+        t1[q] = make_float2(u.v.x, u.v.y);
       }
 #pragma unroll
       for (int q = 0; q < kAccelBatch; q++) {
@@ -964,28 +950,25 @@ __device__ __forceinline__ int64_t accel_slot(int& g) {
 
 __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
                                                  const Rec32* __restrict__ pvb,
-                                                 const float* __restrict__ sigr32,
+                                                 const Rec32* __restrict__ sigr32,
                                                  float4* __restrict__ a32,
                                                  const int32_t* __restrict__ nb,
                                                  const int32_t* __restrict__ cnt) {
   int g;
   const int64_t i = accel_slot(g);
   if (i >= P.n) return;
-  const float4* sga;
-  const float2* sgb;
-  sigr32_split(sigr32, P.npad, sga, sgb);
   if (P.pf_ahead > 0 && g == 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(pvb + ia); prefetch_l2(sga + ia);
-      prefetch_l2(sgb + ia); prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
+      prefetch_l2(pvb + ia); prefetch_l2(sigr32 + ia);
+      prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
       prefetch_l2(F.id + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++)
         nb_prefetch(nb, P.npad, ia, b, 2 * kAccelLanes);
     }
   }
   if (F.perm[i] >= P.n_solid) return;
-  const AccelSrc<RecGlobal> src{{pvb}, sga, sgb};
+  const AccelSrc<RecGlobal> src{{pvb}, {sigr32}};
   const float4 af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
   if (g == 0) a32[i] = af;
 }
@@ -997,25 +980,22 @@ __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
 // the new mirrors go to F.pv and th32, which this pass does not read.
 __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
                                                      const Rec32* __restrict__ pvb,
-                                                     const float* __restrict__ sigr32,
+                                                     const Rec32* __restrict__ sigr32,
                                                      const double4* __restrict__ vd2,
                                                      const int32_t* __restrict__ nb,
                                                      const int32_t* __restrict__ cnt, const List16 L16) {
   int g;
   const int64_t i = accel_slot(g);
   if (i >= P.n) return;
-  const float4* sga;
-  const float2* sgb;
-  sigr32_split(sigr32, P.npad, sga, sgb);
-  const AccelSrc<RecGlobal> src{{pvb}, sga, sgb};
+  const AccelSrc<RecGlobal> src{{pvb}, {sigr32}};
   if (P.state_pf && g == 0) {
     prefetch_l2(F.xm + i); prefetch_l2(vd2 + i); prefetch_l2(F.u + i); prefetch_l2(F.T + i);
   }
   if (P.pf_ahead > 0 && g == 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(pvb + ia); prefetch_l2(sga + ia);
-      prefetch_l2(sgb + ia); prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
+      prefetch_l2(pvb + ia); prefetch_l2(sigr32 + ia);
+      prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
       prefetch_l2(F.id + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 2 * kAccelLanes);
     }
@@ -1037,18 +1017,15 @@ __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
 // shared memory, then reads the neighbours from there through the local
 // lists.  Tiles that are not staged gather from global memory.
 __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
-    StepParams P, Fields F, const Rec32* __restrict__ pvb, const float* __restrict__ sigr32,
+    StepParams P, Fields F, const Rec32* __restrict__ pvb, const Rec32* __restrict__ sigr32,
     const double4* __restrict__ vd2, const int32_t* __restrict__ nb,
     const int32_t* __restrict__ cnt, const TileHalo T) {
   static_assert(kAccelLanes == 2, "one tile per block of 2 lanes per slot");
   extern __shared__ __align__(16) uint8_t sac[];
-  const float4* sga;
-  const float2* sgb;
-  sigr32_split(sigr32, P.npad, sga, sgb);
   float4* sp = reinterpret_cast<float4*>(sac);
   float4* sv = sp + T.cap;
   float4* ssa = sv + T.cap;
-  float2* ssb = reinterpret_cast<float2*>(ssa + T.cap);
+  float4* ssb = ssa + T.cap;
   uint16_t* sl = reinterpret_cast<uint16_t*>(ssb + T.cap);
   int staged = -1;
   {
@@ -1060,8 +1037,9 @@ __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
         const float4* rec = reinterpret_cast<const float4*>(pvb + s);
         cp_async16(sp + k, rec);
         cp_async16(sv + k, rec + 1);
-        cp_async16(ssa + k, sga + s);
-        cp_async8(ssb + k, sgb + s);
+        const float4* sig = reinterpret_cast<const float4*>(sigr32 + s);
+        cp_async16(ssa + k, sig);
+        cp_async16(ssb + k, sig + 1);
       }
       stage_lists(T.nbl, P.npad, blockIdx.x, sl);
       cp_async_wait_all();
@@ -1075,10 +1053,10 @@ __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
   float4 af = make_float4(0.f, 0.f, 0.f, 0.f);   // rigid (non-solid) slots: moved by their BCs
   if (F.perm[i] < P.n_solid) {
     if (staged >= 0) {
-      const AccelSrc<RecShared> src{{sp, sv}, ssa, ssb};
+      const AccelSrc<RecShared> src{{sp, sv}, {ssa, ssb}};
       af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbListS{sl, (int)(threadIdx.x >> 1)});
     } else {
-      const AccelSrc<RecGlobal> src{{pvb}, sga, sgb};
+      const AccelSrc<RecGlobal> src{{pvb}, {sigr32}};
       af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
     }
   }
@@ -1122,7 +1100,9 @@ void launch_fp32_density_heat(const StepParams& P, const Fields& F, double4* vd2
   TileHalo Tl = T;
   if (kDensLanes != 1) Tl.cap = 0;
   const size_t smem =
-      Tl.cap > 0 ? (2 * sizeof(float4) + sizeof(float2)) * (size_t)Tl.cap + WF_TILE_LIST_BYTES : 0;
+      Tl.cap > 0 ? 2 * sizeof(float4) * (size_t)Tl.cap + sizeof(float) * (size_t)((Tl.cap + 3) & ~3) +
+                       WF_TILE_LIST_BYTES
+                 : 0;
   static size_t opted[64] = {};     // per device: dynamic shared memory opted in so far
   opt_in_smem(k_density_heat32, smem, opted);
   static size_t c_smem = 0;
@@ -1151,7 +1131,7 @@ void launch_heat_step32(const StepParams& P, const Fields& F, const HeatWork32& 
   k_heat_step32<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, H, F.th32, th_out, N.nb, N.cnt, first,
                                                      last);
 }
-void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, float* sigr32,
+void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, Rec32* sigr32,
                         const NbBuffers& N, int* status, const void* mlp_packed,
                         const MlpL1* mlp_l1, const TileHalo& T, const List16& L16,
                         cudaStream_t s) {
@@ -1178,7 +1158,7 @@ void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, 
   }
 }
 void launch_fp32_accel(const StepParams& P, const Fields& F, const Rec32* pvb,
-                       const float* sigr32, float4* a32, const NbBuffers& N, cudaStream_t s) {
+                       const Rec32* sigr32, float4* a32, const NbBuffers& N, cudaStream_t s) {
   static size_t c_smem = 0;
   static int64_t c_val = 0;
   StepParams Q = P;
@@ -1187,10 +1167,10 @@ void launch_fp32_accel(const StepParams& P, const Fields& F, const Rec32* pvb,
   k_accel32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sigr32, a32, N.nb, N.cnt);
 }
 void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec32* pvb,
-                                 const float* sigr32, const double4* vd2, const NbBuffers& N,
+                                 const Rec32* sigr32, const double4* vd2, const NbBuffers& N,
                                  const TileHalo& T, const List16& L16, cudaStream_t s) {
   if (T.cap > 0) {
-    const size_t smem = (3 * sizeof(float4) + sizeof(float2)) * (size_t)T.cap + WF_TILE_LIST_BYTES;
+    const size_t smem = 4 * sizeof(float4) * (size_t)T.cap + WF_TILE_LIST_BYTES;
     static size_t opted[64] = {};
     opt_in_smem(k_accel_int32_tiles, smem, opted);
     k_accel_int32_tiles<<<blocks_for(P.n * kAccelLanes, 2 * WF_TILE), 2 * WF_TILE, smem, s>>>(

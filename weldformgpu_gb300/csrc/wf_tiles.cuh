@@ -62,9 +62,9 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
   const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -119,10 +119,11 @@ struct NbList32 {                 // 32-bit slot lists
   const int32_t* nb;
   int64_t npad, i;
   __device__ __forceinline__ void block(int b, int* js) const {
-    const int4* q = reinterpret_cast<const int4*>(nb + ((int64_t)b * npad + i) * WF_NB_BLK);
-    const int4 lo = __ldg(q), hi = __ldg(q + 1);
-    js[0] = lo.x; js[1] = lo.y; js[2] = lo.z; js[3] = lo.w;
-    js[4] = hi.x; js[5] = hi.y; js[6] = hi.z; js[7] = hi.w;
+    // the block's 32 bytes as one load (half the L1 accesses of two 16-byte ones)
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(js[0]), "=r"(js[1]), "=r"(js[2]), "=r"(js[3]), "=r"(js[4]), "=r"(js[5]), "=r"(js[6]),
+          "=r"(js[7])
+        : "l"(nb + ((int64_t)b * npad + i) * WF_NB_BLK));
   }
   template <int W>
   __device__ __forceinline__ void sub(int b, int g, int* js) const {
