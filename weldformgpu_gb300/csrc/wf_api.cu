@@ -75,7 +75,7 @@ struct wf_domain {
   double4* vd2 = nullptr;
   Rec32* pvb = nullptr;        // position, mass | velocity, new density: the later passes of a step
   float4* a32 = nullptr;       // mixed-form acceleration
-  Rec32* sigr32 = nullptr;     // stress / rho^2: xx yy zz xy | yz xz
+  Sig32 sig{};                 // stress / rho^2
   float* mlp_w = nullptr;      // device MLP parameters (FP32, packed layout of wf_mlp.cuh)
   void* mlp_packed = nullptr;  // BF16 tensor-core fragment image of mlp_w
   MlpL1 mlp_l1{};              // layer 1 of mlp_w (a kernel parameter of the stress pass)
@@ -430,7 +430,7 @@ static void layout_arena(wf_domain* d, Arena& A) {
     A.take(&F.xh, n); A.take(&F.pv, n); A.take(&F.tl32, n); A.take(&F.m32, n); A.take(&F.ss32, 6 * n);
     A.take(&F.th32, n); A.take(&F.pwn, n);
   }
-  A.take(&d->vd2, n); A.take(&d->pvb, n); A.take(&d->a32, n); A.take(&d->sigr32, n);
+  A.take(&d->vd2, n); A.take(&d->pvb, n); A.take(&d->a32, n); A.take(&d->sig.a, n); A.take(&d->sig.b, n);
   A.take(&d->nb, (int64_t)WF_NB_ALLOC * n); A.take(&d->nbc, n); A.take(&d->inv, n);
   A.take(&d->pf, n); A.take(&d->pf2, n); A.take(&d->cellid, n); A.take(&d->s_src, n);
   A.take(&d->s_orig, n); A.take(&d->d_mm, 8); A.take(&d->d_status, WF_STATUS_WORDS);
@@ -1195,16 +1195,16 @@ static int solve_step_launches(wf_domain* d) {
       d->heat_pending = false;
     }
     { KTimer t(d, KID_STRESS);
-      launch_fp32_stress(P, F, d->pvb, d->sigr32, N, d->d_status,
+      launch_fp32_stress(P, F, d->pvb, d->sig, N, d->d_status,
                          (d->mlp_on && d->mlp_loaded) ? d->mlp_packed : nullptr, &d->mlp_l1, TH, L16,
                          s); }
     if (!P.contact && d->fuse_integrate) {
       { KTimer t(d, KID_ACCEL);
-        launch_fp32_accel_integrate(P, F, d->pvb, d->sigr32, d->vd2, N, TH, L16, s); }
+        launch_fp32_accel_integrate(P, F, d->pvb, d->sig, d->vd2, N, TH, L16, s); }
       integrated = true;
     } else {
       KTimer t(d, KID_ACCEL);
-      launch_fp32_accel(P, F, d->pvb, d->sigr32, d->a32, N, s);
+      launch_fp32_accel(P, F, d->pvb, d->sig, d->a32, N, s);
     }
   }
   if (P.contact) {                                                                    // :233-257

@@ -8,7 +8,7 @@
 // neighbour data are 32-byte FP32 records (Rec32): pv = (x, m/rho | v, T_hi) with
 // T_lo beside it, written by the integration, for the density + heat pass;
 // pvb = (x, m | v, rho_new), written by the density pass, for the stress and
-// acceleration passes; sigr32 = stress / rho^2, written by the stress pass.
+// acceleration passes; sig = stress / rho^2, written by the stress pass.
 // All FP32 constants arrive precomputed in StepParams: on GB300 a per-thread
 // FP64 division or conversion costs as much as the whole FP32 pair loop.
 #include "wf_common.cuh"
@@ -605,7 +605,7 @@ __device__ __forceinline__ int stage_halo16(const TileHalo& T, int64_t npad, int
 template <bool kMlp>
 __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
                                                   const Rec32* __restrict__ pvb,
-                                                  Rec32* __restrict__ sigr32,
+                                                  const Sig32 sig,
                                                   const int32_t* __restrict__ nb,
                                                   const int32_t* __restrict__ cnt,
                                                   int* __restrict__ status,
@@ -794,9 +794,8 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
   const float pf = (float)p;
   const float rf = vi.w;
   const float ir2 = 1.0f / (rf * rf);
-  sigr32[i] = Rec32{make_float4((Sn.xx - pf) * ir2, (Sn.yy - pf) * ir2, (Sn.zz - pf) * ir2,
-                                Sn.xy * ir2),
-                    make_float4(Sn.yz * ir2, Sn.xz * ir2, 0.f, 0.f)};
+  sig.a[i] = make_float4((Sn.xx - pf) * ir2, (Sn.yy - pf) * ir2, (Sn.zz - pf) * ir2, Sn.xy * ir2);
+  sig.b[i] = make_float2(Sn.yz * ir2, Sn.xz * ir2);
   F.eps_p[i] = eps_p;
   F.sy[i] = sy;
   F.seq[i] = seq;
@@ -820,23 +819,23 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
 
 __global__ void __launch_bounds__(128, 6) k_stress32_mlp(StepParams P, Fields F,
                                                       const Rec32* __restrict__ pvb,
-                                                      Rec32* __restrict__ sigr32,
+                                                      const Sig32 sig,
                                                       const int32_t* __restrict__ nb,
                                                       const int32_t* __restrict__ cnt,
                                                       int* __restrict__ status,
                                                       const uint4* __restrict__ mlp,
                                                       const MlpL1 l1, const TileHalo T,
                                                       const List16 L16) {
-  stress32_body<true>(P, F, pvb, sigr32, nb, cnt, status, mlp, l1, T, L16);
+  stress32_body<true>(P, F, pvb, sig, nb, cnt, status, mlp, l1, T, L16);
 }
 __global__ void __launch_bounds__(128, 6) k_stress32(StepParams P, Fields F,
                                                      const Rec32* __restrict__ pvb,
-                                                     Rec32* __restrict__ sigr32,
+                                                     const Sig32 sig,
                                                      const int32_t* __restrict__ nb,
                                                      const int32_t* __restrict__ cnt,
                                                      int* __restrict__ status,
                                                      const TileHalo T, const List16 L16) {
-  stress32_body<false>(P, F, pvb, sigr32, nb, cnt, status, nullptr, MlpL1{}, T, L16);
+  stress32_body<false>(P, F, pvb, sig, nb, cnt, status, nullptr, MlpL1{}, T, L16);
 }
 
 // ---- C32: acceleration + Monaghan viscosity (InteractionAlt.cu:18-150) ----
@@ -854,22 +853,23 @@ static_assert(WF_NB_BLK / kAccelLanes >= kAccelBatch, "batch within the lane's s
 // arrays) or from the tile's halo in shared memory (indexed by local list).
 template <class R>
 struct AccelSrc {
-  R rec, sig;
+  R rec;
+  const float4* sa;
+  const float2* sb;
 };
 
 template <class L, class R>
 __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields& F,
                                               const Rec32* __restrict__ pvb,
-                                              const Rec32* __restrict__ sigr32,
+                                              const Sig32 sig,
                                               const int32_t* __restrict__ cnt, int64_t i, int g,
                                               const AccelSrc<R>& src, const L& list) {
   constexpr int W = WF_NB_BLK / kAccelLanes;
   const Rec32 own = rec_load(pvb + i);
   const float4 pi = own.p, vi = own.v;
   const int32_t idi = F.id[i];
-  const Rec32 own_sig = rec_load(sigr32 + i);
-  const float4 s0 = own_sig.p;
-  const float2 s1 = make_float2(own_sig.v.x, own_sig.v.y);
+  const float4 s0 = sig.a[i];
+  const float2 s1 = sig.b[i];
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
   const float h = P.hf, Cs = P.Csf, alpha = P.alphaf, beta = P.betaf, eps = P.epsf;
   const bool av = alpha != 0.0f || beta != 0.0f;
@@ -894,9 +894,8 @@ __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields&
         const Rec32 r = src.rec.get(j);
         pj[q] = r.p;
         vj[q] = r.v;
-        const Rec32 u = src.sig.get(j);
-        t0[q] = u.p;
-        t1[q] = make_float2(u.v.x, u.v.y);
+        t0[q] = src.sa[j];
+        t1[q] = src.sb[j];
       }
 #pragma unroll
       for (int q = 0; q < kAccelBatch; q++) {
@@ -950,7 +949,7 @@ __device__ __forceinline__ int64_t accel_slot(int& g) {
 
 __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
                                                  const Rec32* __restrict__ pvb,
-                                                 const Rec32* __restrict__ sigr32,
+                                                 const Sig32 sig,
                                                  float4* __restrict__ a32,
                                                  const int32_t* __restrict__ nb,
                                                  const int32_t* __restrict__ cnt) {
@@ -960,7 +959,7 @@ __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
   if (P.pf_ahead > 0 && g == 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(pvb + ia); prefetch_l2(sigr32 + ia);
+      prefetch_l2(pvb + ia); prefetch_l2(sig.a + ia); prefetch_l2(sig.b + ia);
       prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
       prefetch_l2(F.id + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++)
@@ -968,8 +967,8 @@ __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
     }
   }
   if (F.perm[i] >= P.n_solid) return;
-  const AccelSrc<RecGlobal> src{{pvb}, {sigr32}};
-  const float4 af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
+  const AccelSrc<RecGlobal> src{{pvb}, sig.a, sig.b};
+  const float4 af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbList32{nb, P.npad, i});
   if (g == 0) a32[i] = af;
 }
 
@@ -980,21 +979,21 @@ __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
 // the new mirrors go to F.pv and th32, which this pass does not read.
 __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
                                                      const Rec32* __restrict__ pvb,
-                                                     const Rec32* __restrict__ sigr32,
+                                                     const Sig32 sig,
                                                      const double4* __restrict__ vd2,
                                                      const int32_t* __restrict__ nb,
                                                      const int32_t* __restrict__ cnt, const List16 L16) {
   int g;
   const int64_t i = accel_slot(g);
   if (i >= P.n) return;
-  const AccelSrc<RecGlobal> src{{pvb}, {sigr32}};
+  const AccelSrc<RecGlobal> src{{pvb}, sig.a, sig.b};
   if (P.state_pf && g == 0) {
     prefetch_l2(F.xm + i); prefetch_l2(vd2 + i); prefetch_l2(F.u + i); prefetch_l2(F.T + i);
   }
   if (P.pf_ahead > 0 && g == 0) {
     const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
     if (ia < P.n) {
-      prefetch_l2(pvb + ia); prefetch_l2(sigr32 + ia);
+      prefetch_l2(pvb + ia); prefetch_l2(sig.a + ia); prefetch_l2(sig.b + ia);
       prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
       prefetch_l2(F.id + ia);
       for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 2 * kAccelLanes);
@@ -1005,9 +1004,9 @@ __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
   if (F.perm[i] < P.n_solid) {
     const int b16 = L16.base ? L16.base[i / WF_TILE] : -1;   // uniform over the block
     if (b16 >= 0)
-      af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList16{L16.off, P.npad, i, b16});
+      af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbList16{L16.off, P.npad, i, b16});
     else
-      af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
+      af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbList32{nb, P.npad, i});
   }
   if (g == 0) integrate_mixed_one(P, F, vd2, i, af);
 }
@@ -1017,7 +1016,7 @@ __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
 // shared memory, then reads the neighbours from there through the local
 // lists.  Tiles that are not staged gather from global memory.
 __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
-    StepParams P, Fields F, const Rec32* __restrict__ pvb, const Rec32* __restrict__ sigr32,
+    StepParams P, Fields F, const Rec32* __restrict__ pvb, const Sig32 sig,
     const double4* __restrict__ vd2, const int32_t* __restrict__ nb,
     const int32_t* __restrict__ cnt, const TileHalo T) {
   static_assert(kAccelLanes == 2, "one tile per block of 2 lanes per slot");
@@ -1025,7 +1024,7 @@ __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
   float4* sp = reinterpret_cast<float4*>(sac);
   float4* sv = sp + T.cap;
   float4* ssa = sv + T.cap;
-  float4* ssb = ssa + T.cap;
+  float2* ssb = reinterpret_cast<float2*>(ssa + T.cap);
   uint16_t* sl = reinterpret_cast<uint16_t*>(ssb + T.cap);
   int staged = -1;
   {
@@ -1037,9 +1036,8 @@ __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
         const float4* rec = reinterpret_cast<const float4*>(pvb + s);
         cp_async16(sp + k, rec);
         cp_async16(sv + k, rec + 1);
-        const float4* sig = reinterpret_cast<const float4*>(sigr32 + s);
-        cp_async16(ssa + k, sig);
-        cp_async16(ssb + k, sig + 1);
+        cp_async16(ssa + k, sig.a + s);
+        cp_async8(ssb + k, sig.b + s);
       }
       stage_lists(T.nbl, P.npad, blockIdx.x, sl);
       cp_async_wait_all();
@@ -1053,11 +1051,11 @@ __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
   float4 af = make_float4(0.f, 0.f, 0.f, 0.f);   // rigid (non-solid) slots: moved by their BCs
   if (F.perm[i] < P.n_solid) {
     if (staged >= 0) {
-      const AccelSrc<RecShared> src{{sp, sv}, {ssa, ssb}};
-      af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbListS{sl, (int)(threadIdx.x >> 1)});
+      const AccelSrc<RecShared> src{{sp, sv}, ssa, ssb};
+      af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbListS{sl, (int)(threadIdx.x >> 1)});
     } else {
-      const AccelSrc<RecGlobal> src{{pvb}, {sigr32}};
-      af = accel_value(P, F, pvb, sigr32, cnt, i, g, src, NbList32{nb, P.npad, i});
+      const AccelSrc<RecGlobal> src{{pvb}, sig.a, sig.b};
+      af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbList32{nb, P.npad, i});
     }
   }
   if (g == 0) integrate_mixed_one(P, F, vd2, i, af);
@@ -1131,7 +1129,7 @@ void launch_heat_step32(const StepParams& P, const Fields& F, const HeatWork32& 
   k_heat_step32<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, H, F.th32, th_out, N.nb, N.cnt, first,
                                                      last);
 }
-void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, Rec32* sigr32,
+void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, const Sig32& sig,
                         const NbBuffers& N, int* status, const void* mlp_packed,
                         const MlpL1* mlp_l1, const TileHalo& T, const List16& L16,
                         cudaStream_t s) {
@@ -1147,34 +1145,34 @@ void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, 
     opt_in_smem(k_stress32_mlp, smem, opted[1]);
     Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
         k_stress32_mlp, 128, smem, 1, &c_smem[1], &c_val[1]));
-    k_stress32_mlp<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, pvb, sigr32, N.nb, N.cnt,
+    k_stress32_mlp<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, pvb, sig, N.nb, N.cnt,
                                                            status, W, l1, T, L16);
   } else {
     opt_in_smem(k_stress32, smem, opted[0]);
     Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
         k_stress32, 128, smem, 1, &c_smem[0], &c_val[0]));
-    k_stress32<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, pvb, sigr32, N.nb, N.cnt, status,
+    k_stress32<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, pvb, sig, N.nb, N.cnt, status,
                                                        T, L16);
   }
 }
 void launch_fp32_accel(const StepParams& P, const Fields& F, const Rec32* pvb,
-                       const Rec32* sigr32, float4* a32, const NbBuffers& N, cudaStream_t s) {
+                       const Sig32& sig, float4* a32, const NbBuffers& N, cudaStream_t s) {
   static size_t c_smem = 0;
   static int64_t c_val = 0;
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
       k_accel32, 128, 0, kAccelLanes, &c_smem, &c_val));
-  k_accel32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sigr32, a32, N.nb, N.cnt);
+  k_accel32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sig, a32, N.nb, N.cnt);
 }
 void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec32* pvb,
-                                 const Rec32* sigr32, const double4* vd2, const NbBuffers& N,
+                                 const Sig32& sig, const double4* vd2, const NbBuffers& N,
                                  const TileHalo& T, const List16& L16, cudaStream_t s) {
   if (T.cap > 0) {
-    const size_t smem = 4 * sizeof(float4) * (size_t)T.cap + WF_TILE_LIST_BYTES;
+    const size_t smem = (3 * sizeof(float4) + sizeof(float2)) * (size_t)T.cap + WF_TILE_LIST_BYTES;
     static size_t opted[64] = {};
     opt_in_smem(k_accel_int32_tiles, smem, opted);
     k_accel_int32_tiles<<<blocks_for(P.n * kAccelLanes, 2 * WF_TILE), 2 * WF_TILE, smem, s>>>(
-        P, F, pvb, sigr32, vd2, N.nb, N.cnt, T);
+        P, F, pvb, sig, vd2, N.nb, N.cnt, T);
     return;
   }
   static size_t c_smem = 0;
@@ -1182,6 +1180,6 @@ void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
       k_accel_int32, 128, 0, kAccelLanes, &c_smem, &c_val));
-  k_accel_int32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sigr32, vd2, N.nb,
+  k_accel_int32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sig, vd2, N.nb,
                                                                    N.cnt, L16);
 }
