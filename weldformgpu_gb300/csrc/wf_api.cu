@@ -126,6 +126,10 @@ struct wf_domain {
   size_t work_refused = 0;     // a size the device had no memory for
   bool pair_cache = true;      // option "pair_cache"
   int rr_cur = 0;              // which of the two 1/rho arrays is current
+  int* d_zone = nullptr;       // [0] a massive particle has a mesh's zone id, [1] slots near a tool
+  bool zone_checked = false;   // d_zone[0] is of the current ids and masses
+  bool maxdep_kept = false;    // h_maxdep is on its way from the last step (ev_maxdep)
+  cudaEvent_t ev_maxdep = nullptr;
   bool geo_valid = false;      // gk, r2: of the current positions and lists
   bool rr_valid = false;       // rr: of the current density
   int tile_cap_max = WF_TILE_HALO_MAX;   // option "tile_cap_max": largest halo staged
@@ -436,7 +440,7 @@ static void layout_arena(wf_domain* d, Arena& A) {
   A.take(&d->s_orig, n); A.take(&d->d_mm, 8); A.take(&d->d_status, WF_STATUS_WORDS);
   A.take(&d->d_cstat, 2);
   A.take(&d->fr, n); A.take(&d->out_part, wf_out_partial_words(WF_MAX_BC));
-  A.take(&d->e0, 1);
+  A.take(&d->e0, 1); A.take(&d->d_zone, 2);
   d->t_halo_cap = 10 * n;      // halo entries: ~7 per slot on cell-sorted lattices
   A.take(&d->t_hoff, n / WF_TILE); A.take(&d->t_hcnt, n / WF_TILE);
   A.take(&d->t_halo, d->t_halo_cap); A.take(&d->t_nbl, (int64_t)WF_NB_ALLOC * n);
@@ -761,7 +765,10 @@ static size_t work64_bytes(const wf_domain* d) {
 }
 // Kept values are of this call's own steps only: anything may have changed
 // between two calls and in the step hook.
-static void work64_drop(wf_domain* d) { d->geo_valid = d->rr_valid = false; }
+static void kept_drop(wf_domain* d) {
+  d->geo_valid = d->rr_valid = false;
+  d->zone_checked = d->maxdep_kept = false;
+}
 static Work64 work64_of(const wf_domain* d) {
   Work64 W{};
   if (!d->pair_cache || !d->work || d->work_bytes < work64_bytes(d)) return W;
@@ -785,7 +792,7 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
     if (rc) return rc;
   }
   KTimer t(d, KID_REBUILD);
-  work64_drop(d);
+  d->geo_valid = d->rr_valid = false;
   const int64_t n = d->n;
   cudaStream_t s = d->stream;
   Fields& A = d->F[d->cur];
@@ -859,6 +866,7 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
   if (d->F[d->cur].eps_rb) {       // adaptive rebuild: the strain this list was built at
     k_copy_d<<<nblk(n), 256, 0, s>>>(n, d->F[d->cur].eps_p, d->F[d->cur].eps_rb);
     d->launches += 1;
+    if (d->d_maxdep) WF_CUDA_OK(cudaMemsetAsync(d->d_maxdep, 0, sizeof(unsigned long long), s));
   }
   WF_CUDA_OK(cudaGetLastError());
   d->nb_built = true;
@@ -1133,17 +1141,24 @@ static int solve_step_launches(wf_domain* d) {
   bool rb;
   if (d->rb_dep > 0.0) {
     // adaptive: rebuild once the plastic strain grew by rb_dep anywhere since
-    // the last rebuild (one device reduction and a 8-byte read per step)
-    const Fields& F0 = d->F[d->cur];
-    WF_CUDA_OK(cudaMemsetAsync(d->d_maxdep, 0, sizeof(unsigned long long), s));
-    k_max_dep<<<std::min(nblk(d->n), kMaxDepBlocks), 256, 0, s>>>(d->n, F0.eps_p, F0.eps_rb,
-                                                                 d->d_maxdep);
-    WF_CUDA_OK(cudaMemcpyAsync(d->h_maxdep, d->d_maxdep, sizeof(unsigned long long),
-                               cudaMemcpyDeviceToHost, s));
-    WF_CUDA_OK(cudaStreamSynchronize(s));
+    // the last rebuild.  The mixed stress pass keeps the maximum up and its
+    // copy to the host is under way since the last step's stress pass, so the
+    // GPU does not wait for the host; a call's first step and the FP64 form
+    // reduce the strains here (one pass and an 8-byte read).
+    if (d->maxdep_kept) {
+      WF_CUDA_OK(cudaEventSynchronize(d->ev_maxdep));
+    } else {
+      const Fields& F0 = d->F[d->cur];
+      WF_CUDA_OK(cudaMemsetAsync(d->d_maxdep, 0, sizeof(unsigned long long), s));
+      k_max_dep<<<std::min(nblk(d->n), kMaxDepBlocks), 256, 0, s>>>(d->n, F0.eps_p, F0.eps_rb,
+                                                                   d->d_maxdep);
+      WF_CUDA_OK(cudaMemcpyAsync(d->h_maxdep, d->d_maxdep, sizeof(unsigned long long),
+                                 cudaMemcpyDeviceToHost, s));
+      WF_CUDA_OK(cudaStreamSynchronize(s));
+      d->launches += 1;
+    }
     double mx;
     memcpy(&mx, d->h_maxdep, sizeof mx);
-    d->launches += 1;
     rb = mx > d->rb_dep;
   } else {
     rb = d->ts_i == 0 && (d->is_yielding || !d->rebuild_after_yield);   // :166-182
@@ -1173,6 +1188,22 @@ static int solve_step_launches(wf_domain* d) {
   NbBuffers N{d->nb, d->nbc};
   const bool mixed = d->precision == 1;
   bool integrated = false;
+  if (P.contact) {
+    P.zone_mass = d->d_zone;
+    if (mixed && !d->zone_checked) {   // a call's first step
+      WF_CUDA_OK(cudaMemsetAsync(d->d_zone, 0, sizeof(int), s));
+      launch_zone_mass(P, F, d->d_zone, s);
+      d->zone_checked = true;
+      d->launches += 1;
+    }
+  }
+  const bool law1_fused = mixed && P.contact && P.contact_law == 1 && d->fuse_integrate;
+  if (law1_fused) {
+    WF_CUDA_OK(cudaMemsetAsync(d->d_zone + 1, 0, sizeof(int), s));
+    P.near_count = d->d_zone + 1;
+    P.near_list = d->cnb;              // law 0's contact lists: not used by law 1
+  }
+  if (mixed && d->rb_dep > 0.0) P.max_dep = d->d_maxdep;
   const TileHalo TH{d->t_hoff, d->t_hcnt, d->t_halo, d->t_nbl,
                     (mixed && d->tile_staging && !P.contact) ? d->tile_cap : 0};
   const List16 L16{(mixed && d->list16 && d->l16_built) ? d->l16_base : nullptr, d->l16_off};
@@ -1198,9 +1229,19 @@ static int solve_step_launches(wf_domain* d) {
       launch_fp32_stress(P, F, d->pvb, d->sig, N, d->d_status,
                          (d->mlp_on && d->mlp_loaded) ? d->mlp_packed : nullptr, &d->mlp_l1, TH, L16,
                          s); }
-    if (!P.contact && d->fuse_integrate) {
+    if (P.max_dep) {
+      WF_CUDA_OK(cudaMemcpyAsync(d->h_maxdep, d->d_maxdep, sizeof(unsigned long long),
+                                 cudaMemcpyDeviceToHost, s));
+      WF_CUDA_OK(cudaEventRecord(d->ev_maxdep, s));
+      d->maxdep_kept = true;
+    }
+    if (law1_fused) {                  // the acceleration pass looks into the tools' bins
+      KTimer t(d, KID_CONTACT);
+      launch_contact_stage(P, F, N, false, d->a32, s);
+    }
+    if (law1_fused || (!P.contact && d->fuse_integrate)) {
       { KTimer t(d, KID_ACCEL);
-        launch_fp32_accel_integrate(P, F, d->pvb, d->sig, d->vd2, N, TH, L16, s); }
+        launch_fp32_accel_integrate(P, F, d->pvb, d->sig, d->vd2, d->a32, N, TH, L16, s); }
       integrated = true;
     } else {
       KTimer t(d, KID_ACCEL);
@@ -1209,7 +1250,8 @@ static int solve_step_launches(wf_domain* d) {
   }
   if (P.contact) {                                                                    // :233-257
     KTimer t(d, KID_CONTACT);
-    launch_contact_stage(P, F, N, d->ts_i == 0, mixed ? d->a32 : nullptr, s);
+    if (law1_fused) launch_contact_law1_list(P, F, d->vd2, d->a32, s);
+    else launch_contact_stage(P, F, N, d->ts_i == 0, mixed ? d->a32 : nullptr, s);
     d->launches += d->ts_i == 0 ? 3 : 2;
   }
   if (!integrated) {   // :273-287
@@ -1291,7 +1333,7 @@ static int solve_step(wf_domain* d) {
   d->in_callback = true;
   const int r = d->after_fn(d, d->after_user);
   d->in_callback = false;
-  work64_drop(d);
+  kept_drop(d);
   if (r) return wf_fail(d, WF_ERR_STATE, "step callback returned " + std::to_string(r));
   return WF_OK;
 }
@@ -1399,6 +1441,7 @@ int wf_destroy(wf_domain* d) {
   if (d->work) cudaFree(d->work);
   if (d->d_maxdep) cudaFree(d->d_maxdep);
   if (d->h_maxdep) cudaFreeHost(d->h_maxdep);
+  if (d->ev_maxdep) cudaEventDestroy(d->ev_maxdep);
   if (d->cnb) cudaFree(d->cnb);
   if (d->ccnt) cudaFree(d->ccnt);
   void* ptrs[] = {d->log_x, d->log_y, d->log_count, d->cell_count, d->cell_cursor,
@@ -1772,7 +1815,8 @@ int wf_set_option(wf_domain* d, const char* key, double v) {
       for (int f = 0; f < 2; f++)
         if (dalloc(&d->F[f].eps_rb, d->npad, d->stream)) return wf_fail(d, WF_ERR_ALLOC, "eps_rb");
       if (dalloc(&d->d_maxdep, 1, d->stream) ||
-          cudaMallocHost((void**)&d->h_maxdep, sizeof(unsigned long long)) != cudaSuccess)
+          cudaMallocHost((void**)&d->h_maxdep, sizeof(unsigned long long)) != cudaSuccess ||
+          cudaEventCreateWithFlags(&d->ev_maxdep, cudaEventDisableTiming) != cudaSuccess)
         return wf_fail(d, WF_ERR_ALLOC, "rebuild flag");
     }
     d->rb_dep = v;
@@ -1813,7 +1857,7 @@ int wf_set_option(wf_domain* d, const char* key, double v) {
   }
   else if (k == "pair_cache") {
     d->pair_cache = v != 0;
-    work64_drop(d);
+    kept_drop(d);
   }
   else if (k == "tile_staging") d->tile_staging = v != 0;   // takes effect at the next rebuild
   else if (k == "list_prefetch") d->list_prefetch = std::max(0, std::min((int)v, WF_NB_BLOCKS));
@@ -1860,7 +1904,7 @@ int wf_step(wf_domain* d, int64_t nsteps) {
     int rc = solve_begin(d, d->output_interval);
     if (rc) return rc;
   }
-  work64_drop(d);
+  kept_drop(d);
   for (int64_t k = 0; k < nsteps; k++) {
     int rc = solve_step(d);
     if (rc) return rc;
@@ -1897,7 +1941,7 @@ int wf_thermal_solve(wf_domain* d, double tf) {
   if (d->precision == 1) k_mixed_init<<<nblk(d->n), 256, 0, d->stream>>>(d->n, CF(d));
   StepParams P = make_params(d);
   NbBuffers N{d->nb, d->nbc};
-  work64_drop(d);
+  kept_drop(d);
   const bool mixed = d->precision == 1;
   const int64_t entries = (int64_t)WF_NB_ALLOC * d->npad, n = d->npad;
   const bool kept = d->time < tf &&
@@ -2316,7 +2360,7 @@ int wf_time_steps(wf_domain* d, int64_t nsteps, double* elapsed_ms, double* kern
   cudaEventRecord(e0, d->stream);
   int rc = WF_OK;
   d->timing = true;
-  work64_drop(d);
+  kept_drop(d);
   for (int64_t k = 0; k < nsteps && rc == WF_OK; k++) rc = solve_step(d);
   flush_heat(d);   // the timed steps include their whole heat work
   if (rc == WF_OK) rc = segment_end(d);

@@ -213,6 +213,11 @@ struct StepParams {
   double* e0;           // mixed form, energy_mode 0: particle 0's S:D of this step
   const int32_t* inv;   // inv[original id] = slot (particle 0's slot for energy_mode 0)
   int contact;          // contact pass filter active
+  const int* zone_mass; // set when a particle with mass carries a mesh's zone id
+  int* near_count;      // contact law 1 fused into the mixed acceleration pass: slots near a
+  int32_t* near_list;   // tool (null: the contact is a pass of its own)
+  unsigned long long* max_dep;   // adaptive rebuild, mixed form: bits of the largest strain
+                                 // increment since the last rebuild (null: off)
   int ncsid;
   int32_t csid[WF_MAX_MESH];
   MeshDev mesh[WF_MAX_MESH];   // ncsid meshes, zone ids in csid
@@ -330,6 +335,54 @@ __device__ __forceinline__ bool pass_j(const StepParams& P, int32_t idj) {
   return pass;
 }
 
+// The mixed passes' contact filter (pass_ij, pass_j) changes nothing while
+// every particle with a mesh's zone id is massless, as wf_add_trimesh makes
+// them: such a neighbour adds exact zeros.  It then costs an id gathered per
+// neighbour (500k particles: density + heat 154 -> 110 us, stress 134 -> 103), so it runs
+// only when P.zone_mass says otherwise (k_zone_mass).
+__device__ __forceinline__ bool zone_filter(const StepParams& P) {
+  return P.contact && __ldg(P.zone_mass) != 0;
+}
+
+// Contact law 1: is a position (FP32) within a tool's bin grid, widened by one
+// cell (far more than FP32 rounding)?
+__device__ __forceinline__ bool law1_near(const StepParams& P, float px, float py, float pz) {
+  bool near = false;
+  for (int m = 0; m < P.ncsid; m++) {
+    const MeshDev& M = P.mesh[m];
+    const float4 o = M.off32[0];
+    const float tx = px - o.x, ty = py - o.y, tz = pz - o.z;
+    near |= tx >= M.glo[0] && tx <= M.ghi[0] && ty >= M.glo[1] && ty <= M.ghi[1] &&
+            tz >= M.glo[2] && tz <= M.ghi[2];
+  }
+  return near;
+}
+
+// The particle's cell in mesh M's bins, or -1 outside the grid (compared in
+// double first: a particle far outside the grid, or a NaN position, is
+// skipped before any integer conversion; the bins carry a margin of h, so the
+// rounding of the product cannot lose a triangle within h).  Rounds alike in
+// every translation unit.
+__device__ __forceinline__ int tool_cell(const MeshDev& M, double x, double y, double z) {
+  const double4 o = M.node[0];
+  const double fx = floor(__dmul_rn(__dsub_rn(__dsub_rn(x, o.x), M.grel[0]), M.inv_cs));
+  const double fy = floor(__dmul_rn(__dsub_rn(__dsub_rn(y, o.y), M.grel[1]), M.inv_cs));
+  const double fz = floor(__dmul_rn(__dsub_rn(__dsub_rn(z, o.z), M.grel[2]), M.inv_cs));
+  if (!(fx >= 0.0 && fy >= 0.0 && fz >= 0.0 && fx < (double)M.dims[0] &&
+        fy < (double)M.dims[1] && fz < (double)M.dims[2]))
+    return -1;
+  return ((int)fz * M.dims[1] + (int)fy) * M.dims[0] + (int)fx;
+}
+// Does the particle's cell in some tool's bins list a triangle?
+__device__ __forceinline__ bool law1_triangles(const StepParams& P, const double4& x) {
+  bool any = false;
+  for (int m = 0; m < P.ncsid; m++) {
+    const int cell = tool_cell(P.mesh[m], x.x, x.y, x.z);
+    if (cell >= 0) any |= P.mesh[m].cstart[cell + 1] > P.mesh[m].cstart[cell];
+  }
+  return any;
+}
+
 // Kernel launchers (defined in the .cu files, called by wf_api.cu).
 struct NbBuffers {
   int32_t* nb;      // [WF_NB_ALLOC * npad], blocks of 8 (nb_at)
@@ -389,6 +442,12 @@ void launch_thermal(const StepParams& P, const Fields& F, const Work64& W, const
 // after the integration; plane coefficients at solve start
 void launch_contact_stage(const StepParams& P, const Fields& F, const NbBuffers& N, bool list,
                           float4* a32, cudaStream_t s);
+// contact law 1 and integration of the slots that the fused acceleration pass
+// listed (P.near_list)
+void launch_contact_law1_list(const StepParams& P, const Fields& F, const double4* vd2,
+                              float4* a32, cudaStream_t s);
+// *flag = 1 if a particle with mass carries a mesh's zone id (flag zeroed before)
+void launch_zone_mass(const StepParams& P, const Fields& F, int* flag, cudaStream_t s);
 void launch_mesh_update(const StepParams& P, const Fields& F, int mixed, cudaStream_t s);
 void launch_mesh_plane(const StepParams& P, cudaStream_t s);
 struct TileHalo;
@@ -414,5 +473,5 @@ void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb,
 void launch_fp32_accel(const StepParams& P, const Fields& F, const Rec32* pvb,
                        const Sig32& sig, float4* a32, const NbBuffers& N, cudaStream_t s);
 void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec32* pvb,
-                                 const Sig32& sig, const double4* vd2, const NbBuffers& N,
-                                 const TileHalo& T, const List16& L16, cudaStream_t s);
+                                 const Sig32& sig, const double4* vd2, float4* a32,
+                                 const NbBuffers& N, const TileHalo& T, const List16& L16, cudaStream_t s);

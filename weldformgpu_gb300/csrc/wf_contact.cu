@@ -11,7 +11,10 @@
 // right, length = sqrt(dot)), so the plain form matches the oracle bit for bit.
 // One thread per particle (surface, list, force), per node (mesh motion) or
 // per element (element geometry, rigid particles).
+#include <algorithm>
+
 #include "wf_common.cuh"
+#include "wf_integrate.cuh"
 #include "wf_nsearch.cuh"
 
 namespace {
@@ -218,21 +221,6 @@ __device__ __forceinline__ float3 rel32(const float4* r, int q) {
   return make_float3(v.x, v.y, v.z);
 }
 
-// The particle's cell in mesh M's bins, or -1 outside the grid (compared in
-// double first: a particle far outside the grid, or a NaN position, is
-// skipped before any integer conversion; the bins carry a margin of h, so the
-// rounding of the product cannot lose a triangle within h).
-__device__ __forceinline__ int tool_cell(const MeshDev& M, V3 xi) {
-  const V3 r = xi - mk(M.node[0]);
-  const double fx = floor((r.x - M.grel[0]) * M.inv_cs);
-  const double fy = floor((r.y - M.grel[1]) * M.inv_cs);
-  const double fz = floor((r.z - M.grel[2]) * M.inv_cs);
-  if (!(fx >= 0.0 && fy >= 0.0 && fz >= 0.0 && fx < (double)M.dims[0] &&
-        fy < (double)M.dims[1] && fz < (double)M.dims[2]))
-    return -1;
-  return ((int)fz * M.dims[1] + (int)fy) * M.dims[0] + (int)fx;
-}
-
 // Bins of a rotating tool, rebuilt every step from the current nodes: every
 // triangle goes into each cell that its bounding box (relative to node 0)
 // widened by the margin touches, with its vertices relative to node 0 in
@@ -284,138 +272,12 @@ __global__ void k_bins_fill(MeshDev M) {
       }
 }
 
-// Contact law 1 (the 2M-particle contact workload; no reference
-// counterpart).  A solid particle looks up its cell in each tool's triangle
-// bins (built once in the tool's frame; the frame moves with node 0) and takes
-// the nearest triangle whose closest point q lies within h (ties: first mesh,
-// lowest triangle index), searched in FP32 and decided in FP64.  With the gap
-// g = |x - q| along n = (x - q)/g (the face normal and the signed gap for a
-// centre behind the face) and the penetration delta = dx/2 - g > 0 the normal
-// force is
-// kappa K dx delta (pressure kappa K / dx on the face dx^2); friction is
-// Coulomb, regularised below v_reg: F_t = -mu F_n v_t / max(|v_t|, v_reg);
-// eta of the frictional power heats the particle.  Mixed form: the
-// acceleration comes from and returns to the FP32 array.
-__global__ void __launch_bounds__(128) k_contact_law1(StepParams P, Fields F, float4* a32) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= P.n || F.perm[i] >= P.n_solid) return;
-  // FP32 early-out against each tool's bin grid widened by one cell (far
-  // larger than FP32 rounding): most particles are nowhere near a tool and
-  // skip all FP64 work.  The mixed form keeps an FP32 position mirror.
-  float px, py, pz;
-  if (a32) {
-    const float4 p = F.pv[i].p;
-    px = p.x; py = p.y; pz = p.z;
-  } else {
-    const double4 p = F.xm[i];
-    px = (float)p.x; py = (float)p.y; pz = (float)p.z;
-  }
-  bool near = false;
-  for (int m = 0; m < P.ncsid; m++) {
-    const MeshDev& M = P.mesh[m];
-    const float4 o = M.off32[0];
-    const float tx = px - o.x, ty = py - o.y, tz = pz - o.z;
-    near |= tx >= M.glo[0] && tx <= M.ghi[0] && ty >= M.glo[1] && ty <= M.ghi[1] &&
-            tz >= M.glo[2] && tz <= M.ghi[2];
-  }
-  if (!near) {
-    F.cf[i] = make_double4(0.0, 0.0, 0.0, 0.0);
-    F.qf[i] = 0.0;
-    P.ccnt[i] = 0;
-    return;
-  }
-  const double4 x4 = F.xm[i];
+// The force, frictional heat and acceleration of law 1 from the nearest surface
+// point bq (triangle be of mesh bm, squared distance best; bm < 0: none).
+__device__ __forceinline__ void law1_force(const StepParams& P, const Fields& F, int64_t i,
+                                           const double4& x4, float4* a32, double best, int bm,
+                                           int be, V3 bq) {
   const V3 xi = mk(x4);
-  // Pass 1, FP32: the smallest squared distance over the candidate triangles,
-  // in coordinates relative to each tool's node 0 (each bin entry carries its
-  // triangle's FP32 vertices, so the loads of successive entries overlap).
-  float m32 = P.hf * P.hf, tol = 0.f;
-  unsigned n32 = 0, n64 = 0;
-  for (int m = 0; m < P.ncsid; m++) {
-    const MeshDev& M = P.mesh[m];
-    const int cell = tool_cell(M, xi);
-    if (cell < 0) continue;
-    tol = fmaxf(tol, M.tol32);
-    const double4 n0 = M.node[0];
-    const float3 pr = make_float3((float)(xi.x - n0.x), (float)(xi.y - n0.y), (float)(xi.z - n0.z));
-    const int t0 = M.cstart[cell], t1 = M.cstart[cell + 1];
-    n32 += (unsigned)(t1 - t0);
-#pragma unroll 4
-    for (int t = t0; t < t1; t++) {
-      const float4* v = M.cvert + 3 * (int64_t)t;
-      m32 = fminf(m32, closest_sq32(pr, rel32(v, 0), rel32(v, 1), rel32(v, 2)));
-    }
-  }
-  // Pass 2, FP64: the triangles within tol (in distance) of that minimum, in
-  // the order and with the tie rule of a scan of every triangle.  tol is far
-  // above the FP32 distance error, so the FP64 minimum is always among them.
-  // Candidates are collected first (FP32) and evaluated together: inside the
-  // scan, lanes pass the filter at different entries and a warp would run the
-  // FP64 test once per such entry.  A lane with more than kCand candidates
-  // (never seen on tessellated tools) scans again in FP64.
-  constexpr int kCand = 8;
-  const float lim = sqrtf(m32) + tol;
-  const float thr = lim * lim;
-  int cand[kCand];
-  int ncand = 0;
-  for (int m = 0; m < P.ncsid; m++) {
-    const MeshDev& M = P.mesh[m];
-    const int cell = tool_cell(M, xi);
-    if (cell < 0) continue;
-    const double4 n0 = M.node[0];
-    const float3 pr = make_float3((float)(xi.x - n0.x), (float)(xi.y - n0.y), (float)(xi.z - n0.z));
-    const int t1 = M.cstart[cell + 1];
-#pragma unroll 4
-    for (int t = M.cstart[cell]; t < t1; t++) {
-      const float4* v = M.cvert + 3 * (int64_t)t;
-      const float4 v0 = v[0];
-      if (closest_sq32(pr, make_float3(v0.x, v0.y, v0.z), rel32(v, 1), rel32(v, 2)) > thr)
-        continue;
-      if (ncand < kCand) cand[ncand] = (m << 24) | __float_as_int(v0.w);
-      ncand++;
-    }
-  }
-  double best = P.h * P.h;
-  int bm = -1, be = -1;
-  V3 bq = mk(0.0, 0.0, 0.0);
-  auto consider = [&](int m, int e) {
-    const MeshDev& M = P.mesh[m];
-    const int32_t* en = M.elnode + 3 * e;
-    const V3 q = closest_on_tri(xi, mk(M.node[en[0]]), mk(M.node[en[1]]), mk(M.node[en[2]]));
-    const V3 dv = xi - q;
-    const double d2 = dot(dv, dv);
-    if (d2 < best || (d2 == best && bm == m && e < be)) {
-      best = d2; bm = m; be = e; bq = q;
-    }
-  };
-  if (ncand <= kCand) {
-    for (int k = 0; k < ncand; k++) consider(cand[k] >> 24, cand[k] & 0xffffff);
-    n64 += (unsigned)ncand;
-  } else {
-    for (int m = 0; m < P.ncsid; m++) {
-      const MeshDev& M = P.mesh[m];
-      const int cell = tool_cell(M, xi);
-      if (cell < 0) continue;
-      const double4 n0 = M.node[0];
-      const float3 pr = make_float3((float)(xi.x - n0.x), (float)(xi.y - n0.y), (float)(xi.z - n0.z));
-      for (int t = M.cstart[cell]; t < M.cstart[cell + 1]; t++) {
-        const float4* v = M.cvert + 3 * (int64_t)t;
-        const float4 v0 = v[0];
-        if (closest_sq32(pr, make_float3(v0.x, v0.y, v0.z), rel32(v, 1), rel32(v, 2)) > thr)
-          continue;
-        consider(m, __float_as_int(v0.w));
-        n64++;
-      }
-    }
-  }
-  {
-    const unsigned mask = __activemask();
-    const unsigned s32 = __reduce_add_sync(mask, n32), s64 = __reduce_add_sync(mask, n64);
-    if ((int)(threadIdx.x & 31) == __ffs(mask) - 1 && s32) {
-      atomicAdd(P.cstat, (unsigned long long)s32);
-      atomicAdd(P.cstat + 1, (unsigned long long)s64);
-    }
-  }
   V3 f = mk(0.0, 0.0, 0.0);
   double qf = 0.0;
   int cnt = 0;
@@ -466,6 +328,255 @@ __global__ void __launch_bounds__(128) k_contact_law1(StepParams P, Fields F, fl
   F.cf[i] = d4(f);
   F.qf[i] = qf;
   P.ccnt[i] = cnt;
+}
+
+// Contact law 1 (the 2M-particle contact workload; no reference
+// counterpart).  A solid particle looks up its cell in each tool's triangle
+// bins (built once in the tool's frame; the frame moves with node 0) and takes
+// the nearest triangle whose closest point q lies within h (ties: first mesh,
+// lowest triangle index), searched in FP32 and decided in FP64.  With the gap
+// g = |x - q| along n = (x - q)/g (the face normal and the signed gap for a
+// centre behind the face) and the penetration delta = dx/2 - g > 0 the normal
+// force is
+// kappa K dx delta (pressure kappa K / dx on the face dx^2); friction is
+// Coulomb, regularised below v_reg: F_t = -mu F_n v_t / max(|v_t|, v_reg);
+// eta of the frictional power heats the particle.  Mixed form: the
+// acceleration comes from and returns to the FP32 array.
+__device__ void law1_one(const StepParams& P, const Fields& F, int64_t i, float4* a32) {
+  const double4 x4 = F.xm[i];
+  const V3 xi = mk(x4);
+  // Pass 1, FP32: the smallest squared distance over the candidate triangles,
+  // in coordinates relative to each tool's node 0 (each bin entry carries its
+  // triangle's FP32 vertices, so the loads of successive entries overlap).
+  float m32 = P.hf * P.hf, tol = 0.f;
+  unsigned n32 = 0, n64 = 0;
+  for (int m = 0; m < P.ncsid; m++) {
+    const MeshDev& M = P.mesh[m];
+    const int cell = tool_cell(M, xi.x, xi.y, xi.z);
+    if (cell < 0) continue;
+    tol = fmaxf(tol, M.tol32);
+    const double4 n0 = M.node[0];
+    const float3 pr = make_float3((float)(xi.x - n0.x), (float)(xi.y - n0.y), (float)(xi.z - n0.z));
+    const int t0 = M.cstart[cell], t1 = M.cstart[cell + 1];
+    n32 += (unsigned)(t1 - t0);
+#pragma unroll 4
+    for (int t = t0; t < t1; t++) {
+      const float4* v = M.cvert + 3 * (int64_t)t;
+      m32 = fminf(m32, closest_sq32(pr, rel32(v, 0), rel32(v, 1), rel32(v, 2)));
+    }
+  }
+  // Pass 2, FP64: the triangles within tol (in distance) of that minimum, in
+  // the order and with the tie rule of a scan of every triangle.  tol is far
+  // above the FP32 distance error, so the FP64 minimum is always among them.
+  // Candidates are collected first (FP32) and evaluated together: inside the
+  // scan, lanes pass the filter at different entries and a warp would run the
+  // FP64 test once per such entry.  A lane with more than kCand candidates
+  // (never seen on tessellated tools) scans again in FP64.
+  constexpr int kCand = 8;
+  const float lim = sqrtf(m32) + tol;
+  const float thr = lim * lim;
+  int cand[kCand];
+  int ncand = 0;
+  for (int m = 0; m < P.ncsid; m++) {
+    const MeshDev& M = P.mesh[m];
+    const int cell = tool_cell(M, xi.x, xi.y, xi.z);
+    if (cell < 0) continue;
+    const double4 n0 = M.node[0];
+    const float3 pr = make_float3((float)(xi.x - n0.x), (float)(xi.y - n0.y), (float)(xi.z - n0.z));
+    const int t1 = M.cstart[cell + 1];
+#pragma unroll 4
+    for (int t = M.cstart[cell]; t < t1; t++) {
+      const float4* v = M.cvert + 3 * (int64_t)t;
+      const float4 v0 = v[0];
+      if (closest_sq32(pr, make_float3(v0.x, v0.y, v0.z), rel32(v, 1), rel32(v, 2)) > thr)
+        continue;
+      if (ncand < kCand) cand[ncand] = (m << 24) | __float_as_int(v0.w);
+      ncand++;
+    }
+  }
+  double best = P.h * P.h;
+  int bm = -1, be = -1;
+  V3 bq = mk(0.0, 0.0, 0.0);
+  auto consider = [&](int m, int e) {
+    const MeshDev& M = P.mesh[m];
+    const int32_t* en = M.elnode + 3 * e;
+    const V3 q = closest_on_tri(xi, mk(M.node[en[0]]), mk(M.node[en[1]]), mk(M.node[en[2]]));
+    const V3 dv = xi - q;
+    const double d2 = dot(dv, dv);
+    if (d2 < best || (d2 == best && bm == m && e < be)) {
+      best = d2; bm = m; be = e; bq = q;
+    }
+  };
+  if (ncand <= kCand) {
+    for (int k = 0; k < ncand; k++) consider(cand[k] >> 24, cand[k] & 0xffffff);
+    n64 += (unsigned)ncand;
+  } else {
+    for (int m = 0; m < P.ncsid; m++) {
+      const MeshDev& M = P.mesh[m];
+      const int cell = tool_cell(M, xi.x, xi.y, xi.z);
+      if (cell < 0) continue;
+      const double4 n0 = M.node[0];
+      const float3 pr = make_float3((float)(xi.x - n0.x), (float)(xi.y - n0.y), (float)(xi.z - n0.z));
+      for (int t = M.cstart[cell]; t < M.cstart[cell + 1]; t++) {
+        const float4* v = M.cvert + 3 * (int64_t)t;
+        const float4 v0 = v[0];
+        if (closest_sq32(pr, make_float3(v0.x, v0.y, v0.z), rel32(v, 1), rel32(v, 2)) > thr)
+          continue;
+        consider(m, __float_as_int(v0.w));
+        n64++;
+      }
+    }
+  }
+  {
+    const unsigned mask = __activemask();
+    const unsigned s32 = __reduce_add_sync(mask, n32), s64 = __reduce_add_sync(mask, n64);
+    if ((int)(threadIdx.x & 31) == __ffs(mask) - 1 && s32) {
+      atomicAdd(P.cstat, (unsigned long long)s32);
+      atomicAdd(P.cstat + 1, (unsigned long long)s64);
+    }
+  }
+  law1_force(P, F, i, x4, a32, best, bm, be, bq);
+}
+
+__global__ void __launch_bounds__(128) k_contact_law1(StepParams P, Fields F, float4* a32) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= P.n || F.perm[i] >= P.n_solid) return;
+  // most particles are nowhere near a tool and skip all FP64 work; the mixed
+  // form keeps an FP32 position mirror
+  float px, py, pz;
+  if (a32) {
+    const float4 p = F.pv[i].p;
+    px = p.x; py = p.y; pz = p.z;
+  } else {
+    const double4 p = F.xm[i];
+    px = (float)p.x; py = (float)p.y; pz = (float)p.z;
+  }
+  if (!law1_near(P, px, py, pz)) {
+    F.cf[i] = make_double4(0.0, 0.0, 0.0, 0.0);
+    F.qf[i] = 0.0;
+    P.ccnt[i] = 0;
+    return;
+  }
+  law1_one(P, F, i, a32);
+}
+
+// The slots listed by the fused acceleration pass (those whose cell of a tool's
+// bins is not empty): contact, then integration.  kLaw1Lanes lanes per slot
+// share its triangles: the search is a chain of loads and FP64 operations, and
+// a thread per slot of the widened box, most of them with empty cells, walked
+// its few dozen triangles twice and its FP64 candidates one after the other
+// (60 us a step with 500k particles and 10,304 triangles, now 34; a warp per
+// slot repeats the FP64 work on 32 lanes: 342).  The smallest FP32 distance
+// and the smallest (FP64 distance, mesh, triangle) do not depend on the order,
+// so the choice is that of law1_one's scan.
+constexpr int kLaw1Lanes = 4;
+__global__ void __launch_bounds__(64) k_contact_law1_list(StepParams P, Fields F,
+                                                          const double4* __restrict__ vd2,
+                                                          float4* a32) {
+  const int lane = threadIdx.x & (kLaw1Lanes - 1);
+  const int slots = gridDim.x * blockDim.x / kLaw1Lanes;
+  const int count = *P.near_count;
+  const int first = (blockIdx.x * blockDim.x + threadIdx.x) / kLaw1Lanes;
+  const unsigned group = ((1u << kLaw1Lanes) - 1u) << ((threadIdx.x & 31) & ~(kLaw1Lanes - 1));
+  unsigned n32 = 0, n64 = 0;                  // this lane's triangle tests
+  for (int w = first; w < count; w += slots) {
+    const int64_t i = P.near_list[w];
+    const double4 x4 = F.xm[i];
+    const V3 xi = mk(x4);
+    // FP32: the smallest squared distance
+    float m32 = P.hf * P.hf, tol = 0.f;
+    for (int m = 0; m < P.ncsid; m++) {
+      const MeshDev& M = P.mesh[m];
+      const int cell = tool_cell(M, xi.x, xi.y, xi.z);
+      if (cell < 0) continue;
+      tol = fmaxf(tol, M.tol32);
+      const double4 n0 = M.node[0];
+      const float3 pr = make_float3((float)(xi.x - n0.x), (float)(xi.y - n0.y), (float)(xi.z - n0.z));
+      const int t1 = M.cstart[cell + 1];
+#pragma unroll 4
+      for (int t = M.cstart[cell] + lane; t < t1; t += kLaw1Lanes) {
+        const float4* v = M.cvert + 3 * (int64_t)t;
+        m32 = fminf(m32, closest_sq32(pr, rel32(v, 0), rel32(v, 1), rel32(v, 2)));
+        n32++;
+      }
+    }
+#pragma unroll
+    for (int o = kLaw1Lanes / 2; o > 0; o >>= 1)
+      m32 = fminf(m32, __shfl_xor_sync(group, m32, o));
+    // FP64: the triangles within tol of it, with the scan's tie rule; a lane
+    // collects its candidates first, so that the lanes evaluate them together
+    const float lim = sqrtf(m32) + tol;
+    const float thr = lim * lim;
+    double best = P.h * P.h;
+    int bm = -1, be = -1;
+    V3 bq = mk(0.0, 0.0, 0.0);
+    auto consider = [&](int m, int e) {
+      const MeshDev& M = P.mesh[m];
+      const int32_t* en = M.elnode + 3 * e;
+      const V3 q = closest_on_tri(xi, mk(M.node[en[0]]), mk(M.node[en[1]]), mk(M.node[en[2]]));
+      const V3 dv = xi - q;
+      const double d2 = dot(dv, dv);
+      n64++;
+      if (d2 < best || (d2 == best && bm == m && e < be)) {
+        best = d2; bm = m; be = e; bq = q;
+      }
+    };
+    for (int m = 0; m < P.ncsid; m++) {
+      const MeshDev& M = P.mesh[m];
+      const int cell = tool_cell(M, xi.x, xi.y, xi.z);
+      if (cell < 0) continue;
+      const double4 n0 = M.node[0];
+      const float3 pr = make_float3((float)(xi.x - n0.x), (float)(xi.y - n0.y), (float)(xi.z - n0.z));
+      const int t1 = M.cstart[cell + 1];
+      int cand = -1;
+#pragma unroll 4
+      for (int t = M.cstart[cell] + lane; t < t1; t += kLaw1Lanes) {
+        const float4* v = M.cvert + 3 * (int64_t)t;
+        const float4 v0 = v[0];
+        if (closest_sq32(pr, make_float3(v0.x, v0.y, v0.z), rel32(v, 1), rel32(v, 2)) > thr)
+          continue;
+        const int e = __float_as_int(v0.w);
+        if (cand < 0) cand = e;
+        else consider(m, e);                   // a lane's second: rare
+      }
+      if (cand >= 0) consider(m, cand);
+    }
+    // the group's smallest (distance, mesh, triangle); lanes without one hold h^2 and -1
+#pragma unroll
+    for (int o = kLaw1Lanes / 2; o > 0; o >>= 1) {
+      const double d1 = __shfl_xor_sync(group, best, o);
+      const int m1 = __shfl_xor_sync(group, bm, o), e1 = __shfl_xor_sync(group, be, o);
+      const V3 q1 = mk(__shfl_xor_sync(group, bq.x, o), __shfl_xor_sync(group, bq.y, o),
+                       __shfl_xor_sync(group, bq.z, o));
+      if (d1 < best || (d1 == best && (m1 < bm || (m1 == bm && e1 < be)))) {
+        best = d1; bm = m1; be = e1; bq = q1;
+      }
+    }
+    if (lane == 0) {
+      law1_force(P, F, i, x4, a32, best, bm, be, bq);
+      integrate_mixed_one(P, F, vd2, i, a32[i]);
+    }
+  }
+  __syncwarp();
+  n32 = __reduce_add_sync(0xffffffffu, n32);
+  n64 = __reduce_add_sync(0xffffffffu, n64);
+  if ((threadIdx.x & 31) == 0 && n32) {
+    atomicAdd(P.cstat, (unsigned long long)n32);
+    atomicAdd(P.cstat + 1, (unsigned long long)n64);
+  }
+}
+
+// Does a particle with mass carry a mesh's zone id?
+__global__ void __launch_bounds__(256) k_zone_mass(StepParams P, Fields F, int* flag) {
+  bool any = false;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t id = F.id[i];
+    bool zone = false;
+    for (int m = 0; m < P.ncsid; m++) zone |= id == P.csid[m];
+    if (zone && F.xm[i].w != 0.0) any = true;
+  }
+  if (any) *flag = 1;
 }
 
 // TriMesh_d::Move: node velocity m_v + m_w x node, then node += v dt
@@ -534,12 +645,22 @@ void launch_contact_stage(const StepParams& P, const Fields& F, const NbBuffers&
       cudaMemcpyAsync(M.cursor, M.cstart, sizeof(uint32_t) * ncell, cudaMemcpyDeviceToDevice, s);
       k_bins_fill<<<blocks_for(M.ne, 128), 128, 0, s>>>(M);
     }
-    k_contact_law1<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, a32);
+    if (!P.near_count) k_contact_law1<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, a32);
     return;
   }
   k_surface<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, N.nb, N.cnt);
   if (list) k_contact_nb<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, N.nb, N.cnt);
   k_contact_force<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, a32);
+}
+
+void launch_contact_law1_list(const StepParams& P, const Fields& F, const double4* vd2,
+                              float4* a32, cudaStream_t s) {
+  // a few thousand slots in practice (16 a block); a larger list loops
+  k_contact_law1_list<<<std::min(blocks_for(P.n * kLaw1Lanes, 64), 912), 64, 0, s>>>(P, F, vd2,
+                                                                                     a32);
+}
+void launch_zone_mass(const StepParams& P, const Fields& F, int* flag, cudaStream_t s) {
+  k_zone_mass<<<std::min(blocks_for(P.n, 256), 1024), 256, 0, s>>>(P, F, flag);
 }
 
 void launch_mesh_update(const StepParams& P, const Fields& F, int mixed, cudaStream_t s) {

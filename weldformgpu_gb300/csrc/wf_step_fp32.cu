@@ -95,6 +95,7 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
   constexpr int W = WF_NB_BLK / kDensLanes;
   constexpr int NB = W < kDensBatch ? W : kDensBatch;   // neighbours gathered per batch
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
+  const bool filter = zone_filter(P);
   float drho = 0.0f, sf = 0.0f;
   int nx[W];
   if (c > 0) list.template sub<W>(0, g, nx);
@@ -120,8 +121,8 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
       for (int q = 0; q < NB; q++) {
         // Entries past the count are the particle's own slot (list padding):
         // r^2 = 0 gives GK = 0 exactly (gk32_r2), so they add exact zeros and
-        // need no test, except under the contact filter.
-        if (P.contact && h + q >= m) continue;
+        // need no test, except under the zone filter.
+        if (filter && h + q >= m) continue;
         const float xx = pi.x - pj[q].x, xy = pi.y - pj[q].y, xz = pi.z - pj[q].z;
         const float GK = gk32_r2(xx * xx + xy * xy + xz * xz, invh, Ch, C);
         // m_j / rho_j GK, shared by both sums
@@ -134,7 +135,7 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
         }
         // density rate (solid particles, contact filter); rho_i multiplies the sum
         bool pass = solid;
-        if constexpr (L::kSlots) pass = pass && !(P.contact && !pass_ij(P, idi, F.id[js[h + q]]));
+        if constexpr (L::kSlots) pass = pass && !(filter && !pass_ij(P, idi, F.id[js[h + q]]));
         if (pass) {
           const float vx = vi.x - vj[q].x, vy = vi.y - vj[q].y, vz = vi.z - vj[q].z;
           drho += mg * (vx * xx + vy * xy + vz * xz);
@@ -523,6 +524,7 @@ __device__ __forceinline__ void stress_pairs(const StepParams& P, const Fields& 
                                              const L& list, int c,
                                              float4 pi, float4 vi, float* acc) {
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
+  const bool filter = zone_filter(P);
   float Dxx = 0.f, Dyy = 0.f, Dzz = 0.f;
   float Axy = 0.f, Bxy = 0.f, Axz = 0.f, Bxz = 0.f, Ayz = 0.f, Byz = 0.f;
   int nx[8];
@@ -547,10 +549,10 @@ __device__ __forceinline__ void stress_pairs(const StepParams& P, const Fields& 
       for (int q = 0; q < kStressBatch; q++) {
         // Entries past the count are the particle's own slot (list padding):
         // r^2 = 0 gives GK = 0 exactly (gk32_r2), so they add exact zeros and
-        // need no test, except under the contact filter.
-        if (P.contact && h + q >= m) continue;
+        // need no test, except under the zone filter.
+        if (filter && h + q >= m) continue;
         if constexpr (L::kSlots) {
-          if (P.contact && !pass_j(P, F.id[js[h + q]])) continue;
+          if (filter && !pass_j(P, F.id[js[h + q]])) continue;
         }
         const float xx = pi.x - pj[q].x, xy = pi.y - pj[q].y, xz = pi.z - pj[q].z;
         // w = 2 s of the reference's s = -GK m_j / (2 rho_j); the off-diagonal
@@ -813,6 +815,15 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
   } else if (i == (int64_t)P.inv[0]) {
     *P.e0 = (double)sd;
   }
+  if (P.max_dep && dep > 0.0) {
+    // the largest strain since the last rebuild (k_max_dep's maximum, kept up as
+    // the strains grow); most warps see that it is larger than theirs
+    const double v = eps_p - F.eps_rb[i];
+    if (v > 0.0) {
+      const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+      if (bits > *(volatile unsigned long long*)P.max_dep) atomicMax(P.max_dep, bits);
+    }
+  }
   warp_count(status, n_it, n_call, n_mlp, capped, eps_p > 1.e-6);
   if (!isfinite(st)) atomicOr(status, WF_STATUS_NAN);
 }
@@ -873,6 +884,7 @@ __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields&
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
   const float h = P.hf, Cs = P.Csf, alpha = P.alphaf, beta = P.betaf, eps = P.epsf;
   const bool av = alpha != 0.0f || beta != 0.0f;
+  const bool filter = zone_filter(P);
   float ax = 0.f, ay = 0.f, az = 0.f;
   const int c = cnt[i];
   int nx[W];
@@ -901,10 +913,10 @@ __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields&
       for (int q = 0; q < kAccelBatch; q++) {
         // Entries past the count are the particle's own slot (list padding):
         // r^2 = 0 gives GK = 0 exactly (gk32_r2), so they add exact zeros and
-        // need no test, except under the contact filter.
-        if (P.contact && hh + q >= m) continue;
+        // need no test, except under the zone filter.
+        if (filter && hh + q >= m) continue;
         if constexpr (L::kSlots) {
-          if (P.contact && !pass_ij(P, idi, F.id[js[hh + q]])) continue;
+          if (filter && !pass_ij(P, idi, F.id[js[hh + q]])) continue;
         }
         const float xx = pi.x - pj[q].x, xy = pi.y - pj[q].y, xz = pi.z - pj[q].z;
         const float r2 = xx * xx + xy * xy + xz * xz;
@@ -977,10 +989,19 @@ __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
 // FP64 work and traffic overlapping the other warps' neighbour gathers.
 // Neighbours are read from pvb (the density pass's copy of the mirrors) while
 // the new mirrors go to F.pv and th32, which this pass does not read.
+// kLaw1 (contact law 1): only the slots whose cell of a tool's bins lists a
+// triangle take part in the contact, so all others are integrated here as well,
+// and those few leave their
+// acceleration in a32 and their number in the list that k_contact_law1_list
+// (wf_contact.cu) works through, contact and integration.  The separate passes
+// read and wrote every slot again (500k particles: 68 us for the contact and 39
+// for the integration; now 34 for the listed slots).
+template <bool kLaw1>
 __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
                                                      const Rec32* __restrict__ pvb,
                                                      const Sig32 sig,
                                                      const double4* __restrict__ vd2,
+                                                     float4* __restrict__ a32,
                                                      const int32_t* __restrict__ nb,
                                                      const int32_t* __restrict__ cnt, const List16 L16) {
   int g;
@@ -1008,7 +1029,26 @@ __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
     else
       af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbList32{nb, P.npad, i});
   }
-  if (g == 0) integrate_mixed_one(P, F, vd2, i, af);
+  if (g != 0) return;
+  if constexpr (kLaw1) {
+    if (F.perm[i] < P.n_solid) {
+      const float4 p = pvb[i].p;
+      if (law1_near(P, p.x, p.y, p.z) && law1_triangles(P, F.xm[i])) {
+        a32[i] = af;
+        const unsigned mask = __activemask();
+        const int lead = __ffs(mask) - 1, lane = threadIdx.x & 31;
+        int base = 0;
+        if (lane == lead) base = atomicAdd(P.near_count, __popc(mask));
+        base = __shfl_sync(mask, base, lead);
+        P.near_list[base + __popc(mask & ((1u << lane) - 1u))] = (int32_t)i;
+        return;
+      }
+      F.cf[i] = make_double4(0.0, 0.0, 0.0, 0.0);
+      F.qf[i] = 0.0;
+      P.ccnt[i] = 0;
+    }
+  }
+  integrate_mixed_one(P, F, vd2, i, af);
 }
 
 // The same pass for staged tiles: a block of 2 x 128 threads is one tile;
@@ -1165,8 +1205,8 @@ void launch_fp32_accel(const StepParams& P, const Fields& F, const Rec32* pvb,
   k_accel32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sig, a32, N.nb, N.cnt);
 }
 void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec32* pvb,
-                                 const Sig32& sig, const double4* vd2, const NbBuffers& N,
-                                 const TileHalo& T, const List16& L16, cudaStream_t s) {
+                                 const Sig32& sig, const double4* vd2, float4* a32,
+                                 const NbBuffers& N, const TileHalo& T, const List16& L16, cudaStream_t s) {
   if (T.cap > 0) {
     const size_t smem = (3 * sizeof(float4) + sizeof(float2)) * (size_t)T.cap + WF_TILE_LIST_BYTES;
     static size_t opted[64] = {};
@@ -1175,11 +1215,13 @@ void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec
         P, F, pvb, sig, vd2, N.nb, N.cnt, T);
     return;
   }
-  static size_t c_smem = 0;
-  static int64_t c_val = 0;
+  static size_t c_smem[2] = {0, 0};
+  static int64_t c_val[2] = {0, 0};
+  const int law1 = P.near_count ? 1 : 0;
+  const auto kernel = law1 ? k_accel_int32<true> : k_accel_int32<false>;
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
-      k_accel_int32, 128, 0, kAccelLanes, &c_smem, &c_val));
-  k_accel_int32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sig, vd2, N.nb,
-                                                                   N.cnt, L16);
+      kernel, 128, 0, kAccelLanes, &c_smem[law1], &c_val[law1]));
+  kernel<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sig, vd2, a32, N.nb, N.cnt,
+                                                            L16);
 }
