@@ -213,6 +213,7 @@ struct StepParams {
   double* e0;           // mixed form, energy_mode 0: particle 0's S:D of this step
   const int32_t* inv;   // inv[original id] = slot (particle 0's slot for energy_mode 0)
   int contact;          // contact pass filter active
+  int pair_fence;       // always 0: see the mixed acceleration pass
   const int* zone_mass; // set when a particle with mass carries a mesh's zone id
   int* near_count;      // contact law 1 fused into the mixed acceleration pass: slots near a
   int32_t* near_list;   // tool (null: the contact is a pass of its own)

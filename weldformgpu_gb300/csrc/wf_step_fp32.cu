@@ -67,6 +67,15 @@ __device__ __forceinline__ unsigned group_mask() {
   return ((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1));
 }
 
+// Blocks per SM that a pass is compiled for (kWide: few blocks, so many
+// registers per thread and the compiler keeps more loads in flight; else many
+// blocks).  A grid of at most four blocks per SM runs in one wave whatever the
+// bound, and what it waits for is each thread's own chain of loads: 10,752
+// particles 14.5 -> 12.5 us stress, 16.9 -> 14.8 acceleration, 46.3 -> 42.4 a
+// step, while 50,560 (more than one wave of the acceleration pass's two lanes
+// per particle) lose 27 -> 35 us there.
+constexpr int kWideBlocks = 4;
+
 // Density + heat pass: one lane per particle (786k particles: 0.199 ms with
 // one lane and 6 blocks per SM, 0.202-0.213 ms with 2 or 4 lanes).
 constexpr int kDensLanes = 1;
@@ -85,7 +94,7 @@ constexpr int kDensBatch = 4;
 // entries are slots (NbList32 / NbList16: records gathered from the global
 // arrays) or ranks in the tile's halo (NbListS: the arrays are its
 // shared-memory copies).
-template <class L, class R, bool kHeat = true>
+template <bool kFilter, bool kHeat, class L, class R>
 __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fields& F,
                                                    const R& rec, const float* __restrict__ gt,
                                                    const L& list, int g, int c, float4 pi,
@@ -95,7 +104,6 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
   constexpr int W = WF_NB_BLK / kDensLanes;
   constexpr int NB = W < kDensBatch ? W : kDensBatch;   // neighbours gathered per batch
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
-  const bool filter = zone_filter(P);
   float drho = 0.0f, sf = 0.0f;
   int nx[W];
   if (c > 0) list.template sub<W>(0, g, nx);
@@ -122,7 +130,7 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
         // Entries past the count are the particle's own slot (list padding):
         // r^2 = 0 gives GK = 0 exactly (gk32_r2), so they add exact zeros and
         // need no test, except under the zone filter.
-        if (filter && h + q >= m) continue;
+        if (kFilter && h + q >= m) continue;
         const float xx = pi.x - pj[q].x, xy = pi.y - pj[q].y, xz = pi.z - pj[q].z;
         const float GK = gk32_r2(xx * xx + xy * xy + xz * xz, invh, Ch, C);
         // m_j / rho_j GK, shared by both sums
@@ -135,7 +143,7 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
         }
         // density rate (solid particles, contact filter); rho_i multiplies the sum
         bool pass = solid;
-        if constexpr (L::kSlots) pass = pass && !(filter && !pass_ij(P, idi, F.id[js[h + q]]));
+        if constexpr (kFilter) pass = pass && pass_ij(P, idi, F.id[js[h + q]]);
         if (pass) {
           const float vx = vi.x - vj[q].x, vy = vi.y - vj[q].y, vz = vi.z - vj[q].z;
           drho += mg * (vx * xx + vy * xy + vz * xz);
@@ -149,7 +157,8 @@ __device__ __forceinline__ void density_heat_pairs(const StepParams& P, const Fi
 
 // ---- A32: the density pass without a heat pass to fuse (a call's first
 // step; every step when heat is off): the density sum of density_heat_pairs.
-__global__ void __launch_bounds__(128, kDensMinBlocks) k_density32(StepParams P, Fields F,
+template <bool kWide>
+__global__ void __launch_bounds__(128, kWide ? kWideBlocks : kDensMinBlocks) k_density32(StepParams P, Fields F,
                                                                   double4* __restrict__ vd2,
                                                                   Rec32* __restrict__ pvb,
                                                                   const int32_t* __restrict__ nb,
@@ -174,14 +183,16 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density32(StepParams P,
   float drho = 0.0f, sf = 0.0f;
   const int b16 = L16.base ? L16.base[i / WF_TILE] : -1;     // uniform over the block
   const float2 t0 = make_float2(0.f, 0.f);
-  if (b16 >= 0)
-    density_heat_pairs<NbList16, RecGlobal, false>(P, F, RecGlobal{F.pv}, nullptr,
-                                                   NbList16{L16.off, P.npad, i, b16}, 0, c, pi, vi,
-                                                   t0, solid, idi, drho, sf);
+  const RecGlobal rec{F.pv};
+  const NbList32 list{nb, P.npad, i};
+  if (zone_filter(P))
+    density_heat_pairs<true, false>(P, F, rec, nullptr, list, 0, c, pi, vi, t0, solid, idi, drho, sf);
+  else if (b16 >= 0)
+    density_heat_pairs<false, false>(P, F, rec, nullptr, NbList16{L16.off, P.npad, i, b16}, 0, c, pi,
+                                     vi, t0, solid, idi, drho, sf);
   else
-    density_heat_pairs<NbList32, RecGlobal, false>(P, F, RecGlobal{F.pv}, nullptr,
-                                                   NbList32{nb, P.npad, i}, 0, c, pi, vi, t0, solid,
-                                                   idi, drho, sf);
+    density_heat_pairs<false, false>(P, F, rec, nullptr, list, 0, c, pi, vi, t0, solid, idi, drho,
+                                     sf);
   const double4 vdi = F.vd[i];
   drho *= (float)vdi.w;
   double rho_new = vdi.w;
@@ -194,7 +205,8 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density32(StepParams P,
                  make_float4(vi.x, vi.y, vi.z, (float)rho_new)};
 }
 
-__global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepParams P, Fields F,
+template <bool kWide>
+__global__ void __launch_bounds__(128, kWide ? kWideBlocks : kDensMinBlocks) k_density_heat32(StepParams P, Fields F,
                                                         double4* __restrict__ vd2,
                                                         Rec32* __restrict__ pvb,
                                                         const int32_t* __restrict__ nb,
@@ -249,15 +261,18 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_density_heat32(StepPara
   float drho, sf;
   const int c = cnt[i];
   const int b16 = L16.base ? L16.base[i / WF_TILE] : -1;     // uniform over the block
-  if (staged >= 0)
-    density_heat_pairs(P, F, RecShared{sp, sv}, st, NbListS{sl, (int)threadIdx.x}, g, c, pi, vi, ti,
-                       solid, idi, drho, sf);
+  const RecGlobal rec{F.pv};
+  const NbList32 list{nb, P.npad, i};
+  if (zone_filter(P))
+    density_heat_pairs<true, true>(P, F, rec, F.tl32, list, g, c, pi, vi, ti, solid, idi, drho, sf);
+  else if (staged >= 0)
+    density_heat_pairs<false, true>(P, F, RecShared{sp, sv}, st, NbListS{sl, (int)threadIdx.x}, g, c,
+                                    pi, vi, ti, solid, idi, drho, sf);
   else if (b16 >= 0)
-    density_heat_pairs(P, F, RecGlobal{F.pv}, F.tl32, NbList16{L16.off, P.npad, i, b16}, g, c, pi, vi,
-                       ti, solid, idi, drho, sf);
+    density_heat_pairs<false, true>(P, F, rec, F.tl32, NbList16{L16.off, P.npad, i, b16}, g, c, pi,
+                                    vi, ti, solid, idi, drho, sf);
   else
-    density_heat_pairs(P, F, RecGlobal{F.pv}, F.tl32, NbList32{nb, P.npad, i}, g, c, pi, vi, ti, solid,
-                       idi, drho, sf);
+    density_heat_pairs<false, true>(P, F, rec, F.tl32, list, g, c, pi, vi, ti, solid, idi, drho, sf);
   if constexpr (kDensLanes > 1) {
     const unsigned mask = group_mask<kDensLanes>();
 #pragma unroll
@@ -519,12 +534,11 @@ constexpr float kMlpSteep = 0.02f;
 // (halved by the caller).  The off-diagonal terms of a pair are a + b (D) and
 // a - b (W) of two products a = s_k x_l, b = s_l x_k: their two sums are
 // accumulated (one FMA each) and combined once after the loop.
-template <class L, class R>
+template <bool kFilter, class L, class R>
 __device__ __forceinline__ void stress_pairs(const StepParams& P, const Fields& F, const R& rec,
                                              const L& list, int c,
                                              float4 pi, float4 vi, float* acc) {
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
-  const bool filter = zone_filter(P);
   float Dxx = 0.f, Dyy = 0.f, Dzz = 0.f;
   float Axy = 0.f, Bxy = 0.f, Axz = 0.f, Bxz = 0.f, Ayz = 0.f, Byz = 0.f;
   int nx[8];
@@ -550,9 +564,8 @@ __device__ __forceinline__ void stress_pairs(const StepParams& P, const Fields& 
         // Entries past the count are the particle's own slot (list padding):
         // r^2 = 0 gives GK = 0 exactly (gk32_r2), so they add exact zeros and
         // need no test, except under the zone filter.
-        if (filter && h + q >= m) continue;
-        if constexpr (L::kSlots) {
-          if (filter && !pass_j(P, F.id[js[h + q]])) continue;
+        if constexpr (kFilter) {
+          if (h + q >= m || !pass_j(P, F.id[js[h + q]])) continue;
         }
         const float xx = pi.x - pj[q].x, xy = pi.y - pj[q].y, xz = pi.z - pj[q].z;
         // w = 2 s of the reference's s = -GK m_j / (2 rho_j); the off-diagonal
@@ -650,12 +663,16 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
   const int c = solid ? cnt[i] : 0;
   float acc[9];
   const int b16 = L16.base ? L16.base[i0 / WF_TILE] : -1;    // uniform over the block
-  if (staged >= 0)
-    stress_pairs(P, F, RecShared{sp, sv}, NbListS{sl, (int)threadIdx.x}, c, pi, vi, acc);
+  const RecGlobal rec{pvb};
+  const NbList32 list{nb, P.npad, i};
+  if (zone_filter(P))
+    stress_pairs<true>(P, F, rec, list, c, pi, vi, acc);
+  else if (staged >= 0)
+    stress_pairs<false>(P, F, RecShared{sp, sv}, NbListS{sl, (int)threadIdx.x}, c, pi, vi, acc);
   else if (b16 >= 0)
-    stress_pairs(P, F, RecGlobal{pvb}, NbList16{L16.off, P.npad, i, b16}, c, pi, vi, acc);
+    stress_pairs<false>(P, F, rec, NbList16{L16.off, P.npad, i, b16}, c, pi, vi, acc);
   else
-    stress_pairs(P, F, RecGlobal{pvb}, NbList32{nb, P.npad, i}, c, pi, vi, acc);
+    stress_pairs<false>(P, F, rec, list, c, pi, vi, acc);
   float Dxx = acc[0], Dyy = acc[1], Dzz = acc[2], Dxy = acc[3], Dyz = acc[4], Dxz = acc[5];
   float Wxy = acc[6], Wyz = acc[7], Wxz = acc[8];
   Dxy *= 0.5f; Dxz *= 0.5f; Dyz *= 0.5f;
@@ -828,7 +845,8 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
   if (!isfinite(st)) atomicOr(status, WF_STATUS_NAN);
 }
 
-__global__ void __launch_bounds__(128, 6) k_stress32_mlp(StepParams P, Fields F,
+template <bool kWide>
+__global__ void __launch_bounds__(128, kWide ? kWideBlocks : 6) k_stress32_mlp(StepParams P, Fields F,
                                                       const Rec32* __restrict__ pvb,
                                                       const Sig32 sig,
                                                       const int32_t* __restrict__ nb,
@@ -839,7 +857,8 @@ __global__ void __launch_bounds__(128, 6) k_stress32_mlp(StepParams P, Fields F,
                                                       const List16 L16) {
   stress32_body<true>(P, F, pvb, sig, nb, cnt, status, mlp, l1, T, L16);
 }
-__global__ void __launch_bounds__(128, 6) k_stress32(StepParams P, Fields F,
+template <bool kWide>
+__global__ void __launch_bounds__(128, kWide ? kWideBlocks : 6) k_stress32(StepParams P, Fields F,
                                                      const Rec32* __restrict__ pvb,
                                                      const Sig32 sig,
                                                      const int32_t* __restrict__ nb,
@@ -850,12 +869,14 @@ __global__ void __launch_bounds__(128, 6) k_stress32(StepParams P, Fields F,
 }
 
 // ---- C32: acceleration + Monaghan viscosity (InteractionAlt.cu:18-150) ----
-// Lane groups of kAccelLanes (see nb_sub).  Neighbours are gathered per batch
-// of kAccelBatch: each carries 56 bytes (position, velocity, stress/rho^2).
-// 786k particles: 0.278 ms with one lane per particle, 0.272 ms with two
-// (71 registers, 7 blocks per SM), 0.31-0.39 ms with four.  With the L2
-// prefetches the fused pass held to 64 registers (8 blocks per SM, no spill)
-// runs 0.252 -> 0.245 ms; 6 blocks 0.270, 9 blocks spill.
+// Lane groups of kAccelLanes (see nb_sub).  Neighbours are gathered in batches
+// of kAccelBatch, 56 bytes each (position, velocity, stress/rho^2).  Compiled
+// for 8 blocks per SM (kTight) the neighbours of a batch are kept apart by
+// tests that never hold (P.pair_fence, always 0): without them the compiler
+// overlaps them, needs more than the 64 registers that 8 blocks leave and
+// spills (786k particles: 286 us; 231 with the tests, 240 with 6 blocks and
+// without them).  786k particles with records of 16 bytes: 0.278 ms with one
+// lane per particle, 0.272 with two, 0.31-0.39 with four.
 constexpr int kAccelLanes = 2;
 constexpr int kAccelBatch = 2;
 static_assert(WF_NB_BLK / kAccelLanes >= kAccelBatch, "batch within the lane's sub-block");
@@ -869,7 +890,7 @@ struct AccelSrc {
   const float2* sb;
 };
 
-template <class L, class R>
+template <bool kFilter, bool kTight, class L, class R>
 __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields& F,
                                               const Rec32* __restrict__ pvb,
                                               const Sig32 sig,
@@ -884,7 +905,6 @@ __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields&
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
   const float h = P.hf, Cs = P.Csf, alpha = P.alphaf, beta = P.betaf, eps = P.epsf;
   const bool av = alpha != 0.0f || beta != 0.0f;
-  const bool filter = zone_filter(P);
   float ax = 0.f, ay = 0.f, az = 0.f;
   const int c = cnt[i];
   int nx[W];
@@ -914,9 +934,12 @@ __device__ __forceinline__ float4 accel_value(const StepParams& P, const Fields&
         // Entries past the count are the particle's own slot (list padding):
         // r^2 = 0 gives GK = 0 exactly (gk32_r2), so they add exact zeros and
         // need no test, except under the zone filter.
-        if (filter && hh + q >= m) continue;
-        if constexpr (L::kSlots) {
-          if (filter && !pass_ij(P, idi, F.id[js[hh + q]])) continue;
+        if constexpr (kTight && !kFilter) {
+          if (P.pair_fence && hh + q >= m) continue;
+          if (P.pair_fence && !pass_ij(P, idi, F.id[js[hh + q]])) continue;
+        }
+        if constexpr (kFilter) {
+          if (hh + q >= m || !pass_ij(P, idi, F.id[js[hh + q]])) continue;
         }
         const float xx = pi.x - pj[q].x, xy = pi.y - pj[q].y, xz = pi.z - pj[q].z;
         const float r2 = xx * xx + xy * xy + xz * xz;
@@ -959,7 +982,8 @@ __device__ __forceinline__ int64_t accel_slot(int& g) {
   return t / kAccelLanes;
 }
 
-__global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
+template <bool kWide>
+__global__ void __launch_bounds__(128, kWide ? kWideBlocks : 8) k_accel32(StepParams P, Fields F,
                                                  const Rec32* __restrict__ pvb,
                                                  const Sig32 sig,
                                                  float4* __restrict__ a32,
@@ -980,7 +1004,10 @@ __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
   }
   if (F.perm[i] >= P.n_solid) return;
   const AccelSrc<RecGlobal> src{{pvb}, sig.a, sig.b};
-  const float4 af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbList32{nb, P.npad, i});
+  const NbList32 list{nb, P.npad, i};
+  const float4 af = zone_filter(P)
+                        ? accel_value<true, !kWide>(P, F, pvb, sig, cnt, i, g, src, list)
+                        : accel_value<false, !kWide>(P, F, pvb, sig, cnt, i, g, src, list);
   if (g == 0) a32[i] = af;
 }
 
@@ -996,8 +1023,8 @@ __global__ void __launch_bounds__(128, 8) k_accel32(StepParams P, Fields F,
 // (wf_contact.cu) works through, contact and integration.  The separate passes
 // read and wrote every slot again (500k particles: 68 us for the contact and 39
 // for the integration; now 34 for the listed slots).
-template <bool kLaw1>
-__global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
+template <bool kLaw1, bool kWide>
+__global__ void __launch_bounds__(128, kWide ? kWideBlocks : 8) k_accel_int32(StepParams P, Fields F,
                                                      const Rec32* __restrict__ pvb,
                                                      const Sig32 sig,
                                                      const double4* __restrict__ vd2,
@@ -1024,10 +1051,14 @@ __global__ void __launch_bounds__(128, 8) k_accel_int32(StepParams P, Fields F,
   float4 af = make_float4(0.f, 0.f, 0.f, 0.f);
   if (F.perm[i] < P.n_solid) {
     const int b16 = L16.base ? L16.base[i / WF_TILE] : -1;   // uniform over the block
-    if (b16 >= 0)
-      af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbList16{L16.off, P.npad, i, b16});
+    const NbList32 list{nb, P.npad, i};
+    if (kLaw1 && zone_filter(P))
+      af = accel_value<true, !kWide>(P, F, pvb, sig, cnt, i, g, src, list);
+    else if (b16 >= 0)
+      af = accel_value<false, !kWide>(P, F, pvb, sig, cnt, i, g, src,
+                                      NbList16{L16.off, P.npad, i, b16});
     else
-      af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbList32{nb, P.npad, i});
+      af = accel_value<false, !kWide>(P, F, pvb, sig, cnt, i, g, src, list);
   }
   if (g != 0) return;
   if constexpr (kLaw1) {
@@ -1092,10 +1123,10 @@ __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
   if (F.perm[i] < P.n_solid) {
     if (staged >= 0) {
       const AccelSrc<RecShared> src{{sp, sv}, ssa, ssb};
-      af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbListS{sl, (int)(threadIdx.x >> 1)});
+      af = accel_value<false, false>(P, F, pvb, sig, cnt, i, g, src, NbListS{sl, (int)(threadIdx.x >> 1)});
     } else {
       const AccelSrc<RecGlobal> src{{pvb}, sig.a, sig.b};
-      af = accel_value(P, F, pvb, sig, cnt, i, g, src, NbList32{nb, P.npad, i});
+      af = accel_value<false, false>(P, F, pvb, sig, cnt, i, g, src, NbList32{nb, P.npad, i});
     }
   }
   if (g == 0) integrate_mixed_one(P, F, vd2, i, af);
@@ -1123,14 +1154,29 @@ static int64_t wave_slots(K kernel, int threads, size_t smem, int lanes, size_t*
   return *c_val;
 }
 
+// Does a grid run in one wave at kWideBlocks blocks per SM?  (1 or 0; the SM
+// count is that of the device the process first asked about.)
+static int one_wave(int blocks) {
+  static const int sms = [] {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return 0;
+    return v;
+  }();
+  return blocks <= kWideBlocks * sms ? 1 : 0;
+}
+
 void launch_fp32_density(const StepParams& P, const Fields& F, double4* vd2, Rec32* pvb,
                          const NbBuffers& N, const List16& L16, cudaStream_t s) {
-  static size_t c_smem = 0;
-  static int64_t c_val = 0;
+  static size_t c_smem[2] = {0, 0};
+  static int64_t c_val[2] = {0, 0};
+  const int blocks = blocks_for(P.n, 128), w = one_wave(blocks);
+  const auto kernel = w ? k_density32<true> : k_density32<false>;
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
-      k_density32, 128, 0, 1, &c_smem, &c_val));
-  k_density32<<<blocks_for(P.n, 128), 128, 0, s>>>(Q, F, vd2, pvb, N.nb, N.cnt, L16);
+      kernel, 128, 0, 1, &c_smem[w], &c_val[w]));
+  kernel<<<blocks, 128, 0, s>>>(Q, F, vd2, pvb, N.nb, N.cnt, L16);
 }
 void launch_fp32_density_heat(const StepParams& P, const Fields& F, double4* vd2, Rec32* pvb,
                               const NbBuffers& N, int first, int plastic_heat, const TileHalo& T,
@@ -1141,14 +1187,16 @@ void launch_fp32_density_heat(const StepParams& P, const Fields& F, double4* vd2
       Tl.cap > 0 ? 2 * sizeof(float4) * (size_t)Tl.cap + sizeof(float) * (size_t)((Tl.cap + 3) & ~3) +
                        WF_TILE_LIST_BYTES
                  : 0;
-  static size_t opted[64] = {};     // per device: dynamic shared memory opted in so far
-  opt_in_smem(k_density_heat32, smem, opted);
-  static size_t c_smem = 0;
-  static int64_t c_val = 0;
+  static size_t opted[2][64] = {};  // per variant and device: dynamic shared memory opted in so far
+  static size_t c_smem[2] = {0, 0};
+  static int64_t c_val[2] = {0, 0};
+  const int blocks = blocks_for(P.n * kDensLanes, 128), w = one_wave(blocks);
+  const auto kernel = w ? k_density_heat32<true> : k_density_heat32<false>;
+  opt_in_smem(kernel, smem, opted[w]);
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
-      k_density_heat32, 128, smem, kDensLanes, &c_smem, &c_val));
-  k_density_heat32<<<blocks_for(P.n * kDensLanes, 128), 128, smem, s>>>(
+      kernel, 128, smem, kDensLanes, &c_smem[w], &c_val[w]));
+  kernel<<<blocks, 128, smem, s>>>(
       Q, F, vd2, pvb, N.nb, N.cnt, first, plastic_heat, Tl, L16);
 }
 void launch_fp32_heat(const StepParams& P, const Fields& F, const NbBuffers& N, int plastic_heat,
@@ -1177,32 +1225,30 @@ void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, 
   const MlpL1 l1 = (W && mlp_l1) ? *mlp_l1 : MlpL1{};
   const size_t smem = (W ? WF_UMMA_SMEM : 0) +
                       (T.cap > 0 ? 2 * sizeof(float4) * (size_t)T.cap + WF_TILE_LIST_BYTES : 0);
-  static size_t opted[2][64] = {};  // per variant and device: dynamic shared memory opted in
-  static size_t c_smem[2] = {0, 0};
-  static int64_t c_val[2] = {0, 0};
+  static size_t opted[2][2][64] = {};  // per variant and device: dynamic shared memory opted in
+  static size_t c_smem[2][2] = {};
+  static int64_t c_val[2][2] = {};
+  const int blocks = blocks_for(P.n, 128), w = one_wave(blocks), m = W ? 1 : 0;
   StepParams Q = P;
-  if (W) {
-    opt_in_smem(k_stress32_mlp, smem, opted[1]);
+  const auto run = [&](auto kernel, auto... args) {
+    opt_in_smem(kernel, smem, opted[m][w]);
     Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
-        k_stress32_mlp, 128, smem, 1, &c_smem[1], &c_val[1]));
-    k_stress32_mlp<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, pvb, sig, N.nb, N.cnt,
-                                                           status, W, l1, T, L16);
-  } else {
-    opt_in_smem(k_stress32, smem, opted[0]);
-    Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
-        k_stress32, 128, smem, 1, &c_smem[0], &c_val[0]));
-    k_stress32<<<blocks_for(P.n, 128), 128, smem, s>>>(Q, F, pvb, sig, N.nb, N.cnt, status,
-                                                       T, L16);
-  }
+        kernel, 128, smem, 1, &c_smem[m][w], &c_val[m][w]));
+    kernel<<<blocks, 128, smem, s>>>(Q, F, pvb, sig, N.nb, N.cnt, status, args...);
+  };
+  if (W) run(w ? k_stress32_mlp<true> : k_stress32_mlp<false>, W, l1, T, L16);
+  else run(w ? k_stress32<true> : k_stress32<false>, T, L16);
 }
 void launch_fp32_accel(const StepParams& P, const Fields& F, const Rec32* pvb,
                        const Sig32& sig, float4* a32, const NbBuffers& N, cudaStream_t s) {
-  static size_t c_smem = 0;
-  static int64_t c_val = 0;
+  static size_t c_smem[2] = {0, 0};
+  static int64_t c_val[2] = {0, 0};
+  const int blocks = blocks_for(P.n * kAccelLanes, 128), w = one_wave(blocks);
+  const auto kernel = w ? k_accel32<true> : k_accel32<false>;
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
-      k_accel32, 128, 0, kAccelLanes, &c_smem, &c_val));
-  k_accel32<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sig, a32, N.nb, N.cnt);
+      kernel, 128, 0, kAccelLanes, &c_smem[w], &c_val[w]));
+  kernel<<<blocks, 128, 0, s>>>(Q, F, pvb, sig, a32, N.nb, N.cnt);
 }
 void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec32* pvb,
                                  const Sig32& sig, const double4* vd2, float4* a32,
@@ -1215,13 +1261,14 @@ void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec
         P, F, pvb, sig, vd2, N.nb, N.cnt, T);
     return;
   }
-  static size_t c_smem[2] = {0, 0};
-  static int64_t c_val[2] = {0, 0};
+  static size_t c_smem[2][2] = {};
+  static int64_t c_val[2][2] = {};
+  const int blocks = blocks_for(P.n * kAccelLanes, 128), w = one_wave(blocks);
   const int law1 = P.near_count ? 1 : 0;
-  const auto kernel = law1 ? k_accel_int32<true> : k_accel_int32<false>;
+  const auto kernel = law1 ? (w ? k_accel_int32<true, true> : k_accel_int32<true, false>)
+                           : (w ? k_accel_int32<false, true> : k_accel_int32<false, false>);
   StepParams Q = P;
   Q.pf_ahead = !P.wave_pf ? 0 : (int64_t)(P.wave_dist * (double)wave_slots(
-      kernel, 128, 0, kAccelLanes, &c_smem[law1], &c_val[law1]));
-  kernel<<<blocks_for(P.n * kAccelLanes, 128), 128, 0, s>>>(Q, F, pvb, sig, vd2, a32, N.nb, N.cnt,
-                                                            L16);
+      kernel, 128, 0, kAccelLanes, &c_smem[law1][w], &c_val[law1][w]));
+  kernel<<<blocks, 128, 0, s>>>(Q, F, pvb, sig, vd2, a32, N.nb, N.cnt, L16);
 }
