@@ -212,7 +212,7 @@ int wf_find_neighbors(wf_domain* d);
  *   lists   device, n*WF_MAX_NEIGHBORS int32, row-major; row i holds particle
  *           i's neighbour indices, entries past counts[i] are left untouched
  *   stream  cudaStream_t to run on (NULL: the legacy default stream); the call
- *           returns once the lists are written (it waits for the stream twice)
+ *           returns once the lists are written (it waits for the stream once)
  *   err     optional buffer of err_len bytes for a one-line message
  * Temporaries live in one fixed device array inside the library,
  * WF_STATIC_SCRATCH_BYTES (about 4.5 MiB), which every GPU that loads the

@@ -733,7 +733,7 @@ static int ensure_cells(wf_domain* d, int64_t ncell) {
   int64_t cap = (ncell + 1) + (ncell + 1) / 4 + 1024;
   WF_CUDA_OK(dalloc(&d->cell_count, cap, d->stream));
   WF_CUDA_OK(dalloc(&d->cell_cursor, cap, d->stream));
-  d->scan_cap = scan_tmp_words(cap) + 16;
+  d->scan_cap = cell_scan_words(cap) + 16;
   WF_CUDA_OK(dalloc(&d->scan_tmp, d->scan_cap, d->stream));
   d->cell_cap = cap;
   return WF_OK;
@@ -797,42 +797,41 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
   cudaStream_t s = d->stream;
   Fields& A = d->F[d->cur];
   Fields& B = d->F[1 - d->cur];
-  launch_prep_positions(n, A, use_current ? 1 : 0, d->pf, s);
-  int mm_init[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
-  WF_CUDA_OK(cudaMemcpyAsync(d->d_mm, mm_init, sizeof mm_init, cudaMemcpyHostToDevice, s));
   const float r = (float)(2.0 * d->h);                // SolverFraser.cu:72-82
-  launch_minmax(n, d->pf, r, d->d_mm, s);
-  int mm[8];   // bounds, then the largest halo of the previous tile build
+  launch_prep_bounds(n, A, use_current ? 1 : 0, d->pf, r, reinterpret_cast<unsigned*>(d->d_mm), s);
+  int mm[8];   // the bounds' codes, then the largest halo of the previous tile build
   WF_CUDA_OK(cudaMemcpyAsync(mm, d->d_mm, sizeof mm, cudaMemcpyDeviceToHost, s));
   WF_CUDA_OK(cudaStreamSynchronize(s));
   if (d->tile_cap > 0) d->tile_hmax = mm[6];
-  grid_from_minmax(mm, r, &d->grid);
+  int bounds[6];
+  bounds_from_codes(reinterpret_cast<const unsigned*>(mm), bounds);
+  grid_from_bounds(bounds, r, &d->grid);
   const int64_t ncell = (int64_t)d->grid.dim[0] * d->grid.dim[1] * d->grid.dim[2];
   if (ncell > (int64_t)2000000000) return wf_fail(d, WF_ERR_NUMERIC, "neighbour grid too large");
   int rc = ensure_cells(d, ncell);
   if (rc) return rc;
-  WF_CUDA_OK(cudaMemsetAsync(d->cell_count, 0, sizeof(uint32_t) * (ncell + 1), s));
-  WF_CUDA_OK(cudaMemsetAsync(d->cell_cursor, 0, sizeof(uint32_t) * (ncell + 1), s));
-  launch_cell_count(n, d->pf, d->grid, d->cellid, d->cell_count, d->d_status, s);
-  device_exclusive_scan(d->cell_count, ncell + 1, d->scan_tmp, s);
-  launch_cell_scatter(n, d->cellid, d->cell_count, d->cell_cursor, A.perm, d->s_src, d->s_orig, s);
-  launch_cell_sort(ncell, d->cell_count, d->s_src, d->s_orig, s);
   // The lists hold the same particles in the same order whether or not the
   // state is moved into the sorted order, so the arithmetic is identical;
   // moving it keeps warps' particles close in space.  Inside the step loop
   // the state is moved at every kReorderEvery-th rebuild only (solids move
   // little in between); otherwise the lists name the particles' current slots.
   const bool full = !light || ++d->light_rebuilds >= kReorderEvery;
+  {
+    // pf2 lends its memory to the ranks until the sorted positions go there
+    const CellWork W{d->cellid, reinterpret_cast<uint32_t*>(d->pf2), d->cell_cursor, d->scan_tmp + 1,
+                     d->scan_tmp, d->cell_count, 0};
+    WF_CUDA_OK(cudaMemsetAsync(d->cell_cursor, 0, sizeof(uint32_t) * ncell, s));
+    launch_cell_sort(n, d->pf, d->grid, nullptr, A.perm, W, d->s_src, d->s_orig,
+                     full ? nullptr : d->pf2, d->d_status, s);
+  }
   if (full) {
     launch_reorder(n, d->s_src, A, B, d->pf, d->pf2, d->inv, s);
     d->cur = 1 - d->cur;
     d->light_rebuilds = 0;
-  } else {
-    launch_gather_pf(n, d->s_src, d->pf, d->pf2, s);
   }
   launch_nblist(n, d->npad, d->pf2, d->grid, d->cell_count, full ? nullptr : d->s_src, d->nb,
                 d->nbc, d->d_status, s);
-  d->launches += 8;
+  d->launches += full ? 7 : 6;
   if (d->debug_checks) {
     if (d->inject_list_error >= 0) {
       int32_t slot = -1;

@@ -25,60 +25,126 @@ __device__ __forceinline__ int cell_coord(float p, float gmin, float gdelta) {
   return (int)floorf(__fmul_rn(__fsub_rn(p, gmin), gdelta));
 }
 
-// float positions the search reads: x_h snapshot or the current positions
-__global__ void k_prep_positions(int64_t n, const Fields F, int use_current, float4* pf) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (use_current) {
-    double4 x = F.xm[i];
-    pf[i] = make_float4(__double2float_rn(x.x), __double2float_rn(x.y), __double2float_rn(x.z), 0.f);
-  } else {
-    pf[i] = F.xh[i];
+// Cell bounds of the particles, floor(p / r) per axis (kComputeMinMax), as six
+// unsigned maxima that start at zero: mm[a] of the complement (so of the
+// minimum), mm[3 + a] of the value, both with the sign bit flipped.
+__device__ __forceinline__ unsigned bound_code(int c) { return (unsigned)c ^ 0x80000000u; }
+
+// One thread's bounds into mm: warp, block, one atomic per block and axis.
+__device__ __forceinline__ void reduce_bounds(const unsigned* lo, const unsigned* hi,
+                                              unsigned* mm) {
+  __shared__ unsigned smx[6][32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int a = 0; a < 3; a++) {
+    const unsigned u = __reduce_max_sync(0xffffffffu, lo[a]);
+    const unsigned v = __reduce_max_sync(0xffffffffu, hi[a]);
+    if (l == 0) { smx[a][w] = u; smx[3 + a][w] = v; }
+  }
+  __syncthreads();
+  if (w < 6) {
+    const unsigned u = __reduce_max_sync(0xffffffffu, l < nw ? smx[w][l] : 0u);
+    if (l == 0) atomicMax(mm + w, u);
+  }
+}
+__device__ __forceinline__ void add_bounds(float4 p, float r, unsigned* lo, unsigned* hi) {
+  const float c[3] = {p.x, p.y, p.z};
+  for (int a = 0; a < 3; a++) {
+    const unsigned u = bound_code((int)floorf(__fdiv_rn(c[a], r)));
+    lo[a] = max(lo[a], ~u);
+    hi[a] = max(hi[a], u);
   }
 }
 
-// kComputeMinMax: integer cell bounds of floor(p / r), block-reduced first
-__global__ void k_minmax(int64_t n, const float4* __restrict__ pf, float r, int* mm) {
-  __shared__ int smn[3][32], smx[3][32];
-  int mn[3] = {INT_MAX, INT_MAX, INT_MAX}, mx[3] = {INT_MIN, INT_MIN, INT_MIN};
-  // grid-stride over the particles: one block-reduced atomic per block
+// The float positions the search reads (x_h snapshot or the current ones) and
+// their cell bounds, in one pass.
+__global__ void __launch_bounds__(256) k_prep_bounds(int64_t n, const Fields F, int use_current,
+                                                     float4* __restrict__ pf, float r,
+                                                     unsigned* mm) {
+  unsigned lo[3] = {0u, 0u, 0u}, hi[3] = {0u, 0u, 0u};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const float4 p = pf[i];
-    const int c0 = (int)floorf(__fdiv_rn(p.x, r)), c1 = (int)floorf(__fdiv_rn(p.y, r)),
-              c2 = (int)floorf(__fdiv_rn(p.z, r));
-    mn[0] = min(mn[0], c0); mx[0] = max(mx[0], c0);
-    mn[1] = min(mn[1], c1); mx[1] = max(mx[1], c1);
-    mn[2] = min(mn[2], c2); mx[2] = max(mx[2], c2);
-  }
-  for (int a = 0; a < 3; a++) {
-    for (int o = 16; o > 0; o >>= 1) {
-      mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-      mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
+    float4 p;
+    if (use_current) {
+      const double4 x = F.xm[i];
+      p = make_float4(__double2float_rn(x.x), __double2float_rn(x.y), __double2float_rn(x.z), 0.f);
+    } else {
+      p = F.xh[i];
     }
+    pf[i] = p;
+    add_bounds(p, r, lo, hi);
   }
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0)
-    for (int a = 0; a < 3; a++) { smn[a][w] = mn[a]; smx[a][w] = mx[a]; }
-  __syncthreads();
-  if (w == 0) {
-    int nw = blockDim.x >> 5;
-    for (int a = 0; a < 3; a++) {
-      int v = l < nw ? smn[a][l] : INT_MAX, u = l < nw ? smx[a][l] : INT_MIN;
-      for (int o = 16; o > 0; o >>= 1) {
-        v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-        u = max(u, __shfl_xor_sync(0xffffffffu, u, o));
-      }
-      if (l == 0) { atomicMin(mm + a, v); atomicMax(mm + 3 + a, u); }
-    }
-  }
+  reduce_bounds(lo, hi, mm);
 }
 
+// The same for a caller's double3 array (wf_find_neighbors_static), which also
+// zeroes the cell counters; the last block to finish sizes the search grid
+// (grid_from_bounds) and notes whether it fits: the kernels behind it read it
+// from device memory, so the host waits once, at the end (with the cell sort
+// and the lists one warp per cell: 19,488 particles 192 -> 72 us a call, of
+// which the kernels take 48).
+__global__ void __launch_bounds__(256) k_static_prep(int64_t n, const double* __restrict__ x,
+                                                     float4* __restrict__ pf, float r,
+                                                     StaticHeader* __restrict__ hdr,
+                                                     uint32_t* __restrict__ count,
+                                                     int64_t max_cells) {
+  __shared__ bool last;
+  unsigned lo[3] = {0u, 0u, 0u}, hi[3] = {0u, 0u, 0u};
+  bool bad = false;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  for (int64_t i = i0; i < n; i += step) {
+    const double x0 = x[3 * i], x1 = x[3 * i + 1], x2 = x[3 * i + 2];
+    bad |= !isfinite(x0) || !isfinite(x1) || !isfinite(x2);
+    const float4 p =
+        make_float4(__double2float_rn(x0), __double2float_rn(x1), __double2float_rn(x2), 0.0f);
+    pf[i] = p;
+    add_bounds(p, r, lo, hi);
+  }
+  for (int64_t k = i0; k < max_cells; k += step) count[k] = 0u;
+  if (bad) atomicOr(&hdr->status, WF_STATUS_GRID);
+  reduce_bounds(lo, hi, hdr->mm);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&hdr->ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last || threadIdx.x != 0) return;
+  unsigned mm[6];
+  for (int k = 0; k < 6; k++) mm[k] = atomicMax(hdr->mm + k, 0u);
+  int64_t ncell = 0;
+  bool fits = !(atomicOr(&hdr->status, 0) & WF_STATUS_GRID);
+  int b[6];
+  bounds_from_codes(mm, b);
+  for (int a = 0; a < 3 && fits; a++) {
+    const int64_t span = (int64_t)b[3 + a] - (int64_t)b[a];
+    fits = span >= 0 && span + 5 <= max_cells;
+  }
+  if (fits) {
+    GridDev g;
+    grid_from_bounds(b, r, &g);
+    ncell = 1;
+    for (int a = 0; a < 3 && fits; a++) {
+      fits = g.dim[a] > 0 && g.dim[a] <= max_cells;
+      ncell *= g.dim[a];
+      fits = fits && ncell <= max_cells;
+    }
+    hdr->grid = g;
+  }
+  hdr->ncell = fits ? (int)ncell : 0;
+}
+
+// Each particle's cell and its rank of arrival there (the order inside a cell
+// is settled by k_cell_sort).  The grid comes from the host (g) or, with its
+// number of cells, from device memory (hdr).
 __global__ void k_cell_count(int64_t n, const float4* __restrict__ pf, GridDev g,
-                             uint32_t* __restrict__ cellid, uint32_t* __restrict__ count,
+                             const StaticHeader* __restrict__ hdr, uint32_t* __restrict__ cellid,
+                             uint32_t* __restrict__ rank, uint32_t* __restrict__ count,
                              int* status) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
+  if (hdr) {
+    if (hdr->ncell == 0) return;
+    g = hdr->grid;
+  }
   float4 p = pf[i];
   int cx = cell_coord(p.x, g.gmin[0], g.gdelta[0]);
   int cy = cell_coord(p.y, g.gmin[1], g.gdelta[1]);
@@ -91,7 +157,67 @@ __global__ void k_cell_count(int64_t n, const float4* __restrict__ pf, GridDev g
   }
   uint32_t c = ((uint32_t)cz * g.dim[1] + cy) * g.dim[0] + cx;
   cellid[i] = c;
-  atomicAdd(count + c, 1u);
+  rank[i] = atomicAdd(count + c, 1u);
+}
+
+// The block-local half of an exclusive scan over the cell counts (1,024 per
+// block, in place); the last block to finish scans the blocks' totals, so a
+// cell's offset is its local one plus bsum[cell / 1024] (k_cell_scatter adds
+// them).  bsum: blocks + 1 words, the last one a ticket that starts and ends
+// at zero.
+__global__ void __launch_bounds__(256) k_cell_scan(uint32_t* __restrict__ data, int64_t cells,
+                                                   const StaticHeader* __restrict__ hdr,
+                                                   uint32_t* __restrict__ bsum,
+                                                   uint32_t* __restrict__ ticket) {
+  __shared__ uint32_t warp_tot[8];
+  __shared__ bool last;
+  if (hdr) cells = hdr->ncell;
+  const int64_t blocks = (cells + 1023) / 1024;
+  if (blockIdx.x >= blocks) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // exclusive prefix of t over the block; *total on every thread
+  const auto scan = [&](uint32_t t, uint32_t* total) {
+    uint32_t incl = t;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    __syncthreads();
+    if (lane == 31) warp_tot[w] = incl;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+    for (int k = 0; k < 8; k++) {
+      if (k < w) before += warp_tot[k];
+      all += warp_tot[k];
+    }
+    *total = all;
+    return before + incl - t;
+  };
+  const int64_t base = (int64_t)blockIdx.x * 1024 + threadIdx.x * 4;
+  uint32_t v[4], total;
+  for (int k = 0; k < 4; k++) v[k] = base + k < cells ? data[base + k] : 0u;
+  uint32_t run = scan(v[0] + v[1] + v[2] + v[3], &total);
+  for (int k = 0; k < 4; k++) {
+    if (base + k < cells) data[base + k] = run;
+    run += v[k];
+  }
+  if (threadIdx.x == 0) {
+    bsum[blockIdx.x] = total;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == (uint32_t)blocks - 1u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  uint32_t carry = 0;
+  for (int64_t b0 = 0; b0 < blocks; b0 += 256) {
+    const int64_t b = b0 + threadIdx.x;
+    const uint32_t t = b < blocks ? *(volatile uint32_t*)(bsum + b) : 0u;
+    const uint32_t e = scan(t, &total);
+    if (b < blocks) bsum[b] = carry + e;
+    carry += total;
+  }
+  if (threadIdx.x == 0) *ticket = 0u;
 }
 
 // exclusive scan, 1024 elements per block (256 threads x 4)
@@ -134,55 +260,74 @@ __global__ void k_scan_add(uint32_t* data, int64_t n, const uint32_t* block_sums
     if (base + k < n) data[base + k] += add;
 }
 
-__global__ void k_cell_scatter(int64_t n, const uint32_t* __restrict__ cellid,
-                               const uint32_t* __restrict__ start, uint32_t* __restrict__ cursor,
-                               const int32_t* __restrict__ perm, int32_t* __restrict__ s_src,
+// Particles to their cells' ranges, and the cells' final offsets (start[ncell] = n).
+// orig: original ids (null: the index itself).
+__global__ void k_cell_scatter(int64_t n, int64_t cells, const StaticHeader* __restrict__ hdr,
+                               const uint32_t* __restrict__ cellid,
+                               const uint32_t* __restrict__ rank,
+                               const uint32_t* __restrict__ local,
+                               const uint32_t* __restrict__ bsum, uint32_t* __restrict__ start,
+                               const int32_t* __restrict__ orig, int32_t* __restrict__ s_src,
                                int32_t* __restrict__ s_orig) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t c = cellid[i];
-  uint32_t pos = start[c] + atomicAdd(cursor + c, 1u);
-  s_src[pos] = (int32_t)i;
-  s_orig[pos] = perm[i];
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (hdr) cells = hdr->ncell;
+  if (cells == 0) return;
+  if (i < n) {
+    const uint32_t c = cellid[i];
+    const uint32_t pos = local[c] + bsum[c >> 10] + rank[i];
+    s_src[pos] = (int32_t)i;
+    s_orig[pos] = orig ? orig[i] : (int32_t)i;
+  }
+  for (int64_t c = i; c < cells; c += (int64_t)gridDim.x * blockDim.x)
+    start[c] = local[c] + bsum[c >> 10];
+  if (i == 0) start[cells] = (uint32_t)n;
 }
 
 // Orders each cell's slots by original id, one warp per cell: original ids
 // are distinct, so an element's place is the number of smaller ids in its
 // cell (32 broadcast compares for a cell of at most 32; the cells hold ~14).
 // Every lane reads before any writes.  A larger cell is insertion-sorted by
-// one lane.
-__global__ void k_cell_sort(int64_t ncell, const uint32_t* __restrict__ start,
-                            int32_t* __restrict__ s_src, int32_t* __restrict__ s_orig) {
-  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+// one lane.  With pf2 not null the search positions follow into the order.
+__global__ void k_cell_sort(int64_t cells, const StaticHeader* __restrict__ hdr,
+                            const uint32_t* __restrict__ start, int32_t* s_src, int32_t* s_orig,
+                            const float4* __restrict__ pf, float4* __restrict__ pf2) {
   const int lane = threadIdx.x & 31;
-  if (c >= ncell) return;                      // whole warps leave together
-  const uint32_t b = start[c], e = start[c + 1];
-  const uint32_t m = e - b;
-  if (m <= 1u) return;
-  if (m <= 32u) {
-    const bool v = (uint32_t)lane < m;
-    const int32_t o = v ? s_orig[b + lane] : 0;
-    const int32_t sv = v ? s_src[b + lane] : 0;
-    uint32_t rank = 0;
-    for (uint32_t t = 0; t < m; t++) rank += __shfl_sync(0xffffffffu, o, (int)t) < o;
+  if (hdr) cells = hdr->ncell;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; c < cells; c += warps) {
+    const uint32_t b = start[c], e = start[c + 1];
+    const uint32_t m = e - b;
+    if (m == 0u) continue;
+    if (m <= 32u) {
+      const bool v = (uint32_t)lane < m;
+      const int32_t o = v ? s_orig[b + lane] : 0;
+      const int32_t sv = v ? s_src[b + lane] : 0;
+      uint32_t rank = 0;
+      for (uint32_t t = 0; t < m; t++) rank += __shfl_sync(0xffffffffu, o, (int)t) < o;
+      __syncwarp();
+      if (v) {
+        s_orig[b + rank] = o;
+        s_src[b + rank] = sv;
+        if (pf2) pf2[b + rank] = pf[sv];
+      }
+      continue;
+    }
+    if (lane == 0) {
+      for (uint32_t k = b + 1; k < e; k++) {
+        const int32_t ko = s_orig[k], ks = s_src[k];
+        uint32_t q = k;
+        while (q > b && s_orig[q - 1] > ko) {
+          s_orig[q] = s_orig[q - 1];
+          s_src[q] = s_src[q - 1];
+          q--;
+        }
+        s_orig[q] = ko;
+        s_src[q] = ks;
+      }
+    }
     __syncwarp();
-    if (v) {
-      s_orig[b + rank] = o;
-      s_src[b + rank] = sv;
-    }
-    return;
-  }
-  if (lane != 0) return;
-  for (uint32_t k = b + 1; k < e; k++) {
-    const int32_t ko = s_orig[k], ks = s_src[k];
-    uint32_t q = k;
-    while (q > b && s_orig[q - 1] > ko) {
-      s_orig[q] = s_orig[q - 1];
-      s_src[q] = s_src[q - 1];
-      q--;
-    }
-    s_orig[q] = ko;
-    s_src[q] = ks;
+    if (pf2)
+      for (uint32_t k = b + lane; k < e; k += 32) pf2[k] = pf[s_src[k]];
   }
 }
 
@@ -252,8 +397,10 @@ __global__ void k_reorder(int64_t n, const int32_t* __restrict__ s_src, const Fi
 constexpr int kNbWarps = 4;      // warps (cells in flight) per block
 // List entry index (nb_at) in the index type I: 32-bit when the lists hold
 // fewer than 2^31 entries (fewer than ~29M particles), else 64-bit.
-template <class I>
+// kRows: the caller's row-major lists instead (wf_find_neighbors_static).
+template <class I, bool kRows>
 __device__ __forceinline__ I nb_at_i(I npad, I i, int k) {
+  if constexpr (kRows) return i * (I)WF_NB + (I)k;
   return ((I)(k >> 3) * npad + i) * (I)WF_NB_BLK + (I)(k & 7);
 }
 constexpr int kNbStage = 192;    // staged candidates per warp and round
@@ -265,7 +412,7 @@ constexpr int kNbStage = 192;    // staged candidates per warp and round
 // below it, so the entries keep candidate order.  The counts advance once per
 // chunk (lane j keeps particle j's mask of the chunk), which leaves no chain
 // between the particles' iterations.
-template <class I>
+template <class I, bool kRows>
 __device__ __forceinline__ void nb_append_round(int nstaged, const float4* __restrict__ sp,
                                                 const int32_t* __restrict__ sid, int gn,
                                                 const float4* __restrict__ part, float r2,
@@ -290,16 +437,17 @@ __device__ __forceinline__ void nb_append_round(int nstaged, const float4* __res
       const bool acc = v && sq < r2 && sq > 0.0f;
       const unsigned m = __ballot_sync(0xffffffffu, acc);
       const int k = base + __popc(m & lt);
-      if (acc && k < WF_NB) nb[nb_at_i<I>((I)npad, (I)ij, k)] = qid;
+      if (acc && k < WF_NB) nb[nb_at_i<I, kRows>((I)npad, (I)ij, k)] = qid;
       mine = lane == j ? m : mine;
     }
     count += __popc(mine);
   }
 }
 
-template <class I>
+template <class I, bool kRows>
 __global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t npad,
                                                           const float4* __restrict__ pf, GridDev g,
+                                                          const StaticHeader* __restrict__ hdr,
                                                           const uint32_t* __restrict__ start,
                                                           const int32_t* __restrict__ slot_of,
                                                           int32_t* __restrict__ nb,
@@ -308,10 +456,14 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t
   __shared__ int32_t s_id[kNbWarps][kNbStage];
   __shared__ float4 s_part[kNbWarps][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t c = blockIdx.x * (int64_t)kNbWarps + w;
-  if (c >= ncell) return;                      // whole warps leave together
+  if constexpr (kRows) {                       // the grid is in device memory
+    ncell = hdr->ncell;
+    g = hdr->grid;
+  }
+  for (int64_t c = blockIdx.x * (int64_t)kNbWarps + w; c < ncell;
+       c += (int64_t)gridDim.x * kNbWarps) {   // whole warps together
   const uint32_t ps = start[c], pe = start[c + 1];
-  if (ps >= pe) return;
+  if (ps >= pe) continue;
   // cell coordinates in 32-bit arithmetic (the grid holds at most 2e9 cells;
   // a 64-bit division is a long software sequence in this issue-bound kernel)
   const uint32_t cu = (uint32_t)c, dx = (uint32_t)g.dim[0], dy = (uint32_t)g.dim[1];
@@ -366,7 +518,7 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t
       for (uint32_t t0 = 0; t0 < nr; t0 += 32) {
         if (nstaged > kNbStage - 32) {          // staging full: test what is staged
           __syncwarp();
-          nb_append_round<I>(nstaged, sp, sid, gn, s_part[w], r2, npad, nb, count);
+          nb_append_round<I, kRows>(nstaged, sp, sid, gn, s_part[w], r2, npad, nb, count);
           __syncwarp();
           nstaged = 0;
         }
@@ -393,24 +545,19 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t
       }
     }
     __syncwarp();
-    nb_append_round<I>(nstaged, sp, sid, gn, s_part[w], r2, npad, nb, count);
+    nb_append_round<I, kRows>(nstaged, sp, sid, gn, s_part[w], r2, npad, nb, count);
     __syncwarp();
     if (lane < gn) {
       if (count >= WF_NB) atomicOr(status, WF_STATUS_NB_CAP);
       const int cn = min(count, WF_NB);
       cnt[myslot] = cn;
       // pad the last block with the particle's own slot (see nb_at)
+      if constexpr (!kRows)
       for (int k = cn; k < ((cn + WF_NB_BLK - 1) & ~(WF_NB_BLK - 1)); k++)
         nb[nb_at(npad, myslot, k)] = myslot;
     }
   }
-}
-
-// the search positions in sorted order, for a rebuild that keeps the state in place
-__global__ void k_gather_pf(int64_t n, const int32_t* __restrict__ s_src,
-                            const float4* __restrict__ pf, float4* __restrict__ pf2) {
-  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k < n) pf2[k] = pf[s_src[k]];
+  }
 }
 
 __global__ void k_snapshot(int64_t n, Fields F) {
@@ -423,19 +570,6 @@ __global__ void k_snapshot(int64_t n, Fields F) {
 inline int nblocks(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
-
-// host-side grid set-up, computeCellInformation (cuNSearchDeviceData.cu:80-123)
-void grid_from_minmax(const int mm[6], float r, GridDev* g) {
-  for (int a = 0; a < 3; a++) {
-    float Min = (float)mm[a] * r, Max = (float)mm[3 + a] * r;
-    float gridSize = Max - Min;
-    g->dim[a] = (int)((unsigned)ceilf(gridSize / r) + 4u);
-    g->gmin[a] = Min - r * 2.0f;
-    float gs2 = (float)(unsigned)g->dim[a] * r;
-    g->gdelta[a] = (float)(unsigned)g->dim[a] / gs2;
-  }
-  g->r2 = r * r;
-}
 
 void device_exclusive_scan(uint32_t* data, int64_t n, uint32_t* tmp, cudaStream_t s) {
   int64_t nb = (n + 1023) / 1024;
@@ -457,25 +591,30 @@ int64_t scan_tmp_words(int64_t n) {
   return w + 1;
 }
 
-void launch_prep_positions(int64_t n, const Fields& F, int use_current, float4* pf,
-                           cudaStream_t s) {
-  k_prep_positions<<<nblocks(n, 256), 256, 0, s>>>(n, F, use_current, pf);
+int64_t cell_scan_words(int64_t cells) { return (cells + 1023) / 1024 + 1; }
+
+void launch_prep_bounds(int64_t n, const Fields& F, int use_current, float4* pf, float r,
+                        unsigned* mm, cudaStream_t s) {
+  cudaMemsetAsync(mm, 0, 6 * sizeof(unsigned), s);
+  k_prep_bounds<<<std::min(nblocks(n, 256), 1024), 256, 0, s>>>(n, F, use_current, pf, r, mm);
 }
-void launch_minmax(int64_t n, const float4* pf, float r, int* mm, cudaStream_t s) {
-  k_minmax<<<std::min(nblocks(n, 256), 1024), 256, 0, s>>>(n, pf, r, mm);
+void launch_static_prep(int64_t n, const double* x, float4* pf, float r, StaticHeader* hdr,
+                        uint32_t* count, int64_t max_cells, cudaStream_t s) {
+  cudaMemsetAsync(hdr, 0, sizeof(StaticHeader), s);
+  k_static_prep<<<std::min(nblocks(n, 256), 304), 256, 0, s>>>(n, x, pf, r, hdr, count, max_cells);
 }
-void launch_cell_count(int64_t n, const float4* pf, const GridDev& g, uint32_t* cellid,
-                       uint32_t* count, int* status, cudaStream_t s) {
-  k_cell_count<<<nblocks(n, 256), 256, 0, s>>>(n, pf, g, cellid, count, status);
-}
-void launch_cell_scatter(int64_t n, const uint32_t* cellid, const uint32_t* start,
-                         uint32_t* cursor, const int32_t* perm, int32_t* s_src, int32_t* s_orig,
-                         cudaStream_t s) {
-  k_cell_scatter<<<nblocks(n, 256), 256, 0, s>>>(n, cellid, start, cursor, perm, s_src, s_orig);
-}
-void launch_cell_sort(int64_t ncell, const uint32_t* start, int32_t* s_src, int32_t* s_orig,
-                      cudaStream_t s) {
-  k_cell_sort<<<nblocks(ncell * 32, 256), 256, 0, s>>>(ncell, start, s_src, s_orig);
+void launch_cell_sort(int64_t n, const float4* pf, const GridDev& g, const StaticHeader* hdr,
+                      const int32_t* orig, const CellWork& W, int32_t* s_src, int32_t* s_orig,
+                      float4* pf2, int* status, cudaStream_t s) {
+  // with the grid in device memory the launches are sized for the most cells
+  const int64_t cells = hdr ? W.max_cells : (int64_t)g.dim[0] * g.dim[1] * g.dim[2];
+  k_cell_count<<<nblocks(n, 256), 256, 0, s>>>(n, pf, g, hdr, W.cellid, W.rank, W.count, status);
+  k_cell_scan<<<nblocks(cells, 1024), 256, 0, s>>>(W.count, cells, hdr, W.bsum, W.ticket);
+  k_cell_scatter<<<nblocks(n, 256), 256, 0, s>>>(n, cells, hdr, W.cellid, W.rank, W.count, W.bsum,
+                                                 W.start, orig, s_src, s_orig);
+  const int blocks = nblocks(cells * 32, 256);
+  k_cell_sort<<<hdr ? std::min(blocks, 1216) : blocks, 256, 0, s>>>(cells, hdr, W.start, s_src,
+                                                                    s_orig, pf, pf2);
 }
 void launch_reorder(int64_t n, const int32_t* s_src, const Fields& A, const Fields& B,
                     const float4* pf, float4* pf2, int32_t* inv, cudaStream_t s) {
@@ -487,15 +626,17 @@ void launch_nblist(int64_t n, int64_t npad, const float4* pf, const GridDev& g,
   (void)n;
   const int64_t ncell = (int64_t)g.dim[0] * g.dim[1] * g.dim[2];
   if ((int64_t)WF_NB_ALLOC * npad < ((int64_t)1 << 31))
-    k_nblist<uint32_t><<<nblocks(ncell, kNbWarps), 32 * kNbWarps, 0, s>>>(
-        ncell, npad, pf, g, start, slot_of, nb, cnt, status);
+    k_nblist<uint32_t, false><<<nblocks(ncell, kNbWarps), 32 * kNbWarps, 0, s>>>(
+        ncell, npad, pf, g, nullptr, start, slot_of, nb, cnt, status);
   else
-    k_nblist<int64_t><<<nblocks(ncell, kNbWarps), 32 * kNbWarps, 0, s>>>(
-        ncell, npad, pf, g, start, slot_of, nb, cnt, status);
+    k_nblist<int64_t, false><<<nblocks(ncell, kNbWarps), 32 * kNbWarps, 0, s>>>(
+        ncell, npad, pf, g, nullptr, start, slot_of, nb, cnt, status);
 }
-void launch_gather_pf(int64_t n, const int32_t* s_src, const float4* pf, float4* pf2,
-                      cudaStream_t s) {
-  k_gather_pf<<<nblocks(n, 256), 256, 0, s>>>(n, s_src, pf, pf2);
+void launch_static_lists(const float4* pf, const StaticHeader* hdr, const uint32_t* start,
+                         const int32_t* order, int32_t* lists, int32_t* counts, int* status,
+                         cudaStream_t s) {
+  k_nblist<uint32_t, true><<<2432, 32 * kNbWarps, 0, s>>>(0, 0, pf, GridDev{}, hdr, start, order,
+                                                          lists, counts, status);
 }
 void launch_snapshot(int64_t n, const Fields& F, cudaStream_t s) {
   k_snapshot<<<nblocks(n, 256), 256, 0, s>>>(n, F);
