@@ -1,6 +1,7 @@
 """The FP64 passes' variants against the oracle, bit for bit: one lane per
-particle (domains that fill the GPU) and eight lanes (small ones), with the pair
-geometry kept between a step's passes and without."""
+particle (domains that fill the GPU) and 8, 16 or 32 lanes (small ones), with the
+pair geometry kept between a step's passes and without, and with values that keep
+pairs off the integer pipes."""
 import numpy as np
 import pytest
 
@@ -29,8 +30,8 @@ def _lattice(R, H, thermal):
     return sc, opts
 
 
-# ~700 and ~3,000 particles take eight lanes each (with a last warp that is not
-# full); ~24,500 take one lane, just above the line between the two at 24,000
+# ~700 particles take 32 lanes each, ~3,000 take 16, ~24,500 take eight (the last
+# warp is not full)
 @pytest.mark.parametrize("R,H", [(0.0024, 0.0045), (0.0041, 0.0073), (0.0079, 0.0156)])
 @pytest.mark.parametrize("thermal", [0, 1])
 @pytest.mark.parametrize("cache", [1, 0])
@@ -44,10 +45,45 @@ def test_fp64_passes_bit_exact_vs_oracle(R, H, thermal, cache):
         _same(g, o)
 
 
+# above and below the line between one and eight lanes at 64,000
+@pytest.mark.parametrize("R,H", [(0.0111, 0.0214), (0.0107, 0.0214)])
+def test_fp64_passes_bit_exact_at_the_one_lane_line(R, H):
+    sc, opts = _lattice(R, H, 1)
+    assert (sc["n"] >= 64000) == (R > 0.011) and abs(sc["n"] - 64000) < 6000
+    o = S.load(O.OracleDomain(sc["n"]), sc, opts)
+    g = S.load(Domain_d(sc["n"]), sc, opts)
+    o.step(5)
+    g.step(5)
+    _same(g, o)
+
+
+# (2^-120, 2^120 are the ends of the range in which a pair's arithmetic runs on
+# the integer pipes)
+@pytest.mark.parametrize("field,scale", [("v", 0.0), ("v", 2.0**-124), ("v", 2.0**-119),
+                                         ("m", 2.0**-125), ("T", 2.0**-122)])
+@pytest.mark.parametrize("R,H", [(0.0024, 0.0045), (0.0060, 0.0090)])
+def test_fp64_passes_bit_exact_outside_the_integer_range(field, scale, R, H):
+    sc, opts = _lattice(R, H, 1)
+    rng = np.random.default_rng(3)
+    some = rng.random(sc["n"]) < 0.5
+    sc["alpha"], sc["beta"] = 0.7, 0.4
+    val = rng.normal(0.0, 30.0, (sc["n"], 3)) if field == "v" else np.array(sc[field], dtype=float)
+    val[some] *= scale
+    o = S.load(O.OracleDomain(sc["n"]), sc, opts)
+    g = S.load(Domain_d(sc["n"]), sc, opts)
+    for d in (o, g):
+        d.set_field(field, val)
+    for k in (1, 3):
+        o.step(k)
+        g.step(k)
+        for f in FIELDS:
+            assert np.array_equal(g.get_field(f), o.get_field(f), equal_nan=True), f
+
+
 @pytest.mark.parametrize("cache", [1, 0])
-def test_fp64_contact_passes_bit_exact_with_one_lane(cache):
+def test_fp64_contact_passes_bit_exact_with_eight_lanes(cache):
     sc = S.contact_cylinder(R=0.0083, H=0.0160, dens=12, gap=-2.0e-6, mu=(0.1, 0.1))
-    assert sc["n"] > 24000
+    assert 5000 < sc["n"] < 64000
     o = S.load(O.OracleDomain(sc["n"]), sc)
     g = S.load(Domain_d(sc["n"]), sc, {"pair_cache": cache})
     o.step(8)

@@ -125,13 +125,11 @@ struct wf_domain {
   size_t work_bytes = 0;       // allocated
   size_t work_refused = 0;     // a size the device had no memory for
   bool pair_cache = true;      // option "pair_cache"
-  int rr_cur = 0;              // which of the two 1/rho arrays is current
   int* d_zone = nullptr;       // [0] a massive particle has a mesh's zone id, [1] slots near a tool
   bool zone_checked = false;   // d_zone[0] is of the current ids and masses
   bool maxdep_kept = false;    // h_maxdep is on its way from the last step (ev_maxdep)
   cudaEvent_t ev_maxdep = nullptr;
   bool geo_valid = false;      // gk, r2: of the current positions and lists
-  bool rr_valid = false;       // rr: of the current density
   int tile_cap_max = WF_TILE_HALO_MAX;   // option "tile_cap_max": largest halo staged
   int tile_cap = 0;            // halo capacity the current tiles were built for (0: none)
   int tile_hmax = 0;           // largest halo of the last build (read at the next rebuild)
@@ -531,8 +529,7 @@ static StepParams make_params(const wf_domain* d) {
   P.npad = d->npad;
   P.h = d->h;
   P.gkC = 1.0 / (d->h * d->h * d->h * d->h * WF_PI);   // Functions.cu:83 with h_ = h
-  P.invh = 1.0 / d->h;
-  P.h_known = d->h > 1.0e-100 && d->h < 1.0e100;
+  P.h_tame = d->h > 1.0e-36 && d->h < 1.0e36 && P.gkC > 1.0e-36 && P.gkC < 1.0e36;
   P.dt = d->dt;
   P.Cs = d->Cs;
   P.G = d->G;
@@ -749,7 +746,7 @@ static bool work_reserve(wf_domain* d, size_t bytes) {
     cudaStreamSynchronize(d->stream);   // the passes that still read it
     cudaFree(d->work);
     d->work = nullptr;
-    d->geo_valid = d->rr_valid = false;
+    d->geo_valid = false;
   }
   if (cudaMalloc((void**)&d->work, bytes) != cudaSuccess) {
     cudaGetLastError();
@@ -761,12 +758,12 @@ static bool work_reserve(wf_domain* d, size_t bytes) {
   return true;
 }
 static size_t work64_bytes(const wf_domain* d) {
-  return sizeof(double) * (size_t)(2 * WF_NB_ALLOC + 9) * (size_t)d->npad;
+  return sizeof(double) * (size_t)(2 * WF_NB_ALLOC + 8) * (size_t)d->npad;
 }
 // Kept values are of this call's own steps only: anything may have changed
 // between two calls and in the step hook.
 static void kept_drop(wf_domain* d) {
-  d->geo_valid = d->rr_valid = false;
+  d->geo_valid = false;
   d->zone_checked = d->maxdep_kept = false;
 }
 static Work64 work64_of(const wf_domain* d) {
@@ -776,11 +773,9 @@ static Work64 work64_of(const wf_domain* d) {
   W.gk = reinterpret_cast<double*>(d->work);
   W.r2 = W.gk + e;
   W.mr = W.r2 + e;
-  W.rr = W.mr + n + d->rr_cur * n;
-  W.rr_out = W.mr + n + (1 - d->rr_cur) * n;
-  W.sa6 = W.mr + 3 * n;
+  W.sa6 = W.mr + n;
+  W.tame = reinterpret_cast<uint8_t*>(W.mr + 7 * n);
   W.geo = d->geo_valid;
-  W.recip = d->rr_valid;
   return W;
 }
 
@@ -792,7 +787,7 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
     if (rc) return rc;
   }
   KTimer t(d, KID_REBUILD);
-  d->geo_valid = d->rr_valid = false;
+  d->geo_valid = false;
   const int64_t n = d->n;
   cudaStream_t s = d->stream;
   Fields& A = d->F[d->cur];
@@ -1212,8 +1207,6 @@ static int solve_step_launches(wf_domain* d) {
     { KTimer t(d, KID_STRESS);                                                      // :204-218
       d->launches += launch_fp64_stress(P, F, W, d->vd2, N, d->d_status, s) - 1; }
     { KTimer t(d, KID_ACCEL); launch_fp64_accel(P, F, W, d->vd2, N, s); }            // :221
-    d->rr_cur ^= 1;
-    d->rr_valid = W.gk != nullptr;
   } else {
     {
       KTimer t(d, KID_DENSITY);
@@ -1945,7 +1938,7 @@ int wf_thermal_solve(wf_domain* d, double tf) {
   const int64_t entries = (int64_t)WF_NB_ALLOC * d->npad, n = d->npad;
   const bool kept = d->time < tf &&
                     work_reserve(d, mixed ? (size_t)(4 * entries + 16 * n)
-                                          : sizeof(double) * (size_t)(3 * entries + 5 * n));
+                                          : sizeof(double) * (size_t)(2 * entries + 5 * n));
   HeatWork64 H64{};
   HeatWork32 H32{};
   if (kept && mixed) {
@@ -1955,8 +1948,8 @@ int wf_thermal_solve(wf_domain* d, double tf) {
     d->launches += 1;
   } else if (kept) {
     double* w = reinterpret_cast<double*>(d->work);
-    H64.dot = w; H64.r2 = w + entries; H64.ir2 = w + 2 * entries;
-    w += 3 * entries;
+    H64.dot = w; H64.r2 = w + entries;
+    w += 2 * entries;
     H64.mr = w; H64.scale = w + n; H64.icp = w + 2 * n; H64.conv = w + 3 * n; H64.fric = w + 4 * n;
     launch_heat_pairs64(P, CF(d), H64, N, d->stream);
     d->launches += 1;

@@ -198,8 +198,7 @@ struct StepParams {
   int64_t n_solid;      // original ids below this are solid (solid_part_count)
   int64_t npad;         // slot stride of the neighbour-list blocks (nb_at)
   double h, gkC;        // smoothing length (uniform) and 1/(h^4 pi)
-  double invh;          // 1/h rounded to nearest (FP64 form's division by h)
-  int h_known;          // h is far enough inside the range for that division
+  int h_tame;           // h and 1/(h^4 pi) are within 2^+-120 (products on the integer pipe)
   double dt;
   double Cs, G, rho0;   // uniform sound speed, shear modulus, reference density
   double alpha, beta;   // Monaghan artificial viscosity
@@ -396,17 +395,15 @@ struct Work64 {
   double* gk;        // per list entry (nb_at): kernel factor GK
   double* r2;        // per list entry: r_ij^2
   double* mr;        // m / rho of the step's new density
-  double* rr;        // 1 / rho of the density the step starts from
-  double* rr_out;    // 1 / rho of the new density, rr of the next step
   double* sa6;       // sigma / rho^2, 6 per slot
+  uint8_t* tame;     // per slot: sa6 is zero or in the middle of the range (wf_step_fp64.cu)
   double* mr_heat;   // m / rho as the heat pass needs it (mr behind a step; null: divide)
   int geo;           // gk and r2 hold the current positions' and lists' values
-  int recip;         // rr holds the current density's reciprocals
 };
 // What a heat solve keeps for its steps (ThermalSolve: positions, densities
 // and lists are fixed inside one solve).
 struct HeatWork64 {
-  double *dot, *r2, *ir2;            // per list entry: x_ij . grad W, r^2, 1 / r^2
+  double *dot, *r2;                  // per list entry: x_ij . grad W, r^2
   double *mr, *scale, *icp, *conv, *fric;   // per slot: m/rho, 1/(rho cp), 1/cp, h_conv dS^2,
                                             // frictional heat rate
 };

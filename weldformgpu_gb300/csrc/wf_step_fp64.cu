@@ -5,19 +5,25 @@
 // the same neighbour order the sums are bit-identical to the CPU oracle.
 // Each kernel states the reference kernel(s) it replaces.
 //
-// What bounds these passes is the FP64 pipe (2 operations per clock and SM,
+// What bounded these passes is the FP64 pipe (2 operations per clock and SM,
 // 1/64 of the FP32 rate): ncu showed it 86-87 % busy in every pair pass at
-// 170k particles with 72 / 113 / 133 / 90 FP64 instructions a pair (density,
-// stress, acceleration, heat).  Memory is nearly idle there, so whatever can be
-// computed once and read back is:
-//   - the kernel factor GK and r^2 of each pair (a square root, a division by
-//     h, a division by q h: about half of a density pass) by the first pass
-//     that sees the positions, kept in two arrays of the lists' layout for the
-//     other passes of the step (Work64);
-//   - m / rho, 1 / rho and sigma / rho^2 once per particle instead of a
-//     division per pair; the remaining rho_i / rho_j divides by a number whose
-//     reciprocal is known (div_known).
-// Every value is rounded exactly as where it was computed per pair.
+// 170k particles, with 72 / 113 / 133 / 90 FP64 instructions a pair (density,
+// stress, acceleration, heat), and memory and the integer pipes nearly idle.
+// So
+//   - whatever can be computed once is read back: the kernel factor GK and r^2
+//     of each pair by the first pass that sees the positions, kept in two
+//     arrays of the lists' layout for the other passes of the step (Work64);
+//     m / rho and sigma / rho^2 once per particle;
+//   - products, quotients and square roots run on the integer pipes (mul_int,
+//     div_int, sqrt_int below), additions on the FP64 pipe.
+// 9 / 21 / 28 / 11 FP64 instructions a pair are left.  Times at 170k, in us,
+// all on the FP64 pipe with nothing kept -> with the kept values -> now:
+// density 1,066 -> 540 -> 247, stress 1,737 -> 1,070 -> 604, acceleration
+// 2,178 -> 1,358 -> 683, heat 1,367 -> 1,354 -> 394 (it computes the geometry
+// that the next step's density pass reads).  Stress and acceleration keep the
+// FP64 pipe 78-80 % busy and the integer ALUs 42-45 %; density and heat the
+// ALUs 61-67 % and FP64 43-71 %.
+// Every value is rounded exactly as where it was computed on the FP64 pipe.
 #include "wf_common.cuh"
 #include "wf_heat.cuh"
 #include "wf_mlp.cuh"
@@ -25,20 +31,147 @@
 
 namespace {
 
-// a / b, correctly rounded, from y = 1 / b correctly rounded: one
-// multiplication and two fused multiply-adds (Brisebarre, Muller and Raina,
-// "Accelerating correctly rounded floating-point division when the divisor is
-// known in advance", IEEE Trans. Computers 53(8), 2004; the last step is
-// Markstein's).  Needs a, b and a / b well inside the normal range.
-__device__ __forceinline__ double div_known(double a, double b, double y) {
-  const double q = __dmul_rn(a, y);
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
+// |x| in [2^-kE, 2^kE], from the exponent bits (a comparison of doubles would
+// run on the FP64 pipe); within: that, or zero
+template <unsigned kE>
+__device__ __forceinline__ bool in_range(double x) {
+  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - (1023u - kE) <= 2u * kE;
 }
-// |x| in [2^-400, 2^400], from the exponent bits (a comparison of doubles
-// would run on the FP64 pipe)
-__device__ __forceinline__ bool mid_range(double x) {
-  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 623u <= 800u;
+template <unsigned kE>
+__device__ __forceinline__ bool within(double x) {
+  return in_range<kE>(x) || (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
 }
+
+// ---- arithmetic on the integer pipes ------------------------------------------
+// A warp's FP64 addition or multiplication takes ~19 cycles of an SM, a
+// division ~140 and a square root ~140 (measured, 1.92 GHz); in 32-bit integer
+// operations a product takes 12, a quotient 17 (known divisor) to 21 and a
+// root 23, on pipes that are otherwise idle here and beside FP64 additions
+// nearly for free.  The results are the same bits: 1.2e9 random and adversarial
+// operands (ties, neighbours of quotients and squares) against the FP64 pipe.
+//
+// a b rounded to nearest even: the 53-bit significands' 106-bit product (one of
+// them shifted up by 11, so that the upper 64 bits hold the 52 or 53 result
+// bits), normalised by one bit, rounded by a carry out of the bits below, the
+// exponents and signs added as one word.  For operands that are zero (a zero
+// result is +0) or whose exponents keep the product inside the normal range.
+__device__ __forceinline__ double mul_int(double a, double b) {
+  const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+  const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
+  const unsigned ua = (ah & 0xfffffu) | 0x100000u, ub = (bh & 0xfffffu) | 0x100000u;
+  const unsigned xh = __funnelshift_l(al, ua, 11), xl = al << 11;
+  const uint64_t p = (uint64_t)xl * bl;
+  const uint64_t t = (uint64_t)xh * bl + (p >> 32);
+  const uint64_t u = (uint64_t)xl * ub + (uint32_t)t;
+  const uint64_t v = (uint64_t)xh * ub + (t >> 32) + (u >> 32);
+  const unsigned w0 = (unsigned)p, w1 = (unsigned)u, w2 = (unsigned)v, w3 = (unsigned)(v >> 32);
+  const unsigned k = w3 < 0x100000u ? 1u : 0u;          // 52 bits: shift up by one
+  const unsigned mh = __funnelshift_l(w2, w3, k), ml = __funnelshift_l(w1, w2, k);
+  const unsigned r1 = __funnelshift_l(w0, w1, k), r0 = w0 << k;
+  const unsigned e = (ah & 0xfff00000u) + (bh & 0xfff00000u) - 0x3ff00000u - (k << 20);
+  // up: the bits below (r1, r0) are over a half, or a half with an odd result:
+  // r1 + 0x7fffffff + (r0 != 0 or odd) carries; the carry runs into the exponent
+  unsigned lo, hi;
+  asm("{\n\t.reg .u32 d;\n\t"
+      "add.cc.u32 d, %2, 0xffffffff;\n\taddc.cc.u32 d, %3, 0x7fffffff;\n\t"
+      "addc.cc.u32 %0, %4, 0;\n\taddc.u32 %1, %5, %6;\n\t}"
+      : "=r"(lo), "=r"(hi)
+      : "r"((ml & 1u) | r0), "r"(r1), "r"(ml), "r"(mh), "r"(e));
+  const bool zero = (ah << 1) == 0u || (bh << 1) == 0u;
+  return __hiloint2double(zero ? 0 : (int)hi, zero ? 0 : (int)lo);
+}
+
+// The significand of a normal number with its hidden bit, and its 24 upper
+// bits as a float of [1, 2)
+__device__ __forceinline__ uint64_t whole_bits(double x) {
+  return (uint64_t)(((unsigned)__double2hiint(x) & 0xfffffu) | 0x100000u) << 32 |
+         (unsigned)__double2loint(x);
+}
+__device__ __forceinline__ unsigned lead_bits(double x) {
+  return (__funnelshift_l((unsigned)__double2loint(x), (unsigned)__double2hiint(x), 3) &
+          0x7fffffu) | 0x3f800000u;
+}
+__device__ __forceinline__ unsigned word(uint64_t v, int shift) {   // bits shift .. shift + 31
+  return __funnelshift_r((unsigned)v, (unsigned)(v >> 32), shift);
+}
+// 2^32 y of a float approximation 0.5 < y <= 1, from below: y (1 - 2^-21) + 1
+// has its bits in the fraction field
+__device__ __forceinline__ unsigned seed(float y) {
+  return __float_as_uint(__fmaf_rn(y, 1.0f - 4.76837158203125e-7f, 1.0f)) << 9;
+}
+
+// a / b rounded to nearest even by long division with digits of 31 and 23
+// bits (Knuth, The Art of Computer Programming 2, 4.3.1): the reciprocal of b
+// to 29 bits from the float one and a Newton step, always from below, so a
+// digit is at most a few units low; the next remainder takes them up, the last
+// one decides the last bit.  q = N 2^-53 is then floored and N + 1 >> 1 is the
+// rounded significand (a quotient of 53-bit numbers never lies in the middle).
+// Operands as for mul_int, b not zero.
+__device__ __forceinline__ double div_int(double a, double b) {
+  const unsigned ah = (unsigned)__double2hiint(a), bh = (unsigned)__double2hiint(b);
+  const uint64_t B = whole_bits(b);
+  uint64_t A = whole_bits(a);
+  const unsigned c = A < B ? 1u : 0u;
+  A <<= c;                                              // A / B in [1, 2)
+  float y0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(__uint_as_float(lead_bits(b))));
+  const unsigned Y = seed(y0);
+  const unsigned y = Y + __umulhi(Y, 0u - 2u * __umulhi(Y, word(B, 21)) - 4u);
+  const unsigned q1 = __umulhi(word(A, 22), y);         // at most 5 low
+  const uint64_t R = (A << 30) - (uint64_t)q1 * B;
+  const unsigned q2 = __umulhi(word(R, 24), y) >> 5;    // at most 1 low
+  const uint64_t R2 = (R << 23) - (uint64_t)q2 * B;
+  const uint64_t M = (((uint64_t)q1 << 23) + q2 + (R2 >= B ? 2u : 1u)) >> 1;
+  const unsigned e = (ah & 0xfff00000u) - (bh & 0xfff00000u) + 0x3fe00000u - (c << 20);
+  const bool zero = (ah << 1) == 0u;
+  return __hiloint2double(zero ? 0 : (int)((unsigned)(M >> 32) + e), zero ? 0 : (int)(unsigned)M);
+}
+
+// sqrt(x) rounded to nearest even, digit by digit the same way (x = 0 or
+// normal): s1 of 31 bits from x / sqrt(x), the rest from the remainder over
+// 2 s1, and N^2 <= x < (N + 1)^2 settled with the last remainder.
+__device__ __forceinline__ double sqrt_int(double x) {
+  const unsigned xh = (unsigned)__double2hiint(x);
+  const unsigned odd = ~(xh >> 20) & 1u;                // of the unbiased exponent
+  const uint64_t X = whole_bits(x) << odd;             // [1, 4) 2^52
+  float y0;
+  asm("rsqrt.approx.ftz.f32 %0, %1;"
+      : "=f"(y0) : "f"(__uint_as_float(lead_bits(x) + (odd << 23))));
+  const unsigned Y = seed(y0), x32 = word(X, 22);
+  const unsigned y =
+      Y + __umulhi(Y, 0x80000000u - 6u - 2u * __umulhi(__umulhi(Y, Y), x32));
+  const unsigned s1 = __umulhi(x32, y);                 // at most 6 low
+  const uint64_t R = (X << 8) - (uint64_t)s1 * s1;
+  const int s2 = (int)(__umulhi(word(R, 3), y) - 8u) >> 5;   // at most 1 low, may be -1
+  const uint64_t K = ((uint64_t)s1 << 24) + (uint64_t)(int64_t)s2;
+  const uint64_t R2 = ((uint64_t)((unsigned)R << 14) << 32) - K * (uint64_t)(int64_t)s2;
+  const uint64_t N = ((uint64_t)s1 << 23) + (uint64_t)(int64_t)s2;
+  const uint64_t M = (N + (R2 > 2 * N ? 2u : 1u)) >> 1;
+  const unsigned e = ((((xh >> 20) + 1023u) >> 1) - 1u) << 20;
+  return __hiloint2double(xh == 0u ? 0 : (int)((unsigned)(M >> 32) + e),
+                          xh == 0u ? 0 : (int)(unsigned)M);
+}
+
+// Both forms of the pair terms: kInt on the integer pipes, else on the FP64 pipe.
+template <bool kInt>
+__device__ __forceinline__ double mul(double a, double b) {
+  if constexpr (kInt) return mul_int(a, b);
+  return a * b;
+}
+template <bool kInt>
+__device__ __forceinline__ double quot(double a, double b) {
+  if constexpr (kInt) return div_int(a, b);
+  return a / b;
+}
+template <bool kInt>
+__device__ __forceinline__ double root(double x) {
+  if constexpr (kInt) return sqrt_int(x);
+  return sqrt(x);
+}
+// A pair takes the integer form if it is tame: its loaded values are zero or
+// within 2^+-kTame, so that every product and quotient of the pair, and every
+// remainder of a sum in it, stays normal.  Any other pair takes the FP64 pipe.
+constexpr unsigned kTame = 120;
 // -0.5 x and 2 x: exact, so only the sign and exponent bits change (zeros,
 // subnormals and the ends of the range take the multiplication)
 __device__ __forceinline__ double neg_half(double x) {
@@ -58,53 +191,74 @@ __device__ __forceinline__ double twice(double x) {
 // shared by its two branches (so a warp whose lanes fall on both sides of
 // q = 1 divides once) and the comparisons on the bits of q >= 0.  q >= 2,
 // infinite or NaN gives 0.
+template <bool kInt>
 __device__ __forceinline__ double spline64(double q, double h, double C) {
   const unsigned hi = (unsigned)__double2hiint(q);
   if (hi >= 0x40000000u) return 0.0;
   if ((hi | (unsigned)__double2loint(q)) == 0u) return C / h * (-3.0 + (9.0 / 2.0) * q);
   const bool in = hi < 0x3ff00000u;
   const double s = in ? q : 2.0 - q;
-  const double c = ((in ? 9.0 / 4.0 : -3.0 / 4.0) * s) * s;
-  return C / (q * h) * (in ? -3.0 * q + c : c);
+  const double c = mul<kInt>(mul<kInt>(in ? 9.0 / 4.0 : -3.0 / 4.0, s), s);
+  const double d = in ? mul<kInt>(-3.0, q) + c : c;
+  return mul<kInt>(quot<kInt>(C, mul<kInt>(q, h)), d);
 }
 
 // GK and RN(r r) of a pair from x_i - x_j
+// (kIntSquares: with one lane the integer ALUs bound the passes that compute
+// it, 67 % busy, and four of its products are better on the FP64 pipe: heat
+// pass at 170k 427 -> 395 us; with eight lanes the other way, 114 -> 106 at
+// 37k.)
+template <bool kInt, bool kIntSquares = kInt>
 __device__ __forceinline__ void pair_geometry(const StepParams& P, double xx, double xy, double xz,
                                               double& GK, double& r2) {
-  const double rij = sqrt(xx * xx + xy * xy + xz * xz);
-  GK = spline64(P.h_known ? div_known(rij, P.h, P.invh) : rij / P.h, P.h, P.gkC);
-  r2 = rij * rij;
+  const double rij = root<kInt>(mul<kIntSquares>(xx, xx) + mul<kIntSquares>(xy, xy) +
+                               mul<kIntSquares>(xz, xz));
+  GK = spline64<kInt>(quot<kInt>(rij, P.h), P.h, P.gkC);
+  r2 = mul<kIntSquares>(rij, rij);
 }
 
 // Where the pair geometry of a pass comes from: computed (the work arrays
 // could not be allocated), computed and kept for the passes behind it, or read.
 enum { GEO_NONE = 0, GEO_STORE = 1, GEO_LOAD = 2 };
 
-template <int kGeo>
-__device__ __forceinline__ void geometry(const StepParams& P, const Work64& W, int64_t e, double xx,
-                                         double xy, double xz, double& GK, double& r2) {
+// GK is never positive, so the sign bit of a kept GK is free to say that the
+// pair is tame: its position difference, GK and the neighbour's mass are zero
+// or within 2^+-kTame (cleared: not, or GK = 0).
+template <int kG, int kGeo>
+__device__ __forceinline__ bool geometry(const StepParams& P, const Work64& W, int64_t e, double xx,
+                                         double xy, double xz, double mj, double& GK, double& r2) {
   if constexpr (kGeo == GEO_LOAD) {
-    GK = __ldg(W.gk + e);
+    const double k = __ldg(W.gk + e);
     r2 = __ldg(W.r2 + e);
+    GK = __hiloint2double(__double2hiint(k) | (int)0x80000000, __double2loint(k));
+    return __double2hiint(k) < 0;
   } else {
-    pair_geometry(P, xx, xy, xz, GK, r2);
+    bool tame = P.h_tame && within<kTame>(xx) && within<kTame>(xy) && within<kTame>(xz) &&
+                within<kTame>(mj);
+    if (kGeo != GEO_NONE && tame) pair_geometry<true, kG != 1>(P, xx, xy, xz, GK, r2);
+    else pair_geometry<false>(P, xx, xy, xz, GK, r2);
+    tame = tame && in_range<kTame>(GK) && in_range<2 * kTame>(r2);
     if constexpr (kGeo == GEO_STORE) {
-      W.gk[e] = GK;
+      W.gk[e] = tame ? GK : fabs(GK);
       W.r2[e] = r2;
     }
+    return tame;
   }
 }
 
 // ---- lanes of a particle ---------------------------------------------------
-// kG = 1: one thread per particle walks its list.  kG = 8: eight lanes per
-// particle, lane g takes entry 8 b + g of list block b (one coalesced read of
-// the block's indices and geometry), and the block's terms are added in list
-// order, term by term, so the sums round as in the walk.  Eight lanes spread a
-// small domain over the chip (540 particles are 5 blocks of 128 threads, 135
-// warps with eight lanes each) and shorten the chain of dependent pairs; the
-// ordered sums cost up to 8 additions per list block and accumulator set, so
-// a domain that fills the SMs is faster with one lane.
-constexpr int kLanes64 = 8;
+// kG = 1: one thread per particle walks its list.  kG = 8, 16 or 32: so many
+// lanes per particle, lane g takes entry kG b + g in round b (one coalesced
+// read of the round's indices and geometry), and the round's terms are added
+// in list order, term by term, so the sums round as in the walk.  More lanes
+// spread a small domain over the chip (800 particles: 13 blocks of 64 threads,
+// 800 of a warp) and shorten the chain of dependent loads and pairs, 27-57
+// deep in the walk and one or two rounds with a warp; the ordered sums use
+// fewer lanes for the more additions (8 lanes: up to 8 a round and accumulator
+// set).  Step with the heat pass, us, with 32 / 16 / 8 / 1 lanes: n = 800 74 /
+// 87 / 111 / -, 2,184 99 / 97 / 111 / -, 3,328 127 / 110 / 121 / -, 6,320 201
+// / 157 / 144 / -, 36,720 - / - / 528 / 584, 86,592 - / - / 1,174 / 1,150:
+// the lines of lanes64.
 
 // this thread's slot, lane and list length; threads past the end or without a
 // list keep c = 0 and stay for the warp's shuffles
@@ -114,33 +268,56 @@ __device__ __forceinline__ int64_t slot64(int& g) {
   g = (int)(t & (kG - 1));
   return t / kG;
 }
-// list blocks the warp walks together (eight lanes per particle)
-__device__ __forceinline__ int warp_blocks(int c) {
-  return (__reduce_max_sync(0xffffffffu, c) + WF_NB_BLK - 1) / WF_NB_BLK;
+// rounds of kG entries that the warp walks together
+template <int kG>
+__device__ __forceinline__ int warp_rounds(int c) {
+  return (__reduce_max_sync(0xffffffffu, c) + kG - 1) / kG;
 }
-// acc + t_0 + ... + t_7 over the lanes of a group, in lane order, on every lane
-__device__ __forceinline__ double add_in_order(double acc, double t) {
+// acc + t_0 + ... over the lanes of a group, in lane order: on every lane of
+// eight; of a warp, on lane 0, through shared memory (32 doubles).  m: terms
+// of the round (a warp's are all its own particle's)
+template <int kG>
+__device__ __forceinline__ double add_in_order(double* sh, double acc, double t, int m) {
+  if constexpr (kG == 32) {
+    const int lane = threadIdx.x & 31;
+    sh[lane] = t;
+    __syncwarp();
+    if (lane == 0)
 #pragma unroll
-  for (int k = 0; k < kLanes64; k++) acc += __shfl_sync(0xffffffffu, t, k, kLanes64);
+      for (int b = 0; b < kG; b += 8) {
+        if (b >= m) break;
+#pragma unroll
+        for (int k = 0; k < 8; k++) acc += sh[b + k];
+      }
+    __syncwarp();
+  } else {
+#pragma unroll
+    for (int k = 0; k < kG; k++) acc += __shfl_sync(0xffffffffu, t, k, kG);
+  }
   return acc;
 }
 // The same for kA accumulators through shared memory (32 rows of kA doubles,
 // kA odd: no bank conflicts): lane a of the group adds accumulator a, lane
-// a - 8 accumulator a >= 8.
-template <int kA>
-__device__ __forceinline__ void add_in_order(double* sh, const double* t, int g, double* acc) {
-  static_assert(kA % 2 == 1 && kA <= 2 * kLanes64, "accumulators of a group");
+// a - kG accumulator a >= kG.
+template <int kG, int kA>
+__device__ __forceinline__ void add_in_order(double* sh, const double* t, int g, double* acc,
+                                             int m) {
+  static_assert(kA % 2 == 1 && kA <= 2 * kG, "accumulators of a group");
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int a = 0; a < kA; a++) sh[lane * kA + a] = t[a];
   __syncwarp();
   const double* row = sh + (lane - g) * kA;
-  if (g < kA)
 #pragma unroll
-    for (int k = 0; k < kLanes64; k++) acc[0] += row[k * kA + g];
-  if (kA > kLanes64 && g < kA - kLanes64)
+  for (int b = 0; b < kG; b += 8) {
+    if (kG == 32 && b >= m) break;
+    if (g < kA)
 #pragma unroll
-    for (int k = 0; k < kLanes64; k++) acc[1] += row[k * kA + g + kLanes64];
+      for (int k = 0; k < 8; k++) acc[0] += row[(b + k) * kA + g];
+    if (kA > kG && g < kA - kG)
+#pragma unroll
+      for (int k = 0; k < 8; k++) acc[1] += row[(b + k) * kA + g + kG];
+  }
   __syncwarp();
 }
 
@@ -148,28 +325,35 @@ __device__ __forceinline__ void add_in_order(double* sh, const double* t, int g,
 // src/cuda/InteractionAlt.cu:166-246, src/cuda/Mechanical.cu:198-203.
 // Writes vd2 = (v, rho + dt*drho): the density the later passes of the step
 // read, next to the velocity so one 32-byte load serves both; with the work
-// arrays also m / rho and 1 / rho of the new density.
-template <int kGeo>
+// arrays also m / rho of the new density.
+template <bool kInt>
+__device__ __forceinline__ double density_sum(double xx, double xy, double xz, double GK, double vx,
+                                              double vy, double vz, double mj, double di,
+                                              double dj) {
+  const double temp1 = mul<kInt>(vx, mul<kInt>(xx, GK)) + mul<kInt>(vy, mul<kInt>(xy, GK)) +
+                       mul<kInt>(vz, mul<kInt>(xz, GK));
+  return mul<kInt>(mul<kInt>(mj, quot<kInt>(di, dj)), temp1);
+}
+template <int kG, int kGeo>
 __device__ __forceinline__ double density_term(const StepParams& P, const Fields& F,
                                                const Work64& W, int64_t e, int j, const double4& xi,
-                                               const double4& vi, bool known_i, bool pass) {
+                                               const double4& vi, bool pass) {
   const double4 xj = F.xm[j];
   const double xx = xi.x - xj.x, xy = xi.y - xj.y, xz = xi.z - xj.z;
+  const double mj = xj.w;
   double GK, r2;
-  geometry<kGeo>(P, W, e, xx, xy, xz, GK, r2);   // kept for the other passes whatever the filter
+  // kept for the other passes whatever the filter
+  const bool tame = geometry<kG, kGeo>(P, W, e, xx, xy, xz, mj, GK, r2);
   if (!pass) return 0.0;
   const double4 vj = F.vd[j];
-  const double di = vi.w, dj = vj.w, mj = xj.w;
+  const double di = vi.w, dj = vj.w;
   const double vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
-  const double temp1 = vx * (xx * GK) + vy * (xy * GK) + vz * (xz * GK);
-  double ratio;
-  if (kGeo != GEO_NONE && known_i) {
-    const double y = __ldg(W.rr + j);
-    ratio = mid_range(y) ? div_known(di, dj, y) : di / dj;
-  } else {
-    ratio = di / dj;
+  if constexpr (kGeo != GEO_NONE) {
+    if (tame && within<kTame>(vx) && within<kTame>(vy) && within<kTame>(vz) &&
+        in_range<kTame>(di) && in_range<kTame>(dj))
+      return density_sum<true>(xx, xy, xz, GK, vx, vy, vz, mj, di, dj);
   }
-  return mj * ratio * temp1;
+  return density_sum<false>(xx, xy, xz, GK, vx, vy, vz, mj, di, dj);
 }
 
 template <int kG, int kGeo>
@@ -177,6 +361,7 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_density64(StepParams P, F
                                                    double4* __restrict__ vd2,
                                                    const int32_t* __restrict__ nb,
                                                    const int32_t* __restrict__ cnt) {
+  __shared__ double sh[kG == 32 ? 32 : 1];
   int g;
   const int64_t i0 = slot64<kG>(g);
   if (kG == 1 && i0 >= P.n) return;
@@ -187,27 +372,26 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_density64(StepParams P, F
   const bool solid = valid && F.perm[i] < P.n_solid;
   const int32_t idi = F.id[i];
   const int c = solid ? cnt[i] : 0;
-  const bool known_i = W.recip && mid_range(vi.w);
   double drho = 0.0;
   if constexpr (kG == 1) {
     for (int k = 0; k < c; k++) {
       const int64_t e = nb_at(P.npad, i, k);
       const int j = __ldg(nb + e);
       const bool pass = !P.contact || pass_ij(P, idi, F.id[j]);
-      const double t = density_term<kGeo>(P, F, W, e, j, xi, vi, known_i, pass);
+      const double t = density_term<kG, kGeo>(P, F, W, e, j, xi, vi, pass);
       if (pass) drho += t;
     }
   } else {
-    const int blocks = warp_blocks(c);
-    for (int b = 0; b < blocks; b++) {
+    const int rounds = warp_rounds<kG>(c);
+    for (int b = 0; b < rounds; b++) {
       double t = 0.0;
-      if (WF_NB_BLK * b + g < c) {
-        const int64_t e = nb_at(P.npad, i, WF_NB_BLK * b + g);
+      if (kG * b + g < c) {
+        const int64_t e = nb_at(P.npad, i, kG * b + g);
         const int j = __ldg(nb + e);
         const bool pass = !P.contact || pass_ij(P, idi, F.id[j]);
-        t = density_term<kGeo>(P, F, W, e, j, xi, vi, known_i, pass);
+        t = density_term<kG, kGeo>(P, F, W, e, j, xi, vi, pass);
       }
-      drho = add_in_order(drho, t);
+      drho = add_in_order<kG>(sh, drho, t, c - kG * b);
     }
     if (!valid || g != 0) return;
   }
@@ -217,16 +401,31 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_density64(StepParams P, F
     rho_new = vi.w + P.dt * drho;
   }
   vd2[i] = make_double4(vi.x, vi.y, vi.z, rho_new);
-  if (kGeo != GEO_NONE) {
-    W.mr[i] = xi.w / rho_new;
-    W.rr_out[i] = 1.0 / rho_new;
-  }
+  if (kGeo != GEO_NONE) W.mr[i] = xi.w / rho_new;
 }
 
 // ---- B: CalcRateTensors + PressureKernelExt + StressStrainOne -----------
 // src/cuda/InteractionAlt.cu:262-383, src/cuda/Mechanical.cu:289-298 and
 // :458-554.  The terms of one pair: D xx yy zz xy yz xz, W xy yz xz.
-template <int kGeo>
+template <bool kInt>
+__device__ __forceinline__ void rate_terms(double xx, double xy, double xz, double ax, double ay,
+                                           double az, double GK, double mj_dj, double* t) {
+  const double s = neg_half(GK);
+  // StrainRate (symmetric) scaled by -GK/2, then by mj/dj
+  t[0] = mul<kInt>(mul<kInt>(mul<kInt>(twice(ax), xx), s), mj_dj);
+  t[1] = mul<kInt>(mul<kInt>(mul<kInt>(twice(ay), xy), s), mj_dj);
+  t[2] = mul<kInt>(mul<kInt>(mul<kInt>(twice(az), xz), s), mj_dj);
+  const double pxy = mul<kInt>(ax, xy), qxy = mul<kInt>(ay, xx), pxz = mul<kInt>(ax, xz),
+               qxz = mul<kInt>(az, xx), pyz = mul<kInt>(ay, xz), qyz = mul<kInt>(az, xy);
+  t[3] = mul<kInt>(mul<kInt>(pxy + qxy, s), mj_dj);
+  t[4] = mul<kInt>(mul<kInt>(pyz + qyz, s), mj_dj);
+  t[5] = mul<kInt>(mul<kInt>(pxz + qxz, s), mj_dj);
+  // RotationRate with the reference's xz sign flip (zx left 0), :358-365
+  t[6] = mul<kInt>(mul<kInt>(pxy - qxy, s), mj_dj);
+  t[7] = mul<kInt>(mul<kInt>(pyz - qyz, s), mj_dj);
+  t[8] = mul<kInt>(mul<kInt>(-(pxz - qxz), s), mj_dj);
+}
+template <int kG, int kGeo>
 __device__ __forceinline__ void stress_terms(const StepParams& P, const Fields& F, const Work64& W,
                                              const double4* __restrict__ vd2, int64_t e, int j,
                                              const double4& xi, const double4& vi, double* t) {
@@ -234,29 +433,30 @@ __device__ __forceinline__ void stress_terms(const StepParams& P, const Fields& 
   const double4 vj = vd2[j];
   const double xx = xi.x - xj.x, xy = xi.y - xj.y, xz = xi.z - xj.z;
   const double ax = vi.x - vj.x, ay = vi.y - vj.y, az = vi.z - vj.z;
-  double GK, mj_dj;
-  if constexpr (kGeo == GEO_NONE) {
-    double r2;
-    pair_geometry(P, xx, xy, xz, GK, r2);
-    mj_dj = xj.w / vj.w;
-  } else {
-    GK = __ldg(W.gk + e);
-    mj_dj = __ldg(W.mr + j);
+  double GK, r2, mj_dj;
+  const bool tame = geometry<kG, kGeo>(P, W, e, xx, xy, xz, xj.w, GK, r2);
+  if constexpr (kGeo == GEO_NONE) mj_dj = xj.w / vj.w;
+  else mj_dj = __ldg(W.mr + j);
+  if constexpr (kGeo != GEO_NONE) {
+    if (tame && within<kTame>(ax) && within<kTame>(ay) && within<kTame>(az) &&
+        within<kTame>(mj_dj)) {
+      rate_terms<true>(xx, xy, xz, ax, ay, az, GK, mj_dj, t);
+      return;
+    }
   }
-  const double s = neg_half(GK);
-  // StrainRate (symmetric) scaled by -GK/2, then by mj/dj
-  t[0] = (twice(ax) * xx) * s * mj_dj;
-  t[1] = (twice(ay) * xy) * s * mj_dj;
-  t[2] = (twice(az) * xz) * s * mj_dj;
-  const double pxy = ax * xy, qxy = ay * xx, pxz = ax * xz, qxz = az * xx, pyz = ay * xz,
-               qyz = az * xy;
-  t[3] = (pxy + qxy) * s * mj_dj;
-  t[4] = (pyz + qyz) * s * mj_dj;
-  t[5] = (pxz + qxz) * s * mj_dj;
-  // RotationRate with the reference's xz sign flip (zx left 0), :358-365
-  t[6] = (pxy - qxy) * s * mj_dj;
-  t[7] = (pyz - qyz) * s * mj_dj;
-  t[8] = (-(pxz - qxz)) * s * mj_dj;
+  rate_terms<false>(xx, xy, xz, ax, ay, az, GK, mj_dj, t);
+}
+
+// sigma / rho^2 of a slot (ai = 1 / rho^2), and whether all of it is tame
+__device__ __forceinline__ void keep_sigma(const Work64& W, int64_t i, const double* sigma,
+                                           double ai) {
+  bool tame = true;
+  for (int k = 0; k < 6; k++) {
+    const double q = sigma[k] * ai;
+    W.sa6[6 * i + k] = q;
+    tame = tame && within<kTame>(q);
+  }
+  W.tame[i] = tame ? 1 : 0;
 }
 
 // The per-particle EOS and stress update from the particle's own rates
@@ -296,9 +496,8 @@ __device__ __forceinline__ void stress_point(const StepParams& P, const Fields& 
   t3_store_flat(out.S, ss);
   if (W.sa6) {
     const double ai = 1.0 / (rho * rho);
-    double* sa = W.sa6 + 6 * i;
-    sa[0] = out.Sig.xx * ai; sa[1] = out.Sig.yy * ai; sa[2] = out.Sig.zz * ai;
-    sa[3] = out.Sig.xy * ai; sa[4] = out.Sig.yz * ai; sa[5] = out.Sig.xz * ai;
+    const double q[6] = {out.Sig.xx, out.Sig.yy, out.Sig.zz, out.Sig.xy, out.Sig.yz, out.Sig.xz};
+    keep_sigma(W, i, q, ai);
   }
   // strain += dt * D (the reference accumulates into an uninitialised local)
   ep[0] += SRS.xx * P.dt; ep[1] += SRS.yy * P.dt; ep[2] += SRS.zz * P.dt;
@@ -327,28 +526,24 @@ __device__ __forceinline__ void store_rates(const Fields& F, int64_t i, const do
   rr[0] = 0.0; rr[1] = 0.0; rr[2] = 0.0; rr[3] = r[6]; rr[4] = r[7]; rr[5] = r[8];
 }
 
-// sigma / rho^2 of a slot that the stress update skips (a rigid one), as stored
-__device__ __forceinline__ void keep_sigma(const Fields& F, const Work64& W, int64_t i, double rho) {
-  if (!W.sa6) return;
-  const double ai = 1.0 / (rho * rho);
-  for (int k = 0; k < 6; k++) W.sa6[6 * i + k] = F.sig6[6 * i + k] * ai;
-}
-
 // One lane per particle: the pair loop with the stress update behind it.
+// Twelve blocks an SM (80 registers) hide the update's chains of operations:
+// 170k particles 640 us with the 98 registers it would take, 604 with 80; the
+// update as a kernel of its own, 624.
 template <int kGeo>
-__global__ void __launch_bounds__(64) k_stress64(StepParams P, Fields F, Work64 W,
-                                                  const double4* __restrict__ vd2,
-                                                  const int32_t* __restrict__ nb,
-                                                  const int32_t* __restrict__ cnt,
-                                                  int* __restrict__ status) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(64, 12) k_stress64(StepParams P, Fields F, Work64 W,
+                                                     const double4* __restrict__ vd2,
+                                                     const int32_t* __restrict__ nb,
+                                                     const int32_t* __restrict__ cnt,
+                                                     int* __restrict__ status) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= P.n) return;
   const double4 xi = F.xm[i];
   const double4 vi = vd2[i];
   // PressureKernelExt runs over every particle (EOS case 0, P0 = 0)
   F.p[i] = 0.0 + (P.Cs * P.Cs) * (vi.w - P.rho0);
   if (F.perm[i] >= P.n_solid) {
-    keep_sigma(F, W, i, vi.w);
+    if (W.sa6) keep_sigma(W, i, F.sig6 + 6 * i, 1.0 / (vi.w * vi.w));   // as stored
     return;
   }
   double r[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -358,7 +553,7 @@ __global__ void __launch_bounds__(64) k_stress64(StepParams P, Fields F, Work64 
     const int j = __ldg(nb + e);
     if (P.contact && !pass_j(P, F.id[j])) continue;
     double t[9];
-    stress_terms<kGeo>(P, F, W, vd2, e, j, xi, vi, t);
+    stress_terms<1, kGeo>(P, F, W, vd2, e, j, xi, vi, t);
 #pragma unroll
     for (int a = 0; a < 9; a++) r[a] += t[a];
   }
@@ -366,38 +561,38 @@ __global__ void __launch_bounds__(64) k_stress64(StepParams P, Fields F, Work64 
   stress_point(P, F, W, i, vi.w, r, status);
 }
 
-// Eight lanes per particle: the pair loop alone (the rates go to sr6, rr6).
+// Several lanes per particle: the pair loop alone (the rates go to sr6, rr6).
 // The stress update is a kernel of its own, one lane per particle: behind the
-// pair loop it would run on 4 of a warp's 32 lanes.
-template <int kGeo>
+// pair loop it would run on 1 to 4 of a warp's 32 lanes.
+template <int kG, int kGeo>
 __global__ void __launch_bounds__(32) k_rates64(StepParams P, Fields F, Work64 W,
                                                 const double4* __restrict__ vd2,
                                                 const int32_t* __restrict__ nb,
                                                 const int32_t* __restrict__ cnt) {
   __shared__ double sh[32 * 9];
   int g;
-  const int64_t i0 = slot64<kLanes64>(g);
+  const int64_t i0 = slot64<kG>(g);
   const bool solid = i0 < P.n && F.perm[i0] < P.n_solid;
   const int64_t i = solid ? i0 : 0;
   const double4 xi = F.xm[i];
   const double4 vi = vd2[i];
   const int c = solid ? cnt[i] : 0;
-  const int blocks = warp_blocks(c);
+  const int rounds = warp_rounds<kG>(c);
   double acc[2] = {0.0, 0.0};
-  for (int b = 0; b < blocks; b++) {
+  for (int b = 0; b < rounds; b++) {
     double t[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (WF_NB_BLK * b + g < c) {
-      const int64_t e = nb_at(P.npad, i, WF_NB_BLK * b + g);
+    if (kG * b + g < c) {
+      const int64_t e = nb_at(P.npad, i, kG * b + g);
       const int j = __ldg(nb + e);
-      if (!P.contact || pass_j(P, F.id[j])) stress_terms<kGeo>(P, F, W, vd2, e, j, xi, vi, t);
+      if (!P.contact || pass_j(P, F.id[j])) stress_terms<kG, kGeo>(P, F, W, vd2, e, j, xi, vi, t);
     }
-    add_in_order<9>(sh, t, g, acc);
+    add_in_order<kG, 9>(sh, t, g, acc, c - kG * b);
   }
   if (!solid) return;
   // accumulators 0-5 are D (sr6), 6-8 W (rr6 3-5); rr6 0-2 are zero
   if (g < 6) F.sr6[6 * i + g] = acc[0];
-  else F.rr6[6 * i + g - 3] = acc[0];
-  if (g == 0) F.rr6[6 * i + 5] = acc[1];
+  else if (g < 9) F.rr6[6 * i + g - 3] = acc[0];
+  if (kG < 9 && g == 0) F.rr6[6 * i + 5] = acc[1];
   if (g < 3) F.rr6[6 * i + g] = 0.0;
 }
 
@@ -409,7 +604,7 @@ __global__ void __launch_bounds__(32) k_stress_point64(StepParams P, Fields F, W
   const double rho = vd2[i].w;
   F.p[i] = 0.0 + (P.Cs * P.Cs) * (rho - P.rho0);
   if (F.perm[i] >= P.n_solid) {
-    keep_sigma(F, W, i, rho);
+    if (W.sa6) keep_sigma(W, i, F.sig6 + 6 * i, 1.0 / (rho * rho));   // as stored
     return;
   }
   const double* sr = F.sr6 + 6 * i;
@@ -420,51 +615,83 @@ __global__ void __launch_bounds__(32) k_stress_point64(StepParams P, Fields F, W
 
 // ---- C: Domain_d::CalcAccel (src/cuda/InteractionAlt.cu:18-150) ---------
 // si = sigma_i / rho_i^2 (xx yy zz xy yz xz)
-template <int kGeo>
+template <bool kInt>
+__device__ __forceinline__ void force_terms(double xx, double xy, double xz, double GK, double mj,
+                                            const double* T, double* t) {
+  const double gx = mul<kInt>(xx, GK), gy = mul<kInt>(xy, GK), gz = mul<kInt>(xz, GK);
+  const double Mxx = mul<kInt>(T[0], mj), Myy = mul<kInt>(T[1], mj), Mzz = mul<kInt>(T[2], mj);
+  const double Mxy = mul<kInt>(T[3], mj), Myz = mul<kInt>(T[4], mj), Mxz = mul<kInt>(T[5], mj);
+  t[0] = mul<kInt>(Mxx, gx) + mul<kInt>(Mxy, gy) + mul<kInt>(Mxz, gz);
+  t[1] = mul<kInt>(Mxy, gx) + mul<kInt>(Myy, gy) + mul<kInt>(Myz, gz);
+  t[2] = mul<kInt>(Mxz, gx) + mul<kInt>(Myz, gy) + mul<kInt>(Mzz, gz);
+}
+// The artificial viscosity of a tame pair: false where a value in it leaves
+// the range.
+__device__ __forceinline__ bool viscosity_int(const StepParams& P, double xx, double xy, double xz,
+                                              double vx, double vy, double vz, double r2, double di,
+                                              double dj, double& PI) {
+  const double vdx = mul_int(vx, xx) + mul_int(vy, xy) + mul_int(vz, xz);
+  if (__double2hiint(vdx) >= 0) return true;
+  const double den = r2 + 0.01 * P.h * P.h, aC = P.alpha * (0.5 * (P.Cs + P.Cs));
+  const double rho2 = di + dj;
+  const double MU = div_int(mul_int(P.h, vdx), den);
+  double num = mul_int(aC, MU);
+  if (P.beta != 0.0) num = num + mul_int(mul_int(P.beta, MU), MU);
+  PI = div_int(num, mul_int(0.5, rho2));
+  return in_range<kTame>(MU) && within<kTame>(aC) && within<kTame>(P.beta) &&
+         within<4 * kTame>(num) && in_range<kTame>(rho2) && in_range<2 * kTame>(den);
+}
+template <int kG, int kGeo>
 __device__ __forceinline__ void accel_terms(const StepParams& P, const Fields& F, const Work64& W,
                                             const double4* __restrict__ vd2, int64_t e, int j,
                                             const double4& xi, const double4& vi, const double* si,
-                                            double* t) {
+                                            bool tame_i, double* t) {
   const double4 xj = F.xm[j];
   const double4 vj = vd2[j];
   const double xx = xi.x - xj.x, xy = xi.y - xj.y, xz = xi.z - xj.z;
   const double di = vi.w, dj = vj.w, mj = xj.w;
   const double vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
   double GK, r2;
+  bool tame = geometry<kG, kGeo>(P, W, e, xx, xy, xz, mj, GK, r2) && tame_i;
   double2 s01, s23, s45;
   if constexpr (kGeo == GEO_NONE) {
-    pair_geometry(P, xx, xy, xz, GK, r2);
     const double2* q = reinterpret_cast<const double2*>(F.sig6 + 6 * (int64_t)j);
     const double aj = 1.0 / (dj * dj);
     s01 = make_double2(q[0].x * aj, q[0].y * aj);
     s23 = make_double2(q[1].x * aj, q[1].y * aj);
     s45 = make_double2(q[2].x * aj, q[2].y * aj);
   } else {
-    GK = __ldg(W.gk + e);
-    r2 = __ldg(W.r2 + e);
     const double2* q = reinterpret_cast<const double2*>(W.sa6 + 6 * (int64_t)j);
     s01 = q[0]; s23 = q[1]; s45 = q[2];
+    tame = tame && __ldg(W.tame + j) != 0;
   }
   // Si/di^2 + Sj/dj^2 + PI*I, times mj, then times GK*xij (tensor3.cu:225)
-  double Txx = si[0] + s01.x, Tyy = si[1] + s01.y, Tzz = si[2] + s23.x;
-  const double Txy = si[3] + s23.y, Tyz = si[4] + s45.x, Txz = si[5] + s45.y;
+  double T[6] = {si[0] + s01.x, si[1] + s01.y, si[2] + s23.x,
+                 si[3] + s23.y, si[4] + s45.x, si[5] + s45.y};
   if (P.alpha != 0.0 || P.beta != 0.0) {
-    const double vdx = vx * xx + vy * xy + vz * xz;
-    if (vdx < 0) {
-      const double MU = P.h * vdx / (r2 + 0.01 * P.h * P.h);
-      const double Cij = 0.5 * (P.Cs + P.Cs);
-      const double PI = (P.alpha * Cij * MU + P.beta * MU * MU) / (0.5 * (di + dj));
-      Txx = Txx + PI;
-      Tyy = Tyy + PI;
-      Tzz = Tzz + PI;
+    bool done = false;
+    double PI = 0.0;
+    if constexpr (kGeo != GEO_NONE) {
+      if (tame && within<kTame>(vx) && within<kTame>(vy) && within<kTame>(vz))
+        done = viscosity_int(P, xx, xy, xz, vx, vy, vz, r2, di, dj, PI);
     }
+    if (!done) {
+      const double vdx = vx * xx + vy * xy + vz * xz;
+      PI = 0.0;
+      if (vdx < 0) {
+        const double MU = P.h * vdx / (r2 + 0.01 * P.h * P.h);
+        const double Cij = 0.5 * (P.Cs + P.Cs);
+        PI = (P.alpha * Cij * MU + P.beta * MU * MU) / (0.5 * (di + dj));
+      }
+    }
+    // (adding the zero of a pair that moves apart changes no term)
+    T[0] = T[0] + PI;
+    T[1] = T[1] + PI;
+    T[2] = T[2] + PI;
+    tame = tame && within<kTame>(PI);
   }
-  const double gx = xx * GK, gy = xy * GK, gz = xz * GK;
-  const double Mxx = Txx * mj, Myy = Tyy * mj, Mzz = Tzz * mj;
-  const double Mxy = Txy * mj, Myz = Tyz * mj, Mxz = Txz * mj;
-  t[0] = Mxx * gx + Mxy * gy + Mxz * gz;
-  t[1] = Mxy * gx + Myy * gy + Myz * gz;
-  t[2] = Mxz * gx + Myz * gy + Mzz * gz;
+  if (kGeo != GEO_NONE && tame) force_terms<true>(xx, xy, xz, GK, mj, T, t);
+  else force_terms<false>(xx, xy, xz, GK, mj, T, t);
 }
 
 template <int kGeo>
@@ -495,6 +722,7 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_accel64(StepParams P, Fie
   const int32_t idi = F.id[i];
   double si[6];
   own_sigma<kGeo>(F, W, i, vi.w, si);
+  const bool tame_i = kGeo != GEO_NONE && W.tame[i] != 0;
   const int c = solid ? cnt[i] : 0;
   double t[3];
   if constexpr (kG == 1) {
@@ -503,22 +731,22 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_accel64(StepParams P, Fie
       const int64_t e = nb_at(P.npad, i, k);
       const int j = __ldg(nb + e);
       if (P.contact && !pass_ij(P, idi, F.id[j])) continue;
-      accel_terms<kGeo>(P, F, W, vd2, e, j, xi, vi, si, t);
+      accel_terms<kG, kGeo>(P, F, W, vd2, e, j, xi, vi, si, tame_i, t);
       a[0] += t[0]; a[1] += t[1]; a[2] += t[2];
     }
     F.a[i] = make_double4(a[0], a[1], a[2], 0.0);
   } else {
-    const int blocks = warp_blocks(c);
+    const int rounds = warp_rounds<kG>(c);
     double acc[2] = {0.0, 0.0};
-    for (int b = 0; b < blocks; b++) {
+    for (int b = 0; b < rounds; b++) {
       t[0] = t[1] = t[2] = 0.0;
-      if (WF_NB_BLK * b + g < c) {
-        const int64_t e = nb_at(P.npad, i, WF_NB_BLK * b + g);
+      if (kG * b + g < c) {
+        const int64_t e = nb_at(P.npad, i, kG * b + g);
         const int j = __ldg(nb + e);
         if (!P.contact || pass_ij(P, idi, F.id[j]))
-          accel_terms<kGeo>(P, F, W, vd2, e, j, xi, vi, si, t);
+          accel_terms<kG, kGeo>(P, F, W, vd2, e, j, xi, vi, si, tame_i, t);
       }
-      add_in_order<3>(sh, t, g, acc);
+      add_in_order<kG, 3>(sh, t, g, acc, c - kG * b);
     }
     if (solid && g < 4) reinterpret_cast<double*>(F.a + i)[g] = acc[0];   // lane 3: 0
   }
@@ -530,17 +758,28 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_accel64(StepParams P, Fie
 // (wf_step_fp32.cu): pair flux in FP32 with the temperature difference taken
 // from the (hi, lo) float pair; dT/dt and T stay FP64.  It runs behind the
 // integration, so the geometry that it computes is that of the next step.
-template <int kGeo>
+template <bool kInt>
+__device__ __forceinline__ double heat_flux(double xx, double xy, double xz, double GK, double r2,
+                                            double mj_dj, double kk, double dT) {
+  return quot<kInt>(mul<kInt>(mul<kInt>(mj_dj, mul<kInt>(kk, dT)),
+                              mul<kInt>(xx, mul<kInt>(xx, GK)) + mul<kInt>(xy, mul<kInt>(xy, GK)) +
+                                  mul<kInt>(xz, mul<kInt>(xz, GK))), r2);
+}
+template <int kG, int kGeo>
 __device__ __forceinline__ double heat_term(const StepParams& P, const Fields& F, const Work64& W,
                                             int64_t e, int j, const double4& xi, double Ti,
                                             double kk) {
   const double4 xj = F.xm[j];
   const double xx = xi.x - xj.x, xy = xi.y - xj.y, xz = xi.z - xj.z;
   double GK, r2;
-  geometry<kGeo>(P, W, e, xx, xy, xz, GK, r2);
+  const bool tame = geometry<kG, kGeo>(P, W, e, xx, xy, xz, xj.w, GK, r2);
   const double mj_dj = W.mr_heat ? __ldg(W.mr_heat + j) : xj.w / F.vd[j].w;
-  return mj_dj * (kk * (Ti - F.T[j])) *
-         (xx * (xx * GK) + xy * (xy * GK) + xz * (xz * GK)) / r2;
+  const double dT = Ti - F.T[j];
+  if constexpr (kGeo != GEO_NONE) {
+    if (tame && within<kTame>(mj_dj) && within<kTame>(dT) && within<kTame>(kk))
+      return heat_flux<true>(xx, xy, xz, GK, r2, mj_dj, kk, dT);
+  }
+  return heat_flux<false>(xx, xy, xz, GK, r2, mj_dj, kk, dT);
 }
 
 template <int kG, int kGeo>
@@ -548,6 +787,7 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_rate(StepParams P, F
                                                    const int32_t* __restrict__ nb,
                                                    const int32_t* __restrict__ cnt,
                                                    int plastic_heat) {
+  __shared__ double sh[kG == 32 ? 32 : 1];
   int g;
   const int64_t i0 = slot64<kG>(g);
   if (kG == 1 && i0 >= P.n) return;
@@ -564,17 +804,17 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_rate(StepParams P, F
   if constexpr (kG == 1) {
     for (int k = 0; k < c; k++) {
       const int64_t e = nb_at(P.npad, i, k);
-      s += heat_term<kGeo>(P, F, W, e, __ldg(nb + e), xi, Ti, kk);
+      s += heat_term<kG, kGeo>(P, F, W, e, __ldg(nb + e), xi, Ti, kk);
     }
   } else {
-    const int blocks = warp_blocks(c);
-    for (int b = 0; b < blocks; b++) {
+    const int rounds = warp_rounds<kG>(c);
+    for (int b = 0; b < rounds; b++) {
       double t = 0.0;
-      if (WF_NB_BLK * b + g < c) {
-        const int64_t e = nb_at(P.npad, i, WF_NB_BLK * b + g);
-        t = heat_term<kGeo>(P, F, W, e, __ldg(nb + e), xi, Ti, kk);
+      if (kG * b + g < c) {
+        const int64_t e = nb_at(P.npad, i, kG * b + g);
+        t = heat_term<kG, kGeo>(P, F, W, e, __ldg(nb + e), xi, Ti, kk);
       }
-      s = add_in_order(s, t);
+      s = add_in_order<kG>(sh, s, t, c - kG * b);
     }
     if (!valid || g != 0) return;
   }
@@ -585,13 +825,13 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_rate(StepParams P, F
 // ---- ThermalSolve in FP64 (src/cuda/Thermal.cu:188-260) --------------------
 // Positions, densities and lists do not change inside a heat solve, so what a
 // pair contributes apart from the temperatures is computed once per solve:
-// the product of the position difference with the kernel gradient, r^2 and
-// its reciprocal (three arrays of the lists' layout), m / rho, and the
-// particle's own factors.  A step is then eight FP64 operations a pair instead
-// of 90 (the FP64 pipe bounds both: 64,000 particles 761 -> 68 us a step, 80 %
-// of the pipe's peak; the factors take 364 us a solve) and takes the leapfrog
-// update with it; the neighbours' temperatures are read
-// from one array while the new ones go to another.
+// the product of the position difference with the kernel gradient and r^2 (two
+// arrays of the lists' layout), m / rho, and the particle's own factors.  A
+// step is then two FP64 operations, three integer products and a quotient a
+// pair, and takes the leapfrog update with it; the neighbours' temperatures
+// are read from one array while the new ones go to another.  64,000
+// particles, 20 steps: 15.5 ms recomputing the pairs on the FP64 pipe, 1.88
+// with the kept factors, 1.42 on the integer pipes.
 __global__ void __launch_bounds__(64) k_heat_pairs64(StepParams P, Fields F, HeatWork64 H,
                                                      const int32_t* __restrict__ nb,
                                                      const int32_t* __restrict__ cnt) {
@@ -610,20 +850,29 @@ __global__ void __launch_bounds__(64) k_heat_pairs64(StepParams P, Fields F, Hea
     const double4 xj = F.xm[__ldg(nb + e)];
     const double xx = xi.x - xj.x, xy = xi.y - xj.y, xz = xi.z - xj.z;
     double GK, r2;
-    pair_geometry(P, xx, xy, xz, GK, r2);
+    if (P.h_tame && within<kTame>(xx) && within<kTame>(xy) && within<kTame>(xz)) {
+      pair_geometry<true, false>(P, xx, xy, xz, GK, r2);
+      if (in_range<kTame>(GK)) {
+        H.dot[e] = mul_int(xx, mul_int(xx, GK)) + mul_int(xy, mul_int(xy, GK)) +
+                   mul_int(xz, mul_int(xz, GK));
+        H.r2[e] = r2;
+        continue;
+      }
+    }
+    pair_geometry<false>(P, xx, xy, xz, GK, r2);
     H.dot[e] = xx * (xx * GK) + xy * (xy * GK) + xz * (xz * GK);
     H.r2[e] = r2;
-    H.ir2[e] = 1.0 / r2;
   }
 }
 
 __device__ __forceinline__ double heat_step_term(const HeatWork64& H, const double* __restrict__ T,
                                                  int64_t e, int j, double Ti, double kk) {
-  const double num = __ldg(H.mr + j) * (kk * (Ti - __ldg(T + j))) * __ldg(H.dot + e);
-  const double r2 = __ldg(H.r2 + e), y = __ldg(H.ir2 + e);
-  // zero and the middle of the range divide by the known reciprocal
-  const bool easy = mid_range(num) || ((__double2hiint(num) << 1) | __double2loint(num)) == 0;
-  return easy && mid_range(y) ? div_known(num, r2, y) : num / r2;
+  const double mr = __ldg(H.mr + j), dT = Ti - __ldg(T + j), dot = __ldg(H.dot + e);
+  const double r2 = __ldg(H.r2 + e);
+  if (within<kTame>(mr) && within<kTame>(dT) && within<kTame>(dot) && within<kTame>(kk) &&
+      in_range<kTame>(r2))
+    return div_int(mul_int(mul_int(mr, mul_int(kk, dT)), dot), r2);
+  return mr * (kk * dT) * dot / r2;
 }
 
 template <int kG>
@@ -632,6 +881,7 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_step64(StepParams P,
                                                      double* __restrict__ T_out,
                                                      const int32_t* __restrict__ nb,
                                                      const int32_t* __restrict__ cnt, int first) {
+  __shared__ double sh[kG == 32 ? 32 : 1];
   int g;
   const int64_t i0 = slot64<kG>(g);
   if (kG == 1 && i0 >= P.n) return;
@@ -647,14 +897,14 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_step64(StepParams P,
       s += heat_step_term(H, T, e, __ldg(nb + e), Ti, kk);
     }
   } else {
-    const int blocks = warp_blocks(c);
-    for (int b = 0; b < blocks; b++) {
+    const int rounds = warp_rounds<kG>(c);
+    for (int b = 0; b < rounds; b++) {
       double t = 0.0;
-      if (WF_NB_BLK * b + g < c) {
-        const int64_t e = nb_at(P.npad, i, WF_NB_BLK * b + g);
+      if (kG * b + g < c) {
+        const int64_t e = nb_at(P.npad, i, kG * b + g);
         t = heat_step_term(H, T, e, __ldg(nb + e), Ti, kk);
       }
-      s = add_in_order(s, t);
+      s = add_in_order<kG>(sh, s, t, c - kG * b);
     }
     if (!valid || g != 0) return;
   }
@@ -680,16 +930,19 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_step64(StepParams P,
 
 static inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
-// Below this many particles eight lanes share one (see kLanes64).
-constexpr int64_t kWide64 = 24000;
+// Lanes of a particle for a domain of n (the times stand at slot64).
+static inline int lanes64(int64_t n) {
+  return n >= 64000 ? 1 : n >= 5000 ? 8 : n >= 2000 ? 16 : 32;
+}
 
-// Launches K<lanes, geometry> with one or eight lanes per particle.
+// Launches K<lanes, geometry>.
 #define WF_LAUNCH64(K, GEO, ...)                                                               \
   do {                                                                                         \
-    if (P.n < kWide64)                                                                         \
-      K<kLanes64, GEO><<<blocks_for(P.n * kLanes64, 32), 32, 0, s>>>(P, F, W, __VA_ARGS__);    \
-    else                                                                                       \
-      K<1, GEO><<<blocks_for(P.n, 64), 64, 0, s>>>(P, F, W, __VA_ARGS__);                      \
+    const int lanes = lanes64(P.n), grid = blocks_for(P.n * lanes, lanes == 1 ? 64 : 32);      \
+    if (lanes == 32) K<32, GEO><<<grid, 32, 0, s>>>(P, F, W, __VA_ARGS__);                     \
+    else if (lanes == 16) K<16, GEO><<<grid, 32, 0, s>>>(P, F, W, __VA_ARGS__);                \
+    else if (lanes == 8) K<8, GEO><<<grid, 32, 0, s>>>(P, F, W, __VA_ARGS__);                  \
+    else K<1, GEO><<<grid, 64, 0, s>>>(P, F, W, __VA_ARGS__);                                  \
   } while (0)
 
 void launch_fp64_density(const StepParams& P, const Fields& F, const Work64& W, double4* vd2,
@@ -700,16 +953,24 @@ void launch_fp64_density(const StepParams& P, const Fields& F, const Work64& W, 
 }
 int launch_fp64_stress(const StepParams& P, const Fields& F, const Work64& W, const double4* vd2,
                        const NbBuffers& N, int* status, cudaStream_t s) {
-  if (P.n < kWide64) {
-    const int blocks = blocks_for(P.n * kLanes64, 32);
-    if (W.gk) k_rates64<GEO_LOAD><<<blocks, 32, 0, s>>>(P, F, W, vd2, N.nb, N.cnt);
-    else k_rates64<GEO_NONE><<<blocks, 32, 0, s>>>(P, F, W, vd2, N.nb, N.cnt);
-    k_stress_point64<<<blocks_for(P.n, 32), 32, 0, s>>>(P, F, W, vd2, status);
-    return 2;
+  const int lanes = lanes64(P.n), grid = blocks_for(P.n * lanes, lanes == 1 ? 64 : 32);
+  if (lanes == 1) {
+    if (W.gk) k_stress64<GEO_LOAD><<<grid, 64, 0, s>>>(P, F, W, vd2, N.nb, N.cnt, status);
+    else k_stress64<GEO_NONE><<<grid, 64, 0, s>>>(P, F, W, vd2, N.nb, N.cnt, status);
+    return 1;
   }
-  if (W.gk) k_stress64<GEO_LOAD><<<blocks_for(P.n, 64), 64, 0, s>>>(P, F, W, vd2, N.nb, N.cnt, status);
-  else k_stress64<GEO_NONE><<<blocks_for(P.n, 64), 64, 0, s>>>(P, F, W, vd2, N.nb, N.cnt, status);
-  return 1;
+  if (lanes == 32) {
+    if (W.gk) k_rates64<32, GEO_LOAD><<<grid, 32, 0, s>>>(P, F, W, vd2, N.nb, N.cnt);
+    else k_rates64<32, GEO_NONE><<<grid, 32, 0, s>>>(P, F, W, vd2, N.nb, N.cnt);
+  } else if (lanes == 16) {
+    if (W.gk) k_rates64<16, GEO_LOAD><<<grid, 32, 0, s>>>(P, F, W, vd2, N.nb, N.cnt);
+    else k_rates64<16, GEO_NONE><<<grid, 32, 0, s>>>(P, F, W, vd2, N.nb, N.cnt);
+  } else {
+    if (W.gk) k_rates64<8, GEO_LOAD><<<grid, 32, 0, s>>>(P, F, W, vd2, N.nb, N.cnt);
+    else k_rates64<8, GEO_NONE><<<grid, 32, 0, s>>>(P, F, W, vd2, N.nb, N.cnt);
+  }
+  k_stress_point64<<<blocks_for(P.n, 32), 32, 0, s>>>(P, F, W, vd2, status);
+  return 2;
 }
 void launch_fp64_accel(const StepParams& P, const Fields& F, const Work64& W, const double4* vd2,
                        const NbBuffers& N, cudaStream_t s) {
@@ -727,9 +988,13 @@ void launch_heat_pairs64(const StepParams& P, const Fields& F, const HeatWork64&
 }
 void launch_heat_step64(const StepParams& P, const Fields& F, const HeatWork64& H, double* T_out,
                         const NbBuffers& N, int first, cudaStream_t s) {
-  if (P.n < kWide64)
-    k_heat_step64<kLanes64><<<blocks_for(P.n * kLanes64, 32), 32, 0, s>>>(P, F, H, F.T, T_out,
-                                                                          N.nb, N.cnt, first);
+  const int lanes = lanes64(P.n), grid = blocks_for(P.n * lanes, lanes == 1 ? 64 : 32);
+  if (lanes == 32)
+    k_heat_step64<32><<<grid, 32, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
+  else if (lanes == 16)
+    k_heat_step64<16><<<grid, 32, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
+  else if (lanes == 8)
+    k_heat_step64<8><<<grid, 32, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
   else
-    k_heat_step64<1><<<blocks_for(P.n, 64), 64, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
+    k_heat_step64<1><<<grid, 64, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
 }
