@@ -1110,7 +1110,7 @@ static int solve_begin(wf_domain* d, double dt_out) {
     if (rc) return rc;
     d->totmass = 0.0;
     for (double mm : hm) d->totmass += mm;
-    launch_mesh_plane(make_params(d), d->stream);  // CalcSpheresKernel, :129-141
+    launch_mesh_plane(make_params(d), d->F[d->cur], d->stream);  // CalcSpheresKernel, :129-141
     if (d->contact_law == 1) {
       if (!(d->c_dx > 0.0)) return wf_fail(d, WF_ERR_STATE, "contact law 1 needs the option contact_dx");
       for (const MeshDev& M : d->meshes)
@@ -1267,8 +1267,8 @@ static int solve_step_launches(wf_domain* d) {
   }
   if (P.contact) {                                                                    // :289-316
     KTimer t(d, KID_CONTACT);
-    launch_mesh_update(P, F, mixed ? 1 : 0, s);
-    d->launches += 3 * P.ncsid;
+    launch_mesh_update(P, F, mixed ? 1 : 0, !integrated, s);
+    d->launches += (integrated ? 2 : 1) * P.ncsid;
   }
   if (d->debug_checks) {
     k_check_finite<<<nblk(d->n), 256, 0, s>>>(d->n, F.xm, F.vd, d->d_status);

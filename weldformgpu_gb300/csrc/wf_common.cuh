@@ -446,8 +446,10 @@ void launch_contact_law1_list(const StepParams& P, const Fields& F, const double
                               float4* a32, cudaStream_t s);
 // *flag = 1 if a particle with mass carries a mesh's zone id (flag zeroed before)
 void launch_zone_mass(const StepParams& P, const Fields& F, int* flag, cudaStream_t s);
-void launch_mesh_update(const StepParams& P, const Fields& F, int mixed, cudaStream_t s);
-void launch_mesh_plane(const StepParams& P, cudaStream_t s);
+// moved: launch_integrate moved the nodes
+void launch_mesh_update(const StepParams& P, const Fields& F, int mixed, bool moved,
+                        cudaStream_t s);
+void launch_mesh_plane(const StepParams& P, const Fields& F, cudaStream_t s);
 struct TileHalo;
 struct List16;
 // density pass alone (mixed form; a call's first step, or heat off)

@@ -9,12 +9,13 @@
 // Compiled with -fmad=false: the FP64 arithmetic follows the reference's
 // operation order (vector_math.h: a / s is a * (1.0 / s), dot sums left to
 // right, length = sqrt(dot)), so the plain form matches the oracle bit for bit.
-// One thread per particle (surface, list, force), per node (mesh motion) or
-// per element (element geometry, rigid particles).
+// 1 to 32 lanes per particle (surface, list, force; wf_lanes64.cuh), one thread
+// per node (mesh motion) or element (element geometry and rigid particle).
 #include <algorithm>
 
 #include "wf_common.cuh"
 #include "wf_integrate.cuh"
+#include "wf_lanes64.cuh"
 #include "wf_nsearch.cuh"
 
 namespace {
@@ -47,23 +48,53 @@ __device__ __forceinline__ int mesh_of(const StepParams& P, int32_t orig) {
 // with n' <= 46 tags the particle as free surface unless its zone is protected.
 // Other threads may turn a neighbour's id into the free-surface id meanwhile;
 // that id is never a mesh zone id, so the test on ID[j] does not change.
-__global__ void __launch_bounds__(128) k_surface(StepParams P, Fields F,
-                                                 const int32_t* __restrict__ nb,
-                                                 const int32_t* __restrict__ cnt) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= P.n || F.perm[i] >= P.n_solid) return;
+// Several lanes share a particle as in the pair passes (5.4k particles: 37 us
+// with one thread each, 17 us so).
+template <int kG>
+__global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_surface(StepParams P, Fields F,
+                                                               const int32_t* __restrict__ nb,
+                                                               const int32_t* __restrict__ cnt) {
+  __shared__ double sh[kG == 1 ? 1 : 32 * 3];
+  int g;
+  const int64_t i0 = slot64<kG>(g);
+  const bool solid = i0 < P.n && F.perm[i0] < P.n_solid;
+  if (kG == 1 && !solid) return;
+  const int64_t i = solid ? i0 : 0;
   const V3 xi = mk(F.xm[i]);
   V3 nrm = mk(0.0, 0.0, 0.0);
   int corr = 0;
-  const int c = cnt[i];
-  for (int k = 0; k < c; k++) {
-    const int j = __ldg(nb + nb_at(P.npad, i, k));
-    const double4 xj = F.xm[j];
-    const V3 xij = xi - mk(xj);
-    if (F.id[j] != P.csid[0]) {
-      nrm = nrm + scale(xij, xj.w);
-      corr++;
+  const int c = solid ? cnt[i] : 0;
+  if constexpr (kG == 1) {
+    for (int k = 0; k < c; k++) {
+      const int j = __ldg(nb + nb_at(P.npad, i, k));
+      const double4 xj = F.xm[j];
+      const V3 xij = xi - mk(xj);
+      if (F.id[j] != P.csid[0]) {
+        nrm = nrm + scale(xij, xj.w);
+        corr++;
+      }
     }
+  } else {
+    const int rounds = warp_rounds<kG>(c);
+    double acc[2] = {0.0, 0.0};
+    for (int b = 0; b < rounds; b++) {
+      double t[3] = {0.0, 0.0, 0.0};
+      if (kG * b + g < c) {
+        const int j = __ldg(nb + nb_at(P.npad, i, kG * b + g));
+        const double4 xj = F.xm[j];
+        const V3 xij = scale(xi - mk(xj), xj.w);
+        if (F.id[j] != P.csid[0]) {
+          t[0] = xij.x; t[1] = xij.y; t[2] = xij.z;
+          corr++;
+        }
+      }
+      add_in_order<kG, 3>(sh, t, g, acc, c - kG * b);
+    }
+#pragma unroll
+    for (int k = kG / 2; k > 0; k /= 2) corr += __shfl_xor_sync(0xffffffffu, corr, k);
+    nrm = mk(__shfl_sync(0xffffffffu, acc[0], 0, kG), __shfl_sync(0xffffffffu, acc[0], 1, kG),
+             __shfl_sync(0xffffffffu, acc[0], 2, kG));
+    if (!solid || g != 0) return;
   }
   nrm = scale(nrm, (double)P.n / (P.totmass * (double)corr));
   F.nrm[i] = d4(nrm);
@@ -73,25 +104,40 @@ __global__ void __launch_bounds__(128) k_surface(StepParams P, Fields F,
 // CalcContactNb: rigid neighbours within 2h of a free-surface particle, in
 // neighbour order, once per mesh whose zone id matches; at most WF_CONT_NB
 // (the reference writes past its 20 slots).  Column-major: cnb[k * npad + i].
-__global__ void __launch_bounds__(128) k_contact_nb(StepParams P, Fields F,
-                                                    const int32_t* __restrict__ nb,
-                                                    const int32_t* __restrict__ cnt) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= P.n || F.perm[i] >= P.n_solid) return;
+// The distance is computed of rigid neighbours only, the lanes of a particle
+// append in list order (5.4k particles 47 us with one thread each and all
+// distances, 36 without, 12 so).
+template <int kG>
+__global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_contact_nb(StepParams P, Fields F,
+                                                                  const int32_t* __restrict__ nb,
+                                                                  const int32_t* __restrict__ cnt) {
+  int g;
+  const int64_t i0 = slot64<kG>(g);
+  const bool solid = i0 < P.n && F.perm[i0] < P.n_solid;
+  const int64_t i = solid ? i0 : 0;
   int cc = 0;
-  if (F.id[i] == P.id_free_surf) {
-    const V3 xi = mk(F.xm[i]);
-    const int c = cnt[i];
-    for (int k = 0; k < c; k++) {
-      const int j = __ldg(nb + nb_at(P.npad, i, k));
+  const int c = solid && F.id[i] == P.id_free_surf ? cnt[i] : 0;
+  const V3 xi = mk(F.xm[i]);
+  const int rounds = warp_rounds<kG>(c);
+  for (int b = 0; b < rounds; b++) {
+    int j = 0, meshes = 0;
+    if (kG * b + g < c) {
+      j = __ldg(nb + nb_at(P.npad, i, kG * b + g));
       const int32_t idj = F.id[j];
-      const double r = len(xi - mk(F.xm[j]));
-      for (int mc = 0; mc < P.ncsid; mc++)
-        if (idj == P.csid[mc] && r < 2. * P.h && cc < WF_CONT_NB)
-          P.cnb[(int64_t)(cc++) * P.npad + i] = j;
+      for (int mc = 0; mc < P.ncsid; mc++) meshes += idj == P.csid[mc];
+      if (meshes && !(len(xi - mk(F.xm[j])) < 2. * P.h)) meshes = 0;
     }
+    int upto = meshes;                                   // of the lanes up to this one
+#pragma unroll
+    for (int k = 1; k < kG; k *= 2) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, k, kG);
+      if (g >= k) upto += v;
+    }
+    for (int q = cc + upto - meshes; q < cc + upto && q < WF_CONT_NB; q++)
+      P.cnb[(int64_t)q * P.npad + i] = j;
+    cc += __shfl_sync(0xffffffffu, upto, kG - 1, kG);
   }
-  P.ccnt[i] = cc;
+  if (solid && g == 0) P.ccnt[i] = cc < WF_CONT_NB ? cc : WF_CONT_NB;
 }
 
 // CalcContactForcesWang: for each contact neighbour j (the centroid particle of
@@ -102,62 +148,94 @@ __global__ void __launch_bounds__(128) k_contact_nb(StepParams P, Fields F,
 // acceleration accumulates all of them, and later contacts see the earlier
 // ones through the predicted position.  Mixed form: the acceleration comes
 // from and returns to the FP32 array.
-__global__ void __launch_bounds__(128) k_contact_force(StepParams P, Fields F, float4* a32) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= P.n || F.perm[i] >= P.n_solid) return;
-  const int cc = P.ccnt[i];
+//
+// Eight lanes share a particle in domains that do not fill the GPU (lanes64):
+// they test eight contacts in a row against the acceleration so far, the first
+// that hits applies its force, and the contacts behind it are tested anew.  A
+// hit is rare, so the chain of contacts (each some 100 operations at 19 cycles)
+// shrinks by up to 8: 5.4k particles 44 -> 15 us.
+struct ContactHit {
+  V3 x_pred, n;
+  double dist;
+  int j;
+};
+__device__ __forceinline__ bool contact_test(const StepParams& P, const Fields& F, int64_t i, int k,
+                                             V3 xi, V3 vi, V3 a, ContactHit& H) {
+  const double dt = P.dt, h = P.h;
+  const int j = P.cnb[(int64_t)k * P.npad + i];
+  const int32_t oj = F.perm[j];
+  const int mid = mesh_of(P, oj);
+  const MeshDev& M = P.mesh[mid];
+  const int e = oj - M.first;
+  const V3 x_pred = (xi + scale(vi, dt)) + divide(scale(scale(a, dt), dt), 2.);
+  const V3 n = mk(M.normal[e]);
+  const double dist = dot(n, x_pred) - M.pplane[e];
+  H = ContactHit{x_pred, n, dist, j};
+  if (!(dist < h)) return false;
+  const V3 Qj = xi - scale(n, dist);
+  for (int l = 0; l < 3; l++) {
+    const int nx = l + 1 > 2 ? 0 : l + 1;
+    const V3 pl = mk(M.node[M.elnode[3 * e + l]]);
+    const V3 pn = mk(M.node[M.elnode[3 * e + nx]]);
+    if (dot(cross(pn - pl, Qj - pl), n) < 0.0) return false;
+  }
+  return true;
+}
+// the force of one contact: cf becomes its force, a gains it
+__device__ __forceinline__ void contact_apply(const StepParams& P, const Fields& F,
+                                              const ContactHit& H, V3 xi, double mi, V3& a,
+                                              V3& cf) {
+  const double dt = P.dt, delta = P.h - H.dist;
+  const double kij = 2.0 * mi / (dt * dt);
+  cf = scale(H.n, 0.4 * kij * delta);
+  a = a + divide(cf, mi);
+  if (P.mu_s > 0.) {
+    const V3 du = (H.x_pred - xi) - scale(mk(F.vd[H.j]), dt);
+    const V3 dtg = du - scale(H.n, dot(du, H.n));
+    const V3 ft = scale(dtg, kij);
+    if (len(ft) < P.mu_s * len(cf)) {
+      a = a - divide(ft, mi);
+    } else {
+      const V3 fd = divide(scale(ft, P.mu_d * len(cf)), len(ft));
+      cf = cf - fd;
+      a = a - divide(fd, mi);
+    }
+  }
+}
+
+template <int kG>
+__global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_contact_force(StepParams P, Fields F,
+                                                                     float4* a32) {
+  constexpr unsigned kAll = 0xffffffffu;
+  int g;
+  const int64_t i0 = slot64<kG>(g);
+  const bool solid = i0 < P.n && F.perm[i0] < P.n_solid;
+  const int64_t i = solid ? i0 : 0;
+  const int cc = solid ? P.ccnt[i] : 0;
   V3 cf = mk(0.0, 0.0, 0.0);
-  if (cc > 0) {
+  if (__any_sync(kAll, cc > 0)) {
     const double4 x4 = F.xm[i];
     const V3 xi = mk(x4), vi = mk(F.vd[i]);
-    const double mi = x4.w, dt = P.dt, h = P.h;
-    V3 a;
-    if (a32) {
-      const float4 af = a32[i];
-      a = mk(af.x, af.y, af.z);
-    } else {
-      a = mk(F.a[i]);
+    V3 a = a32 ? mk(a32[i].x, a32[i].y, a32[i].z) : mk(F.a[i]);
+    const int base = (threadIdx.x & 31) - g;             // the group's first lane
+    for (int pos = 0; __any_sync(kAll, pos < cc);) {
+      ContactHit H;
+      const bool hit = pos + g < cc && contact_test(P, F, i, pos + g, xi, vi, a, H);
+      const unsigned m = (__ballot_sync(kAll, hit) >> base) & ((1u << kG) - 1u);
+      const int first = m ? __ffs(m) - 1 : 0;
+      if (hit && g == first) contact_apply(P, F, H, xi, x4.w, a, cf);
+      a = mk(__shfl_sync(kAll, a.x, first, kG), __shfl_sync(kAll, a.y, first, kG),
+             __shfl_sync(kAll, a.z, first, kG));
+      cf = mk(__shfl_sync(kAll, cf.x, first, kG), __shfl_sync(kAll, cf.y, first, kG),
+              __shfl_sync(kAll, cf.z, first, kG));
+      pos += m ? first + 1 : kG;
     }
-    for (int k = 0; k < cc; k++) {
-      const int j = P.cnb[(int64_t)k * P.npad + i];
-      const int32_t oj = F.perm[j];
-      const int mid = mesh_of(P, oj);
-      const MeshDev& M = P.mesh[mid];
-      const int e = oj - M.first;
-      const V3 x_pred = (xi + scale(vi, dt)) + divide(scale(scale(a, dt), dt), 2.);
-      const V3 n = mk(M.normal[e]);
-      const double dist = dot(n, x_pred) - M.pplane[e];
-      if (!(dist < h)) continue;
-      const V3 Qj = xi - scale(n, dist);
-      bool inside = true;
-      for (int l = 0; l < 3 && inside; l++) {
-        const int nx = l + 1 > 2 ? 0 : l + 1;
-        const V3 pl = mk(M.node[M.elnode[3 * e + l]]);
-        const V3 pn = mk(M.node[M.elnode[3 * e + nx]]);
-        if (dot(cross(pn - pl, Qj - pl), n) < 0.0) inside = false;
-      }
-      if (!inside) continue;
-      const double delta = h - dist;
-      const double kij = 2.0 * mi / (dt * dt);
-      cf = scale(n, 0.4 * kij * delta);
-      a = a + divide(cf, mi);
-      if (P.mu_s > 0.) {
-        const V3 du = (x_pred - xi) - scale(mk(F.vd[j]), dt);
-        const V3 dtg = du - scale(n, dot(du, n));
-        const V3 ft = scale(dtg, kij);
-        if (len(ft) < P.mu_s * len(cf)) {
-          a = a - divide(ft, mi);
-        } else {
-          const V3 fd = divide(scale(ft, P.mu_d * len(cf)), len(ft));
-          cf = cf - fd;
-          a = a - divide(fd, mi);
-        }
-      }
+    if (cc > 0 && g == 0) {
+      if (a32) a32[i] = make_float4((float)a.x, (float)a.y, (float)a.z, 0.f);
+      else F.a[i] = d4(a);
     }
-    if (a32) a32[i] = make_float4((float)a.x, (float)a.y, (float)a.z, 0.f);
-    else F.a[i] = d4(a);
   }
-  F.cf[i] = d4(cf);
+  if (solid && g == 0) F.cf[i] = d4(cf);
 }
 
 // Closest point of triangle abc to p (Ericson, Real-Time Collision Detection,
@@ -579,49 +657,37 @@ __global__ void __launch_bounds__(256) k_zone_mass(StepParams P, Fields F, int* 
   if (any) *flag = 1;
 }
 
-// TriMesh_d::Move: node velocity m_v + m_w x node, then node += v dt
 __global__ void k_mesh_move(MeshDev M, double dt) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= M.nn) return;
-  const V3 nd = mk(M.node[q]);
-  const V3 vr = cross(mk(M.mw[0], M.mw[1], M.mw[2]), nd);
-  const V3 nv = mk(M.mv[0], M.mv[1], M.mv[2]) + vr;
-  M.node_v[q] = d4(nv);
-  const V3 moved = nd + scale(nv, dt);
-  M.node[q] = d4(moved);
-  if (q == 0 && M.off32)   // node 0 in FP32 for the law-1 early-out
-    M.off32[0] = make_float4((float)moved.x, (float)moved.y, (float)moved.z, 0.f);
+  mesh_move_one(M, dt, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // CalcCentroids, CalcNormals and UpdatePlaneCoeff of one element from the
 // moved nodes; the plane coefficient reads node[elnode[3e] + nfar] with
-// nfar = 2, the index CalcSpheres leaves (Mesh.cu:205-231)
-__global__ void k_mesh_elems(MeshDev M, int geometry) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= M.ne) return;
-  if (geometry) {
-    const V3 n0 = mk(M.node[M.elnode[3 * e]]), n1 = mk(M.node[M.elnode[3 * e + 1]]),
-             n2 = mk(M.node[M.elnode[3 * e + 2]]);
-    M.centroid[e] = d4(divide((n0 + n1) + n2, 3.));
-    const V3 w = cross(n1 - n0, n2 - n0);
-    M.normal[e] = d4(divide(w, len(w)));
-  }
-  M.pplane[e] = dot(mk(M.node[M.elnode[3 * e] + 2]), mk(M.normal[e]));
-}
-
+// nfar = 2, the index CalcSpheres leaves (Mesh.cu:205-231).  Then
 // UpdateContactParticles: the element's rigid particle takes the mean node
-// velocity, zero acceleration and the element normal
-__global__ void k_contact_particles(StepParams P, Fields F, MeshDev M, int mixed) {
+// velocity, zero acceleration and the element normal.  `plane`: only the plane
+// coefficient.
+__global__ void k_mesh_elems(StepParams P, Fields F, MeshDev M, int plane, int mixed) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= M.ne) return;
+  if (plane) {
+    M.pplane[e] = dot(mk(M.node[M.elnode[3 * e] + 2]), mk(M.normal[e]));
+    return;
+  }
+  const int e0 = M.elnode[3 * e], e1 = M.elnode[3 * e + 1], e2 = M.elnode[3 * e + 2];
+  const V3 n0 = mk(M.node[e0]), n1 = mk(M.node[e1]), n2 = mk(M.node[e2]);
+  M.centroid[e] = d4(divide((n0 + n1) + n2, 3.));
+  const V3 w = cross(n1 - n0, n2 - n0);
+  const V3 normal = divide(w, len(w));
+  M.normal[e] = d4(normal);
+  M.pplane[e] = dot(mk(M.node[e0 + 2]), normal);
   const int32_t s = P.inv[M.first + e];
-  V3 vv = mk(0.0, 0.0, 0.0);
-  for (int q = 0; q < 3; q++) vv = vv + mk(M.node_v[M.elnode[3 * e + q]]);
+  const V3 vv = ((mk(0.0, 0.0, 0.0) + mk(M.node_v[e0])) + mk(M.node_v[e1])) + mk(M.node_v[e2]);
   const V3 v = divide(vv, 3.);
   const double rho = F.vd[s].w;
   F.vd[s] = d4(v, rho);
   F.a[s] = make_double4(0.0, 0.0, 0.0, 0.0);
-  F.nrm[s] = M.normal[e];
+  F.nrm[s] = d4(normal);
   if (mixed) {
     float4& m = F.pv[s].v;
     m.x = (float)v.x; m.y = (float)v.y; m.z = (float)v.z;
@@ -648,9 +714,19 @@ void launch_contact_stage(const StepParams& P, const Fields& F, const NbBuffers&
     if (!P.near_count) k_contact_law1<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, a32);
     return;
   }
-  k_surface<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, N.nb, N.cnt);
-  if (list) k_contact_nb<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, N.nb, N.cnt);
-  k_contact_force<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, a32);
+  const int lanes = lanes64(P.n), grid = blocks_for(P.n * lanes, lanes == 1 ? 64 : 32);
+  if (lanes == 32) k_surface<32><<<grid, 32, 0, s>>>(P, F, N.nb, N.cnt);
+  else if (lanes == 16) k_surface<16><<<grid, 32, 0, s>>>(P, F, N.nb, N.cnt);
+  else if (lanes == 8) k_surface<8><<<grid, 32, 0, s>>>(P, F, N.nb, N.cnt);
+  else k_surface<1><<<grid, 64, 0, s>>>(P, F, N.nb, N.cnt);
+  if (lanes > 1) {
+    const int grid8 = blocks_for(P.n * 8, 32);
+    if (list) k_contact_nb<8><<<grid8, 32, 0, s>>>(P, F, N.nb, N.cnt);
+    k_contact_force<8><<<grid8, 32, 0, s>>>(P, F, a32);
+  } else {
+    if (list) k_contact_nb<1><<<grid, 64, 0, s>>>(P, F, N.nb, N.cnt);
+    k_contact_force<1><<<grid, 64, 0, s>>>(P, F, a32);
+  }
 }
 
 void launch_contact_law1_list(const StepParams& P, const Fields& F, const double4* vd2,
@@ -663,17 +739,15 @@ void launch_zone_mass(const StepParams& P, const Fields& F, int* flag, cudaStrea
   k_zone_mass<<<std::min(blocks_for(P.n, 256), 1024), 256, 0, s>>>(P, F, flag);
 }
 
-void launch_mesh_update(const StepParams& P, const Fields& F, int mixed, cudaStream_t s) {
-  for (int m = 0; m < P.ncsid; m++) {
-    const MeshDev& M = P.mesh[m];
-    k_mesh_move<<<blocks_for(M.nn, 128), 128, 0, s>>>(M, P.dt);
-    k_mesh_elems<<<blocks_for(M.ne, 128), 128, 0, s>>>(M, 1);
-  }
+void launch_mesh_update(const StepParams& P, const Fields& F, int mixed, bool moved,
+                        cudaStream_t s) {
+  for (int m = 0; m < P.ncsid && !moved; m++)
+    k_mesh_move<<<blocks_for(P.mesh[m].nn, 128), 128, 0, s>>>(P.mesh[m], P.dt);
   for (int m = 0; m < P.ncsid; m++)
-    k_contact_particles<<<blocks_for(P.mesh[m].ne, 128), 128, 0, s>>>(P, F, P.mesh[m], mixed);
+    k_mesh_elems<<<blocks_for(P.mesh[m].ne, 64), 64, 0, s>>>(P, F, P.mesh[m], 0, mixed);
 }
 
-void launch_mesh_plane(const StepParams& P, cudaStream_t s) {
+void launch_mesh_plane(const StepParams& P, const Fields& F, cudaStream_t s) {
   for (int m = 0; m < P.ncsid; m++)
-    k_mesh_elems<<<blocks_for(P.mesh[m].ne, 128), 128, 0, s>>>(P.mesh[m], 0);
+    k_mesh_elems<<<blocks_for(P.mesh[m].ne, 64), 64, 0, s>>>(P, F, P.mesh[m], 1, 0);
 }

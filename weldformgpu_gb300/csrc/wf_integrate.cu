@@ -12,11 +12,22 @@ namespace {
 // GeneralAfter/ApplyBCVel (src/WeldFormGPU.cu:103-106, src/cuda/Mechanical.cu:572-584),
 // UpdatePosFraser (:179-187), UpdateVel (:142-148), CalcIntEnergy
 // (src/cuda/Energy.cu:5-19), in SolverFraser.cu:273-287 order.
+// The blocks behind the particles' move the rigid meshes' nodes (nothing here
+// reads them), which saves a launch per mesh.
 __global__ void __launch_bounds__(256) k_integrate(StepParams P, Fields F,
                                                    const double4* __restrict__ vd2,
                                                    const float4* __restrict__ a32) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= P.n) return;
+  if (i >= P.n) {
+    int b = (int)blockIdx.x - (int)((P.n + blockDim.x - 1) / blockDim.x);
+    if (b < 0) return;
+    for (int m = 0; m < P.ncsid; m++) {
+      const int blocks = (P.mesh[m].nn + (int)blockDim.x - 1) / (int)blockDim.x;
+      if (b < blocks) return mesh_move_one(P.mesh[m], P.dt, b * (int)blockDim.x + (int)threadIdx.x);
+      b -= blocks;
+    }
+    return;
+  }
   if (a32) {
     // rigid (non-solid) slots keep the acceleration the BCs left (zero)
     const float4 af = F.perm[i] < P.n_solid ? a32[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -72,15 +83,23 @@ __global__ void __launch_bounds__(256) k_heat_leapfrog(StepParams P, Fields F, i
 }  // namespace
 
 static inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
+// Threads of a block: one warp in domains that give no SM two blocks of 256,
+// so that their few FP64 operations run on every SM (540 particles: integration
+// 7.5 -> 6.3 us).
+static inline int threads64(int64_t n) { return n < 77824 ? 32 : 256; }
 
 void launch_integrate(const StepParams& P, const Fields& F, const double4* vd2,
                       const float4* a32, cudaStream_t s) {
-  k_integrate<<<blocks_for(P.n, 256), 256, 0, s>>>(P, F, vd2, a32);
+  const int t = threads64(P.n);
+  int grid = blocks_for(P.n, t);
+  for (int m = 0; P.contact && m < P.ncsid; m++) grid += blocks_for(P.mesh[m].nn, t);
+  k_integrate<<<grid, t, 0, s>>>(P, F, vd2, a32);
 }
 
 void launch_thermal(const StepParams& P, const Fields& F, const Work64& W, const NbBuffers& N,
                     int first, int plastic_heat, int mixed, cudaStream_t s) {
   if (mixed) launch_fp32_heat(P, F, N, plastic_heat, s);
   else launch_fp64_heat_rate(P, F, W, N, plastic_heat, s);
-  k_heat_leapfrog<<<blocks_for(P.n, 256), 256, 0, s>>>(P, F, first, mixed);
+  const int t = threads64(P.n);
+  k_heat_leapfrog<<<blocks_for(P.n, t), t, 0, s>>>(P, F, first, mixed);
 }

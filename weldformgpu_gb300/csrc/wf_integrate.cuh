@@ -67,3 +67,18 @@ __device__ __forceinline__ void integrate_mixed_one(const StepParams& P, const F
   F.pv[i].v = make_float4((float)vx, (float)vy, (float)vz, thi);
   F.tl32[i] = (float)(T - (double)thi);
 }
+
+// TriMesh_d::Move of node q: velocity m_v + m_w x node, then node += v dt
+// (only in units without FMA contraction)
+__device__ __forceinline__ void mesh_move_one(const MeshDev& M, double dt, int q) {
+  if (q >= M.nn) return;
+  const double4 nd = M.node[q];
+  const double vx = M.mv[0] + (M.mw[1] * nd.z - M.mw[2] * nd.y);
+  const double vy = M.mv[1] + (M.mw[2] * nd.x - M.mw[0] * nd.z);
+  const double vz = M.mv[2] + (M.mw[0] * nd.y - M.mw[1] * nd.x);
+  M.node_v[q] = make_double4(vx, vy, vz, 0.0);
+  const double x = nd.x + vx * dt, y = nd.y + vy * dt, z = nd.z + vz * dt;
+  M.node[q] = make_double4(x, y, z, 0.0);
+  if (q == 0 && M.off32)   // node 0 in FP32 for the law-1 early-out
+    M.off32[0] = make_float4((float)x, (float)y, (float)z, 0.f);
+}
