@@ -26,8 +26,8 @@ def _same(a, b):
             assert np.array_equal(p, q)
 
 
-# 11^3 and 27^3 particles take eight lanes each in FP64, 29^3 one (the line is at 24,000)
-@pytest.mark.parametrize("side", [3, 11, 27, 29])
+# 3^3 and 11^3 particles take 32 lanes each in FP64, 13^3 16, 27^3 and 29^3 eight, 40^3 one
+@pytest.mark.parametrize("side", [3, 11, 13, 27, 29, 40])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_heat_solve_with_kept_factors_is_bit_identical(side, precision):
     sc = S.heat_box(n_side=side)
@@ -47,3 +47,10 @@ def test_heat_solve_fp64_far_below_the_normal_temperatures(side):
     sc["T"] = np.where(x < 0.2, 0.0, 10.0 ** (-320.0 * x) * 1.0e3)
     sc["T_inf"] = 0.0
     _same(_solve(sc, 0, 1, (6,)), _solve(sc, 0, 0, (6,)))
+
+
+def test_heat_solve_mixed_with_lists_beyond_16_bits():
+    """A box whose cell layers hold more than 32,768 particles: the lists of most tiles span more
+    than 65,536 slots and stay 32 bits wide, those of the outer layers are kept as 16-bit offsets."""
+    sc = S.heat_box(n_side=120)
+    _same(_solve(sc, 1, 1, (1, 3)), _solve(sc, 1, 0, (1, 3)))

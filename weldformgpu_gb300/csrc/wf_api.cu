@@ -1937,13 +1937,15 @@ int wf_thermal_solve(wf_domain* d, double tf) {
   const bool mixed = d->precision == 1;
   const int64_t entries = (int64_t)WF_NB_ALLOC * d->npad, n = d->npad;
   const bool kept = d->time < tf &&
-                    work_reserve(d, mixed ? (size_t)(4 * entries + 16 * n)
+                    work_reserve(d, mixed ? (size_t)(6 * entries + 17 * n)
                                           : sizeof(double) * (size_t)(2 * entries + 5 * n));
   HeatWork64 H64{};
   HeatWork32 H32{};
   if (kept && mixed) {
     H32.own = reinterpret_cast<float4*>(d->work);
     H32.mg = reinterpret_cast<float*>(H32.own + n);
+    H32.off = reinterpret_cast<uint16_t*>(H32.mg + entries);
+    H32.base = reinterpret_cast<int32_t*>(H32.off + entries);   // one per 128 slots
     launch_heat_pairs32(P, CF(d), H32, N, d->stream);
     d->launches += 1;
   } else if (kept) {

@@ -409,6 +409,8 @@ struct HeatWork64 {
 };
 struct HeatWork32 {
   float* mg;       // per list entry: m_j / rho_j GK
+  uint16_t* off;   // per list entry: slot - base of its tile of 128 slots
+  int32_t* base;   // per tile; -1: its lists span more than 65,536 slots (32-bit lists)
   float4* own;     // per slot: rho cp, h_conv dS^2 (0: no convection), m cp, frictional heat rate
 };
 void launch_heat_pairs64(const StepParams& P, const Fields& F, const HeatWork64& H,

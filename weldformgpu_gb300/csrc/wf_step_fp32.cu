@@ -378,19 +378,54 @@ __global__ void __launch_bounds__(128, kDensMinBlocks) k_heat32(StepParams P, Fi
 // to another.  T, Tb and dT/dt feed nothing inside a solve and are written by
 // its last step only.  Same operations in the same order as k_heat32 and
 // k_heat_leapfrog.
+// A step streams the lists and factors and is bound by HBM, so the lists are
+// kept as 16-bit offsets from the tile's smallest slot where they span no more
+// than 65,536 (in cell order a tile's lists reach one cell layer down and up:
+// boxes up to ~115 particles a side; other tiles keep the 32-bit lists):
+// 428 bytes a particle instead of 556, a million particles 80 -> 75 us a step
+// (70 with lists and factors read past L1; 48 registers, and a bound that
+// forces fewer spills: 12 blocks an SM 88 us; blocks of 256 72 us).
 __global__ void __launch_bounds__(128) k_heat_pairs32(StepParams P, Fields F, HeatWork32 H,
                                                       const int32_t* __restrict__ nb,
                                                       const int32_t* __restrict__ cnt) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= P.n) return;
+  static_assert(WF_TILE == 128, "a block is a tile");
+  __shared__ int s_lo[4], s_hi[4];
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const bool valid = i0 < P.n;
+  const int64_t i = valid ? i0 : P.n - 1;
+  const int c = valid ? cnt[i] : 0;
+  const NbList32 list{nb, P.npad, i};
+  // the tile's smallest and largest slot
+  int lo = (int)i, hi = (int)i;
+  for (int b = 0; WF_NB_BLK * b < c; b++) {
+    int js[WF_NB_BLK];
+    list.block(b, js);
+#pragma unroll
+    for (int q = 0; q < WF_NB_BLK; q++) {
+      lo = min(lo, js[q]);
+      hi = max(hi, js[q]);
+    }
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) { s_lo[threadIdx.x >> 5] = lo; s_hi[threadIdx.x >> 5] = hi; }
+  __syncthreads();
+  for (int w = 0; w < 4; w++) { lo = min(lo, s_lo[w]); hi = max(hi, s_hi[w]); }
+  const bool near = hi - lo < 65536;
+  if (threadIdx.x == 0) H.base[blockIdx.x] = near ? lo : -1;
+  if (!valid) return;
   const float4 pi = F.pv[i].p;
   const float invh = P.invhf, C = P.Cf, Ch = P.Chf;
-  const int c = cnt[i];
-  const NbList32 list{nb, P.npad, i};
   for (int b = 0; WF_NB_BLK * b < c; b++) {
     int js[WF_NB_BLK];
     float mg[WF_NB_BLK];
     list.block(b, js);
+    if (near)
+      *reinterpret_cast<uint4*>(H.off + ((int64_t)b * P.npad + i) * WF_NB_BLK) =
+          make_uint4((unsigned)(js[0] - lo) | (unsigned)(js[1] - lo) << 16,
+                     (unsigned)(js[2] - lo) | (unsigned)(js[3] - lo) << 16,
+                     (unsigned)(js[4] - lo) | (unsigned)(js[5] - lo) << 16,
+                     (unsigned)(js[6] - lo) | (unsigned)(js[7] - lo) << 16);
 #pragma unroll
     for (int q = 0; q < WF_NB_BLK; q++) {
       const float4 pj = __ldg(&F.pv[js[q]].p);
@@ -409,7 +444,40 @@ __global__ void __launch_bounds__(128) k_heat_pairs32(StepParams P, Fields F, He
   H.own[i] = make_float4(rf * cpf, conv, mf * cpf, fric);
 }
 
-__global__ void __launch_bounds__(128) k_heat_step32(StepParams P, Fields F, HeatWork32 H,
+// four values read once: past L1
+__device__ __forceinline__ void ld_stream4(const float* p, float* v) {
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+      : "l"(p));
+}
+// the heat sum from the kept factors over the list L
+template <class L>
+__device__ __forceinline__ float heat_step_pairs(const float* __restrict__ factors,
+                                                 const float2* __restrict__ th, const L& list,
+                                                 int64_t npad, int64_t i, int c, float2 ti) {
+  float sf = 0.0f;
+  int nx[WF_NB_BLK];
+  if (c > 0) list.block(0, nx);
+  for (int b = 0; WF_NB_BLK * b < c; b++) {
+    float2 tj[WF_NB_BLK];
+#pragma unroll
+    for (int q = 0; q < WF_NB_BLK; q++) tj[q] = __ldg(th + nx[q]);
+    float mg[WF_NB_BLK];
+    const float* f = factors + ((int64_t)b * npad + i) * WF_NB_BLK;
+    ld_stream4(f, mg);
+    ld_stream4(f + 4, mg + 4);
+    if (c > WF_NB_BLK * (b + 1)) list.block(b + 1, nx);
+#pragma unroll
+    for (int q = 0; q < WF_NB_BLK; q++) {
+      const float dT = (ti.x - tj[q].x) + (ti.y - tj[q].y);
+      sf += mg[q] * dT;
+    }
+  }
+  return sf;
+}
+
+constexpr int kHeatStepThreads = 128;
+__global__ void __launch_bounds__(kHeatStepThreads) k_heat_step32(StepParams P, Fields F, HeatWork32 H,
                                                      const float2* __restrict__ th,
                                                      float2* __restrict__ th_out,
                                                      const int32_t* __restrict__ nb,
@@ -419,25 +487,10 @@ __global__ void __launch_bounds__(128) k_heat_step32(StepParams P, Fields F, Hea
   if (i >= P.n) return;
   const float2 ti = th[i];
   const int c = cnt[i];
-  const NbList32 list{nb, P.npad, i};
-  float sf = 0.0f;
-  int nx[WF_NB_BLK];
-  if (c > 0) list.block(0, nx);
-  for (int b = 0; WF_NB_BLK * b < c; b++) {
-    float2 tj[WF_NB_BLK];
-#pragma unroll
-    for (int q = 0; q < WF_NB_BLK; q++) tj[q] = __ldg(th + nx[q]);
-    const float4* m4 =
-        reinterpret_cast<const float4*>(H.mg + ((int64_t)b * P.npad + i) * WF_NB_BLK);
-    const float4 ma = __ldg(m4), mb = __ldg(m4 + 1);
-    if (c > WF_NB_BLK * (b + 1)) list.block(b + 1, nx);
-    const float mg[WF_NB_BLK] = {ma.x, ma.y, ma.z, ma.w, mb.x, mb.y, mb.z, mb.w};
-#pragma unroll
-    for (int q = 0; q < WF_NB_BLK; q++) {
-      const float dT = (ti.x - tj[q].x) + (ti.y - tj[q].y);
-      sf += mg[q] * dT;
-    }
-  }
+  const int b16 = H.base[i / WF_TILE];         // uniform over the warp
+  const float sf =
+      b16 >= 0 ? heat_step_pairs(H.mg, th, NbList16{H.off, P.npad, i, b16}, P.npad, i, c, ti)
+               : heat_step_pairs(H.mg, th, NbList32{nb, P.npad, i}, P.npad, i, c, ti);
   const float4 own = H.own[i];
   float sm = P.k2f * sf / own.x;
   if (own.w > 0.0f) sm += own.w;
@@ -1214,7 +1267,7 @@ void launch_heat_pairs32(const StepParams& P, const Fields& F, const HeatWork32&
 }
 void launch_heat_step32(const StepParams& P, const Fields& F, const HeatWork32& H, float2* th_out,
                         const NbBuffers& N, int first, int last, cudaStream_t s) {
-  k_heat_step32<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, H, F.th32, th_out, N.nb, N.cnt, first,
+  k_heat_step32<<<blocks_for(P.n, kHeatStepThreads), kHeatStepThreads, 0, s>>>(P, F, H, F.th32, th_out, N.nb, N.cnt, first,
                                                      last);
 }
 void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, const Sig32& sig,
