@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(128) k_mlp_newton_iters(StepParams P, double G
 // the latency of its two kernels, not arithmetic (0.1 GFLOP) or memory.  The
 // kernel before this one took a sample per thread and walked 64 x 64 products
 // serially on 32 blocks: 372 -> 16 us per 4,096 samples (a step with Adam 382
-// -> 21 us; 256 threads per block: 17 us).
+// -> 21 us; 256 threads per block: 17 us; as k_mlp_train 16.5).
 constexpr int kTile = 32;              // samples per tile
 constexpr int kGradThreads = 512;
 constexpr int kGradBlocks = 304;       // most blocks (rows of partial sums): 2 per SM
@@ -199,35 +200,52 @@ __device__ __forceinline__ float dot4(float acc, const float4& a, const float4& 
   return acc;
 }
 
-__global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const float* __restrict__ P,
-                                                          const float4* __restrict__ X,
-                                                          const float* __restrict__ Yt,
-                                                          int64_t offset, int64_t count,
-                                                          float inv_total,
-                                                          float* __restrict__ part) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+// The block's sums over its tiles into its row of partial sums.  The parameters
+// are read from L2: inside k_mlp_train other blocks have just written them.
+__device__ __forceinline__ void grad_block(unsigned char* smem_raw, const float* P,
+                                           const float4* __restrict__ X,
+                                           const float* __restrict__ Yt, int64_t offset,
+                                           int64_t count, float inv_total, int rows, float* row) {
   GradShared& S = *reinterpret_cast<GradShared*>(smem_raw);
   const int t = threadIdx.x;
-  for (int k = t; k < WF_MLP_H * WF_MLP_H; k += kGradThreads)
-    S.W2[(k / WF_MLP_H) * LDA + k % WF_MLP_H] = P[WF_MLP_OFF_W2 + k];
-  if (t < 4 * WF_MLP_H) S.W1[t] = P[WF_MLP_OFF_W1 + t];
-  if (t < WF_MLP_H) {
-    S.b1[t] = P[WF_MLP_OFF_B1 + t];
-    S.b2[t] = P[WF_MLP_OFF_B2 + t];
-    S.w3[t] = P[WF_MLP_OFF_W3 + t];
-  }
-  const float b3 = P[WF_MLP_OFF_B3];
   const int ts = t >> 4, to = t & 15;          // sample ts; 16 threads share it
+  const int64_t tiles = (count + kTile - 1) / kTile;
+  // the first tile's samples are on their way while the weights are loaded
+  float4 x_next = make_float4(0.f, 0.f, 0.f, 0.f);
+  float target_next = 0.0f;
+  const auto fetch = [&](int64_t tile) {
+    const int64_t gi = tile * kTile + ts;
+    const bool v = tile < tiles && gi < count;
+    x_next = v ? X[offset + gi] : make_float4(0.f, 0.f, 0.f, 0.f);
+    target_next = v ? Yt[offset + gi] : 0.0f;
+  };
+  fetch(blockIdx.x);
+  static_assert(WF_MLP_OFF_W2 % 4 == 0 && WF_MLP_H * WF_MLP_H == 8 * kGradThreads, "16-byte loads");
+  float4 wv[2];
+#pragma unroll
+  for (int q = 0; q < 2; q++)
+    wv[q] = __ldcg(reinterpret_cast<const float4*>(P + WF_MLP_OFF_W2) + t + q * kGradThreads);
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int k = 4 * (t + q * kGradThreads);
+    *reinterpret_cast<float4*>(S.W2 + (k / WF_MLP_H) * LDA + k % WF_MLP_H) = wv[q];
+  }
+  if (t < 4 * WF_MLP_H) S.W1[t] = __ldcg(P + WF_MLP_OFF_W1 + t);
+  if (t < WF_MLP_H) {
+    S.b1[t] = __ldcg(P + WF_MLP_OFF_B1 + t);
+    S.b2[t] = __ldcg(P + WF_MLP_OFF_B2 + t);
+    S.w3[t] = __ldcg(P + WF_MLP_OFF_W3 + t);
+  }
+  const float b3 = __ldcg(P + WF_MLP_OFF_B3);
   float4 gW2[2] = {}, gW1[4] = {};             // gW2 rows 2 ts + r, columns 4 to; gW1 of unit 4 to + r
   float4 gb1 = {};                             // units 4 to ..
   float gb2[4] = {}, gw3[4] = {};              // units to + 16 r
   float gb3 = 0.0f, loss = 0.0f;
-  const int64_t tiles = (count + kTile - 1) / kTile;
-  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int64_t gi = tile * kTile + ts;
-    const bool valid = gi < count;
-    const float4 x = valid ? X[offset + gi] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float target = valid ? Yt[offset + gi] : 0.0f;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += rows) {
+    const bool valid = tile * kTile + ts < count;
+    const float4 x = x_next;
+    const float target = target_next;
+    fetch(tile + rows);
     __syncthreads();                           // the last tile's arrays are done with
     if (to == 0) S.X[ts] = x;
     {  // layer 1: units 4 to .. 4 to + 3
@@ -305,7 +323,6 @@ __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const float* __restri
       fma4(gW2[1], g.y, h);
     }
   }
-  float* row = part + (int64_t)blockIdx.x * kPartRow;
 #pragma unroll
   for (int r = 0; r < 2; r++)
     *reinterpret_cast<float4*>(row + WF_MLP_OFF_W2 + (2 * ts + r) * WF_MLP_H + 4 * to) = gW2[r];
@@ -349,15 +366,27 @@ __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const float* __restri
   row[at] = a;
 }
 
-// The rows' sum of value k on the first 32 threads of a block of 256, value
-// 32 blockIdx.x + lane: eight threads per value, each every eighth row.
-__device__ __forceinline__ float total_of_rows(const float* __restrict__ part, int rows) {
-  __shared__ float sum[8][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const float* p = part + blockIdx.x * 32 + lane;
+__global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const float* __restrict__ P,
+                                                          const float4* __restrict__ X,
+                                                          const float* __restrict__ Yt,
+                                                          int64_t offset, int64_t count,
+                                                          float inv_total,
+                                                          float* __restrict__ part) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  grad_block(smem_raw, P, X, Yt, offset, count, inv_total, (int)gridDim.x,
+             part + (int64_t)blockIdx.x * kPartRow);
+}
+
+// The rows' sum of value 32 chunk + lane, on every thread of the eight warps w
+// that share a chunk: eight threads per value, each every eighth row.  Every
+// thread of the block takes part.
+__device__ __forceinline__ float total_of_rows(float (*sum)[32], const float* part, int rows,
+                                               int chunk, int w) {
+  const int lane = threadIdx.x & 31;
+  const float* p = part + chunk * 32 + lane;
   float a = 0.0f;
-#pragma unroll 8
-  for (int r = w; r < rows; r += 8) a += p[(int64_t)r * kPartRow];
+#pragma unroll 16
+  for (int r = w; r < rows; r += 8) a += __ldcg(p + (int64_t)r * kPartRow);
   sum[w][lane] = a;
   __syncthreads();
   a = 0.0f;
@@ -368,29 +397,117 @@ __device__ __forceinline__ float total_of_rows(const float* __restrict__ part, i
 __global__ void __launch_bounds__(256) k_grad_total(const float* __restrict__ part, int rows,
                                                     float* __restrict__ grad,
                                                     float* __restrict__ loss) {
-  const float a = total_of_rows(part, rows);
+  __shared__ float sum[8][32];
+  const float a = total_of_rows(sum, part, rows, blockIdx.x, threadIdx.x >> 5);
   const int k = blockIdx.x * 32 + threadIdx.x;
   if (threadIdx.x >= 32) return;
   if (k < WF_MLP_NPARAM) grad[k] = a;
   else if (k == WF_MLP_NPARAM) *loss = a;
 }
 
-// one Adam step from the blocks' partial sums
-__global__ void __launch_bounds__(256) k_adam(float* __restrict__ P, const float* __restrict__ part,
-                                              int rows, float* __restrict__ m,
-                                              float* __restrict__ v, float* __restrict__ loss,
-                                              float lr, float b1, float b2, float eps, float c1,
-                                              float c2) {
-  const float gk = total_of_rows(part, rows);
-  const int k = blockIdx.x * 32 + threadIdx.x;
-  if (threadIdx.x >= 32) return;
-  if (k == WF_MLP_NPARAM) *loss = gk;
-  if (k >= WF_MLP_NPARAM) return;
-  const float mk = b1 * m[k] + (1.0f - b1) * gk;
-  const float vk = b2 * v[k] + (1.0f - b2) * gk * gk;
-  m[k] = mk;
-  v[k] = vk;
-  P[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+// A step's learning rate and the moments' bias corrections
+struct AdamStep {
+  float lr, c1, c2;
+};
+struct AdamState {
+  float *P, *m, *v;
+};
+// one Adam step of value k (the value behind the last parameter is the loss): its
+// state is loaded while the gradient is summed
+struct AdamValue {
+  float p = 0.0f, m = 0.0f, v = 0.0f;
+  __device__ __forceinline__ void load(const AdamState& A, int k) {
+    if (k >= WF_MLP_NPARAM) return;
+    p = __ldcg(A.P + k);
+    m = A.m[k];
+    v = A.v[k];
+  }
+  __device__ __forceinline__ void step(const AdamState& A, int k, float gk, const AdamStep& c,
+                                       float* loss) const {
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    if (k == WF_MLP_NPARAM) *loss = gk;
+    if (k >= WF_MLP_NPARAM) return;
+    const float mk = b1 * m + (1.0f - b1) * gk;
+    const float vk = b2 * v + (1.0f - b2) * gk * gk;
+    A.m[k] = mk;
+    A.v[k] = vk;
+    A.P[k] = p - c.lr * (mk / c.c1) / (sqrtf(vk / c.c2) + eps);
+  }
+};
+
+__global__ void __launch_bounds__(256) k_adam(AdamState A, const float* __restrict__ part, int rows,
+                                              float* __restrict__ loss, AdamStep c) {
+  __shared__ float sum[8][32];
+  const int k = threadIdx.x < 32 ? blockIdx.x * 32 + threadIdx.x : INT_MAX;
+  AdamValue value;
+  value.load(A, k);
+  const float gk = total_of_rows(sum, part, rows, blockIdx.x, threadIdx.x >> 5);
+  value.step(A, k, gk, c, loss);
+}
+
+// ---- many training steps in one cooperative launch ------------------------------
+// As two launches a step, 4,096 samples take 21 us, several of them the launches
+// and the kernels' ramps.  Here the blocks stay: each step is the gradient of
+// its rows, a barrier of the grid, Adam on 32 values per half block, and a
+// second barrier; the sums and their order are those of the two kernels.
+// 16.5 us a step: gradient 10.5 (the tile's products 7, by shared memory reads
+// and their latency), Adam 3.7, the barriers 2.4.  The blocks must all be
+// resident (a cooperative launch, one block an SM: batches of up to 32 samples
+// an SM; larger ones take the two kernels).  A barrier gives up after
+// kSpinLimit polls (seconds): the block sets `bad` and leaves, and so do the
+// others.
+constexpr int kSpinLimit = 1 << 22;
+constexpr int64_t kTrainChunk = 1024;        // most steps of a launch
+
+__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned goal, int* bad) {
+  __syncthreads();
+  bool ok = true;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrived, 1u);
+    int n = 0;
+    unsigned v;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+    } while ((int)(v - goal) < 0 && ++n < kSpinLimit);
+    ok = (int)(v - goal) >= 0;
+    if (!ok) atomicExch(bad, 1);
+  }
+  return __syncthreads_and(ok);
+}
+
+__global__ void __launch_bounds__(kGradThreads) k_mlp_train(
+    AdamState A, const float4* __restrict__ X, const float* __restrict__ Yt, int64_t n,
+    int64_t batch, int64_t off, const AdamStep* __restrict__ sched, int steps, float* part,
+    float* loss, unsigned* arrived, int* bad) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ float sum[2][8][32];
+  const int half = threadIdx.x >> 8, w = (threadIdx.x >> 5) & 7, lane = threadIdx.x & 31;
+  unsigned goal = 0;
+  for (int st = 0; st < steps; st++) {
+    const int64_t cnt = min(batch, n - off);
+    const int rows = (int)min((cnt + kTile - 1) / kTile, (int64_t)kGradBlocks);
+    if ((int)blockIdx.x < rows)
+      grad_block(smem_raw, A.P, X, Yt, off, cnt, 1.0f / (float)cnt, rows,
+                 part + (int64_t)blockIdx.x * kPartRow);
+    goal += gridDim.x;
+    if (!grid_barrier(arrived, goal, bad)) return;
+    const AdamStep c = sched[st];
+    for (int base = 0; base < kPartRow / 32; base += 2 * gridDim.x) {     // whole blocks together
+      const int chunk = base + 2 * blockIdx.x + half;
+      const bool mine = chunk < kPartRow / 32;
+      const int k = mine && w == 0 ? chunk * 32 + lane : INT_MAX;
+      AdamValue value;
+      value.load(A, k);
+      const float gk = total_of_rows(sum[half], part, mine ? rows : 0, mine ? chunk : 0, w);
+      value.step(A, k, gk, c, loss + st);
+      __syncthreads();
+    }
+    goal += gridDim.x;
+    if (!grid_barrier(arrived, goal, bad)) return;
+    off += cnt;
+    if (off >= n) off = 0;
+  }
 }
 
 // partial-sum rows (blocks) of a gradient over `count` samples
@@ -399,8 +516,22 @@ int grad_rows(int64_t count) {
 }
 // the opt-in for the gradient kernel's shared memory, on the current device
 cudaError_t grad_ready() {
-  return cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sizeof(GradShared));
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradShared));
+  return e != cudaSuccess ? e
+                          : cudaFuncSetAttribute(k_mlp_train,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)sizeof(GradShared));
+}
+// do `blocks` blocks of k_mlp_train run at once on the current device?
+bool train_fits(int blocks) {
+  int dev = 0, coop = 0, sms = 0, per = 0;
+  return cudaGetDevice(&dev) == cudaSuccess &&
+         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mlp_train, kGradThreads,
+                                                       sizeof(GradShared)) == cudaSuccess &&
+         blocks <= per * sms;
 }
 
 StepParams jc_params(const wf_material* m, double rtol) {
@@ -503,42 +634,71 @@ int wf_mlp_grad(const float* params, const float* X, const float* Y, int64_t n, 
 int wf_mlp_train(float* params, const float* X, const float* Y, int64_t n, int64_t steps,
                  int64_t batch, float lr, float* final_loss) {
   if (!params || !X || !Y || n <= 0 || steps <= 0 || batch <= 0) return WF_ERR_ARG;
-  // one device block: samples, targets, parameters and moments, partial sums, losses
+  // one device block: samples, targets, parameters and moments, partial sums, losses, the steps'
+  // rates, the barrier's words
   const int most = grad_rows(std::min<int64_t>(batch, n));
   const auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t bX = up(sizeof(float4) * n), bY = up(sizeof(float) * n),
-               bP = up(sizeof(float) * WF_MLP_NPARAM), bR = up(sizeof(float) * most * kPartRow);
+               bP = up(sizeof(float) * WF_MLP_NPARAM), bR = up(sizeof(float) * most * kPartRow),
+               bL = up(sizeof(float) * steps), bS = up(sizeof(AdamStep) * steps);
   DevBufs B;
-  char* base = B.get<char>(bX + bY + 3 * bP + bR + sizeof(float) * steps);
+  char* base = B.get<char>(bX + bY + 3 * bP + bR + bL + bS + 256);
   if (!base) return WF_ERR_ALLOC;
   float4* dX = (float4*)base;
   float* dY = (float*)(base + bX);
   float* dP = (float*)(base + bX + bY);
-  float* dM = (float*)((char*)dP + bP);
-  float* dV = (float*)((char*)dM + bP);
-  float* dR = (float*)((char*)dV + bP);
+  const AdamState A{dP, (float*)((char*)dP + bP), (float*)((char*)dP + 2 * bP)};
+  float* dR = (float*)((char*)dP + 3 * bP);
   float* dL = (float*)((char*)dR + bR);
+  AdamStep* dS = (AdamStep*)((char*)dL + bL);
+  unsigned* dB = (unsigned*)((char*)dS + bS);          // barrier arrivals, failure
+  std::vector<AdamStep> sched(steps);
+  double p1 = 1.0, p2 = 1.0;
+  for (int64_t st = 0; st < steps; st++) {
+    p1 *= 0.9f;
+    p2 *= 0.999f;
+    // cosine decay of the learning rate
+    sched[st] = AdamStep{lr * 0.5f * (1.0f + cosf(3.14159265f * (float)st / (float)steps)),
+                         (float)(1.0 - p1), (float)(1.0 - p2)};
+  }
   cudaMemcpy(dP, params, sizeof(float) * WF_MLP_NPARAM, cudaMemcpyHostToDevice);
   cudaMemcpy(dX, X, sizeof(float) * 4 * n, cudaMemcpyHostToDevice);
   cudaMemcpy(dY, Y, sizeof(float) * n, cudaMemcpyHostToDevice);
-  cudaMemset(dM, 0, 2 * bP);
+  cudaMemset(A.m, 0, 2 * bP);
   if (grad_ready() != cudaSuccess) return WF_ERR_CUDA;
-  const float b1 = 0.9f, b2 = 0.999f;
-  double p1 = 1.0, p2 = 1.0;
   int64_t off = 0;
-  for (int64_t st = 0; st < steps; st++) {
-    const int64_t cnt = std::min<int64_t>(batch, n - off);
-    const int rows = grad_rows(cnt);
-    k_mlp_grad<<<rows, kGradThreads, sizeof(GradShared)>>>(dP, dX, dY, off, cnt, 1.0f / (float)cnt,
-                                                          dR);
-    p1 *= b1;
-    p2 *= b2;
-    // cosine decay of the learning rate
-    const float lr_t = lr * 0.5f * (1.0f + cosf(3.14159265f * (float)st / (float)steps));
-    k_adam<<<kPartRow / 32, 256>>>(dP, dR, rows, dM, dV, dL + st, lr_t, b1, b2, 1e-8f,
-                                   (float)(1.0 - p1), (float)(1.0 - p2));
-    off += cnt;
-    if (off >= n) off = 0;
+  if (train_fits(most)) {
+    cudaMemcpy(dS, sched.data(), sizeof(AdamStep) * steps, cudaMemcpyHostToDevice);
+    cudaMemset(dB, 0, 2 * sizeof(unsigned));
+    for (int64_t st = 0; st < steps; st += kTrainChunk) {
+      int count = (int)std::min<int64_t>(kTrainChunk, steps - st);
+      cudaMemsetAsync(dB, 0, sizeof(unsigned));
+      const AdamStep* s0 = dS + st;
+      float* l0 = dL + st;
+      int* bad = (int*)dB + 1;
+      AdamState state = A;
+      void* args[] = {&state, &dX, &dY, &n, &batch, &off, &s0, &count, &dR, &l0, &dB, &bad};
+      if (cudaLaunchCooperativeKernel((const void*)k_mlp_train, dim3(most), dim3(kGradThreads),
+                                      args, sizeof(GradShared), nullptr) != cudaSuccess)
+        return WF_ERR_CUDA;
+      for (int k = 0; k < count; k++) {                // where the next launch begins
+        off += std::min<int64_t>(batch, n - off);
+        if (off >= n) off = 0;
+      }
+    }
+    int bad = 0;
+    if (cudaMemcpy(&bad, dB + 1, sizeof bad, cudaMemcpyDeviceToHost) != cudaSuccess || bad)
+      return WF_ERR_CUDA;
+  } else {
+    for (int64_t st = 0; st < steps; st++) {
+      const int64_t cnt = std::min<int64_t>(batch, n - off);
+      const int rows = grad_rows(cnt);
+      k_mlp_grad<<<rows, kGradThreads, sizeof(GradShared)>>>(dP, dX, dY, off, cnt,
+                                                            1.0f / (float)cnt, dR);
+      k_adam<<<kPartRow / 32, 256>>>(A, dR, rows, dL + st, sched[st]);
+      off += cnt;
+      if (off >= n) off = 0;
+    }
   }
   cudaMemcpy(params, dP, sizeof(float) * WF_MLP_NPARAM, cudaMemcpyDeviceToHost);
   if (final_loss) {
