@@ -93,9 +93,13 @@ struct wf_domain {
   uint32_t *cell_count = nullptr, *cell_cursor = nullptr, *scan_tmp = nullptr;
   int64_t cell_cap = 0;
   int32_t *s_src = nullptr, *s_orig = nullptr;
-  int* d_mm = nullptr;
+  int* d_mm = nullptr;         // flags; [6], [7]: largest halo and halo entries of a tile build
+  StaticHeader* d_hdr = nullptr;   // search grid of a rebuild
+  cudaEvent_t ev_rb = nullptr;     // its host copy is written
+  int64_t ncell_last = 0;          // cells of the last grid
+  bool rb_pending = false;         // lists built on a grid that the host has not seen yet
   int* d_status = nullptr;     // WF_STATUS_WORDS words (wf_common.cuh)
-  int* h_status = nullptr;     // pinned mirror
+  int* h_status = nullptr;     // pinned mirror, and behind it that of the search grid
   // FP64 output rows (wf_outputs.cu): recorded at output times, or every step
   // with option output_every_step; the series holds up to series_cap rows
   double4* fr = nullptr;       // m a before the BCs at BC-zone slots (written on row steps)
@@ -436,6 +440,7 @@ static void layout_arena(wf_domain* d, Arena& A) {
   A.take(&d->nb, (int64_t)WF_NB_ALLOC * n); A.take(&d->nbc, n); A.take(&d->inv, n);
   A.take(&d->pf, n); A.take(&d->pf2, n); A.take(&d->cellid, n); A.take(&d->s_src, n);
   A.take(&d->s_orig, n); A.take(&d->d_mm, 8); A.take(&d->d_status, WF_STATUS_WORDS);
+  A.take(&d->d_hdr, 1);
   A.take(&d->d_cstat, 2);
   A.take(&d->fr, n); A.take(&d->out_part, wf_out_partial_words(WF_MAX_BC));
   A.take(&d->e0, 1); A.take(&d->d_zone, 2);
@@ -657,13 +662,17 @@ static StepParams make_params(const wf_domain* d) {
 // replay does the same work in the same order.  The instantiated graph is
 // kept and updated in place when the next segment has the same launches.
 // Not used with the adaptive rebuild or CSV snapshots (host reads every step).
+static bool segments(const wf_domain* d) {
+  return d->graph && !(d->rb_dep > 0.0) && !d->csv_on && !d->after_fn;
+}
 static int segment_begin(wf_domain* d) {
-  if (!d->graph || d->capturing || d->rb_dep > 0.0 || d->csv_on || d->after_fn) return WF_OK;
+  if (d->capturing || !segments(d)) return WF_OK;
   WF_CUDA_OK(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeRelaxed));
   d->capturing = true;
   return WF_OK;
 }
 
+static int rebuild_verify(wf_domain* d);
 static int segment_end(wf_domain* d) {
   if (!d->capturing) return WF_OK;
   d->capturing = false;
@@ -677,7 +686,7 @@ static int segment_end(wf_domain* d) {
   cudaGraphGetNodes(g, nullptr, &nodes);
   if (nodes == 0) {
     cudaGraphDestroy(g);
-    return WF_OK;
+    return rebuild_verify(d);
   }
   bool updated = false;
   if (d->gexec) {
@@ -699,6 +708,8 @@ static int segment_end(wf_domain* d) {
     d->graph_instantiations++;
   }
   cudaGraphDestroy(g);
+  const int rc = rebuild_verify(d);      // the lists that the segment's steps read
+  if (rc) return rc;
   WF_CUDA_OK(cudaGraphLaunch(d->gexec, d->stream));
   d->graph_launches++;
   return WF_OK;
@@ -797,42 +808,34 @@ static Work64 work64_of(const wf_domain* d) {
 
 constexpr int kReorderEvery = 20;   // physical reorder at every 20th rebuild of a solve
 
-static int rebuild(wf_domain* d, bool use_current, bool light = false) {
-  {
-    const int rc = segment_end(d);
-    if (rc) return rc;
-  }
-  KTimer t(d, KID_REBUILD);
-  d->geo_valid = false;
+static StaticHeader* host_header(const wf_domain* d) {
+  return reinterpret_cast<StaticHeader*>(d->h_status + WF_STATUS_WORDS);
+}
+// the grid from the bounds' codes, and room for its cells
+static int grid_from_codes(wf_domain* d, const unsigned* codes) {
+  int bounds[6];
+  bounds_from_codes(codes, bounds);
+  grid_from_bounds(bounds, (float)(2.0 * d->h), &d->grid);
+  const int64_t ncell = (int64_t)d->grid.dim[0] * d->grid.dim[1] * d->grid.dim[2];
+  if (ncell > (int64_t)2000000000) return wf_fail(d, WF_ERR_NUMERIC, "neighbour grid too large");
+  d->ncell_last = ncell;
+  return ensure_cells(d, ncell);
+}
+
+// The cell sort, reorder (full) and lists of the positions in pf, on the grid
+// d->grid, or the device's (hdr) of about ncell_last cells.
+static int build_lists(wf_domain* d, const StaticHeader* hdr, bool full) {
   const int64_t n = d->n;
   cudaStream_t s = d->stream;
   Fields& A = d->F[d->cur];
   Fields& B = d->F[1 - d->cur];
-  const float r = (float)(2.0 * d->h);                // SolverFraser.cu:72-82
-  launch_prep_bounds(n, A, use_current ? 1 : 0, d->pf, r, reinterpret_cast<unsigned*>(d->d_mm), s);
-  int mm[8];   // the bounds' codes, then the largest halo of the previous tile build
-  WF_CUDA_OK(cudaMemcpyAsync(mm, d->d_mm, sizeof mm, cudaMemcpyDeviceToHost, s));
-  WF_CUDA_OK(cudaStreamSynchronize(s));
-  if (d->tile_cap > 0) d->tile_hmax = mm[6];
-  int bounds[6];
-  bounds_from_codes(reinterpret_cast<const unsigned*>(mm), bounds);
-  grid_from_bounds(bounds, r, &d->grid);
-  const int64_t ncell = (int64_t)d->grid.dim[0] * d->grid.dim[1] * d->grid.dim[2];
-  if (ncell > (int64_t)2000000000) return wf_fail(d, WF_ERR_NUMERIC, "neighbour grid too large");
-  int rc = ensure_cells(d, ncell);
-  if (rc) return rc;
-  // The lists hold the same particles in the same order whether or not the
-  // state is moved into the sorted order, so the arithmetic is identical;
-  // moving it keeps warps' particles close in space.  Inside the step loop
-  // the state is moved at every kReorderEvery-th rebuild only (solids move
-  // little in between); otherwise the lists name the particles' current slots.
-  const bool full = !light || ++d->light_rebuilds >= kReorderEvery;
   {
     // pf2 lends its memory to the ranks until the sorted positions go there
     const CellWork W{d->cellid, reinterpret_cast<uint32_t*>(d->pf2), d->cell_cursor, d->scan_tmp + 1,
-                     d->scan_tmp, d->cell_count, 0};
-    WF_CUDA_OK(cudaMemsetAsync(d->cell_cursor, 0, sizeof(uint32_t) * ncell, s));
-    launch_cell_sort(n, d->pf, d->grid, nullptr, A.perm, W, d->s_src, d->s_orig,
+                     d->scan_tmp, d->cell_count, d->cell_cap - 1};
+    WF_CUDA_OK(cudaMemsetAsync(d->cell_cursor, 0,
+                               sizeof(uint32_t) * (hdr ? d->cell_cap : d->ncell_last), s));
+    launch_cell_sort(n, d->pf, d->grid, hdr, A.perm, W, d->s_src, d->s_orig,
                      full ? nullptr : d->pf2, d->d_status, s);
   }
   if (full) {
@@ -840,8 +843,8 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
     d->cur = 1 - d->cur;
     d->light_rebuilds = 0;
   }
-  launch_nblist(n, d->npad, d->pf2, d->grid, d->cell_count, full ? nullptr : d->s_src, d->nb,
-                d->nbc, d->d_status, s);
+  launch_nblist(d->ncell_last, d->npad, d->pf2, d->grid, hdr, d->cell_count,
+                full ? nullptr : d->s_src, d->nb, d->nbc, d->d_status, s);
   d->launches += full ? 7 : 6;
   if (d->debug_checks) {
     if (d->inject_list_error >= 0) {
@@ -881,6 +884,65 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
   WF_CUDA_OK(cudaGetLastError());
   d->nb_built = true;
   return WF_OK;
+}
+
+// Inside the step loop a rebuild does not make the GPU wait for the host: its
+// kernels read the grid from device memory, and the host looks at the bounds
+// only when it has captured the steps behind them, before it launches those.
+// If the grid did not fit the cells allocated (a quarter more than the last one
+// that did not), nothing was searched, and the lists are built then with the
+// cells they need.  (10,752 particles: 55 -> 44 us a rebuild, of which the
+// kernels take most.)
+static int rebuild_verify(wf_domain* d) {
+  if (!d->rb_pending) return WF_OK;
+  d->rb_pending = false;
+  WF_CUDA_OK(cudaEventSynchronize(d->ev_rb));
+  const StaticHeader* h = host_header(d);
+  if (h->ncell > 0) {
+    d->ncell_last = h->ncell;
+    return WF_OK;
+  }
+  const int rc = grid_from_codes(d, h->mm);
+  return rc ? rc : build_lists(d, nullptr, false);
+}
+
+static int rebuild(wf_domain* d, bool use_current, bool light = false) {
+  {
+    const int rc = segment_end(d);
+    if (rc) return rc;
+  }
+  KTimer t(d, KID_REBUILD);
+  d->geo_valid = false;
+  d->rb_pending = false;
+  const int64_t n = d->n;
+  cudaStream_t s = d->stream;
+  Fields& A = d->F[d->cur];
+  // The lists hold the same particles in the same order whether or not the
+  // state is moved into the sorted order, so the arithmetic is identical;
+  // moving it keeps warps' particles close in space.  Inside the step loop
+  // the state is moved at every kReorderEvery-th rebuild only (solids move
+  // little in between); otherwise the lists name the particles' current slots.
+  const bool full = !light || ++d->light_rebuilds >= kReorderEvery;
+  const bool tiles = d->precision == 1 && d->tile_staging && d->meshes.empty();
+  const bool deferred = !full && segments(d) && d->ncell_last > 0 && !d->debug_checks && !tiles &&
+                        d->tile_cap == 0;
+  if (deferred && !d->ev_rb)
+    WF_CUDA_OK(cudaEventCreateWithFlags(&d->ev_rb, cudaEventDisableTiming));
+  const float r = (float)(2.0 * d->h);                // SolverFraser.cu:72-82
+  launch_prep_bounds(n, A, use_current ? 1 : 0, d->pf, r, d->d_hdr, d->cell_cap - 1,
+                     deferred ? host_header(d) : nullptr, s);
+  if (deferred) {
+    WF_CUDA_OK(cudaEventRecord(d->ev_rb, s));
+    d->rb_pending = true;
+    return build_lists(d, d->d_hdr, false);
+  }
+  unsigned mm[6];
+  WF_CUDA_OK(cudaMemcpyAsync(mm, d->d_hdr->mm, sizeof mm, cudaMemcpyDeviceToHost, s));
+  if (d->tile_cap > 0)     // the largest halo of the previous tile build
+    WF_CUDA_OK(cudaMemcpyAsync(&d->tile_hmax, d->d_mm + 6, sizeof(int), cudaMemcpyDeviceToHost, s));
+  WF_CUDA_OK(cudaStreamSynchronize(s));
+  const int rc = grid_from_codes(d, mm);
+  return rc ? rc : build_lists(d, nullptr, full);
 }
 
 // The triangles of each tool binned once in the tool's frame as it stands
@@ -1190,6 +1252,10 @@ static int solve_step_launches(wf_domain* d) {
     const int rc = segment_begin(d);
     if (rc) return rc;
   }
+  if (!d->capturing) {
+    const int rc = rebuild_verify(d);
+    if (rc) return rc;
+  }
   StepParams P = make_params(d);
   // an output row is due after this step: the integration records the BC forces
   const bool row_due = d->out_every_step || d->time + d->dt >= d->t_out;
@@ -1426,7 +1492,8 @@ int wf_create(wf_domain** out, int64_t n) {
     layout_arena(d, place);
   }
   if (!d->h_status &&
-      cudaMallocHost((void**)&d->h_status, WF_STATUS_WORDS * sizeof(int)) != cudaSuccess)
+      cudaMallocHost((void**)&d->h_status,
+                     WF_STATUS_WORDS * sizeof(int) + sizeof(StaticHeader)) != cudaSuccess)
     return bail(WF_ERR_ALLOC);
   k_iota<<<nblk(n), 256, 0, d->stream>>>(n, d->F[0].perm, d->inv);
   k_fill_d<<<nblk(n), 256, 0, d->stream>>>(n, -1.0, d->F[0].pwn, 1, 0);
@@ -1450,6 +1517,7 @@ int wf_destroy(wf_domain* d) {
   if (d->d_maxdep) cudaFree(d->d_maxdep);
   if (d->h_maxdep) cudaFreeHost(d->h_maxdep);
   if (d->ev_maxdep) cudaEventDestroy(d->ev_maxdep);
+  if (d->ev_rb) cudaEventDestroy(d->ev_rb);
   if (d->cnb) cudaFree(d->cnb);
   if (d->ccnt) cudaFree(d->ccnt);
   void* ptrs[] = {d->log_x, d->log_y, d->log_count, d->cell_count, d->series, d->arena};

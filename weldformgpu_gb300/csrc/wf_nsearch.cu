@@ -55,59 +55,16 @@ __device__ __forceinline__ void add_bounds(float4 p, float r, unsigned* lo, unsi
   }
 }
 
-// The float positions the search reads (x_h snapshot or the current ones) and
-// their cell bounds, in one pass.
-__global__ void __launch_bounds__(256) k_prep_bounds(int64_t n, const Fields F, int use_current,
-                                                     float4* __restrict__ pf, float r,
-                                                     unsigned* mm) {
-  unsigned lo[3] = {0u, 0u, 0u}, hi[3] = {0u, 0u, 0u};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float4 p;
-    if (use_current) {
-      const double4 x = F.xm[i];
-      p = make_float4(__double2float_rn(x.x), __double2float_rn(x.y), __double2float_rn(x.z), 0.f);
-    } else {
-      p = F.xh[i];
-    }
-    pf[i] = p;
-    add_bounds(p, r, lo, hi);
-  }
-  reduce_bounds(lo, hi, mm);
-}
-
-// The same for a caller's double3 array (wf_find_neighbors_static), which also
-// zeroes the cell counters; the last block to finish sizes the search grid
-// (grid_from_bounds) and notes whether it fits: the kernels behind it read it
-// from device memory, so the host waits once, at the end (with the cell sort
-// and the lists one warp per cell: 19,488 particles 192 -> 72 us a call, of
-// which the kernels take 48).
-__global__ void __launch_bounds__(256) k_static_prep(int64_t n, const double* __restrict__ x,
-                                                     float4* __restrict__ pf, float r,
-                                                     StaticHeader* __restrict__ hdr,
-                                                     uint32_t* __restrict__ count,
-                                                     int64_t max_cells) {
+// The last block to come here sizes the search grid from the bounds in hdr->mm
+// (grid_from_bounds) and notes whether it fits max_cells; the kernels behind
+// read it from device memory.  True on its thread 0.
+__device__ __forceinline__ bool size_grid(StaticHeader* hdr, float r, int64_t max_cells) {
   __shared__ bool last;
-  unsigned lo[3] = {0u, 0u, 0u}, hi[3] = {0u, 0u, 0u};
-  bool bad = false;
-  const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  for (int64_t i = i0; i < n; i += step) {
-    const double x0 = x[3 * i], x1 = x[3 * i + 1], x2 = x[3 * i + 2];
-    bad |= !isfinite(x0) || !isfinite(x1) || !isfinite(x2);
-    const float4 p =
-        make_float4(__double2float_rn(x0), __double2float_rn(x1), __double2float_rn(x2), 0.0f);
-    pf[i] = p;
-    add_bounds(p, r, lo, hi);
-  }
-  for (int64_t k = i0; k < max_cells; k += step) count[k] = 0u;
-  if (bad) atomicOr(&hdr->status, WF_STATUS_GRID);
-  reduce_bounds(lo, hi, hdr->mm);
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(&hdr->ticket, 1u) == gridDim.x - 1;
   __syncthreads();
-  if (!last || threadIdx.x != 0) return;
+  if (!last || threadIdx.x != 0) return false;
   unsigned mm[6];
   for (int k = 0; k < 6; k++) mm[k] = atomicMax(hdr->mm + k, 0u);
   int64_t ncell = 0;
@@ -130,6 +87,62 @@ __global__ void __launch_bounds__(256) k_static_prep(int64_t n, const double* __
     hdr->grid = g;
   }
   hdr->ncell = fits ? (int)ncell : 0;
+  return true;
+}
+
+// The float positions the search reads (x_h snapshot or the current ones) and
+// their cell bounds, in one pass; with host not null also the grid, and the
+// bounds and the number of cells go to that page-locked copy.
+__global__ void __launch_bounds__(256) k_prep_bounds(int64_t n, const Fields F, int use_current,
+                                                     float4* __restrict__ pf, float r,
+                                                     StaticHeader* hdr, int64_t max_cells,
+                                                     StaticHeader* host) {
+  unsigned lo[3] = {0u, 0u, 0u}, hi[3] = {0u, 0u, 0u};
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    float4 p;
+    if (use_current) {
+      const double4 x = F.xm[i];
+      p = make_float4(__double2float_rn(x.x), __double2float_rn(x.y), __double2float_rn(x.z), 0.f);
+    } else {
+      p = F.xh[i];
+    }
+    pf[i] = p;
+    add_bounds(p, r, lo, hi);
+  }
+  reduce_bounds(lo, hi, hdr->mm);
+  if (!host || !size_grid(hdr, r, max_cells)) return;
+  for (int k = 0; k < 6; k++) host->mm[k] = hdr->mm[k];
+  host->ncell = hdr->ncell;
+}
+
+// The same for a caller's double3 array (wf_find_neighbors_static), which also
+// zeroes the cell counters; the last block to finish sizes the search grid
+// (grid_from_bounds) and notes whether it fits: the kernels behind it read it
+// from device memory, so the host waits once, at the end (with the cell sort
+// and the lists one warp per cell: 19,488 particles 192 -> 72 us a call, of
+// which the kernels take 48).
+__global__ void __launch_bounds__(256) k_static_prep(int64_t n, const double* __restrict__ x,
+                                                     float4* __restrict__ pf, float r,
+                                                     StaticHeader* __restrict__ hdr,
+                                                     uint32_t* __restrict__ count,
+                                                     int64_t max_cells) {
+  unsigned lo[3] = {0u, 0u, 0u}, hi[3] = {0u, 0u, 0u};
+  bool bad = false;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  for (int64_t i = i0; i < n; i += step) {
+    const double x0 = x[3 * i], x1 = x[3 * i + 1], x2 = x[3 * i + 2];
+    bad |= !isfinite(x0) || !isfinite(x1) || !isfinite(x2);
+    const float4 p =
+        make_float4(__double2float_rn(x0), __double2float_rn(x1), __double2float_rn(x2), 0.0f);
+    pf[i] = p;
+    add_bounds(p, r, lo, hi);
+  }
+  for (int64_t k = i0; k < max_cells; k += step) count[k] = 0u;
+  if (bad) atomicOr(&hdr->status, WF_STATUS_GRID);
+  reduce_bounds(lo, hi, hdr->mm);
+  size_grid(hdr, r, max_cells);
 }
 
 // Each particle's cell and its rank of arrival there (the order inside a cell
@@ -456,7 +469,7 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t
   __shared__ int32_t s_id[kNbWarps][kNbStage];
   __shared__ float4 s_part[kNbWarps][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if constexpr (kRows) {                       // the grid is in device memory
+  if (hdr) {                                   // the grid is in device memory
     ncell = hdr->ncell;
     g = hdr->grid;
   }
@@ -594,9 +607,11 @@ int64_t scan_tmp_words(int64_t n) {
 int64_t cell_scan_words(int64_t cells) { return (cells + 1023) / 1024 + 1; }
 
 void launch_prep_bounds(int64_t n, const Fields& F, int use_current, float4* pf, float r,
-                        unsigned* mm, cudaStream_t s) {
-  cudaMemsetAsync(mm, 0, 6 * sizeof(unsigned), s);
-  k_prep_bounds<<<std::min(nblocks(n, 256), 1024), 256, 0, s>>>(n, F, use_current, pf, r, mm);
+                        StaticHeader* hdr, int64_t max_cells, StaticHeader* host,
+                        cudaStream_t s) {
+  cudaMemsetAsync(hdr, 0, sizeof(StaticHeader), s);
+  k_prep_bounds<<<std::min(nblocks(n, 256), 1024), 256, 0, s>>>(n, F, use_current, pf, r, hdr,
+                                                                max_cells, host);
 }
 void launch_static_prep(int64_t n, const double* x, float4* pf, float r, StaticHeader* hdr,
                         uint32_t* count, int64_t max_cells, cudaStream_t s) {
@@ -620,17 +635,15 @@ void launch_reorder(int64_t n, const int32_t* s_src, const Fields& A, const Fiel
                     const float4* pf, float4* pf2, int32_t* inv, cudaStream_t s) {
   k_reorder<<<nblocks(n, 256), 256, 0, s>>>(n, s_src, A, B, pf, pf2, inv);
 }
-void launch_nblist(int64_t n, int64_t npad, const float4* pf, const GridDev& g,
-                   const uint32_t* start, const int32_t* slot_of, int32_t* nb, int32_t* cnt,
-                   int* status, cudaStream_t s) {
-  (void)n;
-  const int64_t ncell = (int64_t)g.dim[0] * g.dim[1] * g.dim[2];
+void launch_nblist(int64_t ncell, int64_t npad, const float4* pf, const GridDev& g,
+                   const StaticHeader* hdr, const uint32_t* start, const int32_t* slot_of,
+                   int32_t* nb, int32_t* cnt, int* status, cudaStream_t s) {
   if ((int64_t)WF_NB_ALLOC * npad < ((int64_t)1 << 31))
     k_nblist<uint32_t, false><<<nblocks(ncell, kNbWarps), 32 * kNbWarps, 0, s>>>(
-        ncell, npad, pf, g, nullptr, start, slot_of, nb, cnt, status);
+        ncell, npad, pf, g, hdr, start, slot_of, nb, cnt, status);
   else
     k_nblist<int64_t, false><<<nblocks(ncell, kNbWarps), 32 * kNbWarps, 0, s>>>(
-        ncell, npad, pf, g, nullptr, start, slot_of, nb, cnt, status);
+        ncell, npad, pf, g, hdr, start, slot_of, nb, cnt, status);
 }
 void launch_static_lists(const float4* pf, const StaticHeader* hdr, const uint32_t* start,
                          const int32_t* order, int32_t* lists, int32_t* counts, int* status,

@@ -8,7 +8,9 @@ struct GridDev {
   int dim[3];
 };
 
-// What the allocation-free search keeps at the head of its scratch (device).
+// The search grid and what it is sized from, in device memory: the head of the
+// allocation-free search's scratch, and a domain's own for the rebuilds that do
+// not wait for the host.
 struct StaticHeader {
   unsigned mm[6];       // cell bounds (codes)
   int status;           // WF_STATUS_* bits
@@ -63,9 +65,11 @@ struct CellWork {
 void device_exclusive_scan(uint32_t* data, int64_t n, uint32_t* tmp, cudaStream_t s);
 int64_t scan_tmp_words(int64_t n);
 int64_t cell_scan_words(int64_t cells);
-// float positions (x_h or the current ones) into pf, their cell bounds' codes into mm[6]
+// float positions (x_h or the current ones) into pf, their cell bounds' codes into hdr->mm; with
+// host (page-locked) not null also the grid into hdr, if it fits max_cells, and codes and cells
+// into *host
 void launch_prep_bounds(int64_t n, const Fields& F, int use_current, float4* pf, float r,
-                        unsigned* mm, cudaStream_t s);
+                        StaticHeader* hdr, int64_t max_cells, StaticHeader* host, cudaStream_t s);
 void launch_static_prep(int64_t n, const double* x, float4* pf, float r, StaticHeader* hdr,
                         uint32_t* count, int64_t max_cells, cudaStream_t s);
 // Counting sort by cell, original ids ascending inside a cell (orig null: the
@@ -76,9 +80,10 @@ void launch_cell_sort(int64_t n, const float4* pf, const GridDev& g, const Stati
                       float4* pf2, int* status, cudaStream_t s);
 void launch_reorder(int64_t n, const int32_t* s_src, const Fields& A, const Fields& B,
                     const float4* pf, float4* pf2, int32_t* inv, cudaStream_t s);
-void launch_nblist(int64_t n, int64_t npad, const float4* pf, const GridDev& g,
-                   const uint32_t* start, const int32_t* slot_of, int32_t* nb, int32_t* cnt,
-                   int* status, cudaStream_t s);
+// ncell: cells of the grid g, or about as many when the grid is hdr's
+void launch_nblist(int64_t ncell, int64_t npad, const float4* pf, const GridDev& g,
+                   const StaticHeader* hdr, const uint32_t* start, const int32_t* slot_of,
+                   int32_t* nb, int32_t* cnt, int* status, cudaStream_t s);
 // row-major lists and counts by the caller's index (order[k]: index of the k-th sorted particle)
 void launch_static_lists(const float4* pf, const StaticHeader* hdr, const uint32_t* start,
                          const int32_t* order, int32_t* lists, int32_t* counts, int* status,
