@@ -1064,56 +1064,13 @@ __global__ void __launch_bounds__(128, kWide ? kWideBlocks : 8) k_accel32(StepPa
   if (g == 0) a32[i] = af;
 }
 
-// The acceleration pass with the integration of the same slot behind it
-// (no contact stage in between): one pass instead of two, the integration's
-// FP64 work and traffic overlapping the other warps' neighbour gathers.
-// Neighbours are read from pvb (the density pass's copy of the mirrors) while
-// the new mirrors go to F.pv and th32, which this pass does not read.
-// kLaw1 (contact law 1): only the slots whose cell of a tool's bins lists a
-// triangle take part in the contact, so all others are integrated here as well,
-// and those few leave their
-// acceleration in a32 and their number in the list that k_contact_law1_list
-// (wf_contact.cu) works through, contact and integration.  The separate passes
-// read and wrote every slot again (500k particles: 68 us for the contact and 39
-// for the integration; now 34 for the listed slots).
-template <bool kLaw1, bool kWide>
-__global__ void __launch_bounds__(128, kWide ? kWideBlocks : 8) k_accel_int32(StepParams P, Fields F,
-                                                     const Rec32* __restrict__ pvb,
-                                                     const Sig32 sig,
-                                                     const double4* __restrict__ vd2,
-                                                     float4* __restrict__ a32,
-                                                     const int32_t* __restrict__ nb,
-                                                     const int32_t* __restrict__ cnt, const List16 L16) {
-  int g;
-  const int64_t i = accel_slot(g);
-  if (i >= P.n) return;
-  const AccelSrc<RecGlobal> src{{pvb}, sig.a, sig.b};
-  if (P.state_pf && g == 0) {
-    prefetch_l2(F.xm + i); prefetch_l2(vd2 + i); prefetch_l2(F.u + i); prefetch_l2(F.T + i);
-  }
-  if (P.pf_ahead > 0 && g == 0) {
-    const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
-    if (ia < P.n) {
-      prefetch_l2(pvb + ia); prefetch_l2(sig.a + ia); prefetch_l2(sig.b + ia);
-      prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
-      prefetch_l2(F.id + ia);
-      for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 2 * kAccelLanes);
-    }
-  }
-  // rigid (non-solid) slots: zero acceleration, moved by their BCs
-  float4 af = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (F.perm[i] < P.n_solid) {
-    const int b16 = L16.base ? L16.base[i / WF_TILE] : -1;   // uniform over the block
-    const NbList32 list{nb, P.npad, i};
-    if (kLaw1 && zone_filter(P))
-      af = accel_value<true, !kWide>(P, F, pvb, sig, cnt, i, g, src, list);
-    else if (b16 >= 0)
-      af = accel_value<false, !kWide>(P, F, pvb, sig, cnt, i, g, src,
-                                      NbList16{L16.off, P.npad, i, b16});
-    else
-      af = accel_value<false, !kWide>(P, F, pvb, sig, cnt, i, g, src, list);
-  }
-  if (g != 0) return;
+// What follows the acceleration of a slot: with contact law 1 the few slots near
+// a tool go to the list, all others are integrated.
+template <bool kLaw1>
+__device__ __forceinline__ void accel_tail(const StepParams& P, const Fields& F,
+                                           const Rec32* __restrict__ pvb,
+                                           const double4* __restrict__ vd2, float4* a32, int64_t i,
+                                           float4 af) {
   if constexpr (kLaw1) {
     if (F.perm[i] < P.n_solid) {
       const float4 p = pvb[i].p;
@@ -1133,6 +1090,69 @@ __global__ void __launch_bounds__(128, kWide ? kWideBlocks : 8) k_accel_int32(St
     }
   }
   integrate_mixed_one(P, F, vd2, i, af);
+}
+
+// The acceleration pass with the integration of the same slot behind it
+// (no contact stage in between): one pass instead of two, the integration's
+// FP64 work and traffic overlapping the other warps' neighbour gathers.
+// Neighbours are read from pvb (the density pass's copy of the mirrors) while
+// the new mirrors go to F.pv and th32, which this pass does not read.
+// kLaw1 (contact law 1): only the slots whose cell of a tool's bins lists a
+// triangle take part in the contact, so all others are integrated here as well,
+// and those few leave their
+// acceleration in a32 and their number in the list that k_contact_law1_list
+// (wf_contact.cu) works through, contact and integration.  The separate passes
+// read and wrote every slot again (500k particles: 68 us for the contact and 39
+// for the integration; now 34 for the listed slots).
+// Whole warps run that part, the block's first two for its 64 slots: as one of
+// two lanes per slot it issued its ~35 FP64 operations, 16 cycles of an SM each
+// whatever the lanes, twice as often (FP64 pipe 41 % busy at 786k; 50,560
+// particles 31.6 -> 27.5 us, 500k with law 1 0.5 % of a step).
+template <bool kLaw1, bool kWide>
+__global__ void __launch_bounds__(128, kWide ? kWideBlocks : 8) k_accel_int32(StepParams P, Fields F,
+                                                     const Rec32* __restrict__ pvb,
+                                                     const Sig32 sig,
+                                                     const double4* __restrict__ vd2,
+                                                     float4* __restrict__ a32,
+                                                     const int32_t* __restrict__ nb,
+                                                     const int32_t* __restrict__ cnt, const List16 L16) {
+  __shared__ float4 s_af[128 / kAccelLanes];
+  int g;
+  const int64_t i0 = accel_slot(g);
+  const bool valid = i0 < P.n;
+  const int64_t i = valid ? i0 : P.n - 1;
+  const AccelSrc<RecGlobal> src{{pvb}, sig.a, sig.b};
+  if (P.state_pf && g == 0) {
+    prefetch_l2(F.xm + i); prefetch_l2(vd2 + i); prefetch_l2(F.u + i); prefetch_l2(F.T + i);
+  }
+  if (P.pf_ahead > 0 && g == 0) {
+    const int64_t ia = i + P.pf_ahead;      // the slot this thread's successor will take
+    if (ia < P.n) {
+      prefetch_l2(pvb + ia); prefetch_l2(sig.a + ia); prefetch_l2(sig.b + ia);
+      prefetch_l2(cnt + ia); prefetch_l2(F.perm + ia);
+      prefetch_l2(F.id + ia);
+      for (int b = 0; b < P.wave_pf && b < WF_NB_BLOCKS; b++) nb_prefetch(nb, P.npad, ia, b, 2 * kAccelLanes);
+    }
+  }
+  // rigid (non-solid) slots: zero acceleration, moved by their BCs
+  float4 af = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (valid && F.perm[i] < P.n_solid) {
+    const int b16 = L16.base ? L16.base[i / WF_TILE] : -1;   // uniform over the block
+    const NbList32 list{nb, P.npad, i};
+    if (kLaw1 && zone_filter(P))
+      af = accel_value<true, !kWide>(P, F, pvb, sig, cnt, i, g, src, list);
+    else if (b16 >= 0)
+      af = accel_value<false, !kWide>(P, F, pvb, sig, cnt, i, g, src,
+                                      NbList16{L16.off, P.npad, i, b16});
+    else
+      af = accel_value<false, !kWide>(P, F, pvb, sig, cnt, i, g, src, list);
+  }
+  if (g == 0) s_af[threadIdx.x / kAccelLanes] = af;
+  __syncthreads();
+  if (threadIdx.x >= 128 / kAccelLanes) return;
+  const int64_t k = blockIdx.x * (int64_t)(128 / kAccelLanes) + threadIdx.x;
+  if (k >= P.n) return;
+  accel_tail<kLaw1>(P, F, pvb, vd2, a32, k, s_af[threadIdx.x]);
 }
 
 // The same pass for staged tiles: a block of 2 x 128 threads is one tile;
