@@ -666,11 +666,16 @@ int wf_mlp_train(float* params, const float* X, const float* Y, int64_t n, int64
   cudaMemcpy(dY, Y, sizeof(float) * n, cudaMemcpyHostToDevice);
   cudaMemset(A.m, 0, 2 * bP);
   if (grad_ready() != cudaSuccess) return WF_ERR_CUDA;
-  int64_t off = 0;
+  int64_t off = 0, st = 0;
+  const auto advance = [&] {                           // the next step's first sample
+    off += std::min<int64_t>(batch, n - off);
+    if (off >= n) off = 0;
+    st++;
+  };
   if (train_fits(most)) {
     cudaMemcpy(dS, sched.data(), sizeof(AdamStep) * steps, cudaMemcpyHostToDevice);
     cudaMemset(dB, 0, 2 * sizeof(unsigned));
-    for (int64_t st = 0; st < steps; st += kTrainChunk) {
+    while (st < steps) {
       int count = (int)std::min<int64_t>(kTrainChunk, steps - st);
       cudaMemsetAsync(dB, 0, sizeof(unsigned));
       const AdamStep* s0 = dS + st;
@@ -679,26 +684,22 @@ int wf_mlp_train(float* params, const float* X, const float* Y, int64_t n, int64
       AdamState state = A;
       void* args[] = {&state, &dX, &dY, &n, &batch, &off, &s0, &count, &dR, &l0, &dB, &bad};
       if (cudaLaunchCooperativeKernel((const void*)k_mlp_train, dim3(most), dim3(kGradThreads),
-                                      args, sizeof(GradShared), nullptr) != cudaSuccess)
-        return WF_ERR_CUDA;
-      for (int k = 0; k < count; k++) {                // where the next launch begins
-        off += std::min<int64_t>(batch, n - off);
-        if (off >= n) off = 0;
+                                      args, sizeof(GradShared), nullptr) != cudaSuccess) {
+        cudaGetLastError();                            // not all of its blocks run at once here
+        break;
       }
+      for (int k = 0; k < count; k++) advance();
     }
     int bad = 0;
     if (cudaMemcpy(&bad, dB + 1, sizeof bad, cudaMemcpyDeviceToHost) != cudaSuccess || bad)
       return WF_ERR_CUDA;
-  } else {
-    for (int64_t st = 0; st < steps; st++) {
-      const int64_t cnt = std::min<int64_t>(batch, n - off);
-      const int rows = grad_rows(cnt);
-      k_mlp_grad<<<rows, kGradThreads, sizeof(GradShared)>>>(dP, dX, dY, off, cnt,
-                                                            1.0f / (float)cnt, dR);
-      k_adam<<<kPartRow / 32, 256>>>(A, dR, rows, dL + st, sched[st]);
-      off += cnt;
-      if (off >= n) off = 0;
-    }
+  }
+  for (; st < steps; advance()) {
+    const int64_t cnt = std::min<int64_t>(batch, n - off);
+    const int rows = grad_rows(cnt);
+    k_mlp_grad<<<rows, kGradThreads, sizeof(GradShared)>>>(dP, dX, dY, off, cnt, 1.0f / (float)cnt,
+                                                          dR);
+    k_adam<<<kPartRow / 32, 256>>>(A, dR, rows, dL + st, sched[st]);
   }
   cudaMemcpy(params, dP, sizeof(float) * WF_MLP_NPARAM, cudaMemcpyDeviceToHost);
   if (final_loss) {

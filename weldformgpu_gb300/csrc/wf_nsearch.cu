@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256) k_prep_bounds(int64_t n, const Fields F, 
   }
   reduce_bounds(lo, hi, hdr->mm);
   if (!host || !size_grid(hdr, r, max_cells)) return;
-  for (int k = 0; k < 6; k++) host->mm[k] = hdr->mm[k];
+  for (int k = 0; k < 6; k++) host->mm[k] = __ldcg(hdr->mm + k);
   host->ncell = hdr->ncell;
 }
 
