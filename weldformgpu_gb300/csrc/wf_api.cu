@@ -647,6 +647,8 @@ static StepParams make_params(const wf_domain* d) {
   P.chif = (float)P.chi;
   P.h_convf = (float)P.h_conv;
   P.T_inff = (float)P.T_inf;
+  P.visc_eps = 0.01 * P.h * P.h;
+  P.visc_ac = P.alpha * (0.5 * (P.Cs + P.Cs));
   return P;
 }
 

@@ -198,6 +198,7 @@ struct StepParams {
   int64_t n_solid;      // original ids below this are solid (solid_part_count)
   int64_t npad;         // slot stride of the neighbour-list blocks (nb_at)
   double h, gkC;        // smoothing length (uniform) and 1/(h^4 pi)
+  double visc_eps, visc_ac;   // 0.01 h h and alpha (0.5 (Cs + Cs)), in that order
   int h_tame;           // h and 1/(h^4 pi) are within 2^+-120 (products on the integer pipe)
   double dt;
   double Cs, G, rho0;   // uniform sound speed, shear modulus, reference density

@@ -18,11 +18,11 @@
 //     div_int, sqrt_int below), additions on the FP64 pipe.
 // 9 / 21 / 28 / 11 FP64 instructions a pair are left.  Times at 170k, in us,
 // all on the FP64 pipe with nothing kept -> with the kept values -> now:
-// density 1,066 -> 540 -> 247, stress 1,737 -> 1,070 -> 604, acceleration
-// 2,178 -> 1,358 -> 683, heat 1,367 -> 1,354 -> 394 (it computes the geometry
+// density 1,066 -> 540 -> 247, stress 1,737 -> 1,070 -> 549, acceleration
+// 2,178 -> 1,358 -> 601, heat 1,367 -> 1,354 -> 394 (it computes the geometry
 // that the next step's density pass reads).  Stress and acceleration keep the
-// FP64 pipe 78-80 % busy and the integer ALUs 42-45 %; density and heat the
-// ALUs 61-67 % and FP64 43-71 %.
+// FP64 pipe 79 % busy and the integer ALUs 47-51 %; density and heat the ALUs
+// 61-63 % and FP64 64-71 %.
 // Every value is rounded exactly as where it was computed on the FP64 pipe.
 #include "wf_common.cuh"
 #include "wf_heat.cuh"
@@ -173,19 +173,21 @@ __device__ __forceinline__ double root(double x) {
 // within 2^+-kTame, so that every product and quotient of the pair, and every
 // remainder of a sum in it, stays normal.  Any other pair takes the FP64 pipe.
 constexpr unsigned kTame = 120;
-// -0.5 x and 2 x: exact, so only the sign and exponent bits change (zeros,
-// subnormals and the ends of the range take the multiplication)
+// -0.5 x and 2 x: exact, so for zeros and tame values only the sign and exponent
+// bits change (a select of the FP64 operation would still execute it: an
+// eleventh of the stress pass's FP64 operations)
+template <bool kInt>
 __device__ __forceinline__ double neg_half(double x) {
+  if constexpr (!kInt) return -0.5 * x;
   const int hi = __double2hiint(x);
-  const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
-  if (e - 2u < 2045u) return __hiloint2double((hi ^ (int)0x80000000) - 0x00100000, __double2loint(x));
-  return -0.5 * x;
+  return __hiloint2double((hi ^ (int)0x80000000) - ((hi << 1) != 0 ? 0x00100000 : 0),
+                          __double2loint(x));
 }
+template <bool kInt>
 __device__ __forceinline__ double twice(double x) {
+  if constexpr (!kInt) return x + x;
   const int hi = __double2hiint(x);
-  const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
-  if (e - 1u < 2045u) return __hiloint2double(hi + 0x00100000, __double2loint(x));
-  return x + x;
+  return __hiloint2double(hi + ((hi << 1) != 0 ? 0x00100000 : 0), __double2loint(x));
 }
 
 // The cubic-spline gradient factor of gradK64, bit for bit, with the division
@@ -336,11 +338,11 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_density64(StepParams P, F
 template <bool kInt>
 __device__ __forceinline__ void rate_terms(double xx, double xy, double xz, double ax, double ay,
                                            double az, double GK, double mj_dj, double* t) {
-  const double s = neg_half(GK);
+  const double s = neg_half<kInt>(GK);
   // StrainRate (symmetric) scaled by -GK/2, then by mj/dj
-  t[0] = mul<kInt>(mul<kInt>(mul<kInt>(twice(ax), xx), s), mj_dj);
-  t[1] = mul<kInt>(mul<kInt>(mul<kInt>(twice(ay), xy), s), mj_dj);
-  t[2] = mul<kInt>(mul<kInt>(mul<kInt>(twice(az), xz), s), mj_dj);
+  t[0] = mul<kInt>(mul<kInt>(mul<kInt>(twice<kInt>(ax), xx), s), mj_dj);
+  t[1] = mul<kInt>(mul<kInt>(mul<kInt>(twice<kInt>(ay), xy), s), mj_dj);
+  t[2] = mul<kInt>(mul<kInt>(mul<kInt>(twice<kInt>(az), xz), s), mj_dj);
   const double pxy = mul<kInt>(ax, xy), qxy = mul<kInt>(ay, xx), pxz = mul<kInt>(ax, xz),
                qxz = mul<kInt>(az, xx), pyz = mul<kInt>(ay, xz), qyz = mul<kInt>(az, xy);
   t[3] = mul<kInt>(mul<kInt>(pxy + qxy, s), mj_dj);
@@ -454,8 +456,8 @@ __device__ __forceinline__ void store_rates(const Fields& F, int64_t i, const do
 
 // One lane per particle: the pair loop with the stress update behind it.
 // Twelve blocks an SM (80 registers) hide the update's chains of operations:
-// 170k particles 640 us with the 98 registers it would take, 604 with 80; the
-// update as a kernel of its own, 624.
+// 170k particles 640 us with the 98 registers it would take, 604 with 80 (549
+// now); the update as a kernel of its own, 624.
 template <int kGeo>
 __global__ void __launch_bounds__(64, 12) k_stress64(StepParams P, Fields F, Work64 W,
                                                      const double4* __restrict__ vd2,
@@ -558,7 +560,7 @@ __device__ __forceinline__ bool viscosity_int(const StepParams& P, double xx, do
                                               double dj, double& PI) {
   const double vdx = mul_int(vx, xx) + mul_int(vy, xy) + mul_int(vz, xz);
   if (__double2hiint(vdx) >= 0) return true;
-  const double den = r2 + 0.01 * P.h * P.h, aC = P.alpha * (0.5 * (P.Cs + P.Cs));
+  const double den = r2 + P.visc_eps, aC = P.visc_ac;
   const double rho2 = di + dj;
   const double MU = div_int(mul_int(P.h, vdx), den);
   double num = mul_int(aC, MU);
