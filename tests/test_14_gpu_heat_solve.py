@@ -26,8 +26,9 @@ def _same(a, b):
             assert np.array_equal(p, q)
 
 
-# 3^3 and 11^3 particles take 32 lanes each in FP64, 13^3 16, 27^3 and 29^3 eight, 40^3 one
-@pytest.mark.parametrize("side", [3, 11, 13, 27, 29, 40])
+# 3^3 and 11^3 particles take 32 lanes each in FP64, 13^3 16, 20^3 eight, 23^3 (just above the line
+# at 12,000), 27^3, 29^3 and 40^3 two, 47^3 one
+@pytest.mark.parametrize("side", [3, 11, 13, 20, 23, 27, 29, 40, 47])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_heat_solve_with_kept_factors_is_bit_identical(side, precision):
     sc = S.heat_box(n_side=side)

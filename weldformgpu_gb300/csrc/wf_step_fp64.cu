@@ -759,7 +759,17 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_rate(StepParams P, F
 // pair, and takes the leapfrog update with it; the neighbours' temperatures
 // are read from one array while the new ones go to another.  64,000
 // particles, 20 steps: 15.5 ms recomputing the pairs on the FP64 pipe, 1.88
-// with the kept factors, 1.42 on the integer pipes.
+// with the kept factors, 1.38 on the integer pipes, 1.2 with two lanes.
+//
+// Where the factor of entry k of particle i stands: with one or two lanes per
+// particle (kRows) in row k of npad factors, so that a warp's reads and writes
+// of an entry are whole lines (in the lists' blocks they are 16), else where
+// the lists have it, so that a group's are.
+template <bool kRows>
+__device__ __forceinline__ int64_t factor_at(int64_t npad, int64_t i, int k) {
+  return kRows ? k * npad + i : nb_at(npad, i, k);
+}
+template <bool kRows>
 __global__ void __launch_bounds__(64) k_heat_pairs64(StepParams P, Fields F, HeatWork64 H,
                                                      const int32_t* __restrict__ nb,
                                                      const int32_t* __restrict__ cnt) {
@@ -774,8 +784,8 @@ __global__ void __launch_bounds__(64) k_heat_pairs64(StepParams P, Fields F, Hea
   H.fric[i] = F.qf && F.qf[i] > 0.0 ? F.qf[i] / (xi.w * cp) : 0.0;
   const int c = cnt[i];
   for (int k = 0; k < c; k++) {
-    const int64_t e = nb_at(P.npad, i, k);
-    const double4 xj = F.xm[__ldg(nb + e)];
+    const int64_t e = factor_at<kRows>(P.npad, i, k);
+    const double4 xj = F.xm[__ldg(nb + nb_at(P.npad, i, k))];
     const double xx = xi.x - xj.x, xy = xi.y - xj.y, xz = xi.z - xj.z;
     double GK, r2;
     if (P.h_tame && within<kTame>(xx) && within<kTame>(xy) && within<kTame>(xz)) {
@@ -793,10 +803,8 @@ __global__ void __launch_bounds__(64) k_heat_pairs64(StepParams P, Fields F, Hea
   }
 }
 
-__device__ __forceinline__ double heat_step_term(const HeatWork64& H, const double* __restrict__ T,
-                                                 int64_t e, int j, double Ti, double kk) {
-  const double mr = __ldg(H.mr + j), dT = Ti - __ldg(T + j), dot = __ldg(H.dot + e);
-  const double r2 = __ldg(H.r2 + e);
+__device__ __forceinline__ double heat_step_term(double mr, double dT, double dot, double r2,
+                                                 double kk) {
   if (within<kTame>(mr) && within<kTame>(dT) && within<kTame>(dot) && within<kTame>(kk) &&
       in_range<kTame>(r2))
     return div_int(mul_int(mul_int(mr, mul_int(kk, dT)), dot), r2);
@@ -804,7 +812,7 @@ __device__ __forceinline__ double heat_step_term(const HeatWork64& H, const doub
 }
 
 template <int kG>
-__global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_step64(StepParams P, Fields F,
+__global__ void __launch_bounds__(kG <= 2 ? 64 : 32) k_heat_step64(StepParams P, Fields F,
                                                      HeatWork64 H, const double* __restrict__ T,
                                                      double* __restrict__ T_out,
                                                      const int32_t* __restrict__ nb,
@@ -819,18 +827,46 @@ __global__ void __launch_bounds__(kG == 1 ? 64 : 32) k_heat_step64(StepParams P,
   const double kk = 4.0 * ki * ki / (ki + ki);
   const int c = valid ? cnt[i] : 0;
   double s = 0.0;
-  if constexpr (kG == 1) {
-    for (int k = 0; k < c; k++) {
-      const int64_t e = nb_at(P.npad, i, k);
-      s += heat_step_term(H, T, e, __ldg(nb + e), Ti, kk);
+  if constexpr (kG <= 2) {
+    // Four entries a lane at a time, their loads in flight together; with two
+    // lanes the terms of 8 b .. 8 b + 3 are lane 0's, and the sum goes from lane
+    // to lane in list order.
+    const int rounds = (kG == 1 ? c + 3 : __reduce_max_sync(0xffffffffu, c) + 7) / (4 * kG);
+    for (int b = 0; b < rounds; b++) {
+      const int k0 = 4 * (kG * b + g);
+      double t[4] = {0.0, 0.0, 0.0, 0.0};
+      if (k0 < c) {
+        const int4 ja = __ldg(reinterpret_cast<const int4*>(nb + nb_at(P.npad, i, k0)));
+        const int js[4] = {ja.x, ja.y, ja.z, ja.w};        // (past the list: the own slot)
+        double mr[4], Tj[4], dot[4], r2[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int64_t e = factor_at<true>(P.npad, i, k0 + k);
+          mr[k] = __ldg(H.mr + js[k]);
+          Tj[k] = __ldg(T + js[k]);
+          dot[k] = k0 + k < c ? __ldg(H.dot + e) : 0.0;
+          r2[k] = k0 + k < c ? __ldg(H.r2 + e) : 1.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (k0 + k < c) t[k] = heat_step_term(mr[k], Ti - Tj[k], dot[k], r2[k], kk);
+      }
+#pragma unroll
+      for (int turn = 0; turn < kG; turn++) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) s += t[k];
+        if constexpr (kG == 2) s = __shfl_sync(0xffffffffu, s, turn, 2);
+      }
     }
+    if (!valid || g != 0) return;
   } else {
     const int rounds = warp_rounds<kG>(c);
     for (int b = 0; b < rounds; b++) {
       double t = 0.0;
       if (kG * b + g < c) {
-        const int64_t e = nb_at(P.npad, i, kG * b + g);
-        t = heat_step_term(H, T, e, __ldg(nb + e), Ti, kk);
+        const int64_t e = factor_at<false>(P.npad, i, kG * b + g);
+        const int j = __ldg(nb + e);
+        t = heat_step_term(__ldg(H.mr + j), Ti - __ldg(T + j), __ldg(H.dot + e), __ldg(H.r2 + e), kk);
       }
       s = add_in_order<kG>(sh, s, t, c - kG * b);
     }
@@ -905,19 +941,28 @@ void launch_fp64_heat_rate(const StepParams& P, const Fields& F, const Work64& W
   if (W.gk) WF_LAUNCH64(k_heat_rate, GEO_STORE, N.nb, N.cnt, plastic_heat);
   else WF_LAUNCH64(k_heat_rate, GEO_NONE, N.nb, N.cnt, plastic_heat);
 }
+// Lanes of a particle in a heat solve's steps.  A step, us, with 1 / 2 lanes and
+// four entries a lane in flight / the lanes of lanes64: n = 8,000 - / 18.5 /
+// 16.4, 13,824 - / 20.4 / 22.6, 46,656 - / 34.9 / 66.6, 64,000 48.9 / 45.0 /
+// 53.3, 85,184 61.4 / 59.8, 110,592 72.3 / 74.8, a million 500 / 529.
+static int heat_lanes(int64_t n) { return n >= 100000 ? 1 : n >= 12000 ? 2 : lanes64(n); }
+
 void launch_heat_pairs64(const StepParams& P, const Fields& F, const HeatWork64& H,
                          const NbBuffers& N, cudaStream_t s) {
-  k_heat_pairs64<<<blocks_for(P.n, 64), 64, 0, s>>>(P, F, H, N.nb, N.cnt);
+  if (heat_lanes(P.n) <= 2) k_heat_pairs64<true><<<blocks_for(P.n, 64), 64, 0, s>>>(P, F, H, N.nb, N.cnt);
+  else k_heat_pairs64<false><<<blocks_for(P.n, 64), 64, 0, s>>>(P, F, H, N.nb, N.cnt);
 }
 void launch_heat_step64(const StepParams& P, const Fields& F, const HeatWork64& H, double* T_out,
                         const NbBuffers& N, int first, cudaStream_t s) {
-  const int lanes = lanes64(P.n), grid = blocks_for(P.n * lanes, lanes == 1 ? 64 : 32);
+  const int lanes = heat_lanes(P.n), grid = blocks_for(P.n * lanes, lanes <= 2 ? 64 : 32);
   if (lanes == 32)
     k_heat_step64<32><<<grid, 32, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
   else if (lanes == 16)
     k_heat_step64<16><<<grid, 32, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
   else if (lanes == 8)
     k_heat_step64<8><<<grid, 32, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
+  else if (lanes == 2)
+    k_heat_step64<2><<<grid, 64, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
   else
     k_heat_step64<1><<<grid, 64, 0, s>>>(P, F, H, F.T, T_out, N.nb, N.cnt, first);
 }
