@@ -30,8 +30,8 @@ def _lattice(R, H, thermal):
     return sc, opts
 
 
-# ~700 particles take 32 lanes each, ~3,000 take 16, ~24,500 take eight (the last
-# warp is not full)
+# ~700 particles take 32 lanes each, ~3,000 take 16, ~24,500 take eight or, in the
+# density and acceleration passes, four (the last warp is not full)
 @pytest.mark.parametrize("R,H", [(0.0024, 0.0045), (0.0041, 0.0073), (0.0079, 0.0156)])
 @pytest.mark.parametrize("thermal", [0, 1])
 @pytest.mark.parametrize("cache", [1, 0])
@@ -45,7 +45,8 @@ def test_fp64_passes_bit_exact_vs_oracle(R, H, thermal, cache):
         _same(g, o)
 
 
-# above and below the line between one and eight lanes at 64,000
+# above and below the line of the stress and density passes at 64,000 (one lane); the acceleration
+# pass takes four lanes there, so do the passes that compute the geometry
 @pytest.mark.parametrize("R,H", [(0.0111, 0.0214), (0.0107, 0.0214)])
 def test_fp64_passes_bit_exact_at_the_one_lane_line(R, H):
     sc, opts = _lattice(R, H, 1)
@@ -78,6 +79,17 @@ def test_fp64_passes_bit_exact_outside_the_integer_range(field, scale, R, H):
         g.step(k)
         for f in FIELDS:
             assert np.array_equal(g.get_field(f), o.get_field(f), equal_nan=True), f
+
+
+def test_fp64_passes_bit_exact_with_one_lane_everywhere():
+    """A domain above all lines (300,000), against the same passes without the kept geometry."""
+    sc, opts = _lattice(0.0190, 0.0340, 1)
+    assert sc["n"] >= 300000
+    a = S.load(Domain_d(sc["n"]), sc, opts)
+    b = S.load(Domain_d(sc["n"]), sc, dict(opts, pair_cache=0))
+    a.step(5)
+    b.step(5)
+    _same(a, b)
 
 
 @pytest.mark.parametrize("cache", [1, 0])

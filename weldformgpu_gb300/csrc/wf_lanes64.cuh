@@ -1,7 +1,7 @@
 // wf_lanes64.cuh — how many lanes share a particle in the FP64 passes over the
 // neighbour lists, and sums in list order over those lanes.
 //
-// kG = 1: one thread per particle walks its list.  kG = 8, 16 or 32: so many
+// kG = 1: one thread per particle walks its list.  kG = 4, 8, 16 or 32: so many
 // lanes per particle, lane g takes entry kG b + g in round b (one coalesced
 // read of the round's indices and geometry), and the round's terms are added
 // in list order, term by term, so the sums round as in the walk.  More lanes
@@ -74,10 +74,10 @@ __device__ __forceinline__ void add_in_order(double* sh, const double* t, int g,
     if (kG == 32 && b >= m) break;
     if (g < kA)
 #pragma unroll
-      for (int k = 0; k < 8; k++) acc[0] += row[(b + k) * kA + g];
+      for (int k = 0; k < (kG < 8 ? kG : 8); k++) acc[0] += row[(b + k) * kA + g];
     if (kA > kG && g < kA - kG)
 #pragma unroll
-      for (int k = 0; k < 8; k++) acc[1] += row[(b + k) * kA + g + kG];
+      for (int k = 0; k < (kG < 8 ? kG : 8); k++) acc[1] += row[(b + k) * kA + g + kG];
   }
   __syncwarp();
 }

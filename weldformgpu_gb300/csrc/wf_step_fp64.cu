@@ -19,7 +19,7 @@
 // 9 / 21 / 28 / 11 FP64 instructions a pair are left.  Times at 170k, in us,
 // all on the FP64 pipe with nothing kept -> with the kept values -> now:
 // density 1,066 -> 540 -> 247, stress 1,737 -> 1,070 -> 549, acceleration
-// 2,178 -> 1,358 -> 601, heat 1,367 -> 1,354 -> 394 (it computes the geometry
+// 2,178 -> 1,358 -> 577, heat 1,367 -> 1,354 -> 394 (it computes the geometry
 // that the next step's density pass reads).  Stress and acceleration keep the
 // FP64 pipe 79 % busy and the integer ALUs 47-51 %; density and heat the ALUs
 // 61-63 % and FP64 64-71 %.
@@ -894,21 +894,35 @@ __global__ void __launch_bounds__(kG <= 2 ? 64 : 32) k_heat_step64(StepParams P,
 
 static inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
+// Lanes of the passes that have a form with four: in mid-sized domains four lanes
+// hide more of a pair's chain of operations than one and spend fewer additions
+// on the ordered sums than eight.  Pass, us, with 8 / 4 / 1 lanes: density
+// 14,040 particles 38 / 35 / -, 50,560 112 / 95 / -, 86,592 - / 149 / 149,
+// 169,680 - / 273 / 246; acceleration 10,752 52 / 55 / -, 14,040 69 / 62 / -,
+// 50,560 201 / 186 / -, 169,680 - / 577 / 601, 401,920 - / 1,341 / 1,348,
+// 786,000 - / 2,943 / 2,908; heat (and density, where they compute the
+// geometry) 36,720 106 / 108 / -, 50,560 137 / 134 / -, 86,592 - / 210 / 227,
+// 169,680 - / 389 / 384, 786,000 - / 1,705 / 1,505.
+static int density_lanes(int64_t n) { return n >= 64000 ? 1 : n >= 12000 ? 4 : lanes64(n); }
+static int accel_lanes(int64_t n) { return n >= 300000 ? 1 : n >= 12000 ? 4 : lanes64(n); }
+static int geometry_lanes(int64_t n) { return n >= 130000 ? 1 : n >= 45000 ? 4 : lanes64(n); }
+
 // Launches K<lanes, geometry>.
-#define WF_LAUNCH64(K, GEO, ...)                                                               \
+#define WF_LAUNCH64(LANES, K, GEO, ...)                                                        \
   do {                                                                                         \
-    const int lanes = lanes64(P.n), grid = blocks_for(P.n * lanes, lanes == 1 ? 64 : 32);      \
+    const int lanes = LANES, grid = blocks_for(P.n * lanes, lanes == 1 ? 64 : 32);             \
     if (lanes == 32) K<32, GEO><<<grid, 32, 0, s>>>(P, F, W, __VA_ARGS__);                     \
     else if (lanes == 16) K<16, GEO><<<grid, 32, 0, s>>>(P, F, W, __VA_ARGS__);                \
     else if (lanes == 8) K<8, GEO><<<grid, 32, 0, s>>>(P, F, W, __VA_ARGS__);                  \
+    else if (lanes == 4) K<4, GEO><<<grid, 32, 0, s>>>(P, F, W, __VA_ARGS__);                  \
     else K<1, GEO><<<grid, 64, 0, s>>>(P, F, W, __VA_ARGS__);                                  \
   } while (0)
 
 void launch_fp64_density(const StepParams& P, const Fields& F, const Work64& W, double4* vd2,
                          const NbBuffers& N, cudaStream_t s) {
-  if (!W.gk) WF_LAUNCH64(k_density64, GEO_NONE, vd2, N.nb, N.cnt);
-  else if (W.geo) WF_LAUNCH64(k_density64, GEO_LOAD, vd2, N.nb, N.cnt);
-  else WF_LAUNCH64(k_density64, GEO_STORE, vd2, N.nb, N.cnt);
+  if (!W.gk) WF_LAUNCH64(density_lanes(P.n), k_density64, GEO_NONE, vd2, N.nb, N.cnt);
+  else if (W.geo) WF_LAUNCH64(density_lanes(P.n), k_density64, GEO_LOAD, vd2, N.nb, N.cnt);
+  else WF_LAUNCH64(geometry_lanes(P.n), k_density64, GEO_STORE, vd2, N.nb, N.cnt);
 }
 int launch_fp64_stress(const StepParams& P, const Fields& F, const Work64& W, const double4* vd2,
                        const NbBuffers& N, int* status, cudaStream_t s) {
@@ -933,13 +947,13 @@ int launch_fp64_stress(const StepParams& P, const Fields& F, const Work64& W, co
 }
 void launch_fp64_accel(const StepParams& P, const Fields& F, const Work64& W, const double4* vd2,
                        const NbBuffers& N, cudaStream_t s) {
-  if (W.gk) WF_LAUNCH64(k_accel64, GEO_LOAD, vd2, N.nb, N.cnt);
-  else WF_LAUNCH64(k_accel64, GEO_NONE, vd2, N.nb, N.cnt);
+  if (W.gk) WF_LAUNCH64(accel_lanes(P.n), k_accel64, GEO_LOAD, vd2, N.nb, N.cnt);
+  else WF_LAUNCH64(accel_lanes(P.n), k_accel64, GEO_NONE, vd2, N.nb, N.cnt);
 }
 void launch_fp64_heat_rate(const StepParams& P, const Fields& F, const Work64& W,
                            const NbBuffers& N, int plastic_heat, cudaStream_t s) {
-  if (W.gk) WF_LAUNCH64(k_heat_rate, GEO_STORE, N.nb, N.cnt, plastic_heat);
-  else WF_LAUNCH64(k_heat_rate, GEO_NONE, N.nb, N.cnt, plastic_heat);
+  if (W.gk) WF_LAUNCH64(geometry_lanes(P.n), k_heat_rate, GEO_STORE, N.nb, N.cnt, plastic_heat);
+  else WF_LAUNCH64(geometry_lanes(P.n), k_heat_rate, GEO_NONE, N.nb, N.cnt, plastic_heat);
 }
 // Lanes of a particle in a heat solve's steps.  A step, us, with 1 / 2 lanes and
 // four entries a lane in flight / the lanes of lanes64: n = 8,000 - / 18.5 /
