@@ -790,7 +790,8 @@ static size_t work64_bytes(const wf_domain* d) {
   return sizeof(double) * (size_t)(2 * WF_NB_ALLOC + 8) * (size_t)d->npad;
 }
 // Kept values are of this call's own steps only: anything may have changed
-// between two calls and in the step hook.
+// between two calls and in the step hook.  Every stepping call drops them:
+// solve_begin for the solves, the calls that may go on without it themselves.
 static void kept_drop(wf_domain* d) {
   d->geo_valid = false;
   d->zone_checked = d->maxdep_kept = false;
@@ -1150,6 +1151,7 @@ static int print_output_row(wf_domain* d) {
 static int solve_begin(wf_domain* d, double dt_out) {
   int rc = check_ready(d);
   if (rc) return rc;
+  kept_drop(d);
   const bool resume = d->resume != 0;
   if (!resume) {
     d->time = 0.0;
@@ -1219,7 +1221,7 @@ static int solve_step_launches(wf_domain* d) {
     // copy to the host is under way since the last step's stress pass, so the
     // GPU does not wait for the host; a call's first step and the FP64 form
     // reduce the strains here (one pass and an 8-byte read).
-    if (d->maxdep_kept) {
+    if (d->maxdep_kept && d->precision == 1) {
       WF_CUDA_OK(cudaEventSynchronize(d->ev_maxdep));
     } else {
       const Fields& F0 = d->F[d->cur];
