@@ -132,8 +132,8 @@ struct wf_domain {
   size_t work_bytes = 0;       // allocated
   size_t work_refused = 0;     // a size the device had no memory for
   bool pair_cache = true;      // option "pair_cache"
-  int* d_zone = nullptr;       // [0] a massive particle has a mesh's zone id, [1] slots near a tool
-  bool zone_checked = false;   // d_zone[0] is of the current ids and masses
+  int* d_zone = nullptr;       // [0] the mixed passes need the zone filter, [1] slots near a tool
+  bool zone_checked = false;   // d_zone[0] is of the current state
   bool maxdep_kept = false;    // h_maxdep is on its way from the last step (ev_maxdep)
   cudaEvent_t ev_maxdep = nullptr;
   bool geo_valid = false;      // gk, r2: of the current positions and lists

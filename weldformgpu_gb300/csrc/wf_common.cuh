@@ -214,7 +214,7 @@ struct StepParams {
   const int32_t* inv;   // inv[original id] = slot (particle 0's slot for energy_mode 0)
   int contact;          // contact pass filter active
   int pair_fence;       // always 0: see the mixed acceleration pass
-  const int* zone_mass; // set when a particle with mass carries a mesh's zone id
+  const int* zone_mass; // set when a particle of a mesh's zone would not add exact zeros
   int* near_count;      // contact law 1 fused into the mixed acceleration pass: slots near a
   int32_t* near_list;   // tool (null: the contact is a pass of its own)
   unsigned long long* max_dep;   // adaptive rebuild, mixed form: bits of the largest strain
@@ -337,8 +337,9 @@ __device__ __forceinline__ bool pass_j(const StepParams& P, int32_t idj) {
 }
 
 // The mixed passes' contact filter (pass_ij, pass_j) changes nothing while
-// every particle with a mesh's zone id is massless, as wf_add_trimesh makes
-// them: such a neighbour adds exact zeros.  It then costs an id gathered per
+// every particle with a mesh's zone id is rigid, massless and of an ordinary
+// density, as wf_add_trimesh makes and wf_set_density leaves them: such a
+// neighbour adds exact zeros.  It then costs an id gathered per
 // neighbour (500k particles: density + heat 154 -> 110 us, stress 134 -> 103), so it runs
 // only when P.zone_mass says otherwise (k_zone_mass).
 __device__ __forceinline__ bool zone_filter(const StepParams& P) {
@@ -447,7 +448,7 @@ void launch_contact_stage(const StepParams& P, const Fields& F, const NbBuffers&
 // listed (P.near_list)
 void launch_contact_law1_list(const StepParams& P, const Fields& F, const double4* vd2,
                               float4* a32, cudaStream_t s);
-// *flag = 1 if a particle with mass carries a mesh's zone id (flag zeroed before)
+// *flag = 1 if a particle of a mesh's zone would not add exact zeros (flag zeroed before)
 void launch_zone_mass(const StepParams& P, const Fields& F, int* flag, cudaStream_t s);
 // moved: launch_integrate moved the nodes
 void launch_mesh_update(const StepParams& P, const Fields& F, int mixed, bool moved,

@@ -644,7 +644,10 @@ __global__ void __launch_bounds__(64) k_contact_law1_list(StepParams P, Fields F
   }
 }
 
-// Does a particle with mass carry a mesh's zone id?
+// Does a particle carry a mesh's zone id without adding exact zeros?  It does
+// add them if it is rigid (the pair passes of the mixed form skip its own sums,
+// as the filter does), without mass, and with a density and a velocity that
+// FP32 holds: 0 / 0 or 0 times infinity would not be zero.
 __global__ void __launch_bounds__(256) k_zone_mass(StepParams P, Fields F, int* flag) {
   bool any = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.n;
@@ -652,7 +655,11 @@ __global__ void __launch_bounds__(256) k_zone_mass(StepParams P, Fields F, int* 
     const int32_t id = F.id[i];
     bool zone = false;
     for (int m = 0; m < P.ncsid; m++) zone |= id == P.csid[m];
-    if (zone && F.xm[i].w != 0.0) any = true;
+    if (!zone) continue;
+    const double4 v = F.vd[i];
+    const float rho = (float)v.w;
+    any |= F.perm[i] < P.n_solid || F.xm[i].w != 0.0 || !(rho > 0.0f) || !isfinite(rho) ||
+           !isfinite((float)v.x) || !isfinite((float)v.y) || !isfinite((float)v.z);
   }
   if (any) *flag = 1;
 }
