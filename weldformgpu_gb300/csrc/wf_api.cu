@@ -2071,11 +2071,13 @@ int wf_thermal_solve(wf_domain* d, double tf) {
 
 // ---- getters ---------------------------------------------------------------
 // Where a read-back's kernel writes its values: straight into the caller's array
-// if all of it is one page-locked allocation that the device can write, else
-// (null) into the staging buffer, which is then copied.  For a small field the
+// if it starts on a whole double and all of it is one page-locked allocation
+// that the device can write, else (null) into the staging buffer, which is then
+// copied (to any byte address).  For a small field the
 // copy costs more than the writes (10,752 particles: 21 -> 17 us a field, 24 ->
 // 20 sigma's half megabyte).
 static double* direct_out(const void* out, size_t bytes) {
+  if ((uintptr_t)out % alignof(double) != 0) return nullptr;
   using Attribute = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
   static const Attribute attribute = [] {
     void* f = nullptr;
@@ -2101,6 +2103,7 @@ static double* direct_out(const void* out, size_t bytes) {
       attribute(&dev, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, h) != CUDA_SUCCESS)
     return nullptr;
   if (h < start || h - start > size || bytes > size - (h - start)) return nullptr;
+  if (dev % alignof(double) != 0) return nullptr;
   return reinterpret_cast<double*>((uintptr_t)dev);
 }
 static int download(wf_domain* d, double* out, int64_t count, bool direct) {
