@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(128, kWide ? kWideBlocks : kDensMinBlocks) k_d
   float4* sp = reinterpret_cast<float4*>(sdh);
   float4* sv = sp + T.cap;
   float* st = reinterpret_cast<float*>(sv + T.cap);
-  uint16_t* sl = reinterpret_cast<uint16_t*>(st + ((T.cap + 3) & ~3));
+  uint16_t* sl = reinterpret_cast<uint16_t*>(sdh + density_lists_at(T.cap));
   int staged = -1;
   if (kDensLanes == 1 && T.cap > 0) {
     const float4* src = reinterpret_cast<const float4*>(F.pv);
@@ -689,7 +689,7 @@ __device__ __forceinline__ void stress32_body(StepParams P, Fields F,
   if constexpr (kMlp) mlp_umma_begin(smlp, mlp);
   float4* sp = reinterpret_cast<float4*>(smlp + (kMlp ? WF_UMMA_SMEM : 0));
   float4* sv = sp + T.cap;
-  uint16_t* sl = reinterpret_cast<uint16_t*>(sv + T.cap);
+  uint16_t* sl = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(sp) + stress_lists_at(T.cap));
   const int staged = stage_halo16(T, P.npad, blockIdx.x, sp, sv, pvb, sl);
   const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const bool valid = i0 < P.n;
@@ -1169,7 +1169,7 @@ __global__ void __launch_bounds__(2 * WF_TILE, 3) k_accel_int32_tiles(
   float4* sv = sp + T.cap;
   float4* ssa = sv + T.cap;
   float2* ssb = reinterpret_cast<float2*>(ssa + T.cap);
-  uint16_t* sl = reinterpret_cast<uint16_t*>(ssb + T.cap);
+  uint16_t* sl = reinterpret_cast<uint16_t*>(sac + accel_lists_at(T.cap));
   int staged = -1;
   {
     const int H = T.cap > 0 ? T.hcnt[blockIdx.x] : -1;
@@ -1256,10 +1256,7 @@ void launch_fp32_density_heat(const StepParams& P, const Fields& F, double4* vd2
                               const List16& L16, cudaStream_t s) {
   TileHalo Tl = T;
   if (kDensLanes != 1) Tl.cap = 0;
-  const size_t smem =
-      Tl.cap > 0 ? 2 * sizeof(float4) * (size_t)Tl.cap + sizeof(float) * (size_t)((Tl.cap + 3) & ~3) +
-                       WF_TILE_LIST_BYTES
-                 : 0;
+  const size_t smem = Tl.cap > 0 ? density_lists_at(Tl.cap) + WF_TILE_LIST_BYTES : 0;
   static size_t opted[2][64] = {};  // per variant and device: dynamic shared memory opted in so far
   static size_t c_smem[2] = {0, 0};
   static int64_t c_val[2] = {0, 0};
@@ -1296,8 +1293,9 @@ void launch_fp32_stress(const StepParams& P, const Fields& F, const Rec32* pvb, 
                         cudaStream_t s) {
   const uint4* W = reinterpret_cast<const uint4*>(mlp_packed);
   const MlpL1 l1 = (W && mlp_l1) ? *mlp_l1 : MlpL1{};
+  static_assert(WF_UMMA_SMEM % 16 == 0, "the halo records behind the network's region");
   const size_t smem = (W ? WF_UMMA_SMEM : 0) +
-                      (T.cap > 0 ? 2 * sizeof(float4) * (size_t)T.cap + WF_TILE_LIST_BYTES : 0);
+                      (T.cap > 0 ? stress_lists_at(T.cap) + WF_TILE_LIST_BYTES : 0);
   static size_t opted[2][2][64] = {};  // per variant and device: dynamic shared memory opted in
   static size_t c_smem[2][2] = {};
   static int64_t c_val[2][2] = {};
@@ -1327,7 +1325,7 @@ void launch_fp32_accel_integrate(const StepParams& P, const Fields& F, const Rec
                                  const Sig32& sig, const double4* vd2, float4* a32,
                                  const NbBuffers& N, const TileHalo& T, const List16& L16, cudaStream_t s) {
   if (T.cap > 0) {
-    const size_t smem = (3 * sizeof(float4) + sizeof(float2)) * (size_t)T.cap + WF_TILE_LIST_BYTES;
+    const size_t smem = accel_lists_at(T.cap) + WF_TILE_LIST_BYTES;
     static size_t opted[64] = {};
     opt_in_smem(k_accel_int32_tiles, smem, opted);
     k_accel_int32_tiles<<<blocks_for(P.n * kAccelLanes, 2 * WF_TILE), 2 * WF_TILE, smem, s>>>(

@@ -78,6 +78,26 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // slot at sl[(b * WF_TILE + t) * 8] (the global layout with WF_TILE as stride)
 #define WF_TILE_LIST_BYTES (WF_NB_BLOCKS * WF_TILE * WF_NB_BLK * 2)
 
+// Where the lists stand behind a staged halo of `cap` records: float4 position
+// and velocity with a float (density + heat), with nothing more (stress), with
+// a float4 and a float2 of stress (acceleration).  The lists are written and
+// read 16 bytes at a time and cap may be any number (option tile_cap_max), so
+// the last array is rounded up.
+__host__ __device__ constexpr size_t density_lists_at(int cap) {
+  return 32 * (size_t)cap + 4 * (size_t)((cap + 3) & ~3);
+}
+__host__ __device__ constexpr size_t stress_lists_at(int cap) { return 32 * (size_t)cap; }
+__host__ __device__ constexpr size_t accel_lists_at(int cap) {
+  return 48 * (size_t)cap + 8 * (size_t)((cap + 1) & ~1);
+}
+constexpr bool lists_on_16_bytes() {
+  for (int cap = 1; cap <= WF_TILE_HALO_MAX; cap++)
+    if (density_lists_at(cap) % 16 || stress_lists_at(cap) % 16 || accel_lists_at(cap) % 16)
+      return false;
+  return true;
+}
+static_assert(lists_on_16_bytes(), "local lists on 16-byte boundaries for every halo capacity");
+
 // Copies the tile's local lists (all WF_NB_BLOCKS blocks, 2 KB each,
 // contiguous in global memory) into shared memory with 16-byte cp.async;
 // the caller waits (cp_async_wait_all + barrier).
