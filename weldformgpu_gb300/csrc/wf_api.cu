@@ -174,6 +174,14 @@ struct wf_domain {
   double time = 0, t_out = 0, dt_out = 0;
   int64_t step = 0;
   int ts_i = 0;
+  // what the host has counted up to a rebuild that it has not seen yet (rb_pending): a refusal
+  // goes back to it, since the steps captured behind the rebuild then never run
+  struct StepMark {
+    double time, t_out;
+    int64_t step, rebuilds, launches;
+    int ts_i, light_rebuilds;
+    bool isfirst, heat_pending, heat_pending_first, row_recorded, lists_stale, zone_checked;
+  } mark{};
   GridDev grid{};
   // measurement
   int64_t launches = 0;
@@ -889,12 +897,29 @@ static int build_lists(wf_domain* d, const StaticHeader* hdr, bool full) {
   return WF_OK;
 }
 
+static void mark_steps(wf_domain* d) {
+  d->mark = {d->time, d->t_out, d->step, d->rebuilds, d->launches, d->ts_i, d->light_rebuilds,
+             d->isfirst, d->heat_pending, d->heat_pending_first, d->row_recorded, d->lists_stale,
+             d->zone_checked};
+}
+static void back_to_mark(wf_domain* d) {
+  const wf_domain::StepMark& m = d->mark;
+  d->time = m.time; d->t_out = m.t_out; d->step = m.step; d->rebuilds = m.rebuilds;
+  d->launches = m.launches; d->ts_i = m.ts_i; d->light_rebuilds = m.light_rebuilds;
+  d->isfirst = m.isfirst; d->heat_pending = m.heat_pending;
+  d->heat_pending_first = m.heat_pending_first; d->row_recorded = m.row_recorded;
+  d->lists_stale = m.lists_stale; d->zone_checked = m.zone_checked;
+  d->geo_valid = false;
+}
+
 // Inside the step loop a rebuild does not make the GPU wait for the host: its
 // kernels read the grid from device memory, and the host looks at the bounds
 // only when it has captured the steps behind them, before it launches those.
 // If the grid did not fit the cells allocated (a quarter more than the last one
 // that did not), nothing was searched, and the lists are built then with the
-// cells they need.  (10,752 particles: 55 -> 44 us a rebuild, of which the
+// cells they need; if that is refused, the steps captured behind the rebuild are
+// dropped and the host's counts go back to before it, as where the host waits.
+// (10,752 particles: 55 -> 44 us a rebuild, of which the
 // kernels take most.)
 static int rebuild_verify(wf_domain* d) {
   if (!d->rb_pending) return WF_OK;
@@ -905,8 +930,10 @@ static int rebuild_verify(wf_domain* d) {
     d->ncell_last = h->ncell;
     return WF_OK;
   }
-  const int rc = grid_from_codes(d, h->mm);
-  return rc ? rc : build_lists(d, nullptr, false);
+  int rc = grid_from_codes(d, h->mm);
+  if (rc == WF_OK) rc = build_lists(d, nullptr, false);
+  if (rc) back_to_mark(d);
+  return rc;
 }
 
 static int rebuild(wf_domain* d, bool use_current, bool light = false) {
@@ -925,7 +952,7 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
   // moving it keeps warps' particles close in space.  Inside the step loop
   // the state is moved at every kReorderEvery-th rebuild only (solids move
   // little in between); otherwise the lists name the particles' current slots.
-  const bool full = !light || ++d->light_rebuilds >= kReorderEvery;
+  const bool full = !light || d->light_rebuilds + 1 >= kReorderEvery;
   const bool tiles = d->precision == 1 && d->tile_staging && d->meshes.empty();
   const bool deferred = !full && segments(d) && d->ncell_last > 0 && !d->debug_checks && !tiles &&
                         d->tile_cap == 0;
@@ -937,6 +964,8 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
   if (deferred) {
     WF_CUDA_OK(cudaEventRecord(d->ev_rb, s));
     d->rb_pending = true;
+    mark_steps(d);
+    d->light_rebuilds++;
     return build_lists(d, d->d_hdr, false);
   }
   unsigned mm[6];
@@ -945,7 +974,9 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
     WF_CUDA_OK(cudaMemcpyAsync(&d->tile_hmax, d->d_mm + 6, sizeof(int), cudaMemcpyDeviceToHost, s));
   WF_CUDA_OK(cudaStreamSynchronize(s));
   const int rc = grid_from_codes(d, mm);
-  return rc ? rc : build_lists(d, nullptr, full);
+  if (rc) return rc;
+  if (!full) d->light_rebuilds++;
+  return build_lists(d, nullptr, full);
 }
 
 // The triangles of each tool binned once in the tool's frame as it stands
