@@ -827,8 +827,11 @@ static int grid_from_codes(wf_domain* d, const unsigned* codes) {
   int bounds[6];
   bounds_from_codes(codes, bounds);
   grid_from_bounds(bounds, (float)(2.0 * d->h), &d->grid);
-  const int64_t ncell = (int64_t)d->grid.dim[0] * d->grid.dim[1] * d->grid.dim[2];
-  if (ncell > (int64_t)2000000000) return wf_fail(d, WF_ERR_NUMERIC, "neighbour grid too large");
+  int64_t ncell = 1;
+  for (int a = 0; a < 3; a++) {          // axis by axis: three spans may overflow 64 bits
+    ncell = d->grid.dim[a] > 0 ? ncell * d->grid.dim[a] : INT64_MAX;
+    if (ncell > (int64_t)2000000000) return wf_fail(d, WF_ERR_NUMERIC, "neighbour grid too large");
+  }
   d->ncell_last = ncell;
   return ensure_cells(d, ncell);
 }
