@@ -67,8 +67,9 @@ typedef struct wf_domain wf_domain;
 int         wf_create(wf_domain** out, int64_t particle_count);
 /* Domain_d::~Domain_d.  The domain's device arena (one allocation for every
  * per-particle array) is kept for the next wf_create on the same device whose
- * layout needs between 80 and 100 % of it (zeroed there like a fresh one);
- * wf_release_cache() returns it to the driver. */
+ * layout needs between 80 and 100 % of it (zeroed there like a fresh one), and
+ * its pair work arrays (option pair_cache) for the next domain of that size
+ * that asks for such arrays; wf_release_cache() returns both to the driver. */
 int         wf_destroy(wf_domain* d);
 int         wf_release_cache(void);
 const char* wf_last_error(const wf_domain* d);

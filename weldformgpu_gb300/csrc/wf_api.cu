@@ -479,12 +479,15 @@ static void free_fields(Fields& F) {
 // whose layout needs between 80 and 100 % of it takes it over (zeroed on its
 // stream like a fresh one).  cudaMalloc and cudaFree of the ~1 GB arena of a
 // 786k-particle domain cost ~0.5 ms each, paid by every drop-in call that
-// creates and destroys its domain.  A cached block that does not fit is freed
-// before the new allocation; wf_release_cache() frees the cache.
+// creates and destroys its domain.  Its pair work arrays stay too, and go to
+// the next domain only when that asks for such arrays (cache_take_work): a
+// mixed domain never does.  A cached block that does not fit is freed before
+// the new allocation, all of it when an allocation finds no memory;
+// wf_release_cache() frees the cache.
 struct ArenaCache {
   char* arena = nullptr;
   size_t bytes = 0;
-  int dev = -1;
+  int dev = -1;                // of all of it
   int* h_status = nullptr;
   char* work = nullptr;        // the domain's pair work arrays
   size_t work_bytes = 0;
@@ -501,11 +504,11 @@ static std::mutex g_cache_mu;
 static ArenaCache g_cache;
 
 static void cache_free_locked() {
-  if (g_cache.arena) {
+  if (g_cache.arena || g_cache.work) {
     int cur = 0;
     cudaGetDevice(&cur);
     cudaSetDevice(g_cache.dev);
-    cudaFree(g_cache.arena);
+    if (g_cache.arena) cudaFree(g_cache.arena);
     if (g_cache.work) cudaFree(g_cache.work);
     if (g_cache.cells) cudaFree(g_cache.cells);
     cudaSetDevice(cur);
@@ -524,14 +527,34 @@ static void cache_take(wf_domain* d) {
   d->arena = g_cache.arena;
   d->arena_alloc = g_cache.bytes;
   d->h_status = g_cache.h_status;
-  d->work = g_cache.work;
-  d->work_bytes = g_cache.work_bytes;
   if (g_cache.cells) {
     d->cell_count = g_cache.cells;
     cells_place(d, g_cache.cell_cap);
     cudaMemsetAsync(d->cell_count, 0, sizeof(uint32_t) * (size_t)cell_words(d->cell_cap), d->stream);
   }
-  g_cache = ArenaCache{};
+  ArenaCache rest;
+  rest.dev = g_cache.dev;
+  rest.work = g_cache.work;
+  rest.work_bytes = g_cache.work_bytes;
+  g_cache = rest;
+}
+// the cached work arrays if they fit `bytes` as the arena must fit; else they are freed
+static void cache_take_work(wf_domain* d, size_t bytes) {
+  std::lock_guard<std::mutex> lk(g_cache_mu);
+  if (!g_cache.work) return;
+  if (g_cache.dev == d->dev && g_cache.work_bytes >= bytes &&
+      g_cache.work_bytes <= bytes + bytes / 4) {
+    d->work = g_cache.work;
+    d->work_bytes = g_cache.work_bytes;
+  } else {
+    int cur = 0;
+    cudaGetDevice(&cur);
+    cudaSetDevice(g_cache.dev);
+    cudaFree(g_cache.work);
+    cudaSetDevice(cur);
+  }
+  g_cache.work = nullptr;
+  g_cache.work_bytes = 0;
 }
 static void cache_put(wf_domain* d) {
   if (!d->arena) return;
@@ -785,6 +808,8 @@ static bool work_reserve(wf_domain* d, size_t bytes) {
     d->work = nullptr;
     d->geo_valid = false;
   }
+  cache_take_work(d, bytes);
+  if (d->work) return true;
   if (cudaMalloc((void**)&d->work, bytes) != cudaSuccess) {
     cudaGetLastError();
     d->work = nullptr;
