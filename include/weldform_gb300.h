@@ -155,8 +155,9 @@ int wf_add_trimesh(wf_domain* d, const double* nodes, int32_t nn, const int32_t*
  *   contact_dx (0),
  *   contact_stiffness (0.1), contact_vreg (1e-3), contact_heat_fraction (1),
  *   fuse_heat (1), fuse_integrate (1), pair_cache (1; 0: the FP64 passes of a
- *   step each compute the pair geometry instead of keeping it, 1.2 KB less per
- *   particle, same results), tile_staging (0; 1: the mixed pair passes
+ *   step each compute the pair geometry instead of keeping it, same results; kept, it
+ *   takes 1.2 KB per particle from the first step on, which another allocation of the
+ *   domain gets when there is no memory left), tile_staging (0; 1: the mixed pair passes
  *   read neighbours from per-tile halos in shared memory; same results),
  *   tile_cap_max (2048: largest halo staged), list_prefetch (2: L2 prefetch of
  *   the neighbour lists that many blocks ahead; 0 off), state_prefetch (1: L2 prefetch, before
@@ -171,7 +172,9 @@ int wf_add_trimesh(wf_domain* d, const double* nodes, int32_t nn, const int32_t*
  *   for non-finite values; either sets status bit 6 and the call returns
  *   WF_ERR_STATE), debug_inject_list_error (a particle id: its list's first entry is
  *   set out of range after the next list build, for testing the checks; only with
- *   debug_checks = 1). */
+ *   debug_checks = 1), debug_refuse_allocations (a count: so many of the domain's next
+ *   device allocations are refused as if there were no memory, for testing what
+ *   gives way to them). */
 int wf_set_option(wf_domain* d, const char* key, double value);
 
 /* The per-step BC hook: Domain_d::GeneralAfter (src/cuda/Domain_d.cuh:402,

@@ -172,13 +172,14 @@ struct wf_domain {
   bool csv_on = false;
   std::string csv_prefix;
   double time = 0, t_out = 0, dt_out = 0;
-  int64_t step = 0;
+  int64_t step = 0, call_steps = 0;   // since the solve's start; of the present call
   int ts_i = 0;
   // what the host has counted up to a rebuild that it has not seen yet (rb_pending): a refusal
   // goes back to it, since the steps captured behind the rebuild then never run
   struct StepMark {
     double time, t_out;
-    int64_t step, rebuilds, launches;
+    int64_t step, call_steps, rebuilds, launches;
+    size_t ev_used;
     int ts_i, light_rebuilds;
     bool isfirst, heat_pending, heat_pending_first, row_recorded, lists_stale, zone_checked;
   } mark{};
@@ -190,9 +191,11 @@ struct wf_domain {
   bool timing = false;         // inside wf_time_steps
   int debug_checks = 0;        // option "debug_checks"
   int64_t inject_list_error = -1;   // option "debug_inject_list_error" (original id), -1 off
+  int64_t inject_refusals = 0;      // option "debug_refuse_allocations"
   // step-segment graphs (segment_begin / segment_end)
   int graph = 1;                // option "graph"
   bool capturing = false;
+  bool segment_held = false;    // a captured segment waits for its rebuild to be verified
   cudaGraphExec_t gexec = nullptr;
   int64_t graph_launches = 0, graph_instantiations = 0;
   std::string err;
@@ -402,13 +405,33 @@ inline int nblk(int64_t n, int t = 256) { return (int)((n + t - 1) / t); }
 // ---------------------------------------------------------------------------
 // allocation
 // ---------------------------------------------------------------------------
+// A device allocation of the domain.  When there is no memory for it, the
+// optional blocks go first: the cache, then the domain's pair work arrays
+// (the passes then compute what these keep).
+static bool give_back(wf_domain* d);
+static cudaError_t dev_malloc(wf_domain* d, void** p, size_t bytes) {
+  const auto take = [&] {
+    if (d->inject_refusals > 0) {
+      d->inject_refusals--;
+      return cudaErrorMemoryAllocation;
+    }
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+  };
+  *p = nullptr;
+  cudaError_t e = take();
+  if (e == cudaErrorMemoryAllocation && give_back(d)) e = take();
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
 // Zero-filled on the domain's own stream: that stream is non-blocking, so a
 // cudaMemset on the legacy default stream would not be ordered before it.
 template <class T>
-static cudaError_t dalloc(T** p, int64_t count, cudaStream_t s) {
+static cudaError_t dalloc(T** p, int64_t count, wf_domain* d) {
   const size_t bytes = sizeof(T) * (size_t)std::max<int64_t>(count, 1);
-  cudaError_t e = cudaMalloc((void**)p, bytes);
-  if (e == cudaSuccess) e = cudaMemsetAsync(*p, 0, bytes, s);
+  cudaError_t e = dev_malloc(d, (void**)p, bytes);
+  if (e == cudaSuccess) e = cudaMemsetAsync(*p, 0, bytes, d->stream);
   return e;
 }
 
@@ -741,7 +764,9 @@ static int segment_end(wf_domain* d) {
     d->graph_instantiations++;
   }
   cudaGraphDestroy(g);
+  d->segment_held = true;
   const int rc = rebuild_verify(d);      // the lists that the segment's steps read
+  d->segment_held = false;
   if (rc) return rc;
   WF_CUDA_OK(cudaGraphLaunch(d->gexec, d->stream));
   d->graph_launches++;
@@ -791,33 +816,51 @@ static int ensure_cells(wf_domain* d, int64_t ncell) {
   d->cell_count = nullptr;
   d->cell_cap = 0;
   const int64_t cap = (ncell + 1) + (ncell + 1) / 4 + 1024;
-  WF_CUDA_OK(dalloc(&d->cell_count, cell_words(cap), d->stream));
+  WF_CUDA_OK(dalloc(&d->cell_count, cell_words(cap), d));
   cells_place(d, cap);
   return WF_OK;
 }
 
+static void work_drop(wf_domain* d) {
+  if (!d->work) return;
+  cudaStreamSynchronize(d->stream);       // the passes that still read it
+  cudaFree(d->work);
+  d->work = nullptr;
+  d->work_bytes = 0;
+  d->geo_valid = false;
+}
 // Work arrays of at least `bytes`; false when there is no memory for them (the
 // passes then compute the pair geometry themselves).  Not inside a capture.
 static bool work_reserve(wf_domain* d, size_t bytes) {
   if (!d->pair_cache) return false;
   if (d->work && d->work_bytes >= bytes) return true;
   if (d->capturing || (d->work_refused && bytes >= d->work_refused)) return false;
-  if (d->work) {
-    cudaStreamSynchronize(d->stream);   // the passes that still read it
-    cudaFree(d->work);
-    d->work = nullptr;
-    d->geo_valid = false;
-  }
+  work_drop(d);
   cache_take_work(d, bytes);
   if (d->work) return true;
-  if (cudaMalloc((void**)&d->work, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    d->work = nullptr;
+  if (dev_malloc(d, (void**)&d->work, bytes) != cudaSuccess) {
     d->work_refused = bytes;
     return false;
   }
   d->work_bytes = bytes;
   return true;
+}
+// Frees what an allocation of the domain may do without; false when that is
+// nothing.  A held segment's launches name the work arrays (rebuild_verify drops
+// the segment first); while one is being captured nothing is allocated.
+static bool give_back(wf_domain* d) {
+  bool any = false;
+  {
+    std::lock_guard<std::mutex> lk(g_cache_mu);
+    any = g_cache.arena || g_cache.work;
+    cache_free_locked();
+  }
+  if (d->work && !d->segment_held && !d->capturing) {
+    d->work_refused = d->work_bytes;      // not asked for again
+    work_drop(d);
+    any = true;
+  }
+  return any;
 }
 static size_t work64_bytes(const wf_domain* d) {
   return sizeof(double) * (size_t)(2 * WF_NB_ALLOC + 8) * (size_t)d->npad;
@@ -925,15 +968,18 @@ static int build_lists(wf_domain* d, const StaticHeader* hdr, bool full) {
   return WF_OK;
 }
 
+// the steps behind the marked rebuild were dropped and are to run again (run_steps)
+constexpr int kStepsAgain = 1 << 20;
 static void mark_steps(wf_domain* d) {
-  d->mark = {d->time, d->t_out, d->step, d->rebuilds, d->launches, d->ts_i, d->light_rebuilds,
-             d->isfirst, d->heat_pending, d->heat_pending_first, d->row_recorded, d->lists_stale,
-             d->zone_checked};
+  d->mark = {d->time, d->t_out, d->step, d->call_steps, d->rebuilds, d->launches, d->ev_used,
+             d->ts_i, d->light_rebuilds, d->isfirst, d->heat_pending, d->heat_pending_first,
+             d->row_recorded, d->lists_stale, d->zone_checked};
 }
 static void back_to_mark(wf_domain* d) {
   const wf_domain::StepMark& m = d->mark;
-  d->time = m.time; d->t_out = m.t_out; d->step = m.step; d->rebuilds = m.rebuilds;
-  d->launches = m.launches; d->ts_i = m.ts_i; d->light_rebuilds = m.light_rebuilds;
+  d->time = m.time; d->t_out = m.t_out; d->step = m.step; d->call_steps = m.call_steps;
+  d->rebuilds = m.rebuilds; d->launches = m.launches; d->ev_used = m.ev_used;
+  d->ts_i = m.ts_i; d->light_rebuilds = m.light_rebuilds;
   d->isfirst = m.isfirst; d->heat_pending = m.heat_pending;
   d->heat_pending_first = m.heat_pending_first; d->row_recorded = m.row_recorded;
   d->lists_stale = m.lists_stale; d->zone_checked = m.zone_checked;
@@ -960,7 +1006,16 @@ static int rebuild_verify(wf_domain* d) {
   }
   int rc = grid_from_codes(d, h->mm);
   if (rc == WF_OK) rc = build_lists(d, nullptr, false);
-  if (rc) back_to_mark(d);
+  if (rc) {
+    back_to_mark(d);
+    if (!d->cell_count && d->work && d->segment_held) {
+      // no memory for the cells: once more without the work arrays, which the
+      // dropped steps used
+      d->work_refused = d->work_bytes;
+      work_drop(d);
+      return kStepsAgain;
+    }
+  }
   return rc;
 }
 
@@ -982,8 +1037,8 @@ static int rebuild(wf_domain* d, bool use_current, bool light = false) {
   // little in between); otherwise the lists name the particles' current slots.
   const bool full = !light || d->light_rebuilds + 1 >= kReorderEvery;
   const bool tiles = d->precision == 1 && d->tile_staging && d->meshes.empty();
-  const bool deferred = !full && segments(d) && d->ncell_last > 0 && !d->debug_checks && !tiles &&
-                        d->tile_cap == 0;
+  const bool deferred = !full && segments(d) && d->cell_count && d->ncell_last > 0 &&
+                        !d->debug_checks && !tiles && d->tile_cap == 0;
   if (deferred && !d->ev_rb)
     WF_CUDA_OK(cudaEventCreateWithFlags(&d->ev_rb, cudaEventDisableTiming));
   const float r = (float)(2.0 * d->h);                // SolverFraser.cu:72-82
@@ -1055,7 +1110,7 @@ static int build_tool_bins(wf_domain* d) {
       M.glo[k] = (float)(M.grel[k] - cs);
       M.ghi[k] = (float)(M.grel[k] + (M.dims[k] + 1) * cs);
     }
-    if (!M.off32 && dalloc(&M.off32, 1, d->stream) != cudaSuccess)
+    if (!M.off32 && dalloc(&M.off32, 1, d) != cudaSuccess)
       return wf_fail(d, WF_ERR_ALLOC, "tool offset");
     const float4 o = make_float4((float)nd[0].x, (float)nd[0].y, (float)nd[0].z, 0.f);
     WF_CUDA_OK(cudaMemcpyAsync(M.off32, &o, sizeof(float4), cudaMemcpyHostToDevice, d->stream));
@@ -1082,9 +1137,9 @@ static int build_tool_bins(wf_domain* d) {
         cap += span * span * span;
       }
       M.cap = cap;
-      if (dalloc(&M.cstart, ncell + 1, d->stream) || dalloc(&M.cursor, ncell, d->stream) ||
-          dalloc(&M.scan_tmp, scan_tmp_words(ncell + 1), d->stream) ||
-          dalloc(&M.cvert, 3 * cap, d->stream))
+      if (dalloc(&M.cstart, ncell + 1, d) || dalloc(&M.cursor, ncell, d) ||
+          dalloc(&M.scan_tmp, scan_tmp_words(ncell + 1), d) ||
+          dalloc(&M.cvert, 3 * cap, d))
         return wf_fail(d, WF_ERR_ALLOC, "rotating tool bins");
       continue;   // binned on the GPU before every contact stage
     }
@@ -1121,7 +1176,7 @@ static int build_tool_bins(wf_domain* d) {
       }
     }
     M.cap = (int64_t)list.size();
-    if (dalloc(&M.cstart, ncell + 1, d->stream) || dalloc(&M.ctri, std::max<int64_t>(1, (int64_t)list.size()), d->stream))
+    if (dalloc(&M.cstart, ncell + 1, d) || dalloc(&M.ctri, std::max<int64_t>(1, (int64_t)list.size()), d))
       return wf_fail(d, WF_ERR_ALLOC, "tool bins");
     WF_CUDA_OK(cudaMemcpyAsync(M.cstart, start.data(), sizeof(int32_t) * (ncell + 1), cudaMemcpyHostToDevice, d->stream));
     if (!list.empty())
@@ -1137,7 +1192,7 @@ static int build_tool_bins(wf_domain* d) {
         cv[3 * t + k] = make_float4((float)p[0], (float)p[1], (float)p[2], w);
       }
     }
-    if (dalloc(&M.cvert, (int64_t)cv.size(), d->stream) != cudaSuccess)
+    if (dalloc(&M.cvert, (int64_t)cv.size(), d) != cudaSuccess)
       return wf_fail(d, WF_ERR_ALLOC, "tool bin vertices");
     WF_CUDA_OK(cudaMemcpyAsync(M.cvert, cv.data(), sizeof(float4) * cv.size(), cudaMemcpyHostToDevice,
                                d->stream));
@@ -1226,7 +1281,7 @@ static int solve_begin(wf_domain* d, double dt_out) {
     if (!d->series || width != d->series_width) {
       if (d->series) cudaFree(d->series);
       d->series = nullptr;
-      if (dalloc(&d->series, d->series_cap * width, d->stream) != cudaSuccess) {
+      if (dalloc(&d->series, d->series_cap * width, d) != cudaSuccess) {
         d->series = nullptr;
         return wf_fail(d, WF_ERR_ALLOC, "output series");
       }
@@ -1441,6 +1496,7 @@ static int solve_step_launches(wf_domain* d) {
     }
   }
   d->step++;
+  d->call_steps++;
   d->ts_i++;
   if (d->ts_i > d->rebuild_every - 1) d->ts_i = 0;
   // the yield flag matters only for the next rebuild decision
@@ -1473,6 +1529,18 @@ static int solve_step(wf_domain* d) {
   kept_drop(d);
   if (r) return wf_fail(d, WF_ERR_STATE, "step callback returned " + std::to_string(r));
   return WF_OK;
+}
+
+// Steps while `more` says so, then `end`; both again from the mark when the
+// steps behind it were dropped (kStepsAgain).
+template <class More, class End>
+static int run_steps(wf_domain* d, More more, End end) {
+  for (;;) {
+    int rc = WF_OK;
+    while (rc == WF_OK && more()) rc = solve_step(d);
+    if (rc == WF_OK) rc = end();
+    if (rc != kStepsAgain) return rc;
+  }
 }
 
 // the last step's heat pass (mixed form), before any result leaves a call
@@ -1542,10 +1610,8 @@ int wf_create(wf_domain** out, int64_t n) {
     d->arena_bytes = size.off;
     cache_take(d);
     if (!d->arena) {
-      if (cudaMalloc((void**)&d->arena, d->arena_bytes) != cudaSuccess) {
-        d->arena = nullptr;
+      if (dev_malloc(d, (void**)&d->arena, d->arena_bytes) != cudaSuccess)
         return bail(WF_ERR_ALLOC);
-      }
       d->arena_alloc = d->arena_bytes;
     }
     if (cudaMemsetAsync(d->arena, 0, d->arena_bytes, d->stream) != cudaSuccess)
@@ -1805,7 +1871,7 @@ int wf_set_contact(wf_domain* d, double mu_static, double mu_dynamic, int law) {
   if (law == 1) {
     if (!d->F[0].qf)
       for (int f = 0; f < 2; f++)
-        if (dalloc(&d->F[f].qf, d->npad, d->stream)) return wf_fail(d, WF_ERR_ALLOC, "qf");
+        if (dalloc(&d->F[f].qf, d->npad, d)) return wf_fail(d, WF_ERR_ALLOC, "qf");
   }
   d->mu_s = mu_static;
   d->mu_d = mu_dynamic;
@@ -1856,8 +1922,8 @@ int wf_add_trimesh(wf_domain* d, const double* nodes, int32_t nn, const int32_t*
   M.nn = nn; M.ne = ne; M.first = (int32_t)first; M.zone = zone_id;
   for (int k = 0; k < 3; k++) { M.mv[k] = vel[k]; M.mw[k] = angvel[k]; }
   cudaStream_t s = d->stream;
-  if (dalloc(&M.node, nn, s) || dalloc(&M.node_v, nn, s) || dalloc(&M.centroid, ne, s) ||
-      dalloc(&M.normal, ne, s) || dalloc(&M.elnode, 3 * (int64_t)ne, s) || dalloc(&M.pplane, ne, s)) {
+  if (dalloc(&M.node, nn, d) || dalloc(&M.node_v, nn, d) || dalloc(&M.centroid, ne, d) ||
+      dalloc(&M.normal, ne, d) || dalloc(&M.elnode, 3 * (int64_t)ne, d) || dalloc(&M.pplane, ne, d)) {
     void* mp[] = {M.node, M.node_v, M.centroid, M.normal, M.elnode, M.pplane};
     for (void* p : mp) if (p) cudaFree(p);
     return wf_fail(d, WF_ERR_ALLOC, "mesh arrays");
@@ -1870,9 +1936,9 @@ int wf_add_trimesh(wf_domain* d, const double* nodes, int32_t nn, const int32_t*
   WF_CUDA_OK(cudaMemcpyAsync(M.elnode, tris, sizeof(int32_t) * 3 * ne, cudaMemcpyHostToDevice, s));
   if (!d->cnb) {               // per-particle contact state, on the first mesh
     for (int k = 0; k < 2; k++)
-      if (dalloc(&d->F[k].nrm, d->npad, s) || dalloc(&d->F[k].cf, d->npad, s))
+      if (dalloc(&d->F[k].nrm, d->npad, d) || dalloc(&d->F[k].cf, d->npad, d))
         return wf_fail(d, WF_ERR_ALLOC, "contact fields");
-    if (dalloc(&d->cnb, (int64_t)WF_CONT_NB * d->npad, s) || dalloc(&d->ccnt, d->npad, s))
+    if (dalloc(&d->cnb, (int64_t)WF_CONT_NB * d->npad, d) || dalloc(&d->ccnt, d->npad, d))
       return wf_fail(d, WF_ERR_ALLOC, "contact lists");
   }
   k_place_rigid<<<nblk(ne), 256, 0, s>>>(ne, (int32_t)first, d->inv, M.centroid, M.normal,
@@ -1951,8 +2017,8 @@ int wf_set_option(wf_domain* d, const char* key, double v) {
     if (!(v >= 0.0)) return wf_fail(d, WF_ERR_ARG, "rebuild_strain_increment must be >= 0");
     if (v > 0.0 && !d->F[0].eps_rb) {
       for (int f = 0; f < 2; f++)
-        if (dalloc(&d->F[f].eps_rb, d->npad, d->stream)) return wf_fail(d, WF_ERR_ALLOC, "eps_rb");
-      if (dalloc(&d->d_maxdep, 1, d->stream) ||
+        if (dalloc(&d->F[f].eps_rb, d->npad, d)) return wf_fail(d, WF_ERR_ALLOC, "eps_rb");
+      if (dalloc(&d->d_maxdep, 1, d) ||
           cudaMallocHost((void**)&d->h_maxdep, sizeof(unsigned long long)) != cudaSuccess ||
           cudaEventCreateWithFlags(&d->ev_maxdep, cudaEventDisableTiming) != cudaSuccess)
         return wf_fail(d, WF_ERR_ALLOC, "rebuild flag");
@@ -1988,9 +2054,9 @@ int wf_set_option(wf_domain* d, const char* key, double v) {
     d->log_x = nullptr; d->log_y = nullptr; d->log_count = nullptr;
     d->log_cap = (int64_t)v;
     if (d->log_cap > 0) {
-      WF_CUDA_OK(dalloc(&d->log_x, d->log_cap, d->stream));
-      WF_CUDA_OK(dalloc(&d->log_y, d->log_cap, d->stream));
-      WF_CUDA_OK(dalloc(&d->log_count, 1, d->stream));
+      WF_CUDA_OK(dalloc(&d->log_x, d->log_cap, d));
+      WF_CUDA_OK(dalloc(&d->log_y, d->log_cap, d));
+      WF_CUDA_OK(dalloc(&d->log_count, 1, d));
     }
   }
   else if (k == "pair_cache") {
@@ -2008,6 +2074,11 @@ int wf_set_option(wf_domain* d, const char* key, double v) {
     if (!(v >= 0.0) || v >= (double)d->n)
       return wf_fail(d, WF_ERR_ARG, "debug_inject_list_error: a particle id in [0, n)");
     d->inject_list_error = (int64_t)v;
+  }
+  else if (k == "debug_refuse_allocations") {
+    if (!(v >= 0.0) || v > 1.0e9)
+      return wf_fail(d, WF_ERR_ARG, "debug_refuse_allocations: a count in [0, 1e9]");
+    d->inject_refusals = (int64_t)v;
   }
   else if (k == "wave_prefetch") d->wave_prefetch = (int)v;
   else if (k == "wave_prefetch_distance") d->wave_dist = v;
@@ -2043,11 +2114,8 @@ int wf_step(wf_domain* d, int64_t nsteps) {
     if (rc) return rc;
   }
   kept_drop(d);
-  for (int64_t k = 0; k < nsteps; k++) {
-    int rc = solve_step(d);
-    if (rc) return rc;
-  }
-  return finish(d);
+  d->call_steps = 0;
+  return run_steps(d, [&] { return d->call_steps < nsteps; }, [&] { return finish(d); });
 }
 
 int wf_mech_fraser_solve(wf_domain* d, double tf, double dt_out) {
@@ -2055,11 +2123,7 @@ int wf_mech_fraser_solve(wf_domain* d, double tf, double dt_out) {
   if (d->in_callback) return wf_fail(d, WF_ERR_STATE, "solvers cannot be called from the step callback");
   int rc = solve_begin(d, dt_out);
   if (rc) return rc;
-  while (d->time < tf) {
-    rc = solve_step(d);
-    if (rc) return rc;
-  }
-  rc = finish(d);
+  rc = run_steps(d, [&] { return d->time < tf; }, [&] { return finish(d); });
   if (rc == WF_OK && d->csv_on) rc = write_series_csv(d, (d->csv_prefix + "outputs.csv").c_str());
   return rc;
 }
@@ -2326,8 +2390,8 @@ int wf_get_neighbors(wf_domain* d, int32_t* counts, int32_t* lists) {
   if (!d || !counts || !lists) return WF_ERR_ARG;
   if (!d->nb_built) return wf_fail(d, WF_ERR_STATE, "no neighbour list yet");
   int32_t *dc = nullptr, *dl = nullptr;
-  WF_CUDA_OK(cudaMalloc((void**)&dc, sizeof(int32_t) * d->n));
-  cudaError_t e = cudaMalloc((void**)&dl, sizeof(int32_t) * d->n * WF_NB);
+  WF_CUDA_OK(dev_malloc(d, (void**)&dc, sizeof(int32_t) * d->n));
+  cudaError_t e = dev_malloc(d, (void**)&dl, sizeof(int32_t) * d->n * WF_NB);
   if (e != cudaSuccess) { cudaFree(dc); return wf_cuda_fail(d, e, "cudaMalloc"); }
   k_gather_nb<<<nblk(d->n), 256, 0, d->stream>>>(d->n, d->npad, d->inv, CF(d).perm, d->nb, d->nbc, dc, dl);
   cudaMemcpyAsync(counts, dc, sizeof(int32_t) * d->n, cudaMemcpyDeviceToHost, d->stream);
@@ -2548,12 +2612,14 @@ int wf_time_steps(wf_domain* d, int64_t nsteps, double* elapsed_ms, double* kern
   const int64_t l0 = d->launches;
   WF_CUDA_OK(cudaStreamSynchronize(d->stream));
   cudaEventRecord(e0, d->stream);
-  int rc = WF_OK;
   d->timing = true;
   kept_drop(d);
-  for (int64_t k = 0; k < nsteps && rc == WF_OK; k++) rc = solve_step(d);
-  flush_heat(d);   // the timed steps include their whole heat work
-  if (rc == WF_OK) rc = segment_end(d);
+  d->call_steps = 0;
+  const int rc = run_steps(d, [&] { return d->call_steps < nsteps; }, [&] {
+    flush_heat(d);   // the timed steps include their whole heat work
+    return segment_end(d);
+  });
+  flush_heat(d);
   d->timing = false;
   cudaEventRecord(e1, d->stream);
   WF_CUDA_OK(cudaEventSynchronize(e1));
