@@ -157,7 +157,7 @@ int wf_add_trimesh(wf_domain* d, const double* nodes, int32_t nn, const int32_t*
  *   fuse_heat (1), fuse_integrate (1), pair_cache (1; 0: the FP64 passes of a
  *   step each compute the pair geometry instead of keeping it, same results; kept, it
  *   takes 1.2 KB per particle from the first step on, which another allocation of the
- *   domain gets when there is no memory left), tile_staging (0; 1: the mixed pair passes
+ *   domain gets when there is no memory left, and setting 0 frees), tile_staging (0; 1: the mixed pair passes
  *   read neighbours from per-tile halos in shared memory; same results),
  *   tile_cap_max (2048: largest halo staged), list_prefetch (2: L2 prefetch of
  *   the neighbour lists that many blocks ahead; 0 off), state_prefetch (1: L2 prefetch, before

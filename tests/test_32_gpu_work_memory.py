@@ -1,5 +1,5 @@
 """The pair work arrays of the plain form (1.2 KB a particle) stay in the cache behind a destroyed
-domain and go to the next one only when it asks for them."""
+domain and go to the next one only when it asks for them; option pair_cache 0 frees them."""
 import pytest
 
 from weldformgpu_gb300 import Domain_d
@@ -49,4 +49,26 @@ def test_a_plain_domain_takes_the_last_domains_work_arrays():
     assert (b.get_field("a") == x).all()
     release_cache()
     assert _free() == held                   # b holds all of it
+    b.close()
+
+
+def test_the_option_frees_the_work_arrays():
+    _free()
+    release_cache()
+    sc = S.compression_cylinder(R=0.0107, H=0.0214, generator="lattice")
+    a = S.load(Domain_d(sc["n"]), sc, {"precision": 0})
+    b = S.load(Domain_d(sc["n"]), sc, {"precision": 0})
+    for d in (a, b):
+        d.step(2)
+    held = _free()
+    a.set_option("pair_cache", 0)
+    assert _free() - held > 1150 * sc["n"]
+    a.step(1)
+    a.set_option("pair_cache", 1)
+    for d, k in ((a, 2), (b, 3)):
+        d.step(k)
+    assert abs(_free() - held) < 100 * sc["n"]
+    for f in ("x", "v", "sigma"):
+        assert (a.get_field(f) == b.get_field(f)).all(), f
+    a.close()
     b.close()

@@ -2062,6 +2062,8 @@ int wf_set_option(wf_domain* d, const char* key, double v) {
   else if (k == "pair_cache") {
     d->pair_cache = v != 0;
     kept_drop(d);
+    d->work_refused = 0;
+    if (!d->pair_cache) work_drop(d);
   }
   else if (k == "tile_staging") d->tile_staging = v != 0;   // takes effect at the next rebuild
   else if (k == "list_prefetch") d->list_prefetch = std::max(0, std::min((int)v, WF_NB_BLOCKS));
