@@ -906,7 +906,7 @@ static int grid_from_codes(wf_domain* d, const unsigned* codes) {
 
 // The cell sort, reorder (full) and lists of the positions in pf, on the grid
 // d->grid, or the device's (hdr) of about ncell_last cells.
-static int build_lists(wf_domain* d, const StaticHeader* hdr, bool full) {
+static int build_lists(wf_domain* d, StaticHeader* hdr, bool full) {
   const int64_t n = d->n;
   cudaStream_t s = d->stream;
   Fields& A = d->F[d->cur];

@@ -43,7 +43,9 @@ constexpr int64_t kOffCount = kOffStart + align256(4 * (kMaxCells + 1));   // ui
 constexpr int64_t kOffScan = kOffCount + align256(4 * kMaxCells);          // uint32[kScanWords]
 constexpr int64_t kScratchBytes = kOffScan + align256(4 * kScanWords);
 static_assert(kScratchBytes == WF_STATIC_SCRATCH_BYTES, "header and layout disagree");
-static_assert(sizeof(StaticHeader) <= 256 && kMaxCells / 1024 + 1 <= kScanWords, "scratch layout");
+static_assert(sizeof(StaticHeader) <= 256 && kMaxCells / 1024 + 1 <= kScanWords &&
+                  2 * (kMaxParticles / 32) <= kMaxCells,
+              "scratch layout");
 
 }  // namespace
 
@@ -154,7 +156,7 @@ extern "C" int wf_find_neighbors_static(const double* x, int64_t n, double h, in
   const float r = (float)(2.0 * h);
   launch_static_prep(n, x, pf, r, hdr, W.count, kMaxCells, s);
   launch_cell_sort(n, pf, GridDev{}, hdr, nullptr, W, order, order, sorted, &hdr->status, s);
-  launch_static_lists(sorted, hdr, W.start, order, lists, counts, &hdr->status, s);
+  launch_static_lists(sorted, hdr, W.start, order, W.count, lists, counts, &hdr->status, s);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(err, err_len, e, "neighbour search launch");
   StaticHeader head;

@@ -301,9 +301,15 @@ __global__ void k_cell_scatter(int64_t n, int64_t cells, const StaticHeader* __r
 // cell (32 broadcast compares for a cell of at most 32; the cells hold ~14).
 // Every lane reads before any writes.  A larger cell is insertion-sorted by
 // one lane.  With pf2 not null the search positions follow into the order.
-__global__ void k_cell_sort(int64_t cells, const StaticHeader* __restrict__ hdr,
+// kStatic (wf_find_neighbors_static, s_src is s_orig; clouds of any density):
+// a larger cell's ranks are counted by all lanes into tmp, and its particles
+// behind the first 32 are listed in groups of 32, pairs of cell and first
+// index, hdr->groups of them.
+template <bool kStatic>
+__global__ void k_cell_sort(int64_t cells, StaticHeader* hdr,
                             const uint32_t* __restrict__ start, int32_t* s_src, int32_t* s_orig,
-                            const float4* __restrict__ pf, float4* __restrict__ pf2) {
+                            const float4* __restrict__ pf, float4* __restrict__ pf2, int32_t* tmp,
+                            uint32_t* groups) {
   const int lane = threadIdx.x & 31;
   if (hdr) cells = hdr->ncell;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -325,7 +331,25 @@ __global__ void k_cell_sort(int64_t cells, const StaticHeader* __restrict__ hdr,
       }
       continue;
     }
-    if (lane == 0) {
+    if constexpr (kStatic) {
+      for (uint32_t k = b + lane; k < e; k += 32) {
+        const int32_t o = s_src[k];
+        uint32_t rank = 0;
+#pragma unroll 8
+        for (uint32_t t = b; t < e; t++) rank += s_src[t] < o;
+        tmp[b + rank] = o;
+      }
+      __syncwarp();
+      for (uint32_t k = b + lane; k < e; k += 32) s_src[k] = tmp[k];
+      const uint32_t more = (m - 1u) / 32u;
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&hdr->groups, more);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      for (uint32_t k = lane; k < more; k += 32) {
+        groups[2 * (at + k)] = (uint32_t)c;
+        groups[2 * (at + k) + 1] = b + 32u * (k + 1u);
+      }
+    } else if (lane == 0) {
       for (uint32_t k = b + 1; k < e; k++) {
         const int32_t ko = s_orig[k], ks = s_src[k];
         uint32_t q = k;
@@ -457,26 +481,11 @@ __device__ __forceinline__ void nb_append_round(int nstaged, const float4* __res
   }
 }
 
-template <class I, bool kRows>
-__global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t npad,
-                                                          const float4* __restrict__ pf, GridDev g,
-                                                          const StaticHeader* __restrict__ hdr,
-                                                          const uint32_t* __restrict__ start,
-                                                          const int32_t* __restrict__ slot_of,
-                                                          int32_t* __restrict__ nb,
-                                                          int32_t* __restrict__ cnt, int* status) {
-  __shared__ float4 s_pos[kNbWarps][kNbStage];
-  __shared__ int32_t s_id[kNbWarps][kNbStage];
-  __shared__ float4 s_part[kNbWarps][32];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (hdr) {                                   // the grid is in device memory
-    ncell = hdr->ncell;
-    g = hdr->grid;
-  }
-  for (int64_t c = blockIdx.x * (int64_t)kNbWarps + w; c < ncell;
-       c += (int64_t)gridDim.x * kNbWarps) {   // whole warps together
-  const uint32_t ps = start[c], pe = start[c + 1];
-  if (ps >= pe) continue;
+// Row r = 3 (dz + 1) + (dy + 1) of the candidates of cell c: slots [rb, rb + rn)
+// on lane r < 9
+__device__ __forceinline__ void nb_rows(const GridDev& g, const uint32_t* __restrict__ start,
+                                        int64_t c, uint32_t& rb, uint32_t& rn) {
+  const int lane = threadIdx.x & 31;
   // cell coordinates in 32-bit arithmetic (the grid holds at most 2e9 cells;
   // a 64-bit division is a long software sequence in this issue-bound kernel)
   const uint32_t cu = (uint32_t)c, dx = (uint32_t)g.dim[0], dy = (uint32_t)g.dim[1];
@@ -484,8 +493,7 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t
   const int cx = (int)(cu - cyz * dx);
   const int cy = (int)(cyz % dy);
   const int cz = (int)(cyz / dy);
-  // row r = 3 (dz + 1) + (dy + 1): slot range [rb, rb + rn) on lane r
-  uint32_t rb = 0, rn = 0;
+  rb = rn = 0;
   if (lane < 9) {
     const int fz = cz + lane / 3 - 1, fy = cy + lane % 3 - 1;
     if (fz >= 0 && fz < g.dim[2] && fy >= 0 && fy < g.dim[1]) {
@@ -495,81 +503,136 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t
       rn = start[rowc + x1 + 1] - rb;
     }
   }
-  const float r2 = g.r2, thr = r2 * 1.0001f;
-  float4* sp = s_pos[w];
-  int32_t* sid = s_id[w];
-  for (uint32_t g0 = ps; g0 < pe; g0 += 32) {
-    const int gn = (int)min(32u, pe - g0);
-    // this group's particles (lane j < gn holds particle g0 + j) and their box
-    float px = 0.f, py = 0.f, pz = 0.f;
-    int32_t myslot = 0;
-    float lo[3], hi[3];
-    if (lane < gn) {
-      const float4 p = pf[g0 + lane];
-      px = p.x; py = p.y; pz = p.z;
-      myslot = slot_of ? slot_of[g0 + lane] : (int32_t)(g0 + lane);
-      s_part[w][lane] = make_float4(px, py, pz, __int_as_float(myslot));
-    }
-    {
-      const float4 p0 = pf[g0];
-      lo[0] = hi[0] = lane < gn ? px : p0.x;
-      lo[1] = hi[1] = lane < gn ? py : p0.y;
-      lo[2] = hi[2] = lane < gn ? pz : p0.z;
-    }
+}
+
+// The lists of a cell's particles g0 .. g0 + gn - 1 (gn <= 32) from its rows.
+// kRows: the scan ends when every list of the group is full.
+template <class I, bool kRows>
+__device__ __forceinline__ void nb_group(uint32_t g0, int gn, uint32_t rb, uint32_t rn, float r2,
+                                         int64_t npad, const float4* __restrict__ pf,
+                                         const int32_t* __restrict__ slot_of,
+                                         int32_t* __restrict__ nb, int32_t* __restrict__ cnt,
+                                         int* status, float4* sp, int32_t* sid, float4* part) {
+  const int lane = threadIdx.x & 31;
+  const float thr = r2 * 1.0001f;
+  // this group's particles (lane j < gn holds particle g0 + j) and their box
+  float px = 0.f, py = 0.f, pz = 0.f;
+  int32_t myslot = 0;
+  float lo[3], hi[3];
+  if (lane < gn) {
+    const float4 p = pf[g0 + lane];
+    px = p.x; py = p.y; pz = p.z;
+    myslot = slot_of ? slot_of[g0 + lane] : (int32_t)(g0 + lane);
+    part[lane] = make_float4(px, py, pz, __int_as_float(myslot));
+  }
+  {
+    const float4 p0 = pf[g0];
+    lo[0] = hi[0] = lane < gn ? px : p0.x;
+    lo[1] = hi[1] = lane < gn ? py : p0.y;
+    lo[2] = hi[2] = lane < gn ? pz : p0.z;
+  }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+  for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-      for (int a = 0; a < 3; a++) {
-        lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-        hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-      }
-    int count = 0;
-    int nstaged = 0;
-    for (int r = 0; r < 9; r++) {
-      const uint32_t b = __shfl_sync(0xffffffffu, rb, r);
-      const uint32_t nr = __shfl_sync(0xffffffffu, rn, r);
-      for (uint32_t t0 = 0; t0 < nr; t0 += 32) {
-        if (nstaged > kNbStage - 32) {          // staging full: test what is staged
-          __syncwarp();
-          nb_append_round<I, kRows>(nstaged, sp, sid, gn, s_part[w], r2, npad, nb, count);
-          __syncwarp();
-          nstaged = 0;
-        }
-        const bool v = t0 + lane < nr;
-        const uint32_t s = b + t0 + lane;
-        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-        int32_t id = (int32_t)s;
-        bool keep = false;
-        if (v) {
-          q = pf[s];
-          if (slot_of) id = slot_of[s];
-          const float ex = fmaxf(0.f, fmaxf(lo[0] - q.x, q.x - hi[0]));
-          const float ey = fmaxf(0.f, fmaxf(lo[1] - q.y, q.y - hi[1]));
-          const float ez = fmaxf(0.f, fmaxf(lo[2] - q.z, q.z - hi[2]));
-          keep = ex * ex + ey * ey + ez * ez < thr;
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) {
-          const int at = nstaged + __popc(m & ((1u << lane) - 1u));
-          sp[at] = q;
-          sid[at] = id;
-        }
-        nstaged += __popc(m);
-      }
+    for (int a = 0; a < 3; a++) {
+      lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+      hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
     }
-    __syncwarp();
-    nb_append_round<I, kRows>(nstaged, sp, sid, gn, s_part[w], r2, npad, nb, count);
-    __syncwarp();
-    if (lane < gn) {
-      if (count >= WF_NB) atomicOr(status, WF_STATUS_NB_CAP);
-      const int cn = min(count, WF_NB);
-      cnt[myslot] = cn;
-      // pad the last block with the particle's own slot (see nb_at)
-      if constexpr (!kRows)
-      for (int k = cn; k < ((cn + WF_NB_BLK - 1) & ~(WF_NB_BLK - 1)); k++)
-        nb[nb_at(npad, myslot, k)] = myslot;
+  int count = 0;
+  int nstaged = 0;
+  bool full = false;
+  for (int r = 0; r < 9 && !full; r++) {
+    const uint32_t b = __shfl_sync(0xffffffffu, rb, r);
+    const uint32_t nr = __shfl_sync(0xffffffffu, rn, r);
+    for (uint32_t t0 = 0; t0 < nr; t0 += 32) {
+      if (nstaged > kNbStage - 32) {          // staging full: test what is staged
+        __syncwarp();
+        nb_append_round<I, kRows>(nstaged, sp, sid, gn, part, r2, npad, nb, count);
+        __syncwarp();
+        nstaged = 0;
+        if constexpr (kRows) {
+          full = __all_sync(0xffffffffu, lane >= gn || count >= WF_NB);
+          if (full) break;
+        }
+      }
+      const bool v = t0 + lane < nr;
+      const uint32_t s = b + t0 + lane;
+      float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+      int32_t id = (int32_t)s;
+      bool keep = false;
+      if (v) {
+        q = pf[s];
+        if (slot_of) id = slot_of[s];
+        const float ex = fmaxf(0.f, fmaxf(lo[0] - q.x, q.x - hi[0]));
+        const float ey = fmaxf(0.f, fmaxf(lo[1] - q.y, q.y - hi[1]));
+        const float ez = fmaxf(0.f, fmaxf(lo[2] - q.z, q.z - hi[2]));
+        keep = ex * ex + ey * ey + ez * ez < thr;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const int at = nstaged + __popc(m & ((1u << lane) - 1u));
+        sp[at] = q;
+        sid[at] = id;
+      }
+      nstaged += __popc(m);
     }
   }
+  __syncwarp();
+  nb_append_round<I, kRows>(nstaged, sp, sid, gn, part, r2, npad, nb, count);
+  __syncwarp();
+  if (lane < gn) {
+    if (count >= WF_NB) atomicOr(status, WF_STATUS_NB_CAP);
+    const int cn = min(count, WF_NB);
+    cnt[myslot] = cn;
+    // pad the last block with the particle's own slot (see nb_at)
+    if constexpr (!kRows)
+    for (int k = cn; k < ((cn + WF_NB_BLK - 1) & ~(WF_NB_BLK - 1)); k++)
+      nb[nb_at(npad, myslot, k)] = myslot;
+  }
+}
+
+// kRows: a cell's particles behind its first 32 are groups of the list that
+// k_cell_sort left, so that the warps share dense cells, and a group's scan ends
+// when its lists are full.  A call with 25,000 particles, 200 / 500 / 1,500 a
+// cell: 0.28 / 0.49 / 1.15 ms; with a whole cell per warp, its scan to the end
+// and its sort by one lane 2.9 / 10.2 / 53; with a thread per particle that
+// leaves at 70 entries and a thread per cell for the sort 1.7 / 4.5 / 20.6.
+// Up to 14 a cell there are no such groups (74 us).
+template <class I, bool kRows>
+__global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t npad,
+                                                          const float4* __restrict__ pf, GridDev g,
+                                                          const StaticHeader* __restrict__ hdr,
+                                                          const uint32_t* __restrict__ start,
+                                                          const int32_t* __restrict__ slot_of,
+                                                          const uint32_t* __restrict__ groups,
+                                                          int32_t* __restrict__ nb,
+                                                          int32_t* __restrict__ cnt, int* status) {
+  __shared__ float4 s_pos[kNbWarps][kNbStage];
+  __shared__ int32_t s_id[kNbWarps][kNbStage];
+  __shared__ float4 s_part[kNbWarps][32];
+  const int w = threadIdx.x >> 5;
+  if (hdr) {                                   // the grid is in device memory
+    ncell = hdr->ncell;
+    g = hdr->grid;
+  }
+  const int64_t total = ncell + (kRows ? (int64_t)hdr->groups : 0);
+  for (int64_t k = blockIdx.x * (int64_t)kNbWarps + w; k < total;
+       k += (int64_t)gridDim.x * kNbWarps) {   // whole warps together
+    int64_t c = k;
+    uint32_t ps;
+    if (kRows && k >= ncell) {
+      c = groups[2 * (k - ncell)];
+      ps = groups[2 * (k - ncell) + 1];
+    } else {
+      ps = start[c];
+    }
+    const uint32_t end = start[c + 1], pe = kRows ? min(end, ps + 32u) : end;
+    if (ps >= pe) continue;
+    uint32_t rb, rn;
+    nb_rows(g, start, c, rb, rn);
+    for (uint32_t g0 = ps; g0 < pe; g0 += 32)
+      nb_group<I, kRows>(g0, (int)min(32u, pe - g0), rb, rn, g.r2, npad, pf, slot_of, nb, cnt, status,
+                         s_pos[w], s_id[w], s_part[w]);
   }
 }
 
@@ -618,7 +681,7 @@ void launch_static_prep(int64_t n, const double* x, float4* pf, float r, StaticH
   cudaMemsetAsync(hdr, 0, sizeof(StaticHeader), s);
   k_static_prep<<<std::min(nblocks(n, 256), 304), 256, 0, s>>>(n, x, pf, r, hdr, count, max_cells);
 }
-void launch_cell_sort(int64_t n, const float4* pf, const GridDev& g, const StaticHeader* hdr,
+void launch_cell_sort(int64_t n, const float4* pf, const GridDev& g, StaticHeader* hdr,
                       const int32_t* orig, const CellWork& W, int32_t* s_src, int32_t* s_orig,
                       float4* pf2, int* status, cudaStream_t s) {
   // with the grid in device memory the launches are sized for the most cells
@@ -628,8 +691,13 @@ void launch_cell_sort(int64_t n, const float4* pf, const GridDev& g, const Stati
   k_cell_scatter<<<nblocks(n, 256), 256, 0, s>>>(n, cells, hdr, W.cellid, W.rank, W.count, W.bsum,
                                                  W.start, orig, s_src, s_orig);
   const int blocks = nblocks(cells * 32, 256);
-  k_cell_sort<<<hdr ? std::min(blocks, 1216) : blocks, 256, 0, s>>>(cells, hdr, W.start, s_src,
-                                                                    s_orig, pf, pf2);
+  const int grid = hdr ? std::min(blocks, 1216) : blocks;
+  if (orig)
+    k_cell_sort<false><<<grid, 256, 0, s>>>(cells, hdr, W.start, s_src, s_orig, pf, pf2, nullptr,
+                                            nullptr);
+  else   // the cell numbers and counts have done their work
+    k_cell_sort<true><<<grid, 256, 0, s>>>(cells, hdr, W.start, s_src, s_orig, pf, pf2,
+                                           reinterpret_cast<int32_t*>(W.cellid), W.count);
 }
 void launch_reorder(int64_t n, const int32_t* s_src, const Fields& A, const Fields& B,
                     const float4* pf, float4* pf2, int32_t* inv, cudaStream_t s) {
@@ -640,16 +708,16 @@ void launch_nblist(int64_t ncell, int64_t npad, const float4* pf, const GridDev&
                    int32_t* nb, int32_t* cnt, int* status, cudaStream_t s) {
   if ((int64_t)WF_NB_ALLOC * npad < ((int64_t)1 << 31))
     k_nblist<uint32_t, false><<<nblocks(ncell, kNbWarps), 32 * kNbWarps, 0, s>>>(
-        ncell, npad, pf, g, hdr, start, slot_of, nb, cnt, status);
+        ncell, npad, pf, g, hdr, start, slot_of, nullptr, nb, cnt, status);
   else
     k_nblist<int64_t, false><<<nblocks(ncell, kNbWarps), 32 * kNbWarps, 0, s>>>(
-        ncell, npad, pf, g, hdr, start, slot_of, nb, cnt, status);
+        ncell, npad, pf, g, hdr, start, slot_of, nullptr, nb, cnt, status);
 }
 void launch_static_lists(const float4* pf, const StaticHeader* hdr, const uint32_t* start,
-                         const int32_t* order, int32_t* lists, int32_t* counts, int* status,
-                         cudaStream_t s) {
+                         const int32_t* order, const uint32_t* groups, int32_t* lists,
+                         int32_t* counts, int* status, cudaStream_t s) {
   k_nblist<uint32_t, true><<<2432, 32 * kNbWarps, 0, s>>>(0, 0, pf, GridDev{}, hdr, start, order,
-                                                          lists, counts, status);
+                                                          groups, lists, counts, status);
 }
 void launch_snapshot(int64_t n, const Fields& F, cudaStream_t s) {
   k_snapshot<<<nblocks(n, 256), 256, 0, s>>>(n, F);

@@ -16,6 +16,7 @@ struct StaticHeader {
   int status;           // WF_STATUS_* bits
   unsigned ticket, scan_ticket;
   int ncell;            // cells of the grid; 0: it does not fit, nothing is searched
+  unsigned groups;      // static search: groups of particles behind a cell's first 32
   GridDev grid;
 };
 
@@ -54,9 +55,9 @@ __host__ __device__ inline void grid_from_bounds(const int mm[6], float r, GridD
 
 // Work arrays of the cell sort.
 struct CellWork {
-  uint32_t* cellid;    // [n]
+  uint32_t* cellid;    // [n]; static search: a sort's scratch behind that
   uint32_t* rank;      // [n]
-  uint32_t* count;     // [cells], zero on entry
+  uint32_t* count;     // [cells], zero on entry; static search: [2 n / 32] the groups at the end
   uint32_t* bsum;      // [cells / 1024 + 1]
   uint32_t* ticket;    // one word, zero on entry and on return
   uint32_t* start;     // [cells + 1] out: the cells' ranges in sorted order
@@ -75,7 +76,7 @@ void launch_static_prep(int64_t n, const double* x, float4* pf, float r, StaticH
 // Counting sort by cell, original ids ascending inside a cell (orig null: the
 // index): s_src, s_orig in sorted order, W.start, and with pf2 not null the
 // positions in sorted order.  The grid is g, or hdr's when hdr is not null.
-void launch_cell_sort(int64_t n, const float4* pf, const GridDev& g, const StaticHeader* hdr,
+void launch_cell_sort(int64_t n, const float4* pf, const GridDev& g, StaticHeader* hdr,
                       const int32_t* orig, const CellWork& W, int32_t* s_src, int32_t* s_orig,
                       float4* pf2, int* status, cudaStream_t s);
 void launch_reorder(int64_t n, const int32_t* s_src, const Fields& A, const Fields& B,
@@ -84,8 +85,9 @@ void launch_reorder(int64_t n, const int32_t* s_src, const Fields& A, const Fiel
 void launch_nblist(int64_t ncell, int64_t npad, const float4* pf, const GridDev& g,
                    const StaticHeader* hdr, const uint32_t* start, const int32_t* slot_of,
                    int32_t* nb, int32_t* cnt, int* status, cudaStream_t s);
-// row-major lists and counts by the caller's index (order[k]: index of the k-th sorted particle)
+// row-major lists and counts by the caller's index (order[k]: index of the k-th sorted particle;
+// groups: W.count as launch_cell_sort left it)
 void launch_static_lists(const float4* pf, const StaticHeader* hdr, const uint32_t* start,
-                         const int32_t* order, int32_t* lists, int32_t* counts, int* status,
-                         cudaStream_t s);
+                         const int32_t* order, const uint32_t* groups, int32_t* lists,
+                         int32_t* counts, int* status, cudaStream_t s);
 void launch_snapshot(int64_t n, const Fields& F, cudaStream_t s);
