@@ -1429,7 +1429,7 @@ static int solve_step_launches(wf_domain* d) {
     }
     if (law1_fused) {                  // the acceleration pass looks into the tools' bins
       KTimer t(d, KID_CONTACT);
-      launch_contact_stage(P, F, N, false, d->a32, s);
+      d->launches += launch_contact_stage(P, F, N, false, d->a32, s);
     }
     if (law1_fused || (!P.contact && d->fuse_integrate)) {
       { KTimer t(d, KID_ACCEL);
@@ -1442,9 +1442,12 @@ static int solve_step_launches(wf_domain* d) {
   }
   if (P.contact) {                                                                    // :233-257
     KTimer t(d, KID_CONTACT);
-    if (law1_fused) launch_contact_law1_list(P, F, d->vd2, d->a32, s);
-    else launch_contact_stage(P, F, N, d->ts_i == 0, mixed ? d->a32 : nullptr, s);
-    d->launches += d->ts_i == 0 ? 3 : 2;
+    if (law1_fused) {
+      launch_contact_law1_list(P, F, d->vd2, d->a32, s);
+      d->launches += 1;
+    } else {
+      d->launches += launch_contact_stage(P, F, N, d->ts_i == 0, mixed ? d->a32 : nullptr, s);
+    }
   }
   if (!integrated) {   // :273-287
     KTimer t(d, KID_INTEGRATE);

@@ -441,9 +441,10 @@ void launch_thermal(const StepParams& P, const Fields& F, const Work64& W, const
 
 // contact (wf_contact.cu): surface tagging, contact list (when `list`) and
 // penalty forces after the acceleration pass; mesh motion and rigid particles
-// after the integration; plane coefficients at solve start
-void launch_contact_stage(const StepParams& P, const Fields& F, const NbBuffers& N, bool list,
-                          float4* a32, cudaStream_t s);
+// after the integration; plane coefficients at solve start; returns the number
+// of kernels launched
+int launch_contact_stage(const StepParams& P, const Fields& F, const NbBuffers& N, bool list,
+                         float4* a32, cudaStream_t s);
 // contact law 1 and integration of the slots that the fused acceleration pass
 // listed (P.near_list)
 void launch_contact_law1_list(const StepParams& P, const Fields& F, const double4* vd2,

@@ -705,21 +705,24 @@ inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
 
-void launch_contact_stage(const StepParams& P, const Fields& F, const NbBuffers& N, bool list,
-                          float4* a32, cudaStream_t s) {
+int launch_contact_stage(const StepParams& P, const Fields& F, const NbBuffers& N, bool list,
+                         float4* a32, cudaStream_t s) {
   if (P.contact_law == 1) {
+    int launches = 0;
     for (int m = 0; m < P.ncsid; m++) {   // rotating tools: bins from the current nodes
       const MeshDev& M = P.mesh[m];
       if (!M.rot) continue;
       const int64_t ncell = (int64_t)M.dims[0] * M.dims[1] * M.dims[2];
       cudaMemsetAsync(M.cstart, 0, sizeof(uint32_t) * (ncell + 1), s);
       k_bins_count<<<blocks_for(M.ne, 128), 128, 0, s>>>(M);
-      device_exclusive_scan(reinterpret_cast<uint32_t*>(M.cstart), ncell + 1, M.scan_tmp, s);
+      launches +=
+          2 + device_exclusive_scan(reinterpret_cast<uint32_t*>(M.cstart), ncell + 1, M.scan_tmp, s);
       cudaMemcpyAsync(M.cursor, M.cstart, sizeof(uint32_t) * ncell, cudaMemcpyDeviceToDevice, s);
       k_bins_fill<<<blocks_for(M.ne, 128), 128, 0, s>>>(M);
     }
-    if (!P.near_count) k_contact_law1<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, a32);
-    return;
+    if (P.near_count) return launches;
+    k_contact_law1<<<blocks_for(P.n, 128), 128, 0, s>>>(P, F, a32);
+    return launches + 1;
   }
   const int lanes = lanes64(P.n), grid = blocks_for(P.n * lanes, lanes == 1 ? 64 : 32);
   if (lanes == 32) k_surface<32><<<grid, 32, 0, s>>>(P, F, N.nb, N.cnt);
@@ -734,6 +737,7 @@ void launch_contact_stage(const StepParams& P, const Fields& F, const NbBuffers&
     if (list) k_contact_nb<1><<<grid, 64, 0, s>>>(P, F, N.nb, N.cnt);
     k_contact_force<1><<<grid, 64, 0, s>>>(P, F, a32);
   }
+  return list ? 3 : 2;
 }
 
 void launch_contact_law1_list(const StepParams& P, const Fields& F, const double4* vd2,

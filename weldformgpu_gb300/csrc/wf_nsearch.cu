@@ -647,15 +647,16 @@ inline int nblocks(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
 
-void device_exclusive_scan(uint32_t* data, int64_t n, uint32_t* tmp, cudaStream_t s) {
+int device_exclusive_scan(uint32_t* data, int64_t n, uint32_t* tmp, cudaStream_t s) {
   int64_t nb = (n + 1023) / 1024;
   if (nb <= 1) {
     k_scan_block<<<1, 256, 0, s>>>(data, n, nullptr);
-    return;
+    return 1;
   }
   k_scan_block<<<(int)nb, 256, 0, s>>>(data, n, tmp);
-  device_exclusive_scan(tmp, nb, tmp + nb, s);
+  const int inner = device_exclusive_scan(tmp, nb, tmp + nb, s);
   k_scan_add<<<(int)nb, 256, 0, s>>>(data, n, tmp);
+  return inner + 2;
 }
 
 int64_t scan_tmp_words(int64_t n) {

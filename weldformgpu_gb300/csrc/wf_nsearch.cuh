@@ -63,7 +63,8 @@ struct CellWork {
   uint32_t* start;     // [cells + 1] out: the cells' ranges in sorted order
   int64_t max_cells;   // for a grid in device memory
 };
-void device_exclusive_scan(uint32_t* data, int64_t n, uint32_t* tmp, cudaStream_t s);
+// returns the number of kernels launched
+int device_exclusive_scan(uint32_t* data, int64_t n, uint32_t* tmp, cudaStream_t s);
 int64_t scan_tmp_words(int64_t n);
 int64_t cell_scan_words(int64_t cells);
 // float positions (x_h or the current ones) into pf, their cell bounds' codes into hdr->mm; with
