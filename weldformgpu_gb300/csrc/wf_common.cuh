@@ -27,13 +27,6 @@
 __host__ __device__ __forceinline__ int64_t nb_at(int64_t npad, int64_t i, int k) {
   return ((int64_t)(k >> 3) * npad + i) * WF_NB_BLK + (k & 7);
 }
-// block b of slot i as two int4 (entries 8b .. 8b+7)
-__device__ __forceinline__ void nb_block(const int32_t* __restrict__ nb, int64_t npad, int64_t i,
-                                         int b, int4& lo, int4& hi) {
-  const int4* q = reinterpret_cast<const int4*>(nb + ((int64_t)b * npad + i) * WF_NB_BLK);
-  lo = __ldg(q);
-  hi = __ldg(q + 1);
-}
 
 // L2 prefetch of list block b of slot i, two blocks ahead of its use, so
 // that the list stream (read once per pass, from DRAM) meets L2 latency when
@@ -263,22 +256,6 @@ struct StepParams {
     cudaError_t e_ = (call);                               \
     if (e_ != cudaSuccess) return wf_cuda_fail(d, e_, #call); \
   } while (0)
-
-// Cubic-spline kernel gradient (Dim 3) with C = 1/(h^4 pi) hoisted: the
-// reference recomputes C from h_ = (h_i + h_j)/2 = h for every pair
-// (src/cuda/Functions.cu:76-88); with a uniform h the value is identical.
-__device__ __forceinline__ double gradK64(double q, double h, double C) {
-  if (q == 0.0) return C / h * (-3.0 + (9.0 / 2.0) * q);
-  else if (q < 1.0) return C / (q * h) * (-3.0 * q + (9.0 / 4.0) * q * q);
-  else if (q < 2.0) return C / (q * h) * ((-3.0 / 4.0) * (2.0 - q) * (2.0 - q));
-  return 0.0;
-}
-
-__device__ __forceinline__ float gradK32(float q, float h, float C) {
-  if (q < 1.0f) return C / h * (-3.0f + 2.25f * q);
-  else if (q < 2.0f) return C / (q * h) * (-0.75f * (2.0f - q) * (2.0f - q));
-  return 0.0f;
-}
 
 // The mixed form's cubic-spline gradient factor GK (Functions.cu:82-88) from
 // r^2 > 0 (invh = 1/h, Ch = C/h; the q < 1 branch is C/(q h) q (-3 + 9/4 q)

@@ -190,9 +190,11 @@ __device__ __forceinline__ double twice(double x) {
   return __hiloint2double(hi + ((hi << 1) != 0 ? 0x00100000 : 0), __double2loint(x));
 }
 
-// The cubic-spline gradient factor of gradK64, bit for bit, with the division
-// shared by its two branches (so a warp whose lanes fall on both sides of
-// q = 1 divides once) and the comparisons on the bits of q >= 0.  q >= 2,
+// The cubic-spline gradient factor (Dim 3) with C = 1/(h^4 pi) hoisted: the
+// reference recomputes C from h_ = (h_i + h_j)/2 = h for every pair
+// (src/cuda/Functions.cu:76-88); with a uniform h the value is identical.  The
+// division is shared by its two branches (so a warp whose lanes fall on both
+// sides of q = 1 divides once) and the comparisons are on the bits of q >= 0.  q >= 2,
 // infinite or NaN gives 0.
 template <bool kInt>
 __device__ __forceinline__ double spline64(double q, double h, double C) {

@@ -113,16 +113,6 @@ __device__ __forceinline__ void nbl_block_s(const uint16_t* sl, int t, int b, in
   js[6] = (int)(q.w & 0xffffu); js[7] = (int)(q.w >> 16);
 }
 
-// block b (entries 8b .. 8b+7) of slot i's local list as one 16-byte load
-__device__ __forceinline__ void nbl_block(const uint16_t* __restrict__ nbl, int64_t npad,
-                                          int64_t i, int b, int js[8]) {
-  const uint4 q = __ldg(reinterpret_cast<const uint4*>(nbl + ((int64_t)b * npad + i) * WF_NB_BLK));
-  js[0] = (int)(q.x & 0xffffu); js[1] = (int)(q.x >> 16);
-  js[2] = (int)(q.y & 0xffffu); js[3] = (int)(q.y >> 16);
-  js[4] = (int)(q.z & 0xffffu); js[5] = (int)(q.z >> 16);
-  js[6] = (int)(q.w & 0xffffu); js[7] = (int)(q.w >> 16);
-}
-
 __device__ __forceinline__ void stage_lists(const uint16_t* __restrict__ nbl, int64_t npad,
                                             int tile, uint16_t* sl) {
   constexpr int kChunks = WF_NB_BLOCKS * WF_TILE;   // 16-byte pieces
