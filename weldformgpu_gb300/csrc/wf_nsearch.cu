@@ -15,6 +15,7 @@
 // Lists are stored in blocks of 8 entries (nb_at in wf_common.cuh): a thread
 // reads 8 entries with two 16-byte loads and a warp reads contiguous memory.
 #include <algorithm>
+#include <type_traits>
 
 #include "wf_common.cuh"
 #include "wf_nsearch.cuh"
@@ -540,8 +541,7 @@ __device__ __forceinline__ void nb_group(uint32_t g0, int gn, uint32_t rb, uint3
     }
   int count = 0;
   int nstaged = 0;
-  bool full = false;
-  for (int r = 0; r < 9 && !full; r++) {
+  for (int r = 0; r < 9; r++) {
     const uint32_t b = __shfl_sync(0xffffffffu, rb, r);
     const uint32_t nr = __shfl_sync(0xffffffffu, rn, r);
     for (uint32_t t0 = 0; t0 < nr; t0 += 32) {
@@ -550,9 +550,9 @@ __device__ __forceinline__ void nb_group(uint32_t g0, int gn, uint32_t rb, uint3
         nb_append_round<I, kRows>(nstaged, sp, sid, gn, part, r2, npad, nb, count);
         __syncwarp();
         nstaged = 0;
-        if constexpr (kRows) {
-          full = __all_sync(0xffffffffu, lane >= gn || count >= WF_NB);
-          if (full) break;
+        if (kRows && __all_sync(0xffffffffu, lane >= gn || count >= WF_NB)) {
+          rn = 0;                               // nothing of the rows behind either
+          break;
         }
       }
       const bool v = t0 + lane < nr;
@@ -594,12 +594,14 @@ __device__ __forceinline__ void nb_group(uint32_t g0, int gn, uint32_t rb, uint3
 // kRows: a cell's particles behind its first 32 are groups of the list that
 // k_cell_sort left, so that the warps share dense cells, and a group's scan ends
 // when its lists are full.  A call with 25,000 particles, 200 / 500 / 1,500 a
-// cell: 0.28 / 0.49 / 1.15 ms; with a whole cell per warp, its scan to the end
+// cell: 0.22 / 0.36 / 0.86 ms; with a whole cell per warp, its scan to the end
 // and its sort by one lane 2.9 / 10.2 / 53; with a thread per particle that
 // leaves at 70 entries and a thread per cell for the sort 1.7 / 4.5 / 20.6.
-// Up to 14 a cell there are no such groups (74 us).
+// Up to 14 a cell there are no such groups (73 us).
+// (kRows: eight blocks an SM, so 64 registers: 19,488 particles 23.0 us; with
+// the 48 that the compiler takes of itself 25.7.)
 template <class I, bool kRows>
-__global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t npad,
+__global__ void __launch_bounds__(32 * kNbWarps, kRows ? 8 : 0) k_nblist(int64_t ncell, int64_t npad,
                                                           const float4* __restrict__ pf, GridDev g,
                                                           const StaticHeader* __restrict__ hdr,
                                                           const uint32_t* __restrict__ start,
@@ -615,14 +617,15 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_nblist(int64_t ncell, int64_t
     ncell = hdr->ncell;
     g = hdr->grid;
   }
-  const int64_t total = ncell + (kRows ? (int64_t)hdr->groups : 0);
-  for (int64_t k = blockIdx.x * (int64_t)kNbWarps + w; k < total;
-       k += (int64_t)gridDim.x * kNbWarps) {   // whole warps together
-    int64_t c = k;
+  using K = std::conditional_t<kRows, uint32_t, int64_t>;
+  const K cells = (K)ncell, total = cells + (K)(kRows ? hdr->groups : 0u);
+  for (K k = (K)blockIdx.x * kNbWarps + w; k < total;
+       k += (K)gridDim.x * kNbWarps) {         // whole warps together
+    K c = k;
     uint32_t ps;
-    if (kRows && k >= ncell) {
-      c = groups[2 * (k - ncell)];
-      ps = groups[2 * (k - ncell) + 1];
+    if (kRows && k >= cells) {
+      c = groups[2 * (k - cells)];
+      ps = groups[2 * (k - cells) + 1];
     } else {
       ps = start[c];
     }
