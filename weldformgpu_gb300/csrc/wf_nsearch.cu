@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(256) k_prep_bounds(int64_t n, const Fields F, 
 // zeroes the cell counters; the last block to finish sizes the search grid
 // (grid_from_bounds) and notes whether it fits: the kernels behind it read it
 // from device memory, so the host waits once, at the end (with the cell sort
-// and the lists one warp per cell: 19,488 particles 192 -> 72 us a call, of
-// which the kernels take 48).
+// and the lists by warps: 19,488 particles 192 -> 70 us a call, of which the
+// kernels take 47).
 __global__ void __launch_bounds__(256) k_static_prep(int64_t n, const double* __restrict__ x,
                                                      float4* __restrict__ pf, float r,
                                                      StaticHeader* __restrict__ hdr,

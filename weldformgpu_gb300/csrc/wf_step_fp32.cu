@@ -303,7 +303,9 @@ __global__ void __launch_bounds__(128, kWide ? kWideBlocks : kDensMinBlocks) k_d
 // ---- the heat pass alone (ThermalSolveKernel, src/cuda/Thermal.cu:101-142) --
 // A call's last heat pass and every step of the mixed ThermalSolve: the heat
 // sum of density_heat_pairs, the same operations in the same neighbour order
-// (so a separate pass gives the fused pass's sum bit for bit).
+// (so a separate pass gives the fused pass's sum and dT/dt bit for bit; the
+// temperature update behind it, k_heat_leapfrog, is compiled without FMA
+// contraction, so some temperatures differ from the fused pass's in the last bit).
 template <class L>
 __device__ __forceinline__ float heat_pairs(const StepParams& P, const Rec32* __restrict__ pv,
                                             const float* __restrict__ gt, const L& list, int c,
