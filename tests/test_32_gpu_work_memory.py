@@ -52,6 +52,24 @@ def test_a_plain_domain_takes_the_last_domains_work_arrays():
     b.close()
 
 
+def test_work_arrays_outlast_a_mixed_domain_in_between():
+    _free()
+    release_cache()
+    sc = S.compression_cylinder(R=0.0107, H=0.0214, generator="lattice")
+    for precision in (0, 1):
+        d = S.load(Domain_d(sc["n"]), sc, {"precision": precision})
+        d.step(1)
+        d.close()
+    before = _free()
+    d = S.load(Domain_d(sc["n"]), sc, {"precision": 0})
+    d.step(1)
+    assert before - _free() < 400 * sc["n"]
+    d.close()
+    before = _free()
+    release_cache()
+    assert _free() - before > 1150 * sc["n"]     # one block, and it goes with the cache
+
+
 def test_the_option_frees_the_work_arrays():
     _free()
     release_cache()

@@ -582,6 +582,10 @@ static void cache_take_work(wf_domain* d, size_t bytes) {
 static void cache_put(wf_domain* d) {
   if (!d->arena) return;
   std::lock_guard<std::mutex> lk(g_cache_mu);
+  if (!d->work && g_cache.dev == d->dev) {   // a domain without work arrays leaves those there
+    std::swap(d->work, g_cache.work);
+    std::swap(d->work_bytes, g_cache.work_bytes);
+  }
   cache_free_locked();                       // keep the most recent one
   g_cache.arena = d->arena;
   g_cache.bytes = d->arena_alloc;
